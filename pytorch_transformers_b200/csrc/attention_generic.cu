@@ -7,14 +7,36 @@
 // sizes that the tensor-core kernels refuse. Every query row is reduced over its keys in blocks
 // of 64 aligned to absolute positions, in ascending order, whatever else is in the launch: the
 // result of a position does not depend on how tokens were cut into steps or batched.
-#include "common.cuh"
+#include "mma_common.cuh"
 
 namespace {
 
 constexpr int BQ = 16;        // query rows of a tile
-constexpr int THREADS = 128;  // 8 threads per query row
+constexpr int THREADS = 128;  // 16 threads per pair of query rows
 constexpr int MAX_D = 256;    // head sizes up to this
-constexpr int DPT = MAX_D / 8;
+constexpr int PPITCH = PTB_PAGE + 4;
+
+// floats from one row of `n` values to the next: whole 16-byte words, an odd number of them
+__host__ __device__ constexpr int odd_words(int n) { return 4 * ((n + 3) / 4 + ((n + 3) / 4 % 2 == 0 ? 1 : 0)); }
+
+// a page's rows of `d` values into shared rows `pitch` apart, zeros in rows from `valid` on and beyond d; `async`: by cp.async
+// (float32 rows of whole 16-byte words)
+template <typename T>
+__device__ __forceinline__ void load_rows(float* dst, const T* src, int d, int pitch, int valid, int async) {
+  const int words = (d + 3) / 4;
+  if (sizeof(T) == 4 && async) {
+    for (int i = threadIdx.x; i < PTB_PAGE * words; i += THREADS) {
+      const int j = i / words, c = (i - j * words) * 4;
+      if (j < valid) cp_async16(smem_u32(dst + j * pitch + c), src + size_t(j) * d + c);
+      else *reinterpret_cast<float4*>(dst + j * pitch + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    return;
+  }
+  for (int i = threadIdx.x; i < PTB_PAGE * words * 4; i += THREADS) {
+    const int j = i / (words * 4), e = i - j * (words * 4);
+    dst[j * pitch + e] = (j < valid && e < d) ? to_f(src[size_t(j) * d + e]) : 0.f;
+  }
+}
 
 // a float as the tensors' type holds it
 template <typename T> __device__ __forceinline__ float round_store(float v) { return to_f(from_f<T>(v)); }
@@ -140,20 +162,27 @@ __global__ void split_rotate_store_kernel(const T* __restrict__ fused, T* __rest
 // output is multiplied by sigmoid(gate); with `gate_wide` the gate has a number per output entry instead (row t, head h,
 // entry e at gate[t * gate_stride + h * v_dim + e]); `out_scale` multiplies everything. Output row t, head h starts
 // at out[t * out_stride + h * v_dim]. `softcap` > 0: score <- softcap * tanh(score / softcap) after the scale.
-template <typename T>
+//
+// What bounds it on prompts is the FMA pipe behind shared memory, so operands are read as 16-byte words into register
+// tiles: a block is 8 pairs of rows x 16 lanes; a thread forms 2 rows x 4 keys of the scores (6 words for 32 FMAs, the k
+// ascending in one chain a score) and 2 rows x 4 columns of the output a group of 64 columns (2 + 4 words for 32 FMAs).
+// Shared rows lie an odd number of words apart: eight lanes' words meet no bank twice. float32 pages come by cp.async:
+// a page's values while its scores are formed, the next page's keys while the output takes the values.
+// 16 heads of 64 on prompts of 233 and 467 tokens, float32: 516 -> 69 us (before: scalar loads, two a product).
+template <typename T, int COLS>     // COLS: groups of 64 output columns (v_dim <= 64 COLS)
 __global__ void __launch_bounds__(THREADS)
 attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool,
                          T* __restrict__ out, StepBatch sb, const int* __restrict__ tile_seq,
                          const int* __restrict__ tile_q0, const float* __restrict__ alibi_slopes, int heads,
                          int kv_heads, int head_dim, float scale, int window, int v_dim,
                          const float* __restrict__ sinks, const T* __restrict__ gate, int gate_stride, float out_scale,
-                         int out_stride, int keep_first, float* __restrict__ out_wide, float softcap, int gate_wide) {
-  extern __shared__ float smem[];
-  const int wide = max(head_dim, v_dim);
-  float* qs = smem;                                 // [BQ][head_dim]
-  float* kv = qs + BQ * head_dim;                   // [PTB_PAGE][wide + 1], K then V
-  float* ps = kv + PTB_PAGE * (wide + 1);           // [BQ][PTB_PAGE]
-  const int kstride = head_dim + 1, vstride = v_dim + 1;
+                         int out_stride, int keep_first, float* __restrict__ out_wide, float softcap, int gate_wide, int async) {
+  extern __shared__ __align__(16) float smem[];
+  const int kpitch = odd_words(head_dim), vpitch = odd_words(v_dim), kwords = (head_dim + 3) / 4;
+  float* qs = smem;                                 // [BQ][kpitch], zeros beyond head_dim
+  float* ks = qs + BQ * kpitch;                     // [PTB_PAGE][kpitch], likewise
+  float* vs = ks + PTB_PAGE * kpitch;               // [PTB_PAGE][vpitch]
+  float* ps = vs + PTB_PAGE * vpitch;               // [BQ][PPITCH]
 
   const int tile = blockIdx.x, h = blockIdx.y;
   const int seq = tile_seq[tile], q0 = tile_q0[tile];
@@ -164,18 +193,19 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, 
   // head h's own): every head's weights meet every K/V head's values, for a mixing of the heads' weights afterwards
   const int gv = out_wide ? int(blockIdx.z) : g;
   const int tid = threadIdx.x;
-  const int r = tid / 8, c = tid % 8;
-  const int my_pos = (r < rows) ? past + q0 + r : -1;  // -1: no key is visible, nothing is stored
+  const int r0 = (tid / 16) * 2, lane = tid % 16;   // rows r0 and r0 + 1; keys lane + 16 jj; columns 4 lane + 64 c
   const float slope = alibi_slopes ? alibi_slopes[h] : 0.f;
 
-  for (int i = tid; i < BQ * head_dim; i += THREADS) {
-    const int rr = i / head_dim, e = i % head_dim;
-    qs[i] = (rr < rows) ? to_f(q[(size_t(start + q0 + rr) * heads + h) * head_dim + e]) : 0.f;
+  for (int i = tid; i < BQ * kpitch; i += THREADS) {
+    const int rr = i / kpitch, e = i % kpitch;
+    qs[i] = (rr < rows && e < head_dim) ? to_f(q[(size_t(start + q0 + rr) * heads + h) * head_dim + e]) : 0.f;
   }
-  float acc[DPT];
+  float acc[2][4 * COLS];
 #pragma unroll
-  for (int i = 0; i < DPT; ++i) acc[i] = 0.f;
-  float m_run = -INFINITY, l_run = 0.f;
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int i = 0; i < 4 * COLS; ++i) acc[u][i] = 0.f;
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
   const int last_pos = past + q0 + rows - 1;
   const int first_pos = past + q0;
@@ -185,106 +215,138 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, 
   const int* pages = sb.pages + size_t(seq) * sb.pages_stride;
   // the first keep_first positions stay visible left of the window: their pages are walked first
   const int kept_pages = (window > 0 && keep_first > 0) ? min((keep_first + PTB_PAGE - 1) / PTB_PAGE, kb_lo) : 0;
+  auto after = [&](int kb) { return (kb + 1 == kept_pages && kb + 1 < kb_lo) ? kb_lo : kb + 1; };
+  auto load_keys = [&](int kb) {
+    const T* src = k_pool + kv_offset(pages[kb], g, 0, kv_heads, head_dim);
+    load_rows(ks, src, head_dim, kpitch, min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE), async);
+  };
 
-  for (int kb = (kept_pages > 0 ? 0 : kb_lo); kb <= kb_hi; ++kb) {
-    if (kb == kept_pages && kb < kb_lo) kb = kb_lo;
-    const int page = pages[kb];
-    const int valid = min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE);  // keys of this block that exist
-    const T* kp = k_pool + kv_offset(page, g, 0, kv_heads, head_dim);
-    const T* vp = v_pool + kv_offset(page, gv, 0, kv_heads, v_dim);
-    __syncthreads();  // previous block's V and ps are no longer read
-    for (int i = tid; i < PTB_PAGE * head_dim; i += THREADS) {
-      const int j = i / head_dim, e = i % head_dim;
-      kv[j * kstride + e] = (j < valid) ? to_f(kp[i]) : 0.f;
-    }
-    __syncthreads();
-    // scores: this thread owns keys j = c + 8 jj of row r
-    float s[8];
-    float m_blk = -INFINITY;
+  int kb = kept_pages > 0 ? 0 : kb_lo;
+  load_keys(kb);
+  cp_async_commit();
+  while (kb <= kb_hi) {
+    const int next = after(kb);
+    load_rows(vs, v_pool + kv_offset(pages[kb], gv, 0, kv_heads, v_dim), v_dim, vpitch,
+              min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE), async);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();  // this page's keys are here
+    float s[2][4];
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-      const int j = c + 8 * jj;
-      const int key_pos = kb * PTB_PAGE + j;
-      float dot = 0.f;
-      const float* qr = qs + r * head_dim;
-      const float* kr = kv + j * kstride;
-      for (int e = 0; e < head_dim; ++e) dot = fmaf(qr[e], kr[e], dot);
-      bool visible = key_pos <= my_pos;
-      if (window > 0) visible = visible && (key_pos > my_pos - window || key_pos < keep_first);
-      float sc = -INFINITY;
-      if (visible) {
-        if (alibi_slopes) dot += alibi_bias(slope, key_pos);
-        sc = dot * scale;
-        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) s[u][jj] = 0.f;
+    for (int e = 0; e < kwords; ++e) {
+      float4 a[2], b[4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) a[u] = *reinterpret_cast<const float4*>(qs + (r0 + u) * kpitch + 4 * e);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) b[jj] = *reinterpret_cast<const float4*>(ks + (lane + 16 * jj) * kpitch + 4 * e);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+          s[u][jj] = fmaf(a[u].w, b[jj].w, fmaf(a[u].z, b[jj].z, fmaf(a[u].y, b[jj].y, fmaf(a[u].x, b[jj].x, s[u][jj]))));
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int my_pos = (r0 + u < rows) ? first_pos + r0 + u : -1;  // -1: no key is visible, nothing is stored
+      float m_blk = -INFINITY;
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int key_pos = kb * PTB_PAGE + lane + 16 * jj;
+        bool visible = key_pos <= my_pos;
+        if (window > 0) visible = visible && (key_pos > my_pos - window || key_pos < keep_first);
+        float sc = -INFINITY;
+        if (visible) {
+          sc = s[u][jj];
+          if (alibi_slopes) sc += alibi_bias(slope, key_pos);
+          sc *= scale;
+          if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+        }
+        s[u][jj] = sc;
+        m_blk = fmaxf(m_blk, sc);
       }
-      s[jj] = sc;
-      m_blk = fmaxf(m_blk, sc);
+      // row maximum and sum over the 16 lanes of the row
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) m_blk = fmaxf(m_blk, __shfl_xor_sync(0xffffffffu, m_blk, o));
+      const float m_new = fmaxf(m_run[u], m_blk);
+      float corr = 1.f, l_blk = 0.f;
+      float* prow = ps + (r0 + u) * PPITCH + lane;
+      if (m_new == -INFINITY) {
+        // nothing visible so far (rows beyond the tile, or keys left of a window)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) prow[16 * jj] = 0.f;
+      } else {
+        corr = (m_run[u] == -INFINITY) ? 0.f : expf(m_run[u] - m_new);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          const float p = (s[u][jj] == -INFINITY) ? 0.f : expf(s[u][jj] - m_new);
+          prow[16 * jj] = p;
+          l_blk += p;
+        }
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) l_blk += __shfl_xor_sync(0xffffffffu, l_blk, o);
+      l_run[u] = l_run[u] * corr + l_blk;
+      m_run[u] = m_new;
+#pragma unroll
+      for (int i = 0; i < 4 * COLS; ++i) acc[u][i] *= corr;
     }
-    // row maximum and sum over the 8 threads of the row (lanes 8 r' .. 8 r' + 7 of a warp)
+    __syncthreads();  // all scores of this page are written, its keys are no longer read
+    if (next <= kb_hi) load_keys(next);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();  // this page's values are here
+    for (int j = 0; j < PTB_PAGE; j += 4) {
+      float4 p[2];
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) m_blk = fmaxf(m_blk, __shfl_xor_sync(0xffffffffu, m_blk, o));
-    const float m_new = fmaxf(m_run, m_blk);
-    float corr = 1.f, l_blk = 0.f;
-    if (m_new == -INFINITY) {
-      // nothing visible so far (rows beyond the tile, or keys left of a window)
+      for (int u = 0; u < 2; ++u) p[u] = *reinterpret_cast<const float4*>(ps + (r0 + u) * PPITCH + j);
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) ps[r * PTB_PAGE + c + 8 * jj] = 0.f;
-    } else {
-      corr = (m_run == -INFINITY) ? 0.f : expf(m_run - m_new);
+      for (int jj = 0; jj < 4; ++jj) {
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        const float p = (s[jj] == -INFINITY) ? 0.f : expf(s[jj] - m_new);
-        ps[r * PTB_PAGE + c + 8 * jj] = p;
-        l_blk += p;
+        for (int c = 0; c < COLS; ++c) {
+          const int e = 4 * lane + 64 * c;
+          if (e < v_dim) {
+            const float4 v = *reinterpret_cast<const float4*>(vs + (j + jj) * vpitch + e);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const float w = jj == 0 ? p[u].x : jj == 1 ? p[u].y : jj == 2 ? p[u].z : p[u].w;
+              acc[u][4 * c] = fmaf(w, v.x, acc[u][4 * c]);
+              acc[u][4 * c + 1] = fmaf(w, v.y, acc[u][4 * c + 1]);
+              acc[u][4 * c + 2] = fmaf(w, v.z, acc[u][4 * c + 2]);
+              acc[u][4 * c + 3] = fmaf(w, v.w, acc[u][4 * c + 3]);
+            }
+          }
+        }
       }
     }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) l_blk += __shfl_xor_sync(0xffffffffu, l_blk, o);
-    l_run = l_run * corr + l_blk;
-    m_run = m_new;
-    __syncthreads();  // all scores of this block are written, K is no longer read
-    for (int i = tid; i < PTB_PAGE * v_dim; i += THREADS) {
-      const int j = i / v_dim, e = i % v_dim;
-      kv[j * vstride + e] = (j < valid) ? to_f(vp[i]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < DPT; ++i) acc[i] *= corr;
-    for (int j = 0; j < PTB_PAGE; ++j) {
-      const float p = ps[r * PTB_PAGE + j];
-      const float* vr = kv + j * vstride;
-#pragma unroll
-      for (int i = 0; i < DPT; ++i) {
-        const int e = c + 8 * i;
-        if (e < v_dim) acc[i] = fmaf(p, vr[e], acc[i]);
-      }
-    }
+    __syncthreads();  // the values and the scores are no longer read
+    kb = next;
   }
-  if (r < rows) {
-    float keep = 1.f;      // what the keys' share of the denominator shrinks by when the sink raises the reference
-    if (sinks) {
-      const float sink = sinks[h], m_all = fmaxf(m_run, sink);
-      keep = (m_run == -INFINITY) ? 0.f : expf(m_run - m_all);
-      l_run = l_run * keep + expf(sink - m_all);
-    }
-    float inv = (l_run > 0.f ? 1.f / l_run : 0.f) * keep * out_scale;
-    if (gate && !gate_wide) inv *= 1.f / (1.f + expf(-to_f(gate[size_t(start + q0 + r) * gate_stride + h])));
-    if (out_wide) {
-      // float32 [token][head][K/V head][v_dim]
-      float* o = out_wide + ((size_t(start + q0 + r) * heads + h) * kv_heads + gv) * v_dim;
+  cp_async_wait<0>();
 #pragma unroll
-      for (int i = 0; i < DPT; ++i) {
-        const int e = c + 8 * i;
-        if (e < v_dim) o[e] = acc[i] * inv;
-      }
-      return;
+  for (int u = 0; u < 2; ++u) {
+    const int r = r0 + u;
+    if (r >= rows) continue;
+    float keep = 1.f, l = l_run[u];      // keep: what the keys' share of the denominator shrinks by when the sink raises the reference
+    if (sinks) {
+      const float sink = sinks[h], m_all = fmaxf(m_run[u], sink);
+      keep = (m_run[u] == -INFINITY) ? 0.f : expf(m_run[u] - m_all);
+      l = l * keep + expf(sink - m_all);
     }
-    T* o = out + size_t(start + q0 + r) * out_stride + size_t(h) * v_dim;
+    float inv = (l > 0.f ? 1.f / l : 0.f) * keep * out_scale;
+    if (gate && !gate_wide) inv *= 1.f / (1.f + expf(-to_f(gate[size_t(start + q0 + r) * gate_stride + h])));
+    // out_wide: float32 [token][head][K/V head][v_dim]
+    float* ow = out_wide ? out_wide + ((size_t(start + q0 + r) * heads + h) * kv_heads + gv) * v_dim : nullptr;
+    T* o = out_wide ? nullptr : out + size_t(start + q0 + r) * out_stride + size_t(h) * v_dim;
     const T* ge = (gate && gate_wide) ? gate + size_t(start + q0 + r) * gate_stride + size_t(h) * v_dim : nullptr;
 #pragma unroll
-    for (int i = 0; i < DPT; ++i) {
-      const int e = c + 8 * i;
-      if (e < v_dim) o[e] = from_f<T>(acc[i] * inv * (ge ? 1.f / (1.f + expf(-to_f(ge[e]))) : 1.f));
+    for (int i = 0; i < 4 * COLS; ++i) {
+      const int e = 4 * lane + 64 * (i / 4) + i % 4;
+      if (e >= v_dim) continue;
+      if (ow) ow[e] = acc[u][i] * inv;
+      else o[e] = from_f<T>(acc[u][i] * inv * (ge ? 1.f / (1.f + expf(-to_f(ge[e]))) : 1.f));
     }
   }
 }
@@ -530,21 +592,27 @@ int launch_attention(const void* q, const void* k_pool, const void* v_pool, void
                      int kv_heads, int head_dim, float scale, int window, int v_dim, const float* sinks, const void* gate,
                      int gate_stride, float out_scale, int out_stride, int keep_first, float* out_wide, float softcap,
                      int gate_wide, cudaStream_t stream) {
-  const int wide = head_dim > v_dim ? head_dim : v_dim;
-  const size_t smem = sizeof(float) * (size_t(BQ) * head_dim + size_t(PTB_PAGE) * (wide + 1) + BQ * PTB_PAGE);
-  static size_t configured = 48 * 1024;  // per element type: raised when a larger head size first comes
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(attention_generic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-        cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  const size_t smem = sizeof(float) * (size_t(BQ + PTB_PAGE) * odd_words(head_dim) + size_t(PTB_PAGE) * odd_words(v_dim) + BQ * PPITCH);
+  const int async = sizeof(T) == 4 && head_dim % 4 == 0 && v_dim % 4 == 0 && aligned16(k_pool) && aligned16(v_pool);
   dim3 grid(n_tiles, heads, out_wide ? kv_heads : 1);
-  attention_generic_kernel<T><<<grid, THREADS, smem, stream>>>((const T*)q, (const T*)k_pool, (const T*)v_pool,
-                                                               (T*)out, sb, tile_seq, tile_q0, slopes, heads, kv_heads,
-                                                               head_dim, scale, window, v_dim, sinks, (const T*)gate,
-                                                               gate_stride, out_scale, out_stride, keep_first, out_wide,
-                                                               softcap, gate_wide);
+#define PTB_AG(CC)                                                                                                              \
+  do {                                                                                                                          \
+    static size_t configured = 48 * 1024; /* per instance: raised when a larger head size first comes */                       \
+    if (smem > configured) {                                                                                                    \
+      if (cudaFuncSetAttribute(attention_generic_kernel<T, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=      \
+          cudaSuccess)                                                                                                          \
+        return PTB_ERR_LAUNCH;                                                                                                  \
+      configured = smem;                                                                                                        \
+    }                                                                                                                           \
+    attention_generic_kernel<T, CC><<<grid, THREADS, smem, stream>>>(                                                           \
+        (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, sb, tile_seq, tile_q0, slopes, heads, kv_heads, head_dim,     \
+        scale, window, v_dim, sinks, (const T*)gate, gate_stride, out_scale, out_stride, keep_first, out_wide, softcap,         \
+        gate_wide, async);                                                                                                      \
+  } while (0)
+  if (v_dim <= 64) PTB_AG(1);
+  else if (v_dim <= 128) PTB_AG(2);
+  else PTB_AG(4);
+#undef PTB_AG
   return launch_status();
 }
 

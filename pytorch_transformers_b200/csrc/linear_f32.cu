@@ -1,80 +1,176 @@
 // True float32 linear layer on the CUDA cores: y[m, n] = act(sum_k x[m, k] * w[n, k] + bias[n]).
 // No tensor cores and no reduced-precision mode: every product and sum is an IEEE float32 FMA.
-// Each output element is accumulated by one thread over k in ascending order (16 products at a
-// time, then into the total), so a row's result does not depend on how many other rows are in the
-// launch or on the tiling, and the rounding error stays small for K in the tens of thousands.
-#include "common.cuh"
+//
+// The sums of one output element: the k of a step of 32 are summed in two chains (even and odd k, 16 products each, ascending),
+// the two chains join and go into a running total; a K of 1,024 or more is cut into 2 or 4 stretches whose totals are added
+// in order. All of this follows from N and K alone, so a row's result depends neither on how many other rows are in the
+// launch nor on the tile, and the rounding error stays small for K in the tens of thousands.
+//
+// What bounds it is the FMA pipe (128 lanes an SM). A block owns 8 TM rows x 64 outputs, a thread TM x 4 of them: of every
+// 16 bytes that it reads from shared memory (operands stay in [row][k] order, so cp.async brings them without a
+// transposition, and rows lie 36 floats apart, which lets eight rows' 16-byte words meet no bank twice) it makes
+// 2 TM x 4 / (TM + 4) two-wide FMAs (fma.rn.f32x2: the two k chains in one 64-bit register). A three-stage ring keeps two
+// steps of copies in flight. Matrices with few outputs would leave SMs idle: their K is cut among a thread-block cluster
+// whose blocks join their tiles through distributed shared memory.
+// One B200: the four products of a block of width 1,024 on 700 rows 1,057 -> 517 us (700 x 1,024 x 4,096: 152 us, 39 TFLOP/s of
+// 72; 2,048 rows: 43), 20 rows of 1,024 x 4,096 30 us; before, 64 x 64 tiles with two scalar loads a product and no copies in
+// flight. Now the two-wide FMAs of three blocks an SM leave half of the issue slots empty: registers (168 a thread) allow no more
+// warps, and tiles of 8 x 8 a thread, which read less, were as fast (43) at 2,048 rows and slower below.
+#include <cooperative_groups.h>
+
+#include "mma_common.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;  // tile of the output and step along K
-constexpr int TM = 4, TN = 4;             // outputs per thread; 256 threads
+namespace cg = cooperative_groups;
 
+constexpr int TN = 4, LBN = 16 * TN, LBK = 32, LPITCH = LBK + 4, LSTAGES = 3, LTHREADS = 128;
 
-__global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                         const float* __restrict__ bias, float* __restrict__ y, int M,
-                                                         int N, int K, int ldx, int act) {
-  // k-major tiles: xs[k][m], ws[k][n]; +4 padding keeps the transposing stores off one bank
-  __shared__ float xs[BK][BM + 4];
-  __shared__ float ws[BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tm = (tid / 16) * TM, tn = (tid % 16) * TN;
-  // loader mapping: 256 threads fetch 64 rows x 16 k: thread -> (row = tid / 4, k = (tid % 4) * 4 .. +3)
-  const int lrow = tid / 4, lk = (tid % 4) * 4;
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float2 halves(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+// copies that leave zeros where `bytes` is 0 (a row or a k past the end; the address is then any valid one)
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
+
+// rows [row0, row0 + ROWS) x k [k0, k0 + 32) of a matrix with rows ld apart; k_end: the end of this block's stretch
+template <int ROWS, bool VEC>
+__device__ __forceinline__ void stage_rows(float* dst, const float* src, int row0, int n_rows, size_t ld, int k0, int k_end) {
+  constexpr int W = VEC ? 4 : 1, PER_ROW = LBK / W;
+#pragma unroll
+  for (int i = threadIdx.x; i < ROWS * PER_ROW; i += LTHREADS) {
+    const int r = i / PER_ROW, k = k0 + (i % PER_ROW) * W;
+    const bool ok = row0 + r < n_rows && k < k_end;
+    const float* from = ok ? src + size_t(row0 + r) * ld + k : src;
+    const uint32_t to = smem_u32(dst + r * LPITCH + (i % PER_ROW) * W);
+    if (VEC) copy16(to, from, ok ? 16 : 0);
+    else copy4(to, from, ok ? 4 : 0);
+  }
+}
+
+template <int TM, bool VEC>
+__global__ void __launch_bounds__(LTHREADS, 3)
+linear_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                  float* __restrict__ y, int M, int N, int K, int ldx, int act, int stretch) {
+  constexpr int BM = 8 * TM, STAGE = (BM + LBN) * LPITCH;
+  extern __shared__ __align__(16) float lsm[];
+  const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;      // rows ty + 8 i, outputs tx + 16 j
+  const int n0 = blockIdx.x * LBN, m0 = blockIdx.y * BM;
+  const int k_begin = int(blockIdx.z) * stretch, k_end = min(K, k_begin + stretch);
+  const int steps = k_end > k_begin ? (k_end - k_begin + LBK - 1) / LBK : 0;
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  auto load = [&](int s) {
+    float* st = lsm + (s % LSTAGES) * STAGE;
+    stage_rows<BM, VEC>(st, x, m0, M, size_t(ldx), k_begin + s * LBK, k_end);
+    stage_rows<LBN, VEC>(st + BM * LPITCH, w, n0, N, size_t(K), k_begin + s * LBK, k_end);
+  };
+#pragma unroll
+  for (int s = 0; s < LSTAGES - 1; ++s) {
+    if (s < steps) load(s);
+    cp_async_commit();
+  }
+  for (int s = 0; s < steps; ++s) {
+    cp_async_wait<LSTAGES - 2>();
+    __syncthreads();      // step s has landed for everybody, and step s - 1 is no longer read
+    if (s + LSTAGES - 1 < steps) load(s + LSTAGES - 1);
+    cp_async_commit();
+    const float* xs = lsm + (s % LSTAGES) * STAGE + ty * LPITCH;
+    const float* ws = lsm + (s % LSTAGES) * STAGE + (BM + tx) * LPITCH;
+    unsigned long long part[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) part[i][j] = 0ull;
+#pragma unroll
+    for (int k = 0; k < LBK; k += 4) {
+      ulonglong2 b[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + 16 * j * LPITCH + k);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + 8 * i * LPITCH + k);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma2(part[i][j], a.x, b[j].x);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma2(part[i][j], a.y, b[j].y);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const float2 p = halves(part[i][j]);
+        acc[i][j] += p.x + p.y;
+      }
+  }
+  cp_async_wait<0>();
+  auto store = [&](int gm, int gn, float v) {
+    if (gm >= M || gn >= N) return;
+    if (bias) v += bias[gn];
+    y[size_t(gm) * N + gn] = apply_activation(v, act);
+  };
+  if (gridDim.z == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) store(m0 + ty + 8 * i, n0 + tx + 16 * j, acc[i][j]);
+    return;
+  }
+  // the stretches' totals join: every block leaves its tile in its shared memory and finishes a share of the rows
+  cg::cluster_group cluster = cg::this_cluster();
+  __syncthreads();      // the ring is no longer read
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) lsm[(ty + 8 * i) * LBN + tx + 16 * j] = acc[i][j];
+  cluster.sync();
+  const int rank = int(blockIdx.z), ranks = int(gridDim.z), share = BM / ranks;      // ranks: 2 or 4, BM a multiple of 16
+  for (int e = tid; e < share * LBN; e += LTHREADS) {
+    const int at = rank * share * LBN + e;
+    float v = 0.f;
+    for (int r = 0; r < ranks; ++r) v += *cluster.map_shared_rank(lsm + at, r);
+    store(m0 + at / LBN, n0 + at % LBN, v);
+  }
+  cluster.sync();       // no block leaves while its tile is still read
+}
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = k0 + lk + q;
-      const int gm = m0 + lrow, gn = n0 + lrow;
-      xs[lk + q][lrow] = (gm < M && k < K) ? x[size_t(gm) * ldx + k] : 0.f;
-      ws[lk + q][lrow] = (gn < N && k < K) ? w[size_t(gn) * K + k] : 0.f;
-    }
-    __syncthreads();
-    // two levels of summation: the 16 products of this step are summed on their own and then added
-    // to the total, so the rounding error grows with K / 16 + 16 instead of with K
-    float part[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) part[i][j] = 0.f;
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = xs[k][tm + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = ws[k][tn + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) part[i][j] = fmaf(a[i], b[j], part[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] += part[i][j];
-    __syncthreads();
+template <int TM, bool VEC>
+int launch_linear_f32(const float* x, const float* w, const float* bias, float* y, int M, int N, int K, int ldx, int act,
+                      int ranks, cudaStream_t stream) {
+  const size_t smem = size_t(LSTAGES) * (8 * TM + LBN) * LPITCH * sizeof(float);
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(linear_f32_kernel<TM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+      return PTB_ERR_LAUNCH;
+    configured = true;
   }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int gm = m0 + tm + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gn = n0 + tn + j;
-      if (gn >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[gn];
-      y[size_t(gm) * N + gn] = apply_activation(v, act);
-    }
-  }
+  const int steps = (K + LBK - 1) / LBK, stretch = (steps + ranks - 1) / ranks * LBK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((N + LBN - 1) / LBN, (M + 8 * TM - 1) / (8 * TM), ranks);
+  cfg.blockDim = dim3(LTHREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = ranks;
+  cfg.attrs = attr;
+  cfg.numAttrs = ranks > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, linear_f32_kernel<TM, VEC>, x, w, bias, y, M, N, K, ldx, act, stretch);
+  return launch_status();
 }
 
 }  // namespace
@@ -84,8 +180,15 @@ PTB_API int ptb_linear_f32(const float* x, const float* w, const float* bias, fl
                            cudaStream_t stream) {
   if (M <= 0 || N <= 0) return PTB_OK;
   if (K <= 0 || ldx < K || !activation_known(act)) return PTB_ERR_SIZE;
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) return PTB_ERR_SIZE;
-  linear_f32_kernel<<<grid, 256, 0, stream>>>(x, w, bias, y, M, N, K, ldx, act);
-  return launch_status();
+  if ((long(M) + 63) / 64 > 65535) return PTB_ERR_SIZE;
+  // stretches of K, by N and K alone (the order of a row's sums must not follow the number of rows): a matrix of 1,024
+  // outputs and 700 rows has 176 tiles, little more than an SM each, which two or four stretches even out
+  const int ranks = K >= 2048 ? 4 : (K >= 1024 && N < 2048) ? 2 : 1;
+  // 16-byte copies where every row starts at a whole word
+  const bool vec = K % 4 == 0 && ldx % 4 == 0 && aligned16(x) && aligned16(w);
+#define PTB_LF(TT) (vec ? launch_linear_f32<TT, true>(x, w, bias, y, M, N, K, ldx, act, ranks, stream) \
+                        : launch_linear_f32<TT, false>(x, w, bias, y, M, N, K, ldx, act, ranks, stream))
+  // rows of a tile: 64, or 16 or 32 for steps of few rows, which would be computed for padding otherwise
+  return M <= 16 ? PTB_LF(2) : M <= 32 ? PTB_LF(4) : PTB_LF(8);
+#undef PTB_LF
 }

@@ -133,6 +133,21 @@ def test_linear_f32_rows_do_not_depend_on_the_batch(K):
         assert torch.equal(part, full[rows])
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 131])
+@pytest.mark.parametrize("n,k", [(64, 1024), (65, 1056), (2048, 1024), (7, 2048), (130, 2081), (64, 4100)])
+def test_linear_f32_tiles_and_stretches(K, m, n, k):
+    """Tiles of 16, 32 and 64 rows with remainders, K in one, two and four stretches, rows at odd words, rows that lie apart.
+    An element's error: its chains are 16 products long, then about k / 32 sums, each a rounding of 2^-24 of the partial sum."""
+    wide, w = rnd(m, k + 3, seed=1), rnd(n, k, seed=2, scale=0.1)
+    b = rnd(n, seed=3)
+    for x in (wide[:, :k], wide[:, :k].contiguous()):
+        out = K.linear_f32(x, w, b)
+        ref = x.double() @ w.double().T + b.double()
+        bound = (16 + k / 32 + 6) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+        assert ((out.double() - ref).abs() <= bound).all()
+    assert torch.equal(K.linear_f32(wide[-1:, :k], w, b), K.linear_f32(wide[:, :k], w, b)[-1:])
+
+
 def test_to_float(K):
     x = rnd(3, 1000, dtype=torch.bfloat16)
     assert torch.equal(K.to_float(x), x.float())
