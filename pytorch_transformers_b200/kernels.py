@@ -98,7 +98,7 @@ def lib():
                      "ptb_fill_normal", "ptb_selftest_bounded_wait", "ptb_scale", "ptb_selftest_mma_cadence",
                      "ptb_norm_stream", "ptb_add_stream", "ptb_latent_store", "ptb_latent_attention", "ptb_latent_rows",
                      "ptb_rglru_conv", "ptb_rglru_scan", "ptb_block_linear", "ptb_route", "ptb_expert_plan",
-                     "ptb_expert_linear", "ptb_expert_combine", "ptb_expert_linear_mma", "ptb_latent_attention_mma",
+                     "ptb_expert_linear", "ptb_expert_combine", "ptb_expert_linear_tc", "ptb_latent_attention_mma",
                      "ptb_latent_attention_mma_supports", "ptb_rglru_scan_chunks", "ptb_block_epilogue", "ptb_latent_gather",
                      "ptb_latent_unfold", "ptb_latent_q_unfold", "ptb_gate_heads", "ptb_linear_attention_scan",
                      "ptb_linear_attention_chunks", "ptb_linear_attention_chunks_supports", "ptb_norm_gate",
@@ -1040,7 +1040,17 @@ def rglru_scan_chunks(gates: torch.Tensor, u: torch.Tensor, y_act: torch.Tensor,
 # ------------------------------------------------------------------------------------------------
 # Routed experts
 EXPERT_TILE_ROWS = (16, 64)   # rows of a tile of the grouped products: few pairs, many pairs
-EXPERT_MMA_TILE_ROWS = (64, 128)   # rows of a tile of the tensor-core kernel
+EXPERT_MMA_TILE_ROWS = (16, 32, 64, 128, 256)   # most rows of a tile of the tensor-core kernel
+
+
+def expert_tile_rows(pairs: int, n_experts: int) -> int:
+    """Most rows of a tile of the tensor-core kernel: the smallest size that holds an expert's share of the pairs with some
+    room, so that a matrix crosses to the SMs once for all rows of its expert. A tile costs what its rows need, but its
+    ring and tensor memory are as large as its most rows."""
+    share = 1.2 * pairs / max(1, n_experts) + 4
+    return next((t for t in EXPERT_MMA_TILE_ROWS if share <= t), EXPERT_MMA_TILE_ROWS[-1])
+
+
 
 
 ROUTE_SCORES = {"softmax": 0, "sigmoid": 1, "softmax_chosen": 2}
@@ -1095,12 +1105,10 @@ def expert_rows(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
         raise KernelError("expert_rows: a clamped unit belongs to gated experts and has a positive limit")
     limit, alpha = (ctypes.c_float(clamp[0]), ctypes.c_float(clamp[1])) if clamp is not None else (ctypes.c_float(0), ctypes.c_float(0))
     pairs = n_tokens * top
-    # bfloat16 with row sizes in whole 16-byte words: the tensor-core kernel (tiles of 64 rows); else float32 FMAs
+    # bfloat16 with row sizes in whole 16-byte words: the tensor-core kernel; else float32 FMAs
     mma = h.dtype == torch.bfloat16 and width % 8 == 0 and f % 8 == 0
     if mma:
-        # tiles of 64 rows; 128 are built and tested too, but with about 200 rows an expert they were slower
-        # (3.8 against 3.3 ms for four layers of 12,288 pairs over 64 experts): half-empty last tiles, fewer blocks an SM
-        tile_rows = mma_tile_rows or EXPERT_MMA_TILE_ROWS[0]
+        tile_rows = mma_tile_rows or expert_tile_rows(pairs, n_experts)
         if tile_rows not in EXPERT_MMA_TILE_ROWS:
             raise KernelError(f"routed_experts: tiles of {EXPERT_MMA_TILE_ROWS} rows, got {tile_rows}")
     else:
@@ -1114,10 +1122,12 @@ def expert_rows(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
     a = torch.empty((pairs, f), dtype=h.dtype, device=h.device)
     y = torch.empty((pairs, width), dtype=torch.float32, device=h.device)
     if mma:
-        _check(L.ptb_expert_linear_mma(first, _ptr(h), _ptr(w_gate_up), _ptr(a), _ptr(plan), pairs, max_tiles, top, f, width,
-                                       tile_rows, _ptr(scale), act, limit, alpha, stream), "expert_linear_mma (gate, up)")
-        _check(L.ptb_expert_linear_mma(1, _ptr(a), _ptr(w_down), _ptr(y), _ptr(plan), pairs, max_tiles, top, width, f,
-                                       tile_rows, None, 0, ctypes.c_float(0), ctypes.c_float(0), stream), "expert_linear_mma (down)")
+        flag = _ptr(error_flag(h.device))
+        _check(L.ptb_expert_linear_tc(first, _ptr(h), _ptr(w_gate_up), _ptr(a), _ptr(plan), pairs, max_tiles, top, n_experts, f,
+                                      width, tile_rows, _ptr(scale), act, limit, alpha, flag, stream), "expert_linear_tc (gate, up)")
+        _check(L.ptb_expert_linear_tc(1, _ptr(a), _ptr(w_down), _ptr(y), _ptr(plan), pairs, max_tiles, top, n_experts, width, f,
+                                      tile_rows, None, 0, ctypes.c_float(0), ctypes.c_float(0), flag, stream),
+               "expert_linear_tc (down)")
     else:
         _check(L.ptb_expert_linear(code, first, _ptr(h), _ptr(w_gate_up), _ptr(a), _ptr(plan), pairs, max_tiles, top, f, width,
                                    tile_rows, _ptr(scale), act, limit, alpha, stream), "expert_linear (gate, up)")

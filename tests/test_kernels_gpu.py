@@ -320,3 +320,39 @@ def test_a_bounded_wait_that_runs_out_raises_on_the_host_and_leaves_the_device_u
     torch.testing.assert_close(out.double().cpu(), x.double().cpu() @ w.double().cpu().T, **tol(bf))
     with pytest.raises(KernelError):
         K.selftest_bounded_wait(dev, tries=0)
+
+
+@pytest.mark.parametrize("kind", ["gated", "clamped", "plain", "plain on input"])
+@pytest.mark.parametrize("width,inner", [(72, 136), (200, 1000), (1024, 8)])
+@pytest.mark.parametrize("tile_rows", [0, 16, 32, 64, 128, 256])
+def test_expert_tiles(K, kind, width, inner, tile_rows):
+    """Experts with no rows, one, a tile's rows and one more, remainders of 16, several tiles; K and outputs that end within a
+    stage or a block. The inner values are rounded to bfloat16 on both sides, so they may differ by one unit (2^-8 of
+    themselves) where float32 sums fall on either side of a tie: that bounds a result's error through |W_down|."""
+    counts = [0, 1, 15, 16, 17, 255, 256, 257, 0, 300]
+    n_experts, tokens = len(counts), sum(counts)
+    h = rnd(tokens, width, dtype=torch.bfloat16, seed=1)
+    g = torch.Generator().manual_seed(5)
+    ids = torch.repeat_interleave(torch.arange(n_experts), torch.tensor(counts))[torch.randperm(tokens, generator=g)]
+    plain_kind = kind.startswith("plain")
+    up = rnd(n_experts, inner if plain_kind else 2 * inner, width, dtype=torch.bfloat16, scale=width ** -0.5, seed=2)
+    down = rnd(n_experts, width, inner, dtype=torch.bfloat16, scale=inner ** -0.5, seed=3)
+    weights = rnd(tokens, 1, seed=4).abs()
+    on_input = kind == "plain on input"
+    y, rows = K.expert_rows(h, ids.int().reshape(-1, 1).cuda(), up, down, mma_tile_rows=tile_rows, plain_act="gelu" if plain_kind else None,
+                            input_weights=weights if on_input else None, clamp=(1.0, 1.702) if kind == "clamped" else None)
+    got = y[rows.long()]
+    for e in range(n_experts):
+        at = (ids == e).nonzero()[:, 0].cuda()
+        z = h[at].double() @ up[e].double().T
+        if plain_kind:
+            a = plain.activation((z * weights[at].double() if on_input else z).cpu(), "gelu").cuda()
+        elif kind == "clamped":
+            gate, u = z[:, :inner].clamp(max=1.0), z[:, inner:].clamp(-1.0, 1.0)
+            a = gate * torch.sigmoid(1.702 * gate) * (u + 1)
+        else:
+            a = z[:, :inner] * torch.sigmoid(z[:, :inner]) * z[:, inner:]
+        a = a.bfloat16().double()
+        bound = (2.0 ** -8 * a.abs() + 1e-5) @ down[e].double().abs().T + 1e-5
+        assert ((got[at].double() - a @ down[e].double().T).abs() <= bound).all(), (kind, e)
+    K.check_device_errors("cuda:0")
