@@ -92,6 +92,14 @@ struct TcParams {
   int heads, kv_heads;
   float scale;
   const float* slopes;   // per-head score slopes (ALiBi), or null
+  // EXTRAS only
+  int window, keep_first;            // window > 0: a query sees the last `window` keys and the sequence's first `keep_first`
+  float softcap;                     // > 0: score <- softcap * tanh(score / softcap) after the scale
+  const float* sinks;                // per head, or null: exp(sink) joins the softmax's denominator
+  const __nv_bfloat16* gate;         // or null: token t, head h at gate[t * gate_stride + h], or with gate_wide a number per
+  int gate_stride, gate_wide;        // entry at gate[t * gate_stride + h * DV + e]; the result times sigmoid(gate)
+  float out_scale;                   // multiplies everything
+  int out_stride;                    // from one token's results to the next's
 };
 
 constexpr int SOFTMAX_THREADS = TQ;                 // one thread per query row
@@ -105,7 +113,12 @@ constexpr int BLOCK_THREADS = SOFTMAX_THREADS + 64;
 // WIDE: the softmax weights meet V as two bfloat16 terms (the rounded weight, then what the rounding left: 16
 // bits of mantissa). The terms of a page, 32 columns each, together take the place of its S; O += P V is two
 // groups of matrix instructions on the same V tile.
-template <int DK, int DV, bool BIAS, bool WIDE>
+// EXTRAS: a window with kept first positions, a soft cap, sinks, an output gate, an output factor and strided results. A walk
+// takes the kept pages, then the window's: page i of the walk is not page i of the sequence, and a row may see nothing of a
+// page. Nothing else of the pipeline changes. What such a prompt costs is the chain of a page as above (a cap adds an
+// exponential and a reciprocal a score): 16 heads of 128 on 4 K/V heads, 2,048 tokens, window 1,024: 41 us, where
+// the mma.sync kernel took 175; prompts of 500, 1,000 and 1,501 tokens, cap and a gate per entry: 104 us against 261.
+template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS>
 __global__ void __launch_bounds__(BLOCK_THREADS, DK == 64 ? 2 : 1)
 attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_pool,
                     const __nv_bfloat16* __restrict__ v_pool, __nv_bfloat16* __restrict__ out, StepBatch sb,
@@ -149,8 +162,14 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   const bool row_ok = row < tok_valid;
   const int row_pos = row_ok ? past + q0 + row : -1;
   const int last_pos = past + q0 + tok_valid - 1;
-  const int n_blocks = last_pos / KEYS + 1;
   const int* pages = sb.pages + size_t(seq) * sb.pages_stride;
+  int kb_lo = 0, kept_pages = 0;      // the window's first page for the tile's first token; kept pages left of it
+  if (EXTRAS && p.window > 0) {
+    kb_lo = max(0, past + q0 - p.window + 1) / KEYS;
+    kept_pages = min((p.keep_first + KEYS - 1) / KEYS, kb_lo);
+  }
+  const int n_blocks = kept_pages + last_pos / KEYS + 1 - kb_lo;
+  auto block_of = [&](int i) { return EXTRAS ? (i < kept_pages ? i : kb_lo + i - kept_pages) : i; };   // page i of the walk
 
   // A warp may be up to three pages ahead of another one (S of page i + 2 is issued before P of page i is
   // complete, S of page i + 3 only after it): arrivals for pages i + 1 and i + 2 must not count for page
@@ -181,7 +200,7 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   };
   int first_pages = 0;   // the copy warp's lanes: the number of page b = lane
   if (copy_warp) {
-    first_pages = lane < n_blocks ? pages[lane] : 0;
+    first_pages = lane < n_blocks ? pages[block_of(lane)] : 0;
     if (lane == 0) {
       for (int b = 0; b < 3; ++b) {
         mbar_init(bar_s + 8 * b, 1);
@@ -234,7 +253,7 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       int issued = min(n_blocks, STAGES_TC);
       for (int b = STAGES_TC; b < n_blocks; ++b) {
         if (!mbar_wait(bar_free + 8 * (b % STAGES_TC), ((b / STAGES_TC) - 1) & 1, error_flag, 6)) break;
-        ask_page(b, pages[b]);
+        ask_page(b, pages[block_of(b)]);
         issued = b + 1;
       }
       if (issued < n_blocks) {
@@ -300,9 +319,11 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
     int buf = 0, phase = 0;   // S buffer of page i (i % 3) and the parity of its barriers ((i / 3) & 1)
     float m_run = -INFINITY, l_run = 0.f;   // running maximum of the raw scores, the row's sum
     const float slope = BIAS ? p.slopes[h] : 0.f;
-    const float sl2 = p.scale * 1.4426950408889634f;
+    const bool capped = EXTRAS && p.softcap > 0.f;
+    const float sl2 = capped ? 1.f : p.scale * 1.4426950408889634f;      // capped scores are in powers of two already
     const uint64_t sl2_2 = pack2(sl2, sl2);
     for (int i = 0; i < n_blocks; ++i) {
+      const int key0 = block_of(i) * KEYS;
       // (1) this thread's row of S_i: both halves asked for, one wait
       if (alive) alive = mbar_wait(bar_s + buf * 8, phase, error_flag, 1);
       tc_fence_after();
@@ -310,13 +331,24 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       tmem_ld64_once(lane_addr + buf * 64, s);
       if (BIAS) {
 #pragma unroll
-        for (int j = 0; j < KEYS; ++j) s[j] += alibi_bias(slope, i * KEYS + j);
+        for (int j = 0; j < KEYS; ++j) s[j] += alibi_bias(slope, key0 + j);
       }
-      // (2) maximum of the visible scores; only pages that reach past some row's position need the test
-      if (i * KEYS + KEYS - 1 > past + q0 || !row_ok) {   // first part is uniform over the block
-        const int visible = row_pos - i * KEYS;   // columns j <= visible are seen by this row
+      if (capped) {      // tanh(x) = 1 - 2 / (1 + exp(2 x)), times the cap, in powers of two
+        const float in = p.scale * (2.f * 1.4426950408889634f / p.softcap), out2 = p.softcap * 1.4426950408889634f;
+#pragma unroll
+        for (int j = 0; j < KEYS; ++j) s[j] = out2 * (1.f - __fdividef(2.f, fast_exp2(s[j] * in) + 1.f));
+      }
+      // (2) maximum of the visible scores; only pages that reach past some row's position, or left of some row's window,
+      // need the test
+      if (key0 + KEYS - 1 > past + q0 || !row_ok) {   // first part is uniform over the block
+        const int visible = row_pos - key0;   // columns j <= visible are seen by this row
 #pragma unroll
         for (int j = 0; j < KEYS; ++j) s[j] = (j <= visible) ? s[j] : -INFINITY;
+      }
+      if (EXTRAS && p.window > 0 && key0 <= last_pos - p.window) {   // uniform over the block
+        const int left = row_pos - p.window - key0, kept = p.keep_first - key0;   // columns left < j or j < kept are seen
+#pragma unroll
+        for (int j = 0; j < KEYS; ++j) s[j] = (j > left || j < kept) ? s[j] : -INFINITY;
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -384,13 +416,36 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
     // the walk's last O += P V
     if (alive) alive = mbar_wait(bar_o + 8 * ((n_blocks - 1) & 3), ((n_blocks - 1) >> 2) & 1, error_flag, 3);
     tc_fence_after();
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    __nv_bfloat16* dst = out + (size_t(start + q0 + row) * p.heads + h) * DV;
+    float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+    const size_t t = size_t(start + q0 + row);
+    __nv_bfloat16* dst = out + (t * p.heads + h) * DV;
+    const __nv_bfloat16* ge = nullptr;      // a gate per entry
+    if (EXTRAS) {
+      if (p.sinks) {
+        const float m2 = m_run * sl2, sink2 = p.sinks[h] * 1.4426950408889634f, m_all = fmaxf(m2, sink2);
+        const float keep = (m_run == -INFINITY) ? 0.f : fast_exp2(m2 - m_all);
+        const float l = l_run * keep + fast_exp2(sink2 - m_all);
+        inv = (l > 0.f ? 1.f / l : 0.f) * keep;
+      }
+      inv *= p.out_scale;
+      dst = out + t * p.out_stride + size_t(h) * DV;
+      if (p.gate && p.gate_wide) ge = p.gate + t * p.gate_stride + size_t(h) * DV;
+      else if (p.gate && row_ok) inv *= 1.f / (1.f + expf(-__bfloat162float(p.gate[t * p.gate_stride + h])));
+    }
 #pragma unroll
     for (int c0 = 0; c0 < DV; c0 += 32) {
       float o[32];
       tmem_ld32(o_addr + c0, o);
       if (row_ok) {
+        if (EXTRAS && ge) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float gv[8];
+            unpack_bf16x8(*reinterpret_cast<const uint4*>(ge + c0 + c * 8), gv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[c * 8 + e] *= 1.f / (1.f + expf(-gv[e]));
+          }
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t w[4];
@@ -812,7 +867,7 @@ PTB_API int ptb_attention_tc_supports_sizes(int head_dim, int v_dim) {
 PTB_API int ptb_attention_tc_tile_tokens() { return TQ; }
 
 namespace {
-template <int DK, int DV, bool BIAS, bool WIDE>
+template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS = false>
 int launch_tc(const void* q, const void* k_pool, const void* v_pool, int pool_pages, void* out, const StepBatch& sb,
               const int* tile_seq, const int* tile_q0, int n_tiles, const TcParams& p, int* error_flag,
               cudaStream_t stream) {
@@ -822,12 +877,12 @@ int launch_tc(const void* q, const void* k_pool, const void* v_pool, int pool_pa
   const size_t smem = 1024 + TQ * DK * 2 + STAGES_TC * KEYS * (DK + DV) * 2 + 192;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_tc_kernel<DK, DV, BIAS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
       return PTB_ERR_LAUNCH;
     configured = true;
   }
   dim3 grid(p.heads, n_tiles);
-  attention_tc_kernel<DK, DV, BIAS, WIDE><<<grid, BLOCK_THREADS, smem, stream>>>(
+  attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS><<<grid, BLOCK_THREADS, smem, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, sb,
       tile_seq, tile_q0, p, *km, *vm, error_flag);
   return launch_status();
@@ -849,7 +904,7 @@ PTB_API int ptb_attention_tc_sizes(const void* q, const void* k_pool, const void
   if (!ptb_attention_tc_supports_sizes(head_dim, v_dim) || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 ||
       n_tiles > 65535 || error_flag == nullptr)
     return PTB_ERR_SIZE;
-  TcParams p;
+  TcParams p = {};
   p.heads = heads; p.kv_heads = kv_heads; p.scale = scale; p.slopes = slopes;
 #define PTB_TC(DK, DV, B, W) \
   launch_tc<DK, DV, B, W>(q, k_pool, v_pool, pool_pages, out, *sb, tile_seq, tile_q0, n_tiles, p, error_flag, stream)
@@ -879,4 +934,28 @@ PTB_API int ptb_attention_tc(const void* q, const void* k_pool, const void* v_po
   if (!ptb_attention_tc_supports(head_dim)) return PTB_ERR_SIZE;
   return ptb_attention_tc_sizes(q, k_pool, v_pool, pool_pages, out, sb, tile_seq, tile_q0, n_tiles, slopes, heads, kv_heads,
                                 head_dim, head_dim, scale, 0, error_flag, stream);
+}
+
+// The same with what some designs put around the softmax (TcParams), head sizes 64 and 128, weights of two terms. out: rows
+// out_stride apart and a gate per entry's rows at whole 16-byte words.
+PTB_API int ptb_attention_tc_extras(const void* q, const void* k_pool, const void* v_pool, int pool_pages, void* out,
+                                    const StepBatch* sb, const int* tile_seq, const int* tile_q0, int n_tiles, int heads,
+                                    int kv_heads, int head_dim, float scale, int window, int keep_first, float softcap,
+                                    const float* sinks, const void* gate, int gate_stride, int gate_wide, float out_scale,
+                                    int out_stride, int* error_flag, cudaStream_t stream) {
+  if (n_tiles <= 0) return PTB_OK;
+  if (pool_pages <= 0 || !aligned16(k_pool) || !aligned16(v_pool) || !aligned16(q) || !aligned16(out) || out_stride % 8 != 0 ||
+      (gate != nullptr && gate_wide && (!aligned16(gate) || gate_stride % 8 != 0)))
+    return PTB_ERR_ALIGN;
+  if (!ptb_attention_tc_supports(head_dim) || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || n_tiles > 65535 ||
+      error_flag == nullptr || window < 0 || keep_first < 0 || softcap < 0.f || out_stride < heads * head_dim ||
+      (gate != nullptr && gate_stride < (gate_wide ? heads * head_dim : heads)))
+    return PTB_ERR_SIZE;
+  TcParams p = {};
+  p.heads = heads; p.kv_heads = kv_heads; p.scale = scale; p.window = window; p.keep_first = keep_first; p.softcap = softcap;
+  p.sinks = sinks; p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride; p.gate_wide = gate_wide;
+  p.out_scale = out_scale; p.out_stride = out_stride;
+  return head_dim == 64
+             ? launch_tc<64, 64, false, true, true>(q, k_pool, v_pool, pool_pages, out, *sb, tile_seq, tile_q0, n_tiles, p, error_flag, stream)
+             : launch_tc<128, 128, false, true, true>(q, k_pool, v_pool, pool_pages, out, *sb, tile_seq, tile_q0, n_tiles, p, error_flag, stream);
 }

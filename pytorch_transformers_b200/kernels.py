@@ -111,7 +111,7 @@ def lib():
                      "ptb_qk_prepare_store", "ptb_route_grouped", "ptb_expert_combine_shared", "ptb_glu_act",
                      "ptb_head_norm_gate_act", "ptb_gla_decay", "ptb_gla_walk", "ptb_gla_chunks", "ptb_gla_max_dim",
                      "ptb_gla_chunk_tokens", "ptb_delta_prepare", "ptb_delta_walk", "ptb_delta_chunks",
-                     "ptb_delta_chunks_supports", "ptb_post_norm", "ptb_token_gate", "ptb_round_rows", "ptb_route_biased", "ptb_attention_tc_sizes", "ptb_attention_tc_supports_sizes"):
+                     "ptb_delta_chunks_supports", "ptb_post_norm", "ptb_token_gate", "ptb_round_rows", "ptb_route_biased", "ptb_attention_tc_sizes", "ptb_attention_tc_supports_sizes", "ptb_attention_tc_extras"):
             getattr(L, name).restype = ctypes.c_int
         L.ptb_latent_part_floats.restype = ctypes.c_longlong
         L.ptb_expert_plan_words.restype = ctypes.c_longlong
@@ -553,6 +553,35 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ba
                                         _ptr(tile_seq), _ptr(tile_q0), n_tiles, _ptr(slopes), heads, kv_heads, head_dim, v_dim,
                                         ctypes.c_float(scale), 1 if wide_weights else 0, _ptr(error_flag(q.device)),
                                         _stream(q)), "attention_tc")
+    return out
+
+
+def attention_tc_extras_take(out: torch.Tensor, gate: Optional[torch.Tensor] = None, gate_wide: bool = False) -> bool:
+    """Whether ``attention_tc_extras`` can write into ``out`` and read ``gate``: whole 16-byte words (a gate per head is read
+    number by number)."""
+    def words(t):
+        return t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0
+    return words(out) and (gate is None or not gate_wide or words(gate))
+
+
+def attention_tc_extras(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, batch: StepBatchC, tile_seq: torch.Tensor,
+                        tile_q0: torch.Tensor, n_tiles: int, kv_heads: int, scale: float, window: int = 0, keep_first: int = 0,
+                        softcap: float = 0.0, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
+                        gate_wide: bool = False, out_scale: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Prompt attention on tcgen05 in tiles of 128 tokens with what ``attention_generic`` takes around the softmax; the softmax
+    weights meet the values as two bfloat16 terms. bfloat16, head sizes 64 and 128, values of the keys' size."""
+    _need_cuda(q, k_pool, v_pool, tile_seq, tile_q0, sinks)
+    n, heads, head_dim = q.shape
+    if out is None:
+        out = torch.empty((n, heads * head_dim), dtype=q.dtype, device=q.device)
+    _check_rows(out, (n, heads * head_dim), q.dtype, "attention_tc_extras: out")
+    if gate is not None:
+        _check_rows(gate, (n, heads * head_dim if gate_wide else heads), q.dtype, "attention_tc_extras: gate")
+    _check(lib().ptb_attention_tc_extras(_ptr(q), _ptr(k_pool), _ptr(v_pool), k_pool.shape[0], _ptr(out), ctypes.byref(batch),
+                                         _ptr(tile_seq), _ptr(tile_q0), n_tiles, heads, kv_heads, head_dim, ctypes.c_float(scale),
+                                         int(window), int(keep_first), ctypes.c_float(softcap), _ptr(sinks), _ptr(gate),
+                                         0 if gate is None else gate.stride(0), 1 if gate_wide else 0, ctypes.c_float(out_scale),
+                                         out.stride(0), _ptr(error_flag(q.device)), _stream(q)), "attention_tc_extras")
     return out
 
 

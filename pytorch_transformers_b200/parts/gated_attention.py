@@ -163,6 +163,11 @@ class SinkAttention(Part):
         gate = proj[:, self.in_rows() - self.gate_cols:] if self.has_gate else None
         tiles = ctx.plan(AttentionTiles.plan_key)
         extras = {"softcap": self.softcap, "gate_wide": self.gate_wide}
+        if self._tc_takes(q, tiles, out, gate):
+            k.attention_tc_extras(q, k_pool, v_pool, batch, tiles.dev["mtile_seq"], tiles.dev["mtile_q0"], tiles.facts["n_mma_tiles"],
+                                  self.kv_heads, self.scale, self.window, sinks=self.p_sink, gate=gate, out_scale=out_scale,
+                                  out=out, **extras)
+            return
         if (q.dtype == torch.bfloat16 and self.dim == self.vdim and k.attention_mma_supports(self.dim)
                 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and self._gate_fits_mma(gate)):
             # bfloat16 with a head size of the tensor-core kernel: tiles of tokens x heads of a K/V group; a step of
@@ -182,6 +187,13 @@ class SinkAttention(Part):
         k.attention_generic(q, k_pool, v_pool, batch, tiles.dev["tile_seq"], tiles.dev["tile_q0"], tiles.facts["n_tiles"],
                             None, self.kv_heads, self.scale, self.window, sinks=self.p_sink, gate=gate, out_scale=out_scale,
                             out=out, **extras)
+
+    def _tc_takes(self, q, tiles, out, gate) -> bool:
+        """Tiles of 128 tokens (some sequence brings more than 64) of a bfloat16 model with equal head sizes of 64 or 128 run on
+        tcgen05; shorter portions leave most rows of its tile empty and stay with the mma.sync kernel, as do mixed weights."""
+        k = self.build.kernels
+        return (q.dtype == torch.bfloat16 and not self.talk and self.dim == self.vdim and tiles.facts["mma_tokens"] == k.TC_TILE_TOKENS
+                and k.attention_tc_supports(self.dim) and k.attention_tc_extras_take(out, gate, self.gate_wide))
 
     def _gate_fits_mma(self, gate) -> bool:
         """A gate per entry is read two entries at a time by the tensor-core kernel: whole 32-bit words."""
@@ -214,6 +226,11 @@ class SinkAttention(Part):
         extras = {"softcap": self.softcap, "gate_wide": self.gate_wide}
         if self.talk and out_scale != 1.0:
             raise ValueError("sink_attention: mixed softmax weights take no output factor")
+        if self._tc_takes(q, tiles, out, gate):
+            k.attention_tc_extras(q, k_pool, v_pool, batch, tiles.dev["mtile_seq"], tiles.dev["mtile_q0"], tiles.facts["n_mma_tiles"], G,
+                                  self.scale, self.window, keep_first=self.keep_first, sinks=self.p_sink, gate=gate,
+                                  out_scale=out_scale, out=out, **extras)
+            return
         if (q.dtype == torch.bfloat16 and d == vd and k.attention_mma_supports(d) and out.stride(0) % 2 == 0
                 and out.data_ptr() % 4 == 0 and self._gate_fits_mma(gate)):
             # the tensor-core kernel, tiled as in forward_projected; with mixed weights a block forms one K/V group's

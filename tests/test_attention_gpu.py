@@ -413,3 +413,48 @@ def test_tensor_core_kernels_on_random_shapes(K, first_seed):
             assert "does not take" in str(refusal) or "too many" in str(refusal), (seed, kind, refusal)
             continue
         torch.testing.assert_close(out, ref, msg=lambda m: f"seed {seed} {kind}: {m}", **tol(BF))
+
+
+@pytest.mark.parametrize("heads,kv,d", [(4, 1, 64), (6, 2, 128)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (1, 0), (64, 4), (65, 70), (100, 200), (700, 1)])
+@pytest.mark.parametrize("softcap,sinks,gate,strided", [(0.0, False, None, False), (30.0, True, "head", True), (5.0, True, "entry", False),
+                                                        (0.0, False, "entry", True)])
+def test_tc_extras(K, heads, kv, d, window, keep, softcap, sinks, gate, strided):
+    """The tcgen05 prompt kernel with window, kept positions, cap, sinks, gates and strided results against the general kernel on
+    the same bfloat16 inputs: tiles that begin and end inside pages and windows, rows that see nothing of a page. Both round the
+    result to bfloat16: where their float32 results lie on either side of a tie they are one unit apart, and a unit of 8
+    significant bits is up to 2^-7 of the value (at a power of two); the weights' two terms leave 2^-16 of sum p |v| < 5."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.attention import AttentionTiles
+    from pytorch_transformers_b200.parts.base import CacheNeed
+    pasts, news = [0, 190, 64, 700], [300, 129, 1, 128]
+    cache = Cache([(0, CacheNeed("full", kv, d), None)], sum((p + n + 63) // 64 * 64 for p, n in zip(pasts, news)), BF, "cuda")
+    slots = [cache.open() for _ in news]
+    for s, p in zip(slots, pasts):
+        cache.reserve(s, p)
+        cache.commit(s, p)
+    ctx = StepContext(cache, slots, [[0] * n for n in news], 1, [[] for _ in news], [AttentionTiles(K)])
+    g = torch.Generator(device="cuda").manual_seed(window + keep + heads)
+    k_pool, v_pool, gi = cache.entry_storage(0)
+    k_pool.normal_(generator=g), v_pool.normal_(generator=g)
+    n = sum(news)
+    q = torch.randn(n, heads, d, generator=g, device="cuda").to(BF)
+    sink = torch.linspace(-4.0, 6.0, heads, device="cuda") if sinks else None
+    cols = {None: 0, "head": heads, "entry": heads * d}[gate]
+    gates = torch.randn(n, cols + 16, generator=g, device="cuda").to(BF)[:, 16:] if gate else None
+    tiles, batch = ctx.plan(AttentionTiles.plan_key), ctx.batch_c[gi]
+
+    def result(fn, name_seq, name_q0, count):
+        out = torch.full((n, heads * d + (24 if strided else 0)), 7.0, dtype=BF, device="cuda")
+        view = out[:, 8:8 + heads * d] if strided else out
+        fn(q, k_pool, v_pool, batch, tiles.dev[name_seq], tiles.dev[name_q0], tiles.facts[count],
+           *(() if fn is K.attention_tc_extras else (None,)), kv, d ** -0.5, window, keep_first=keep, softcap=softcap, sinks=sink,
+           gate=gates, gate_wide=gate == "entry", out_scale=0.5, out=view)
+        assert not strided or ((out[:, :8] == 7).all() and (out[:, 8 + heads * d:] == 7).all())
+        return view.double()
+    got = result(K.attention_tc_extras, "mtile_seq", "mtile_q0", "n_mma_tiles")
+    ref = result(K.attention_generic, "tile_seq", "tile_q0", "n_tiles")
+    assert K.attention_tc_extras_take(q.view(n, -1), gates, gate == "entry")
+    assert ((got - ref).abs() <= 2.0 ** -7 * ref.abs() + 2e-4).all(), (got - ref).abs().max()
+    K.check_device_errors("cuda:0")
