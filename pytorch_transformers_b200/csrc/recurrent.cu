@@ -188,9 +188,14 @@ __global__ void rglru_scan_kernel(const float* __restrict__ gates, const T* __re
 // memory, so the values of SCAN_AHEAD tokens (or chunks) are asked for before the first is used: 2,048 tokens of 2,560
 // channels 94 us for the three passes (a token at a time: 117).
 constexpr int SCAN_AHEAD = 8;
-template <typename T, int PASS>
-__global__ void rglru_chunk_kernel(const float* __restrict__ gates, const T* __restrict__ u, const T* __restrict__ y_act,
-                                   const float* __restrict__ lam, const T* __restrict__ proj,
+// A chunk goes to SPLIT blocks of consecutive tokens each, as chunks of their own: 32 tokens a thread keep twice as many warps an SM.
+// RAW: `gates` is the gates' product itself [blocks][tokens][2 bw] without bias and sigmoid (`gates_b` [blocks][2 bw]); pass 1
+// forms log a and sqrt(1 - a^2) i u from it and leaves them in its place for pass 3, so that nothing is formed twice and no
+// pass of its own adds the bias (epilogue 23 us and passes 94 -> passes 67 us).
+constexpr int SPLIT = 2;
+template <typename T, int PASS, bool RAW>
+__global__ void rglru_chunk_kernel(float* __restrict__ gates, const float* __restrict__ gates_b, const T* __restrict__ u,
+                                   const T* __restrict__ y_act, const float* __restrict__ lam, const T* __restrict__ proj,
                                    const float* __restrict__ bx, float* __restrict__ state, long long state_stride,
                                    const int* __restrict__ slots, StepBatch sb, const int* __restrict__ chunk_seq,
                                    const int* __restrict__ chunk_q0, const int* __restrict__ seq_chunk0, int n_chunks,
@@ -199,12 +204,13 @@ __global__ void rglru_chunk_kernel(const float* __restrict__ gates, const T* __r
                                    float c_decay) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R) return;
+  const int len = (chunk_len + SPLIT - 1) / SPLIT;
   if (PASS == 2) {
     const int seq = blockIdx.y;
     const int n_new = sb.seq_new[seq], start = sb.seq_start[seq];
     float* st = state + size_t(slots[seq]) * state_stride;
     float S = st[c];
-    const int first = seq_chunk0[seq], count = (n_new + chunk_len - 1) / chunk_len;
+    const int first = seq_chunk0[seq] * SPLIT, count = (n_new + chunk_len - 1) / chunk_len * SPLIT;
     for (int k0 = first; k0 < first + count; k0 += SCAN_AHEAD) {
       float a[SCAN_AHEAD], b[SCAN_AHEAD];
 #pragma unroll
@@ -226,12 +232,14 @@ __global__ void rglru_chunk_kernel(const float* __restrict__ gates, const T* __r
     for (int k = 0; k < taps - 1; ++k) st[R + size_t(k) * R + c] = keep[k];
     return;
   }
-  const int chunk = blockIdx.y;
-  const int seq = chunk_seq[chunk], q0 = chunk_q0[chunk];
-  const int first = sb.seq_start[seq] + q0, count = min(chunk_len, sb.seq_new[seq] - q0);
+  const int chunk = blockIdx.y, part = chunk % SPLIT;
+  const int seq = chunk_seq[chunk / SPLIT], q0 = chunk_q0[chunk / SPLIT] + part * len;
+  const int first = sb.seq_start[seq] + q0, count = min(min(len, chunk_len - part * len), sb.seq_new[seq] - q0);
   const float l = lam[c];
   const float sp = (l > 20.f) ? l : log1pf(expf(l));
-  const size_t goff = size_t(c / bw) * 2 * bw + c % bw;
+  const int t_step = RAW ? 2 * bw : 2 * R;      // from a token's gates to the next one's
+  float* gate = gates + (RAW ? size_t(c / bw) * sb.n_tokens * 2 * bw : size_t(c / bw) * 2 * bw) + c % bw;
+  const float b_r = RAW ? gates_b[size_t(c / bw) * 2 * bw + c % bw] : 0.f, b_i = RAW ? gates_b[size_t(c / bw) * 2 * bw + bw + c % bw] : 0.f;
   float S = (PASS == 3) ? s_start[size_t(chunk) * R + c] : 0.f, A = 0.f;      // A: the chunk's summed log a
   for (int i0 = 0; i0 < count; i0 += SCAN_AHEAD) {
     float r[SCAN_AHEAD], in[SCAN_AHEAD], uv[SCAN_AHEAD], yv[SCAN_AHEAD];
@@ -239,16 +247,27 @@ __global__ void rglru_chunk_kernel(const float* __restrict__ gates, const T* __r
     for (int i = 0; i < SCAN_AHEAD; ++i)
       if (i0 + i < count) {
         const size_t t = size_t(first + i0 + i);
-        r[i] = gates[t * 2 * R + goff], in[i] = gates[t * 2 * R + goff + bw], uv[i] = to_f(u[t * R + c]);
+        r[i] = gate[t * t_step], in[i] = gate[t * t_step + bw];
+        if (!RAW || PASS == 1) uv[i] = to_f(u[t * R + c]);
         if (PASS == 3) yv[i] = to_f(y_act[t * R + c]);
       }
 #pragma unroll
     for (int i = 0; i < SCAN_AHEAD; ++i)
       if (i0 + i < count) {
-        const float log_a = -c_decay * r[i] * sp;
-        S = decayed(S, log_a, sqrtf(-expm1f(2.f * log_a)) * (in[i] * uv[i]));
+        const size_t t = size_t(first + i0 + i);
+        float log_a = r[i], drive = in[i];
+        if (!RAW || PASS == 1) {
+          if (RAW) {
+            r[i] = 1.f / (1.f + expf(-(r[i] + b_r)));
+            in[i] = 1.f / (1.f + expf(-(in[i] + b_i)));
+          }
+          log_a = -c_decay * r[i] * sp;
+          drive = sqrtf(-expm1f(2.f * log_a)) * (in[i] * uv[i]);
+          if (RAW) gate[t * t_step] = log_a, gate[t * t_step + bw] = drive;
+        }
+        S = decayed(S, log_a, drive);
         if (PASS == 1) A += log_a;
-        if (PASS == 3) out[size_t(first + i0 + i) * R + c] = from_f<T>(S * yv[i]);
+        if (PASS == 3) out[t * R + c] = from_f<T>(S * yv[i]);
       }
   }
   if (PASS == 1) {
@@ -257,22 +276,21 @@ __global__ void rglru_chunk_kernel(const float* __restrict__ gates, const T* __r
   }
 }
 
-template <typename T>
-int launch_rglru_chunks(const float* gates, const void* u, const void* y_act, const float* lam, const void* proj,
+template <typename T, bool RAW>
+int launch_rglru_chunks(float* gates, const float* gates_b, const void* u, const void* y_act, const float* lam, const void* proj,
                         const float* bx, float* state, long long state_stride, const int* slots, const StepBatch& sb,
-                        const int* chunk_seq, const int* chunk_q0, const int* seq_chunk0, int n_chunks, int chunk_len,
-                        float* work, void* out, int R, int bw, int taps, float c_decay, cudaStream_t stream) {
-  float* agg_a = work;
-  float* agg_b = work + size_t(n_chunks) * R;
-  float* s_start = work + 2 * size_t(n_chunks) * R;
+                        const int* chunk_seq, const int* chunk_q0, const int* seq_chunk0, int n_chunks, int chunk_len, float* work,
+                        void* out, int R, int bw, int taps, float c_decay, cudaStream_t stream) {
+  const size_t per = size_t(n_chunks) * SPLIT * R;
+  float *agg_a = work, *agg_b = work + per, *s_start = work + 2 * per;
   const int threads = 128, gx = (R + threads - 1) / threads;
-#define PTB_CHUNK_PASS(P, GY)                                                                                      \
-  rglru_chunk_kernel<T, P><<<dim3(gx, GY), threads, 0, stream>>>(                                                   \
-      gates, (const T*)u, (const T*)y_act, lam, (const T*)proj, bx, state, state_stride, slots, sb, chunk_seq, chunk_q0, \
+#define PTB_CHUNK_PASS(P, GY)                                                                                       \
+  rglru_chunk_kernel<T, P, RAW><<<dim3(gx, GY), threads, 0, stream>>>(                                               \
+      gates, gates_b, (const T*)u, (const T*)y_act, lam, (const T*)proj, bx, state, state_stride, slots, sb, chunk_seq, chunk_q0, \
       seq_chunk0, n_chunks, chunk_len, agg_a, agg_b, s_start, (T*)out, R, bw, taps, c_decay)
-  PTB_CHUNK_PASS(1, n_chunks);
+  PTB_CHUNK_PASS(1, n_chunks * SPLIT);
   PTB_CHUNK_PASS(2, sb.n_seqs);
-  PTB_CHUNK_PASS(3, n_chunks);
+  PTB_CHUNK_PASS(3, n_chunks * SPLIT);
 #undef PTB_CHUNK_PASS
   return launch_status();
 }
@@ -617,24 +635,26 @@ PTB_API int ptb_rglru_scan(int dtype, const float* gates, const void* u, const v
   return launch_status();
 }
 
-// `work`: 3 * n_chunks * R float32 values
-PTB_API int ptb_rglru_scan_chunks(int dtype, const float* gates, const void* u, const void* y_act, const float* lam,
+// float32 values of `work` that ptb_rglru_scan_chunks needs
+PTB_API long long ptb_rglru_chunks_work_floats(int n_chunks, int R) { return 3LL * n_chunks * SPLIT * R; }
+
+// gates_b null: `gates` [tokens, blocks, 2 bw] after their sigmoid. gates_b [blocks][2 bw]: `gates` [blocks][tokens][2 bw] is the
+// gates' product without bias and sigmoid, which the scan writes over.
+PTB_API int ptb_rglru_scan_chunks(int dtype, float* gates, const float* gates_b, const void* u, const void* y_act, const float* lam,
                                   const void* proj, const float* bx, float* state, long long state_stride,
                                   const int* slots, const StepBatch* sb, const int* chunk_seq, const int* chunk_q0,
                                   const int* seq_chunk0, int n_chunks, int chunk_len, float* work, void* out, int R,
                                   int blocks_n, int taps, float c_decay, cudaStream_t stream) {
   if (sb->n_tokens <= 0 || n_chunks <= 0) return PTB_OK;
   if (R <= 0 || blocks_n <= 0 || R % blocks_n != 0 || taps < 1 || taps > MAX_TAPS || chunk_len <= 0 ||
-      n_chunks > 65535 || sb->n_seqs > 65535)
+      n_chunks > 65535 / SPLIT || sb->n_seqs > 65535)
     return PTB_ERR_SIZE;
-  if (dtype == PTB_F32)
-    return launch_rglru_chunks<float>(gates, u, y_act, lam, proj, bx, state, state_stride, slots, *sb, chunk_seq,
-                                      chunk_q0, seq_chunk0, n_chunks, chunk_len, work, out, R, R / blocks_n, taps,
-                                      c_decay, stream);
-  if (dtype == PTB_BF16)
-    return launch_rglru_chunks<__nv_bfloat16>(gates, u, y_act, lam, proj, bx, state, state_stride, slots, *sb,
-                                              chunk_seq, chunk_q0, seq_chunk0, n_chunks, chunk_len, work, out, R,
-                                              R / blocks_n, taps, c_decay, stream);
+#define PTB_RSC(TT, RAW)                                                                                                     \
+  launch_rglru_chunks<TT, RAW>(gates, gates_b, u, y_act, lam, proj, bx, state, state_stride, slots, *sb, chunk_seq, chunk_q0, \
+                               seq_chunk0, n_chunks, chunk_len, work, out, R, R / blocks_n, taps, c_decay, stream)
+  if (dtype == PTB_F32) return gates_b ? PTB_RSC(float, true) : PTB_RSC(float, false);
+  if (dtype == PTB_BF16) return gates_b ? PTB_RSC(__nv_bfloat16, true) : PTB_RSC(__nv_bfloat16, false);
+#undef PTB_RSC
   return PTB_ERR_DTYPE;
 }
 

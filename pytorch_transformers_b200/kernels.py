@@ -114,6 +114,7 @@ def lib():
                      "ptb_delta_chunks_supports", "ptb_post_norm", "ptb_token_gate", "ptb_round_rows", "ptb_route_biased", "ptb_attention_tc_sizes", "ptb_attention_tc_supports_sizes", "ptb_attention_tc_extras"):
             getattr(L, name).restype = ctypes.c_int
         L.ptb_latent_part_floats.restype = ctypes.c_longlong
+        L.ptb_rglru_chunks_work_floats.restype = ctypes.c_longlong
         L.ptb_expert_plan_words.restype = ctypes.c_longlong
         L.ptb_mlstm_chunks_scratch_floats.restype = ctypes.c_longlong
         _configured = True
@@ -1044,21 +1045,32 @@ def rglru_scan(gates: torch.Tensor, u: torch.Tensor, y_act: torch.Tensor, lam: t
     return out
 
 
+def block_product(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """``block_linear``'s library product alone: float32 [groups, tokens, N] of bfloat16 ``x`` [tokens, groups, K] and ``w``
+    [groups, N, K], for a kernel that adds the bias itself. None where ``block_linear`` does not take the library's product."""
+    if x.dtype != torch.bfloat16 or x.shape[0] < BLOCK_LINEAR_LIBRARY_ROWS:
+        return None
+    return torch.bmm(x.transpose(0, 1), w.transpose(1, 2), out_dtype=torch.float32)
+
+
 def rglru_scan_chunks(gates: torch.Tensor, u: torch.Tensor, y_act: torch.Tensor, lam: torch.Tensor, proj: torch.Tensor,
                       bx: torch.Tensor, state: torch.Tensor, slots: torch.Tensor, batch: StepBatchC, blocks: int, taps: int,
                       decay: float, chunk_seq: torch.Tensor, chunk_q0: torch.Tensor, seq_chunk0: torch.Tensor,
-                      n_chunks: int, chunk_len: int) -> torch.Tensor:
+                      n_chunks: int, chunk_len: int, gates_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``rglru_scan`` for long prompts: the sequences are cut into chunks of ``chunk_len`` tokens
     (``chunk_seq``, ``chunk_q0``: sequence and first token of each; ``seq_chunk0``: a sequence's first chunk)
-    that run side by side and are joined in order (three passes)."""
-    _need_cuda(gates, u, y_act, lam, proj, bx, slots, chunk_seq, chunk_q0, seq_chunk0)
+    that run side by side and are joined in order (three passes). With ``gates_bias`` (float32 [blocks, 2 * R / blocks]) ``gates`` is
+    the gates' product [blocks, tokens, 2 * R / blocks] without bias and sigmoid; the scan writes over it."""
+    _need_cuda(gates, u, y_act, lam, proj, bx, slots, chunk_seq, chunk_q0, seq_chunk0, gates_bias)
     n, r = u.shape
     if gates.dtype != torch.float32 or gates.numel() != n * 2 * r or state.stride(1) != 1 or state.shape[1] != r * taps:
         raise KernelError("rglru_scan_chunks: gates or state do not fit")
+    if gates_bias is not None and (gates_bias.dtype != torch.float32 or gates_bias.numel() != 2 * r or gates.shape[0] != blocks):
+        raise KernelError("rglru_scan_chunks: the gates' product is [blocks, tokens, 2 R / blocks] and their bias float32")
     out = torch.empty_like(u)
-    work = torch.empty(3 * n_chunks * r, dtype=torch.float32, device=u.device)
-    _check(lib().ptb_rglru_scan_chunks(_dtype_code(u), _ptr(gates), _ptr(u), _ptr(y_act), _ptr(lam), _ptr(proj), _ptr(bx),
-                                       _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(slots), ctypes.byref(batch),
+    work = torch.empty(int(lib().ptb_rglru_chunks_work_floats(n_chunks, r)), dtype=torch.float32, device=u.device)
+    _check(lib().ptb_rglru_scan_chunks(_dtype_code(u), _ptr(gates), _ptr(gates_bias), _ptr(u), _ptr(y_act), _ptr(lam), _ptr(proj),
+                                       _ptr(bx), _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(slots), ctypes.byref(batch),
                                        _ptr(chunk_seq), _ptr(chunk_q0), _ptr(seq_chunk0), n_chunks, chunk_len, _ptr(work),
                                        _ptr(out), r, blocks, taps, ctypes.c_float(decay), _stream(u)), "rglru_scan_chunks")
     global launches

@@ -96,12 +96,15 @@ class GatedLinearRecurrence(Part):
         state = ctx.state_of(entry, self.state_need().numel)
         slots, batch = ctx.dev["slots"], ctx.batch_c[0]
         y_act, u = k.rglru_conv(proj, self.p_y_b, self.p_x_b, self.p_conv, self.p_conv_b, state, slots, batch)
-        gates = k.block_linear(u.view(t, B, R // B), self.p_gates, self.p_gates_b, act="sigmoid", out_dtype=torch.float32)
         chunks = ctx.plan(RecurrenceChunks.plan_key)
+        # long prompts take the gates' bare product: the scan adds bias and sigmoid as it reads
+        product = k.block_product(u.view(t, B, R // B), self.p_gates) if chunks.facts["n_chunks"] else None
+        gates = product if product is not None else k.block_linear(u.view(t, B, R // B), self.p_gates, self.p_gates_b, act="sigmoid",
+                                                                   out_dtype=torch.float32)
         if chunks.facts["n_chunks"]:       # long prompts: chunks side by side, joined in order
             out = k.rglru_scan_chunks(gates, u, y_act, self.p_lam, proj, self.p_x_b, state, slots, batch, B, self.taps,
                                       self.decay, chunks.dev["chunk_seq"], chunks.dev["chunk_q0"], chunks.dev["seq_chunk0"],
-                                      chunks.facts["n_chunks"], SCAN_CHUNK)
+                                      chunks.facts["n_chunks"], SCAN_CHUNK, gates_bias=self.p_gates_b if product is not None else None)
         else:
             out = k.rglru_scan(gates, u, y_act, self.p_lam, proj, self.p_x_b, state, slots, batch, B, self.taps, self.decay)
         return linear(k, out, self.p_o, add=add)

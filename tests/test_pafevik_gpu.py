@@ -196,6 +196,36 @@ def test_latent_attention_finds_one_far_key(dtype, past, new, pos):
     assert (off - got[last]).abs().max() > 0.1      # another needle gives another row
 
 
+@pytest.mark.parametrize("R,blocks,chunk", [(96, 4, 64), (40, 10, 7), (2560, 16, 64)])
+def test_scan_from_the_gates_product(R, blocks, chunk):
+    """The chunked scan that adds bias and sigmoid itself against the one that reads finished gates: the same float32 operations,
+    so the same bits, in outputs and state; chunks whose second half is short or empty."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.base import StateNeed
+    k, bw, taps, news = K(), R // blocks, 4, [300, 33, 1]
+    g = torch.Generator(device="cuda").manual_seed(R)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    n = sum(news)
+    proj, w, b = rand(n, 2 * R).bfloat16(), (rand(blocks, 2 * bw, bw) / math.sqrt(bw)).bfloat16(), 0.3 * rand(blocks, 2 * bw)
+    bias, conv, lam = [0.3 * rand(R) for _ in range(3)], 0.5 * rand(R, taps), 1.5 * rand(R) - 1
+    got = []
+    for product in (False, True):
+        cache = Cache([(0, None, StateNeed(R * taps))], 64 * 16, torch.bfloat16, "cuda", max_slots=3)
+        ctx = StepContext(cache, [cache.open() for _ in news], [[0] * m for m in news], 1, [[] for _ in news])
+        state = cache.entry_state(0)
+        y_act, u = k.rglru_conv(proj, bias[0], bias[1], conv, bias[2], state, ctx.dev["slots"], ctx.batch_c[0])
+        x = u.view(n, blocks, bw)
+        gates = k.block_product(x, w) if product else k.block_linear(x, w, b, act="sigmoid", out_dtype=torch.float32)
+        seqs, firsts = ctx.tiles(chunk)
+        first_of = [sum((m + chunk - 1) // chunk for m in news[:i]) for i in range(len(news))]
+        ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        out = k.rglru_scan_chunks(gates, u, y_act, lam, proj, bias[1], state, ctx.dev["slots"], ctx.batch_c[0], blocks, taps, 8.0,
+                                  ints(seqs), ints(firsts), ints(first_of), len(seqs), chunk, gates_bias=b if product else None)
+        got.append((out, state.clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def rglru_case(dtype, R, blocks, taps, pasts, news, seed=0, chunk=0):
     """The recurrence's kernels from random branch projections in two steps; (kernel output, plain) for the
     second step, and the state rows of the slots."""
