@@ -13,8 +13,8 @@
 // tokens from and to the state area (steps of any length); over one chunk of 64 tokens from zero, leaving the
 // chunk's own sum and its total decay (pass 1 of the chunked form); over one chunk from the state before it, with
 // outputs (pass 3). Pass 2 joins the chunks of a sequence in order. The chunked form differs from the plain walk by
-// the order of float32 operations only. With bfloat16 projections and keys and values of 64 or 128 entries pass 1 is a
-// product on the tensor cores instead (csrc/gla_mma.cu: the decayed keys enter it as two bfloat16 terms).
+// the order of float32 operations only. With bfloat16 projections and keys and values of 64 or 128 entries passes 1
+// and 3 run on the tensor cores instead (csrc/gla_mma.cu: float32 operands enter a product as two bfloat16 terms).
 #include "common.cuh"
 
 namespace {
@@ -50,6 +50,23 @@ __global__ void gla_decay_kernel(float* __restrict__ z, const float* __restrict_
   if (i >= total) return;
   const float v = z[i] + (bias ? bias[i % width] : 0.f);
   z[i] = (fminf(v, 0.f) - log1pf(expf(-fabsf(v)))) * inv_tau;
+}
+
+// The same, four neighbouring values a thread (width a multiple of 4, rows at whole words): 2,900 x 2,048 values 12 us against 21
+__global__ void gla_decay_quad_kernel(float* __restrict__ z, const float* __restrict__ bias, long long quads, int width,
+                                      float inv_tau) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= quads) return;
+  float4 v = reinterpret_cast<float4*>(z)[i];
+  if (bias) {
+    const float4 b = *reinterpret_cast<const float4*>(bias + i * 4 % width);
+    v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+  }
+  v.x = (fminf(v.x, 0.f) - log1pf(expf(-fabsf(v.x)))) * inv_tau;
+  v.y = (fminf(v.y, 0.f) - log1pf(expf(-fabsf(v.y)))) * inv_tau;
+  v.z = (fminf(v.z, 0.f) - log1pf(expf(-fabsf(v.z)))) * inv_tau;
+  v.w = (fminf(v.w, 0.f) - log1pf(expf(-fabsf(v.w)))) * inv_tau;
+  reinterpret_cast<float4*>(z)[i] = v;
 }
 
 // proj row t: [q: heads * dim | k: heads * dim | v: heads * v_dim | ...], `stride` elements apart.
@@ -314,35 +331,43 @@ gla_walk_kernel(const T* __restrict__ proj, int stride, const float* __restrict_
 
 // One thread per (sequence, head, element of S): walks the sequence's chunks in order; sums[c] becomes the state
 // BEFORE chunk c, and the state area receives the state after the last chunk.
+// V: value columns a thread (1, or 4 where rows of S begin at whole 16-byte words: 46 chunks of 16 heads of 128 x 128 12 us
+// against 29)
+template <int V>
 __global__ void gla_chunk_join_kernel(float* __restrict__ sums, const float* __restrict__ chunk_decay,
                                       float* __restrict__ state, int state_stride, const int* __restrict__ slots,
                                       StepBatch sb, const int* __restrict__ seq_chunk0, int heads, int dim, int v_dim) {
   const int seq = blockIdx.y;
   const size_t per_head = size_t(dim) * v_dim, per = per_head * heads;
-  const size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const size_t e = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * V;
   if (e >= per) return;
   const int h = int(e / per_head), d = int((e % per_head) / v_dim);
   const int n_new = sb.seq_new[seq], c0 = seq_chunk0[seq];
   const int n_chunks = (n_new + CH - 1) / CH;
   float* st = state + size_t(slots[seq]) * state_stride + e;
-  float s = *st;
+  struct alignas(4 * V) Word { float v[V]; };
+  Word s = *reinterpret_cast<const Word*>(st);
   constexpr int AHEAD = 8;      // chunks whose own sums are loaded before the chain of updates needs them
   for (int g0 = 0; g0 < n_chunks; g0 += AHEAD) {
-    float own[AHEAD], dec[AHEAD];
+    Word own[AHEAD];
+    float dec[AHEAD];
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
-      const bool on = g0 + i < n_chunks;
-      own[i] = on ? sums[size_t(c0 + g0 + i) * per + e] : 0.f;
-      dec[i] = on ? chunk_decay[(size_t(c0 + g0 + i) * heads + h) * dim + d] : 0.f;
+      if (g0 + i < n_chunks) {
+        own[i] = *reinterpret_cast<const Word*>(sums + size_t(c0 + g0 + i) * per + e);
+        dec[i] = chunk_decay[(size_t(c0 + g0 + i) * heads + h) * dim + d];
+      }
     }
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
       if (g0 + i >= n_chunks) break;
-      sums[size_t(c0 + g0 + i) * per + e] = s;
-      s = fmaf(expf(dec[i]), s, own[i]);
+      *reinterpret_cast<Word*>(sums + size_t(c0 + g0 + i) * per + e) = s;
+      const float f = expf(dec[i]);
+#pragma unroll
+      for (int x = 0; x < V; ++x) s.v[x] = fmaf(f, s.v[x], own[i].v[x]);
     }
   }
-  *st = s;
+  *reinterpret_cast<Word*>(st) = s;
 }
 
 template <typename T>
@@ -381,6 +406,9 @@ int launch_walk(const void* proj, int stride, const float* log_decay, float* sta
 
 // pass 1 on the tensor cores (csrc/gla_mma.cu)
 PTB_API int ptb_gla_chunk_sum_mma_supports(int dtype, const void* proj, int stride, const float* log_decay, int dim, int v_dim);
+PTB_API int ptb_gla_chunk_out_mma(const void* proj, int stride, const float* log_decay, const StepBatch* sb, const int* chunk_seq,
+                                  const int* chunk_q0, int n_chunks, const float* before, float* out, int heads, int dim, int v_dim,
+                                  float q_scale, cudaStream_t stream);
 PTB_API int ptb_gla_chunk_sum_mma(const void* proj, int stride, const float* log_decay, const StepBatch* sb, const int* chunk_seq,
                                   const int* chunk_q0, int n_chunks, float* sums, float* chunk_decay, int heads, int dim,
                                   int v_dim, cudaStream_t stream);
@@ -393,7 +421,10 @@ PTB_API int ptb_gla_decay(float* z, const float* bias, int n, int width, float t
   if (n <= 0) return PTB_OK;
   if (width <= 0 || !(tau > 0.f)) return PTB_ERR_SIZE;
   const long long total = (long long)n * width;
-  gla_decay_kernel<<<unsigned((total + 255) / 256), 256, 0, stream>>>(z, bias, total, width, 1.f / tau);
+  if (width % 4 == 0 && aligned16(z) && aligned16(bias))
+    gla_decay_quad_kernel<<<unsigned((total / 4 + 255) / 256), 256, 0, stream>>>(z, bias, total / 4, width, 1.f / tau);
+  else
+    gla_decay_kernel<<<unsigned((total + 255) / 256), 256, 0, stream>>>(z, bias, total, width, 1.f / tau);
   return launch_status();
 }
 
@@ -423,12 +454,15 @@ PTB_API int ptb_gla_chunks(int dtype, const void* proj, int stride, const float*
   if (heads <= 0 || heads > 65535 || dim <= 0 || dim > 32 * MAX_WARPS || v_dim <= 0 || stride < 2 * heads * dim + heads * v_dim ||
       sb->n_seqs > 65535)
     return PTB_ERR_SIZE;
-  // a chunk's own sum is a product of the decayed keys by the values: on the tensor cores where the sizes allow
-  const bool sum_mma = ptb_gla_chunk_sum_mma_supports(dtype, proj, stride, log_decay, dim, v_dim) != 0;
+  // the first and the last pass run on the tensor cores where the sizes allow (csrc/gla_mma.cu)
+  const bool mma = ptb_gla_chunk_sum_mma_supports(dtype, proj, stride, log_decay, dim, v_dim) != 0;
   for (int role = GLA_CHUNK_SUM; role <= GLA_CHUNK_OUT; ++role) {
     int rc;
-    if (role == GLA_CHUNK_SUM && sum_mma)
+    if (role == GLA_CHUNK_SUM && mma)
       rc = ptb_gla_chunk_sum_mma(proj, stride, log_decay, sb, chunk_seq, chunk_q0, n_chunks, sums, chunk_decay, heads, dim, v_dim,
+                                 stream);
+    else if (role == GLA_CHUNK_OUT && mma)
+      rc = ptb_gla_chunk_out_mma(proj, stride, log_decay, sb, chunk_seq, chunk_q0, n_chunks, sums, out, heads, dim, v_dim, q_scale,
                                  stream);
     else if (dtype == PTB_F32)
       rc = launch_walk<float>(proj, stride, log_decay, state, state_stride, slots, *sb, chunk_seq, chunk_q0, n_chunks, sums,
@@ -441,9 +475,12 @@ PTB_API int ptb_gla_chunks(int dtype, const void* proj, int stride, const float*
     if (rc != PTB_OK) return rc;
     if (role == GLA_CHUNK_SUM) {
       const size_t per = size_t(heads) * dim * v_dim;
-      dim3 grid(unsigned((per + 255) / 256), sb->n_seqs);
-      gla_chunk_join_kernel<<<grid, 256, 0, stream>>>(sums, chunk_decay, state, state_stride, slots, *sb, seq_chunk0, heads,
-                                                      dim, v_dim);
+      if (v_dim % 4 == 0 && state_stride % 4 == 0 && aligned16(state) && aligned16(sums))
+        gla_chunk_join_kernel<4><<<dim3(unsigned((per / 4 + 127) / 128), sb->n_seqs), 128, 0, stream>>>(
+            sums, chunk_decay, state, state_stride, slots, *sb, seq_chunk0, heads, dim, v_dim);
+      else
+        gla_chunk_join_kernel<1><<<dim3(unsigned((per + 255) / 256), sb->n_seqs), 256, 0, stream>>>(
+            sums, chunk_decay, state, state_stride, slots, *sb, seq_chunk0, heads, dim, v_dim);
       if (launch_status() != PTB_OK) return PTB_ERR_LAUNCH;
     }
   }

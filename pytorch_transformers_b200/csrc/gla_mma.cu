@@ -1,5 +1,5 @@
-// Gated linear attention, pass 1 of the chunked form on the tensor cores (bfloat16 projections, mma.m16n8k16 with
-// float32 sums): a chunk's own sum from a zero state.
+// Gated linear attention, passes 1 and 3 of the chunked form on the tensor cores (bfloat16 projections, mma.m16n8k16 with
+// float32 sums). Pass 1: a chunk's own sum from a zero state.
 //
 // A chunk holds n <= 64 tokens j = 0..n-1 with the logarithms l_j [dim] of their decays (float32). Token j's outer
 // product k_j v_j^T reaches the chunk's end decayed by the tokens after it, channel by channel:
@@ -127,9 +127,319 @@ int launch_sum(const void* proj, int stride, const float* log_decay, const StepB
   return launch_status();
 }
 
+// ------------------------------------------------------------------------------------------------
+// Pass 3 on the tensor cores: a chunk's outputs from the state before it,
+//     o_t = q_scale * ( sum_c q_t[c] exp(l_0 + .. + l_t)[c] S0[c]  +  sum_(i <= t) s_ti v_i ),
+//     s_ti = sum_c q_t[c] k_i[c] exp(l_(i+1) + .. + l_t)[c].
+// The decay differs per key channel, so the scores are no plain product of q and k. The chunk is cut into four sub-blocks of
+// 16 tokens. Between sub-blocks u < w the exponent is a sum of three sums of logarithms of one sign, the rest of u after i,
+// the whole sub-blocks between, and w up to t: the first goes into the keys, the others into the queries, all factors are at
+// most 1, nothing is subtracted, and the scores are a product. Inside a sub-block every (t, i, channel) has an exponent of its
+// own: a warp walks t from i on with its lanes' channels' sums in registers. That is what bounds the kernel: 136 (t, i) pairs a sub-block and
+// channel, 70,000 exponentials a block against 16 a clock and SM, and the instructions around them. 2,900 tokens of
+// 16 heads of 128 x 128: 94 us, where the walk on the CUDA cores took 175.
+// Operands of a product that are float32 (scaled queries and keys, scores, the state) enter it as two bfloat16 terms (the product
+// of two such operands leaves out lo x lo, 2^-18 of it).
+// One block = one chunk x one head, 8 warps; 101 KB of shared memory, two blocks an SM:
+//     tiles of q, k (then the keys' hi terms, then the state's quarters), the keys' lo terms (then v), the logarithms (then
+//     their sums inside a sub-block up to t), the scores.
+constexpr int SUB = 16, SUBS = CH / SUB, SPITCH = CH + 4;     // tokens of a sub-block; pitch of the scores' rows
+constexpr float LOG2E = 1.4426950408889634f;
+
+template <int DK, int DV>
+struct OutShape {
+  static constexpr int LP = DK + 8;                            // floats from one token's logarithms to the next's
+  static constexpr int A_BYTES = CH * (DK > DV ? DK : DV) * 2; // a tile, also of v or of a quarter of the state (two terms)
+  static constexpr size_t SMEM = size_t(CH) * DK * 2 + 2 * size_t(A_BYTES) + size_t(CH) * LP * 4 + size_t(SUBS) * DK * 4 + size_t(CH) * SPITCH * 4;
+};
+
+__device__ __forceinline__ float2 pair_f(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(256, 2)
+gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, const float* __restrict__ log_decay, StepBatch sb,
+                         const int* __restrict__ chunk_seq, const int* __restrict__ chunk_q0, const float* __restrict__ before,
+                         float* __restrict__ out, int heads, float q_scale) {
+  using Shape = OutShape<DK, DV>;
+  constexpr int LP = Shape::LP, NT = DV / 16;      // NT: n-tiles of 8 value columns that a warp owns
+  extern __shared__ __align__(128) unsigned char sm[];
+  unsigned char* q_s = sm;                                  // [CH][DK]
+  unsigned char* k_s = q_s + CH * DK * 2;                   // [CH][DK] k, then the scaled keys' hi terms, then quarters of the state
+  unsigned char* b_s = k_s + Shape::A_BYTES;                // [CH][DK] the scaled keys' lo terms, then [CH][DV] v
+  float* l_s = reinterpret_cast<float*>(b_s + Shape::A_BYTES);   // [CH][LP] logarithms (powers of two), then sums up to t
+  float* t_s = l_s + CH * LP;                               // [SUBS][DK] a sub-block's sum
+  float* s_s = t_s + SUBS * DK;                             // [CH][SPITCH] scores
+  const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp8 = tid >> 5, warp = warp8 & 3, half = warp8 >> 2;
+  const int seq = chunk_seq[c], q0 = chunk_q0[c];
+  const int start = sb.seq_start[seq] + q0, n = min(CH, sb.seq_new[seq] - q0);
+  const __nv_bfloat16* row0 = proj + size_t(start) * stride;
+  {
+    StagedWords<DK, 256> qw, kw;
+    qw.load(row0 + h * DK, stride, n, tid);
+    kw.load(row0 + heads * DK + h * DK, stride, n, tid);
+    constexpr int QUADS = DK / 4, PER = CH * QUADS / 256;
+    const float* l0 = log_decay + size_t(start) * heads * DK + h * DK;
+    float4 l[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int i = tid + u * 256, row = i / QUADS, q = i % QUADS;
+      l[u] = row < n ? *reinterpret_cast<const float4*>(l0 + size_t(row) * heads * DK + q * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    qw.store(q_s, 0, tid);
+    kw.store(k_s, 0, tid);
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int i = tid + u * 256, row = i / QUADS, q = i % QUADS;
+      *reinterpret_cast<float4*>(l_s + row * LP + q * 4) = make_float4(l[u].x * LOG2E, l[u].y * LOG2E, l[u].z * LOG2E, l[u].w * LOG2E);
+    }
+  }
+  __syncthreads();
+  {   // scores inside sub-block `warp`: half of its keys (0, 3, 4, 7, .. or 1, 2, 5, 6, ..: 68 pairs each)
+    constexpr int CPL = DK / 32;      // channels of a lane
+    const int c0 = lane * CPL;
+    auto load_row = [&](const unsigned char* tile, int row, float (&f)[CPL]) {
+      const unsigned char* p = tile + swz<DK>(row, c0 / 8) + (c0 % 8) * 2;
+      if (CPL == 4) {
+        const uint2 v = *reinterpret_cast<const uint2*>(p);
+        const float2 a = pair_f(v.x), b = pair_f(v.y);
+        f[0] = a.x; f[1] = a.y; f[CPL - 2] = b.x; f[CPL - 1] = b.y;
+      } else {
+        const float2 a = pair_f(*reinterpret_cast<const uint32_t*>(p));
+        f[0] = a.x; f[1] = a.y;
+      }
+    };
+    for (int ii = 0; ii < SUB / 2; ++ii) {
+      const int i = 2 * ii + (half ^ (ii & 1));
+      float k[CPL], e[CPL], p[SUB];
+      load_row(k_s, warp * SUB + i, k);
+#pragma unroll
+      for (int u = 0; u < CPL; ++u) e[u] = 0.f;
+#pragma unroll
+      for (int t = 0; t < SUB; ++t) {
+        p[t] = 0.f;
+        if (t < i) continue;
+        float q[CPL];
+        load_row(q_s, warp * SUB + t, q);
+        if (t > i) {
+          const float* lt = l_s + (warp * SUB + t) * LP + c0;
+          if (CPL == 4) {
+            const float4 l = *reinterpret_cast<const float4*>(lt);
+            e[0] += l.x; e[1] += l.y; e[CPL - 2] += l.z; e[CPL - 1] += l.w;
+          } else {
+            const float2 l = *reinterpret_cast<const float2*>(lt);
+            e[0] += l.x; e[1] += l.y;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < CPL; ++u) p[t] = fmaf(q[u] * k[u], fast_exp2(e[u]), p[t]);
+      }
+      // sums over the lanes of 16 values at once: at every step a lane hands half of its values on
+#pragma unroll
+      for (int w = SUB / 2; w > 0; w >>= 1) {
+        const bool up = (lane & (2 * w)) != 0;
+#pragma unroll
+        for (int t = 0; t < w; ++t) {
+          const float give = up ? p[t] : p[t + w], keep = up ? p[t + w] : p[t];
+          p[t] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * w);
+        }
+      }
+      p[0] += __shfl_xor_sync(0xffffffffu, p[0], 1);
+      if ((lane & 1) == 0) s_s[(warp * SUB + (lane >> 1)) * SPITCH + warp * SUB + i] = p[0];
+    }
+  }
+  __syncthreads();
+  // the sums inside sub-blocks: up to t in place of the logarithms, and what follows i into the keys (two terms)
+  for (int u = tid; u < SUBS * DK; u += 256) {
+    const int sub = u / DK, ch = u % DK;
+    float l[SUB], up = 0.f;
+#pragma unroll
+    for (int t = 0; t < SUB; ++t) l[t] = l_s[(sub * SUB + t) * LP + ch];
+#pragma unroll
+    for (int t = 0; t < SUB; ++t) {
+      up += l[t];
+      l_s[(sub * SUB + t) * LP + ch] = up;
+    }
+    t_s[sub * DK + ch] = up;
+    float rest = 0.f;
+#pragma unroll
+    for (int t = SUB - 1; t >= 0; --t) {
+      const uint32_t at = swz<DK>(sub * SUB + t, ch / 8) + (ch % 8) * 2;
+      const float k = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(k_s + at)) * fast_exp2(rest);
+      const __nv_bfloat16 hi = __float2bfloat16_rn(k);
+      *reinterpret_cast<__nv_bfloat16*>(k_s + at) = hi;
+      *reinterpret_cast<__nv_bfloat16*>(b_s + at) = __float2bfloat16_rn(k - __bfloat162float(hi));
+      rest += l[t];
+    }
+  }
+  StagedWords<DV, 256> vw;      // on their way under the scores between sub-blocks
+  vw.load(row0 + 2 * heads * DK + h * DV, stride, n, tid);
+  __syncthreads();
+  const uint32_t ks = smem_u32(k_s), bs = smem_u32(b_s);
+  const int g4 = lane >> 2, t4 = lane & 3, m = lane >> 3;
+  // two neighbouring channels (ch, ch + 1) of query row r, times exp2(sum up to r in its sub-block + extra)
+  auto scaled_q = [&](int r, int ch, float2 extra, uint32_t& hi, uint32_t& lo) {
+    const float2 q = pair_f(*reinterpret_cast<const uint32_t*>(q_s + swz<DK>(r, ch / 8) + (ch % 8) * 2));
+    const float2 e = *reinterpret_cast<const float2*>(l_s + r * LP + ch);
+    split_pack(q.x * fast_exp2(e.x + extra.x), q.y * fast_exp2(e.y + extra.y), hi, lo);
+  };
+  if (warp8 < 6) {      // scores of sub-block w with the keys of sub-block u < w: a pair a warp
+    const int w = warp8 == 0 ? 1 : warp8 < 3 ? 2 : 3, u = warp8 == 0 ? 0 : warp8 < 3 ? warp8 - 1 : warp8 - 3;
+    const int r_lo = w * SUB + g4, r_hi = r_lo + 8;
+    float s[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+    for (int kk = 0; kk < DK / 16; ++kk) {
+      uint32_t qh[4], ql[4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int ch = kk * 16 + 8 * x + 2 * t4;
+        float2 mid = make_float2(0.f, 0.f);
+        for (int y = u + 1; y < w; ++y) {
+          const float2 t = *reinterpret_cast<const float2*>(t_s + y * DK + ch);
+          mid.x += t.x;
+          mid.y += t.y;
+        }
+        scaled_q(r_lo, ch, mid, qh[2 * x], ql[2 * x]);
+        scaled_q(r_hi, ch, mid, qh[2 * x + 1], ql[2 * x + 1]);
+      }
+      uint32_t h0, h1, h2, h3, l0, l1, l2, l3;      // keys 0..7 and 8..15 of the sub-block, 16 channels each
+      const uint32_t off = swz<DK>(u * SUB + (m >> 1) * 8 + (lane & 7), kk * 2 + (m & 1));
+      ldmatrix_x4(h0, h1, h2, h3, ks + off);
+      ldmatrix_x4(l0, l1, l2, l3, bs + off);
+      mma_bf16(s[0], qh, h0, h1);
+      mma_bf16(s[1], qh, h2, h3);
+      mma_bf16(s[0], qh, l0, l1);
+      mma_bf16(s[1], qh, l2, l3);
+      mma_bf16(s[0], ql, h0, h1);
+      mma_bf16(s[1], ql, h2, h3);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      *reinterpret_cast<float2*>(s_s + r_lo * SPITCH + u * SUB + j * 8 + 2 * t4) = make_float2(s[j][0], s[j][1]);
+      *reinterpret_cast<float2*>(s_s + r_hi * SPITCH + u * SUB + j * 8 + 2 * t4) = make_float2(s[j][2], s[j][3]);
+    }
+  }
+  __syncthreads();      // the scores are complete; the keys are no longer read
+  // the state before the chunk comes a quarter of its rows at a time, the next one's loads under this one's products
+  constexpr int QR = DK / 4, CHUNKS = DV / 8, PER = QR * CHUNKS / 256 > 0 ? QR * CHUNKS / 256 : 1;
+  const float* S0 = before + (size_t(c) * heads + h) * DK * DV;
+  float4 sx[PER], sy[PER];
+  auto load_state = [&](int quarter) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int i = tid + u * 256, row = i / CHUNKS, cc = i % CHUNKS;
+      if (i < QR * CHUNKS) {
+        sx[u] = *reinterpret_cast<const float4*>(S0 + size_t(quarter * QR + row) * DV + cc * 8);
+        sy[u] = *reinterpret_cast<const float4*>(S0 + size_t(quarter * QR + row) * DV + cc * 8 + 4);
+      }
+    }
+  };
+  load_state(0);
+  vw.store(b_s, 0, tid);
+  float o[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  const int r_lo = warp * SUB + g4, r_hi = r_lo + 8, j0 = half * NT;      // this thread's two tokens; the warp's first n-tile
+  unsigned char* s_hi = k_s;                      // [QR][DV]
+  unsigned char* s_lo = k_s + QR * DV * 2;
+  const uint32_t shi = smem_u32(s_hi), slo = smem_u32(s_lo);
+#pragma unroll 1
+  for (int quarter = 0; quarter < 4; ++quarter) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int i = tid + u * 256, row = i / CHUNKS, cc = i % CHUNKS;
+      if (i < QR * CHUNKS) {
+        uint4 hi, lo;
+        split_pack(sx[u].x, sx[u].y, hi.x, lo.x);
+        split_pack(sx[u].z, sx[u].w, hi.y, lo.y);
+        split_pack(sy[u].x, sy[u].y, hi.z, lo.z);
+        split_pack(sy[u].z, sy[u].w, hi.w, lo.w);
+        *reinterpret_cast<uint4*>(s_hi + swz<DV>(row, cc)) = hi;
+        *reinterpret_cast<uint4*>(s_lo + swz<DV>(row, cc)) = lo;
+      }
+    }
+    __syncthreads();      // this quarter (and v) is staged
+    if (quarter < 3) load_state(quarter + 1);
+#pragma unroll
+    for (int kk = 0; kk < QR / 16; ++kk) {
+      uint32_t qh[4], ql[4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int ch = quarter * QR + kk * 16 + 8 * x + 2 * t4;
+        float2 front = make_float2(0.f, 0.f);
+        for (int y = 0; y < warp; ++y) {
+          const float2 t = *reinterpret_cast<const float2*>(t_s + y * DK + ch);
+          front.x += t.x;
+          front.y += t.y;
+        }
+        scaled_q(r_lo, ch, front, qh[2 * x], ql[2 * x]);
+        scaled_q(r_hi, ch, front, qh[2 * x + 1], ql[2 * x + 1]);
+      }
+#pragma unroll
+      for (int j = 0; j < NT; j += 2) {
+        uint32_t b0, b1, b2, b3;
+        const uint32_t off = swz<DV>(kk * 16 + (m & 1) * 8 + (lane & 7), j0 + j + (m >> 1));
+        ldmatrix_x4_trans(b0, b1, b2, b3, shi + off);
+        mma_bf16(o[j], qh, b0, b1);
+        mma_bf16(o[j + 1], qh, b2, b3);
+        mma_bf16(o[j], ql, b0, b1);
+        mma_bf16(o[j + 1], ql, b2, b3);
+        ldmatrix_x4_trans(b0, b1, b2, b3, slo + off);
+        mma_bf16(o[j], qh, b0, b1);
+        mma_bf16(o[j + 1], qh, b2, b3);
+      }
+    }
+    __syncthreads();      // the quarter is no longer read
+  }
+#pragma unroll
+  for (int kb = 0; kb < SUBS; ++kb) {
+    if (kb > warp) break;
+    uint32_t ph[4], pl[4];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const float2 a = *reinterpret_cast<const float2*>(s_s + r_lo * SPITCH + kb * 16 + 8 * x + 2 * t4);
+      const float2 b = *reinterpret_cast<const float2*>(s_s + r_hi * SPITCH + kb * 16 + 8 * x + 2 * t4);
+      split_pack(a.x, a.y, ph[2 * x], pl[2 * x]);
+      split_pack(b.x, b.y, ph[2 * x + 1], pl[2 * x + 1]);
+    }
+#pragma unroll
+    for (int j = 0; j < NT; j += 2) {
+      uint32_t b0, b1, b2, b3;
+      ldmatrix_x4_trans(b0, b1, b2, b3, bs + swz<DV>(kb * 16 + (m & 1) * 8 + (lane & 7), j0 + j + (m >> 1)));
+      mma_bf16(o[j], ph, b0, b1);
+      mma_bf16(o[j], pl, b0, b1);
+      mma_bf16(o[j + 1], ph, b2, b3);
+      mma_bf16(o[j + 1], pl, b2, b3);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = i ? r_hi : r_lo;
+    if (r >= n) continue;
+    float* dst = out + (size_t(start + r) * heads + h) * DV + j0 * 8 + t4 * 2;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][2 * i] * q_scale, o[j][2 * i + 1] * q_scale);
+  }
+}
+
+template <int DK, int DV>
+int launch_out(const void* proj, int stride, const float* log_decay, const StepBatch& sb, const int* chunk_seq, const int* chunk_q0,
+               int n_chunks, const float* before, float* out, int heads, float q_scale, cudaStream_t stream) {
+  constexpr size_t smem = OutShape<DK, DV>::SMEM;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gla_chunk_out_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+      return PTB_ERR_LAUNCH;
+    configured = true;
+  }
+  gla_chunk_out_mma_kernel<DK, DV><<<dim3(n_chunks, heads), 256, smem, stream>>>((const __nv_bfloat16*)proj, stride, log_decay, sb,
+                                                                                chunk_seq, chunk_q0, before, out, heads, q_scale);
+  return launch_status();
+}
+
 }  // namespace
 
-// Sizes and layouts that this pass takes: bfloat16 projections, keys and values of 64 or 128 entries, rows that start
+// Sizes and layouts that these passes take: bfloat16 projections, keys and values of 64 or 128 entries, rows that start
 // at whole 16-byte words (then q, k, v and the logarithms' rows do too).
 PTB_API int ptb_gla_chunk_sum_mma_supports(int dtype, const void* proj, int stride, const float* log_decay, int dim, int v_dim) {
   return (dtype == PTB_BF16 && (dim == 64 || dim == 128) && (v_dim == 64 || v_dim == 128) && stride % 8 == 0 &&
@@ -148,5 +458,20 @@ PTB_API int ptb_gla_chunk_sum_mma(const void* proj, int stride, const float* log
   if (dim == 128 && v_dim == 64) PTB_GLA_SUM(128, 64);
   if (dim == 128 && v_dim == 128) PTB_GLA_SUM(128, 128);
 #undef PTB_GLA_SUM
+  return PTB_ERR_SIZE;
+}
+
+// Every chunk's outputs from the state before it (`before`: what the join left of the chunks' sums; the same sizes and layouts).
+PTB_API int ptb_gla_chunk_out_mma(const void* proj, int stride, const float* log_decay, const StepBatch* sb, const int* chunk_seq,
+                                  const int* chunk_q0, int n_chunks, const float* before, float* out, int heads, int dim, int v_dim,
+                                  float q_scale, cudaStream_t stream) {
+  if (n_chunks <= 0) return PTB_OK;
+#define PTB_GLA_OUT(DK, DV) \
+  return launch_out<DK, DV>(proj, stride, log_decay, *sb, chunk_seq, chunk_q0, n_chunks, before, out, heads, q_scale, stream)
+  if (dim == 64 && v_dim == 64) PTB_GLA_OUT(64, 64);
+  if (dim == 64 && v_dim == 128) PTB_GLA_OUT(64, 128);
+  if (dim == 128 && v_dim == 64) PTB_GLA_OUT(128, 64);
+  if (dim == 128 && v_dim == 128) PTB_GLA_OUT(128, 128);
+#undef PTB_GLA_OUT
   return PTB_ERR_SIZE;
 }
