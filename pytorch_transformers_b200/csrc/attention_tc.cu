@@ -116,35 +116,45 @@ constexpr int BLOCK_THREADS = SOFTMAX_THREADS + 64;
 // EXTRAS: a window with kept first positions, a soft cap, sinks, an output gate, an output factor and strided results. A walk
 // takes the kept pages, then the window's: page i of the walk is not page i of the sequence, and a row may see nothing of a
 // page. Nothing else of the pipeline changes. What such a prompt costs is the chain of a page as above (a cap adds an
-// exponential and a reciprocal a score): 16 heads of 128 on 4 K/V heads, 2,048 tokens, window 1,024: 41 us, where
-// the mma.sync kernel took 175; prompts of 500, 1,000 and 1,501 tokens, cap and a gate per entry: 104 us against 261.
-template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS>
-__global__ void __launch_bounds__(BLOCK_THREADS, DK == 64 ? 2 : 1)
+// exponential and a reciprocal a score): 16 heads of 128 on 4 K/V heads, 2,048 tokens, window 1,024: 39 us, where
+// the mma.sync kernel took 175; prompts of 500, 1,000 and 1,501 tokens, cap and a gate per entry: 75 us against 261.
+// TWO (head size 128 with weights of two terms): two S buffers and two page stages instead of three and four, 97 KB and 256
+// columns of tensor memory a block, so that two blocks fit on an SM and one's softmax runs under the other's waits. Worth it
+// where the blocks make more than two waves (384 blocks, capped: 104 -> 75 us) or the walks of a window are alike long (256
+// blocks: 41 -> 39 us); with fewer blocks and the triangle of a full context the longest chain counts, and a
+// block with an SM of its own runs it faster (256 blocks: 41 us alone, 52 us two an SM).
+template <bool TWO> struct TcShape {
+  static constexpr int BUFS = TWO ? 2 : 3;                 // S buffers
+  static constexpr int STAGES = TWO ? 2 : STAGES_TC;       // page stages
+};
+template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS, bool TWO>
+__global__ void __launch_bounds__(BLOCK_THREADS, DK == 64 || TWO ? 2 : 1)
 attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_pool,
                     const __nv_bfloat16* __restrict__ v_pool, __nv_bfloat16* __restrict__ out, StepBatch sb,
                     const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, TcParams p,
                     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                     int* __restrict__ error_flag) {
+  constexpr int BUFS = TcShape<TWO>::BUFS, STAGES = TcShape<TWO>::STAGES;
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte alignment: the swizzle pattern is a function of address bits 4..9
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   constexpr int TILE_Q_BYTES = TQ * DK * 2;      // 16, 32 or 48 KB
   constexpr int TILE_K_BYTES = KEYS * DK * 2;    // 8, 16 or 24 KB
   constexpr int TILE_V_BYTES = KEYS * DV * 2;    // 8 or 16 KB
-  // tensor memory: three S buffers of 64 columns (page i uses buffer i % 3), O at [192, 192 + DV). P of a
+  // tensor memory: BUFS (three, or two) S buffers of 64 columns (page i uses buffer i % BUFS), then O. P of a
   // page (64 keys as bfloat16 pairs, 32 columns) takes the place of its S: a thread has its row of S in
   // registers before it writes its row of P, nobody else touches that row, and the S of three pages later
   // is issued after the O += P V that reads this P (the tensor pipe runs in order). With three buffers S
   // runs two pages ahead of the softmax, so the softmax does not wait for a matrix product that was
   // issued only when the slowest warp finished the page before.
-  constexpr uint32_t TMEM_O = 192, TMEM_COLS = (DV == 64) ? 256 : 512;
+  constexpr uint32_t TMEM_O = BUFS * 64, TMEM_COLS = (TMEM_O + DV <= 256) ? 256 : 512;
   unsigned char* q_tile = smem;
-  unsigned char* k_ring = q_tile + TILE_Q_BYTES;                      // STAGES_TC pages
-  unsigned char* v_ring = k_ring + STAGES_TC * TILE_K_BYTES;          // STAGES_TC pages
+  unsigned char* k_ring = q_tile + TILE_Q_BYTES;                      // STAGES pages
+  unsigned char* v_ring = k_ring + STAGES * TILE_K_BYTES;          // STAGES pages
   // barriers: [0..2] S buffer written; [3..6] O updated (page % 4); [7..9] P written (page % 3);
   // then per stage: page landed, stage free again
-  uint64_t* bars = reinterpret_cast<uint64_t*>(v_ring + STAGES_TC * TILE_V_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10 + 2 * STAGES_TC);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(v_ring + STAGES * TILE_V_BYTES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10 + 2 * STAGES);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool mma_warp = warp == SOFTMAX_THREADS / 32;
@@ -178,16 +188,16 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   // page i knows that O += P V of page i - 3 has completed (the tensor pipe runs in order), and so the one
   // of page i - 4: hence four "O updated" barriers that take turns. With two, a warp that reached the end
   // of its walk pages ahead of the others could take the completion of page i - 2 for that of page i and
-  // read O before the last products were in it.
+  // read O before the last products were in it. With two S buffers every distance is one page less.
   const uint32_t bar_s = smem_u32(&bars[0]), bar_o = smem_u32(&bars[3]);
   const uint32_t bar_p = smem_u32(&bars[7]);
-  const uint32_t bar_k = smem_u32(&bars[10]), bar_free = smem_u32(&bars[10 + STAGES_TC]);
+  const uint32_t bar_k = smem_u32(&bars[10]), bar_free = smem_u32(&bars[10 + STAGES]);
   // The copy warp's first lane sets the barriers up and asks for the first pages at once (their numbers
   // read by the warp's lanes, one each): they are on their way while the other warps fetch Q and tensor
   // memory is allocated. Nobody else touches a barrier before the block-wide barrier below.
   constexpr uint32_t PAGE_BYTES = TILE_K_BYTES + TILE_V_BYTES;
   auto ask_page = [&](int b, int page) {
-    const int st = b % STAGES_TC;
+    const int st = b % STAGES;
     const int y = (page * p.kv_heads + g) * KEYS;   // first row of the page in the pool seen as [rows][D]
     const uint32_t full = bar_k + 8 * st;
     mbar_expect_tx(full, PAGE_BYTES);
@@ -207,13 +217,13 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
         mbar_init(bar_p + 8 * b, SOFTMAX_THREADS);
       }
       for (int b = 0; b < 4; ++b) mbar_init(bar_o + 8 * b, 1);
-      for (int s = 0; s < STAGES_TC; ++s) {
+      for (int s = 0; s < STAGES; ++s) {
         mbar_init(bar_k + 8 * s, 1);      // the copy thread's expect_tx; the bytes complete it
         mbar_init(bar_free + 8 * s, 1);   // tcgen05.commit after the stage's O += P V
       }
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    for (int b = 0; b < STAGES_TC && b < n_blocks; ++b) {
+    for (int b = 0; b < STAGES && b < n_blocks; ++b) {
       const int page = __shfl_sync(0xffffffffu, first_pages, b);
       if (lane == 0) ask_page(b, page);
     }
@@ -245,21 +255,21 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
 
   if (copy_warp) {
     // ------------------------------------------------------------ the thread that asks for the pages
-    // Page b goes into stage b % STAGES_TC as DK / 64 and DV / 64 boxes [64 keys x 64 dims] for K and V, in
+    // Page b goes into stage b % STAGES as DK / 64 and DV / 64 boxes [64 keys x 64 dims] for K and V, in
     // the swizzled layout; the stage's barrier counts the bytes. A stage is free again when the
     // O += P V that read it has completed (S of that page completed before it).
     // The first pages were asked for above; the rest is the first lane's alone.
     if (lane == 0) {
-      int issued = min(n_blocks, STAGES_TC);
-      for (int b = STAGES_TC; b < n_blocks; ++b) {
-        if (!mbar_wait(bar_free + 8 * (b % STAGES_TC), ((b / STAGES_TC) - 1) & 1, error_flag, 6)) break;
+      int issued = min(n_blocks, STAGES);
+      for (int b = STAGES; b < n_blocks; ++b) {
+        if (!mbar_wait(bar_free + 8 * (b % STAGES), ((b / STAGES) - 1) & 1, error_flag, 6)) break;
         ask_page(b, pages[block_of(b)]);
         issued = b + 1;
       }
       if (issued < n_blocks) {
         // a wait ran out: what is in flight lands before the block ends (bounded waits again)
-        for (int b = max(0, issued - STAGES_TC); b < issued; ++b)
-          mbar_wait(bar_k + 8 * (b % STAGES_TC), (b / STAGES_TC) & 1, error_flag, 6);
+        for (int b = max(0, issued - STAGES); b < issued; ++b)
+          mbar_wait(bar_k + 8 * (b % STAGES), (b / STAGES) & 1, error_flag, 6);
       }
     }
   } else if (mma_warp) {
@@ -276,47 +286,48 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       const uint64_t desc_v0 = smem_desc(smem_u32(v_ring), KEYS * 128, 1024);
       constexpr uint64_t K_UNITS = TILE_K_BYTES >> 4, V_UNITS = TILE_V_BYTES >> 4;   // the address field counts 16-byte units
       constexpr uint64_t Q_BLOCK = (TQ * 128) >> 4, KV_BLOCK = (KEYS * 128) >> 4;   // blocks of 64 dims
-      // S_b = Q K_b^T into S buffer `buf`; the page sits in stage b % STAGES_TC
+      // S_b = Q K_b^T into S buffer `buf`; the page sits in stage b % STAGES
       auto issue_s = [&](int b, int buf) {
-        const int st = b % STAGES_TC;
+        const int st = b % STAGES;
 #pragma unroll
         for (int blk = 0; blk < DK / 64; ++blk)
           tc_mma4<2, 2>(tmem_base + buf * 64, desc_q + blk * Q_BLOCK, desc_k0 + st * K_UNITS + blk * KV_BLOCK,
                         IDESC_S, blk > 0 ? 1u : 0u);
         tc_commit(bar_s + buf * 8);
       };
-      // S of the first two pages
-      for (int b = 0; b < 2 && b < n_blocks && alive; ++b) {
+      // S of the first pages
+      for (int b = 0; b < BUFS - 1 && b < n_blocks && alive; ++b) {
         alive = mbar_wait(bar_k + 8 * b, 0, error_flag, 4);
         tc_fence_after();
         if (alive) issue_s(b, b);
       }
-      int buf = 0, phase = 0;   // S buffer of page i (i % 3) and the parity of its barriers ((i / 3) & 1)
+      int buf = 0, phase = 0;   // S buffer of page i (i % BUFS) and the parity of its barriers ((i / BUFS) & 1)
       for (int i = 0; i < n_blocks && alive; ++i) {
-        if (i + 2 < n_blocks) {
-          // page i + 2 landed; S_{i+2} goes where S_{i-1} and P_{i-1} were: every thread had read that S
+        const int ahead = i + BUFS - 1;
+        if (ahead < n_blocks) {
+          // page `ahead` landed; its S goes where S_{i-1} and P_{i-1} were: every thread had read that S
           // before it reported P_{i-1}, and the O += P_{i-1} V_{i-1} that reads the P was issued before
-          alive = mbar_wait(bar_k + 8 * ((i + 2) % STAGES_TC), ((i + 2) / STAGES_TC) & 1, error_flag, 4);
+          alive = mbar_wait(bar_k + 8 * (ahead % STAGES), (ahead / STAGES) & 1, error_flag, 4);
           tc_fence_after();
-          issue_s(i + 2, buf == 0 ? 2 : buf - 1);
+          issue_s(ahead, buf == 0 ? BUFS - 1 : buf - 1);
         }
         // P_i is written and O is rescaled: O += P_i V_i (16 keys: 32 bytes along P's rows, 2048 bytes
         // down V's rows)
         if (alive) alive = mbar_wait(bar_p + buf * 8, phase, error_flag, 5);
         tc_fence_after();
-        const int st = i % STAGES_TC;
+        const int st = i % STAGES;
         tc_mma4_ts<128>(tmem_o, tmem_base + buf * 64, desc_v0 + st * V_UNITS, IDESC_PV, i > 0 ? 1u : 0u);
         if (WIDE) tc_mma4_ts<128>(tmem_o, tmem_base + buf * 64 + KEYS / 2, desc_v0 + st * V_UNITS, IDESC_PV, 1u);
         tc_commit(bar_o + 8 * (i & 3));
         tc_commit(bar_free + 8 * st);   // the copy thread may refill this stage
-        if (++buf == 3) { buf = 0; phase ^= 1; }
+        if (++buf == BUFS) { buf = 0; phase ^= 1; }
       }
     }
   } else {
     // ------------------------------------------------------------ softmax threads
     const uint32_t lane_addr = tmem_base + (uint32_t((warp & 3) * 32) << 16);   // this warp's lanes
     const uint32_t o_addr = lane_addr + TMEM_O;
-    int buf = 0, phase = 0;   // S buffer of page i (i % 3) and the parity of its barriers ((i / 3) & 1)
+    int buf = 0, phase = 0;   // S buffer of page i (i % BUFS) and the parity of its barriers ((i / BUFS) & 1)
     float m_run = -INFINITY, l_run = 0.f;   // running maximum of the raw scores, the row's sum
     const float slope = BIAS ? p.slopes[h] : 0.f;
     const bool capped = EXTRAS && p.softcap > 0.f;
@@ -411,7 +422,7 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       l_run = l_run * corr + ((l0 + l1) + (l2 + l3));
       tc_fence_before();
       mbar_arrive(bar_p + buf * 8);   // (5) the issuing thread starts O += P V when all rows have arrived
-      if (++buf == 3) { buf = 0; phase ^= 1; }
+      if (++buf == BUFS) { buf = 0; phase ^= 1; }
     }
     // the walk's last O += P V
     if (alive) alive = mbar_wait(bar_o + 8 * ((n_blocks - 1) & 3), ((n_blocks - 1) >> 2) & 1, error_flag, 3);
@@ -867,22 +878,28 @@ PTB_API int ptb_attention_tc_supports_sizes(int head_dim, int v_dim) {
 PTB_API int ptb_attention_tc_tile_tokens() { return TQ; }
 
 namespace {
-template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS = false>
+template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS = false, bool TWO = false>
 int launch_tc(const void* q, const void* k_pool, const void* v_pool, int pool_pages, void* out, const StepBatch& sb,
               const int* tile_seq, const int* tile_q0, int n_tiles, const TcParams& p, int* error_flag,
               cudaStream_t stream) {
+  if constexpr (DK == 128 && DV == 128 && WIDE && !TWO) {      // the rule of TWO
+    const long long blocks = (long long)p.heads * n_tiles, sms = sm_count();
+    if (blocks > 2 * sms || (p.window > 0 && blocks > sms))
+      return launch_tc<DK, DV, BIAS, WIDE, EXTRAS, true>(q, k_pool, v_pool, pool_pages, out, sb, tile_seq, tile_q0, n_tiles, p,
+                                                         error_flag, stream);
+  }
   const CUtensorMap* km = pool_map(k_pool, pool_pages, p.kv_heads, DK);
   const CUtensorMap* vm = pool_map(v_pool, pool_pages, p.kv_heads, DV);
   if (km == nullptr || vm == nullptr) return PTB_ERR_LAUNCH;
-  const size_t smem = 1024 + TQ * DK * 2 + STAGES_TC * KEYS * (DK + DV) * 2 + 192;
+  const size_t smem = 1024 + TQ * DK * 2 + TcShape<TWO>::STAGES * KEYS * (DK + DV) * 2 + 192;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
       return PTB_ERR_LAUNCH;
     configured = true;
   }
   dim3 grid(p.heads, n_tiles);
-  attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS><<<grid, BLOCK_THREADS, smem, stream>>>(
+  attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO><<<grid, BLOCK_THREADS, smem, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, sb,
       tile_seq, tile_q0, p, *km, *vm, error_flag);
   return launch_status();

@@ -415,7 +415,7 @@ def test_tensor_core_kernels_on_random_shapes(K, first_seed):
         torch.testing.assert_close(out, ref, msg=lambda m: f"seed {seed} {kind}: {m}", **tol(BF))
 
 
-@pytest.mark.parametrize("heads,kv,d", [(4, 1, 64), (6, 2, 128)])
+@pytest.mark.parametrize("heads,kv,d", [(4, 1, 64), (6, 2, 128), (60, 4, 128)])    # 60: more blocks than two an SM
 @pytest.mark.parametrize("window,keep", [(0, 0), (1, 0), (64, 4), (65, 70), (100, 200), (700, 1)])
 @pytest.mark.parametrize("softcap,sinks,gate,strided", [(0.0, False, None, False), (30.0, True, "head", True), (5.0, True, "entry", False),
                                                         (0.0, False, "entry", True)])
