@@ -35,10 +35,12 @@ __global__ void mlstm_gates_kernel(float* __restrict__ gates, const float* __res
 
 // One block per (sequence, head, 32 value columns) walks the sequence's tokens of the step. Thread (warp w, lane v)
 // keeps S[w + 8 i][v0 + v] in registers; lane l of warp w also keeps n[w + 8 l]. One barrier a token: q, k, v of the
-// next token and the partial sums of this one go through buffers that take turns.
+// next token and the partial sums of this one go through buffers that take turns. With bias_i the gates are the products' sums and
+// the walk forms their logarithms itself (steps of single tokens: no launch of its own for 2 heads values a token).
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(VB * WARPS)
-mlstm_scan_kernel(const T* __restrict__ proj, int stride, const float* __restrict__ gates, float* __restrict__ state,
+mlstm_scan_kernel(const T* __restrict__ proj, int stride, const float* __restrict__ gates, const float* __restrict__ bias_i,
+                  const float* __restrict__ bias_f, float cap, float* __restrict__ state,
                   int state_stride, const int* __restrict__ slots, StepBatch sb, float* __restrict__ out, int heads, int dim,
                   int v_dim, float q_scale) {
   __shared__ float qs[2][MAX_DIM], ks[2][MAX_DIM], vs[2][VB], red_o[2][WARPS][VB], red_n[2][WARPS];
@@ -83,13 +85,22 @@ mlstm_scan_kernel(const T* __restrict__ proj, int stride, const float* __restric
     if (col_ok) out[size_t(start + t) * heads * v_dim + size_t(h) * v_dim + v0 + lane] = o / den;
   };
 
+  float gi, gf;      // the token's gates
+  auto load_gates = [&](int t) {
+    gi = gates[size_t(start + t) * 2 * heads + h], gf = gates[size_t(start + t) * 2 * heads + heads + h];
+    if (bias_i) {
+      gi = capped(gi + bias_i[h], cap);
+      gf = log_sigmoid(capped(gf + bias_f[h], cap));
+    }
+  };
   load(0, 0);
+  load_gates(0);
   float m_prev_token = m;
   for (int t = 0; t < n_new; ++t) {
     const int buf = t & 1;
     __syncthreads();
     if (t > 0 && w == 0) finish(t - 1, buf ^ 1, m_prev_token);
-    const float gi = gates[size_t(start + t) * 2 * heads + h], gf = gates[size_t(start + t) * 2 * heads + heads + h];
+    if (t > 0) load_gates(t);
     const float m_new = fmaxf(gf + m, gi);
     const float a = expf(gf + m - m_new), b = expf(gi - m_new);
     m = m_new;
@@ -148,11 +159,11 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ x, const float* 
 }
 
 template <typename T>
-int launch_scan(const void* proj, int stride, const float* gates, float* state, int state_stride, const int* slots,
+int launch_scan(const void* proj, int stride, const float* gates, const float* bias_i, const float* bias_f, float cap, float* state, int state_stride, const int* slots,
                 const StepBatch& sb, float* out, int heads, int dim, int v_dim, float q_scale, cudaStream_t stream) {
   dim3 grid(sb.n_seqs, heads, (v_dim + VB - 1) / VB);
 #define PTB_SCAN(ROWS)                                                                                                       \
-  mlstm_scan_kernel<T, ROWS><<<grid, VB * WARPS, 0, stream>>>((const T*)proj, stride, gates, state, state_stride, slots, sb, \
+  mlstm_scan_kernel<T, ROWS><<<grid, VB * WARPS, 0, stream>>>((const T*)proj, stride, gates, bias_i, bias_f, cap, state, state_stride, slots, sb, \
                                                               out, heads, dim, v_dim, q_scale)
   if (dim <= 8 * WARPS)
     PTB_SCAN(8);
@@ -179,17 +190,18 @@ PTB_API int ptb_mlstm_gates(float* gates, const float* bias_i, const float* bias
 
 // proj [tokens, >= 2 heads dim + heads v_dim] holds q, k, v side by side (rows `stride` apart); gates as ptb_mlstm_gates
 // leaves them; state [slots, >= ptb_mlstm_state_floats(heads, dim, v_dim)] float32; out float32 [tokens, heads * v_dim].
-PTB_API int ptb_mlstm_scan(int dtype, const void* proj, int stride, const float* gates, float* state, int state_stride,
-                           const int* slots, const StepBatch* sb, float* out, int heads, int dim, int v_dim, float q_scale,
+// bias_i, bias_f null: `gates` hold the gates' logarithms; else their products' sums, and the walk adds biases, caps at `cap`
+PTB_API int ptb_mlstm_scan(int dtype, const void* proj, int stride, const float* gates, const float* bias_i, const float* bias_f,
+                           float cap, float* state, int state_stride, const int* slots, const StepBatch* sb, float* out, int heads, int dim, int v_dim, float q_scale,
                            cudaStream_t stream) {
   if (sb->n_tokens <= 0) return PTB_OK;
   if (heads <= 0 || heads > 65535 || dim <= 0 || dim > MAX_DIM || v_dim <= 0 || stride < 2 * heads * dim + heads * v_dim ||
       state_stride < heads * (dim * v_dim + ((v_dim + VB - 1) / VB) * (dim + 1)))
     return PTB_ERR_SIZE;
   if (dtype == PTB_F32)
-    return launch_scan<float>(proj, stride, gates, state, state_stride, slots, *sb, out, heads, dim, v_dim, q_scale, stream);
+    return launch_scan<float>(proj, stride, gates, bias_i, bias_f, cap, state, state_stride, slots, *sb, out, heads, dim, v_dim, q_scale, stream);
   if (dtype == PTB_BF16)
-    return launch_scan<__nv_bfloat16>(proj, stride, gates, state, state_stride, slots, *sb, out, heads, dim, v_dim, q_scale,
+    return launch_scan<__nv_bfloat16>(proj, stride, gates, bias_i, bias_f, cap, state, state_stride, slots, *sb, out, heads, dim, v_dim, q_scale,
                                       stream);
   return PTB_ERR_DTYPE;
 }

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 skinny_linear_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                      const float* __restrict__ bias, const __nv_bfloat16* __restrict__ add,
                      __nv_bfloat16* __restrict__ y_bf16, float* __restrict__ y_f32, int M, int N, int K, int ldx, int act,
-                     int ksplit, float* __restrict__ scratch, int* __restrict__ tickets) {
+                     int ksplit, float* __restrict__ scratch, int* __restrict__ tickets, int n_bf16) {
   __shared__ float red[WARPS][MT * 16][NT * 8 + 1];
   __shared__ int is_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -170,8 +170,8 @@ skinny_linear_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
     if (bias) v += bias[n];
     v = apply_activation(v, act);
     if (add) v += __bfloat162float(add[size_t(m) * N + n]);
-    if (y_f32) y_f32[size_t(m) * N + n] = v;
-    else y_bf16[size_t(m) * N + n] = __float2bfloat16_rn(v);
+    if (n < n_bf16) y_bf16[size_t(m) * n_bf16 + n] = __float2bfloat16_rn(v);
+    else y_f32[size_t(m) * (N - n_bf16) + n - n_bf16] = v;
   }
 }
 
@@ -201,7 +201,7 @@ int k_split(int tiles, int chunks, int round) {
 template <int MT, int NT, int U>
 int launch_skinny(const void* x, const void* w, const float* bias, const void* add, void* y_bf16, float* y_f32,
                   int M, int N, int K, int ldx, int act, float* scratch, size_t scratch_floats, int* tickets, int n_tickets,
-                  size_t* need_floats, cudaStream_t stream) {
+                  size_t* need_floats, int n_bf16, cudaStream_t stream) {
   const int tiles = (N + 16 * MT - 1) / (16 * MT);
   int ksplit = k_split(tiles, K / KC, WARPS * U);
   const size_t need = ksplit > 1 ? size_t(tiles) * ksplit * (MT * 16 * NT * 8) : 0;
@@ -212,13 +212,13 @@ int launch_skinny(const void* x, const void* w, const float* bias, const void* a
   if (scratch == nullptr || tickets == nullptr || scratch_floats < need || n_tickets < tiles) ksplit = 1;
   skinny_linear_kernel<MT, NT, U><<<tiles * ksplit, WARPS * 32, 0, stream>>>(
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, (const __nv_bfloat16*)add, (__nv_bfloat16*)y_bf16,
-      y_f32, M, N, K, ldx, act, ksplit, scratch, tickets);
+      y_f32, M, N, K, ldx, act, ksplit, scratch, tickets, n_bf16);
   return launch_status();
 }
 
 int dispatch_skinny(const void* x, const void* w, const float* bias, const void* add, void* y_bf16, float* y_f32, int M,
                     int N, int K, int ldx, int act, float* scratch, size_t scratch_floats, int* tickets, int n_tickets,
-                    size_t* need_floats, cudaStream_t stream) {
+                    size_t* need_floats, int n_bf16, cudaStream_t stream) {
   // Tile height and chunks in flight per warp, from a sweep over matrices of 4,096 to 65,024 rows (each
   // alone, from HBM): matrices with four tiles or more per SM (many rows, short K) want 32 rows per
   // block and four chunks in flight at up to 8 activation rows, 16 rows and two chunks at up to 16;
@@ -226,7 +226,7 @@ int dispatch_skinny(const void* x, const void* w, const float* bias, const void*
   const bool wide = N >= 16 * sm_count() * 4;   // four 16-row tiles or more per SM
 #define PTB_SKINNY(MT, NT, U) \
   return launch_skinny<MT, NT, U>(x, w, bias, add, y_bf16, y_f32, M, N, K, ldx, act, scratch, scratch_floats, tickets, \
-                                  n_tickets, need_floats, stream)
+                                  n_tickets, need_floats, n_bf16, stream)
   if (M <= 8) {
     if (wide) PTB_SKINNY(2, 1, 4);
     PTB_SKINNY(1, 1, 4);
@@ -247,25 +247,26 @@ PTB_API int ptb_skinny_linear_max_rows() { return 32; }
 PTB_API int ptb_skinny_linear_k_multiple() { return KC; }
 
 // y = act(x w^T + bias) + add. x [M, K] (rows ldx apart, whole 16-byte words), w [N, K], add [M, N] bfloat16; bias float32 [N];
-// exactly one of y_bf16, y_f32 is given. M <= 32, K a multiple of 32, 16-byte aligned x and w.
+// the first n_bf16 outputs go to y_bf16 [M, n_bf16], the others unrounded to y_f32 [M, N - n_bf16] (n_bf16 0 or N: one of the two,
+// the other pointer null; in between: one pass over rows of two matrices that read the same x). M <= 32, K a multiple of 32, 16-byte aligned x and w.
 // scratch (float32, scratch_floats of them) and tickets (int32, n_tickets of them, all zero between
 // launches: the kernel puts them back) let the kernel divide K among several blocks per tile where that
 // balances the SMs; without them it does not divide. ptb_skinny_linear_scratch says how many floats a
 // launch would use.
 PTB_API int ptb_skinny_linear(const void* x, const void* w, const float* bias, const void* add, void* y_bf16,
-                              float* y_f32, int M, int N, int K, int ldx, int act, float* scratch, size_t scratch_floats,
-                              int* tickets, int n_tickets, cudaStream_t stream) {
+                              float* y_f32, int n_bf16, int M, int N, int K, int ldx, int act, float* scratch,
+                              size_t scratch_floats, int* tickets, int n_tickets, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return PTB_OK;
   if (M > 32 || K <= 0 || K % KC != 0 || ldx < K || !activation_known(act)) return PTB_ERR_SIZE;
-  if ((y_bf16 == nullptr) == (y_f32 == nullptr)) return PTB_ERR_SIZE;
+  if (n_bf16 < 0 || n_bf16 > N || (y_bf16 == nullptr) != (n_bf16 == 0) || (y_f32 == nullptr) != (n_bf16 == N)) return PTB_ERR_SIZE;
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) || ldx % 8 != 0) return PTB_ERR_ALIGN;
   return dispatch_skinny(x, w, bias, add, y_bf16, y_f32, M, N, K, ldx, act, scratch, scratch_floats, tickets, n_tickets,
-                         nullptr, stream);
+                         nullptr, n_bf16, stream);
 }
 
 PTB_API long long ptb_skinny_linear_scratch(int M, int N, int K) {
   if (M <= 0 || N <= 0 || M > 32 || K <= 0 || K % KC != 0) return 0;
   size_t need = 0;
-  dispatch_skinny(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, M, N, K, K, 0, nullptr, 0, nullptr, 0, &need, nullptr);
+  dispatch_skinny(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, M, N, K, K, 0, nullptr, 0, nullptr, 0, &need, 0, nullptr);
   return (long long)need;
 }

@@ -409,20 +409,19 @@ class CausalLM:
             if isinstance(x, DeferredSum):
                 x.join(x.base.device)
             return torch.empty((0, self.spec.vocab_size), dtype=torch.float32, device=self.device)
+        def wanted(t):
+            return t if ctx.all_wanted else k.gather_rows(ctx.dev["logits_at"], t, self.status)
         if (isinstance(x, DeferredSum) and hasattr(self.final_norm, "forward_pending") and x.base.dtype == torch.float32
                 and x.pending.dtype == torch.float32):
             # the last sum only at the wanted rows, in the final norm's kernel
             x.join(x.base.device)
-            rows, _ = self.final_norm.forward_pending(k.gather_rows(ctx.dev["logits_at"], x.base, self.status),
-                                                      k.gather_rows(ctx.dev["logits_at"], x.pending, self.status), x.bias)
+            rows, _ = self.final_norm.forward_pending(wanted(x.base), wanted(x.pending), x.bias)
             return self.logits(rows)
         if isinstance(x, DeferredSum) and x.bias is None and hasattr(self.final_norm, "forward_sum"):
             x.join(x.base.device)       # likewise: the last sum at the wanted rows, in the final norm's kernel
-            rows = self.final_norm.forward_sum(k.gather_rows(ctx.dev["logits_at"], x.base, self.status),
-                                               k.gather_rows(ctx.dev["logits_at"], x.pending, self.status))[1]
+            rows = self.final_norm.forward_sum(wanted(x.base), wanted(x.pending))[1]
             return self.logits(rows)
-        x = resolve(k, x)
-        rows = k.gather_rows(ctx.dev["logits_at"], x, self.status)
+        rows = wanted(resolve(k, x))
         rows = self.final_norm.forward(rows)
         return self.logits(rows)
 

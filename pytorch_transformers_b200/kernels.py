@@ -722,17 +722,36 @@ def skinny_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
         raise KernelError(f"skinny_linear: shapes x {list(x.shape)}, w {list(w.shape)} do not fit")
     y = torch.empty((m, n), dtype=out_dtype, device=x.device)
     ybf, yf = (y, None) if out_dtype == torch.bfloat16 else (None, y)
+    _skinny_launch(x, w, bias, act, add, ybf, yf)
+    return y
+
+
+def skinny_linear_split(x: torch.Tensor, w: torch.Tensor, n_bf16: int):
+    """x @ w.T in one pass over w with the first ``n_bf16`` outputs in bfloat16 and the others as unrounded float32 sums: two
+    products of the same rows, (bfloat16 [rows, n_bf16], float32 [rows, the rest])."""
+    _need_cuda(w)
+    _check_rows(x, x.shape, torch.bfloat16, "skinny_linear_split: x")
+    m, n = x.shape[0], w.shape[0]
+    if w.dtype != torch.bfloat16 or w.shape[1] != x.shape[1] or not 0 < n_bf16 < n:
+        raise KernelError("skinny_linear_split takes bfloat16 x [rows, K] and w [N, K] and 0 < n_bf16 < N")
+    y = torch.empty((m, n_bf16), dtype=torch.bfloat16, device=x.device)
+    rest = torch.empty((m, n - n_bf16), dtype=torch.float32, device=x.device)
+    _skinny_launch(x, w, None, "none", None, y, rest)
+    return y, rest
+
+
+def _skinny_launch(x, w, bias, act, add, ybf, yf) -> None:
+    (m, k), n = x.shape, w.shape[0]
     # where the tiles of w do not divide evenly over the SMs the kernel divides K among several blocks per
     # tile; their partial sums meet in scratch memory, a zeroed ticket per tile says who is last
     need = _skinny_scratch_floats(m, n, k)
     scratch = torch.empty(need, dtype=torch.float32, device=x.device) if need else None
     n_tickets = (n + 15) // 16 if need else 0        # a ticket per tile of weight rows; tiles have 16 rows or more
     tickets = _tickets(n_tickets, x.device) if need else None
-    _check(lib().ptb_skinny_linear(_ptr(x), _ptr(w), _ptr(bias), _ptr(add), _ptr(ybf), _ptr(yf), m, n, k,
-                                   x.stride(0) if m > 1 else k,
+    _check(lib().ptb_skinny_linear(_ptr(x), _ptr(w), _ptr(bias), _ptr(add), _ptr(ybf), _ptr(yf), 0 if ybf is None else ybf.shape[1],
+                                   m, n, k, x.stride(0) if m > 1 else k,
                                    ACTIVATIONS[act], _ptr(scratch), ctypes.c_size_t(need), _ptr(tickets),
                                    n_tickets, _stream(x)), "skinny_linear")
-    return y
 
 
 _skinny_scratch_cache = {}
@@ -1441,13 +1460,14 @@ def mlstm_chunks_takes(proj: torch.Tensor, dim: int, v_dim: int) -> bool:
 
 def mlstm(proj: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
           state: torch.Tensor, slots: torch.Tensor, batch: StepBatchC, heads: int, dim: int, v_dim: int,
-          q_scale: float, chunks=None) -> torch.Tensor:
+          q_scale: float, chunks=None, single_tokens: bool = False) -> torch.Tensor:
     """The matrix memory with exponential gates over the step's tokens, continuing and leaving each sequence's state.
     ``proj`` [tokens, >= 2 heads dim + heads v_dim] holds q, k, v side by side (rows may lie wider apart); ``gates``
     float32 [tokens, 2 heads] holds the input and forget gates' projections and is overwritten with the gates'
     logarithms ``cap tanh((g + b) / cap)`` and ``logsigmoid`` of the same; ``state`` [slots, >= mlstm_state_floats]
     float32. ``chunks``: (chunk_seq, chunk_q0, seq_chunk0, n_chunks) for the chunked form on the tensor cores (prompts;
-    ``mlstm_chunks_takes`` says whether it takes the projection), None for the token-by-token form. Returns float32
+    ``mlstm_chunks_takes`` says whether it takes the projection), None for the token-by-token form. ``single_tokens``: every
+    sequence brings one token; the walk forms the gates' logarithms itself (``gates`` stay as they are). Returns float32
     [tokens, heads * v_dim]: S^T q / (max(|n . q|, exp(-m)) + 1e-6)."""
     _need_cuda(gates, bias_i, bias_f, slots)
     _check_rows(proj, proj.shape, proj.dtype, "mlstm: proj")
@@ -1456,8 +1476,10 @@ def mlstm(proj: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor, bias_f:
         raise KernelError("mlstm: the gates are float32 [tokens, 2 * heads]")
     if state.dtype != torch.float32 or state.shape[1] < mlstm_state_floats(heads, dim, v_dim) or state.stride(1) != 1:
         raise KernelError("mlstm: the state is float32 [slots, >= mlstm_state_floats(heads, dim, v_dim)]")
-    _check(lib().ptb_mlstm_gates(_ptr(gates), _ptr(bias_i), _ptr(bias_f), n, heads, ctypes.c_float(cap), _stream(gates)),
-           "mlstm_gates")
+    single = bool(single_tokens) and chunks is None and n == batch.n_seqs
+    if not single:
+        _check(lib().ptb_mlstm_gates(_ptr(gates), _ptr(bias_i), _ptr(bias_f), n, heads, ctypes.c_float(cap), _stream(gates)),
+               "mlstm_gates")
     out = torch.empty((n, heads * v_dim), dtype=torch.float32, device=proj.device)
     if chunks is not None:
         if not mlstm_chunks_takes(proj, dim, v_dim):
@@ -1472,7 +1494,8 @@ def mlstm(proj: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor, bias_f:
         global launches
         launches += 2       # three kernels
         return out
-    _check(lib().ptb_mlstm_scan(_dtype_code(proj), _ptr(proj), proj.stride(0), _ptr(gates), _ptr(state), state.stride(0),
+    _check(lib().ptb_mlstm_scan(_dtype_code(proj), _ptr(proj), proj.stride(0), _ptr(gates), _ptr(bias_i if single else None),
+                                _ptr(bias_f if single else None), ctypes.c_float(cap), _ptr(state), state.stride(0),
                                 _ptr(slots), ctypes.byref(batch), _ptr(out), heads, dim, v_dim, ctypes.c_float(q_scale),
                                 _stream(proj)), "mlstm_scan")
     return out

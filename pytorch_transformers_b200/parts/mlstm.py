@@ -13,7 +13,8 @@ Prompts of 256 tokens or more run in chunks of 64 on the tensor cores where the 
 sum, the chunks joined in order, the outputs); shorter steps and decoding run token by token. Both carry the same
 running maximum m. Per sequence the mixer keeps S, n and m in the cache's state area (float32) and needs no pages. The gates'
 projections are a product of their own whose float32 sums stay unrounded; biases, cap, logarithms, decays, state,
-the division and the heads' norm are float32 whatever the model dtype. q, k, v and the output gate are one product.
+the division and the heads' norm are float32 whatever the model dtype. q, k, v and the output gate are one product; in steps of few rows the gates' rows are part of it
+(their sums stay float32), and a step of single tokens forms the gates' logarithms in the walk.
 """
 from __future__ import annotations
 
@@ -40,7 +41,7 @@ class MatrixMemory(Part):
             raise ValueError(f"the matrix memory's kernel takes keys of 1 to {build.kernels.MLSTM_MAX_DIM} entries, got {dim}")
         if SCAN_CHUNK != build.kernels.MLSTM_CHUNK:
             raise ValueError("the chunk planner and the chunked kernel disagree on the chunk's size")
-        self.p_in = self.p_gates = self.p_i_b = self.p_f_b = self.p_norm = self.p_o = None
+        self.w_all = self.p_in = self.p_gates = self.p_i_b = self.p_f_b = self.p_norm = self.p_o = None
 
     def param_decls(self) -> Dict[str, ParamDecl]:
         H, d, vd = self.heads, self.dim, self.vdim
@@ -54,8 +55,10 @@ class MatrixMemory(Part):
         return decls
 
     def bind(self, t: Dict[str, torch.Tensor]) -> None:
-        self.p_in = torch.cat([t["q"], t["k"], t["v"]] + ([t["g"]] if self.has_gate else [])).contiguous()
-        self.p_gates = torch.cat([t["i"], t["f"]]).contiguous()
+        rows = [t["q"], t["k"], t["v"]] + ([t["g"]] if self.has_gate else [])
+        # one matrix, so that a step of few rows reads both in one pass; two views for the products apart
+        self.w_all = torch.cat(rows + [t["i"], t["f"]]).contiguous()
+        self.p_in, self.p_gates = self.w_all[:-2 * self.heads], self.w_all[-2 * self.heads:]
         self.p_i_b, self.p_f_b, self.p_norm, self.p_o = t["i_b"], t["f_b"], t["norm"], t["o"]
 
     def cache_need(self):
@@ -80,14 +83,16 @@ class MatrixMemory(Part):
     def _heads(self, x, ctx, entry):
         k = self.build.kernels
         H, d, vd = self.heads, self.dim, self.vdim
-        proj = linear(k, x, self.p_in)
-        gates = linear(k, x, self.p_gates, wide_out=True)
+        if x.dtype == torch.bfloat16 and k.skinny_linear_preferred(x.shape[0], x.shape[1], self.w_all.shape[0]):
+            proj, gates = k.skinny_linear_split(x, self.w_all, self.p_in.shape[0])
+        else:
+            proj, gates = linear(k, x, self.p_in), linear(k, x, self.p_gates, wide_out=True)
         state = ctx.state_of(entry, self.state_need().numel)
         plan, chunks = ctx.plan(RecurrenceChunks.plan_key), None
         if plan.facts["n_chunks"] and k.mlstm_chunks_takes(proj, d, vd):
             # a long prompt in bfloat16 with sizes of the tensor-core kernels: chunks of 64 tokens in three passes
             chunks = (plan.dev["chunk_seq"], plan.dev["chunk_q0"], plan.dev["seq_chunk0"], plan.facts["n_chunks"])
         o = k.mlstm(proj, gates, self.p_i_b, self.p_f_b, self.gate_cap, state, ctx.dev["slots"], ctx.batch_c[0], H, d, vd,
-                    d ** -0.5, chunks)
+                    d ** -0.5, chunks, single_tokens=ctx.is_decode)
         gate = proj[:, 2 * H * d + H * vd:] if self.has_gate else None
         return k.head_norm_gate(o, self.p_norm, gate, H, self.eps, proj.dtype)

@@ -356,3 +356,26 @@ def test_expert_tiles(K, kind, width, inner, tile_rows):
         bound = (2.0 ** -8 * a.abs() + 1e-5) @ down[e].double().abs().T + 1e-5
         assert ((got[at].double() - a @ down[e].double().T).abs() <= bound).all(), (kind, e)
     K.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 32])
+@pytest.mark.parametrize("n,n_bf16,k", [(40, 8, 64), (8224, 8192, 2048), (50, 49, 4096), (10000, 9000, 256)])
+def test_skinny_linear_split(K, m, n, n_bf16, k):
+    """One pass over two matrices' rows: the first rounded, the others as float32 sums; borders inside a tile, K divided or not.
+    The same kernel's whole results in either type have the same sums, so the same bits."""
+    x, w = rnd(m, k, dtype=torch.bfloat16, seed=1), rnd(n, k, dtype=torch.bfloat16, scale=0.1, seed=2)
+    a, b = K.skinny_linear_split(x, w, n_bf16)
+    wide, rounded = K.skinny_linear(x, w, out_dtype=torch.float32), K.skinny_linear(x, w)
+    assert torch.equal(a, rounded[:, :n_bf16]) and torch.equal(b, wide[:, n_bf16:])
+
+
+@pytest.mark.parametrize("tokens,heads,kv,v_dim", [(1, 16, 4, 128), (5, 6, 3, 20), (700, 16, 4, 128), (2, 4, 1, 7)])
+def test_talk_mix(K, tokens, heads, kv, v_dim):
+    """Both forms (a thread an output, or four columns of a K/V group's heads) against float64."""
+    wide, talk = rnd(tokens, heads, kv, v_dim, seed=1), rnd(heads, heads, seed=2)
+    out = K.talk_mix(wide, talk, torch.float32).view(tokens, heads, v_dim)
+    own = torch.arange(heads, device="cuda") // (heads // kv)
+    per = wide.double()[:, :, own]                      # [tokens, g, h, v]: head g's weights on head h's values
+    ref = torch.einsum("hg,tghv->thv", talk.double(), per)
+    bound = heads * 2.0 ** -24 * torch.einsum("hg,tghv->thv", talk.double().abs(), per.abs()) + 1e-30
+    assert ((out.double() - ref).abs() <= bound).all()
