@@ -56,6 +56,7 @@ __global__ void split_rotate_store_kernel(const T* __restrict__ fused, T* __rest
                                           const float* __restrict__ rope_cos, const float* __restrict__ rope_sin,
                                           int rot_pairs, int kv_heads, int q_per_kv, int head_dim, int write_cache,
                                           int interleaved) {
+  pdl_entry();
   const int t = blockIdx.x;
   const int pos = sb.tok_pos[t];
   const int seq = sb.tok_seq[t];
@@ -177,6 +178,7 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, 
                          int kv_heads, int head_dim, float scale, int window, int v_dim,
                          const float* __restrict__ sinks, const T* __restrict__ gate, int gate_stride, float out_scale,
                          int out_stride, int keep_first, float* __restrict__ out_wide, float softcap, int gate_wide, int async) {
+  pdl_entry();
   extern __shared__ __align__(16) float smem[];
   const int kpitch = odd_words(head_dim), vpitch = odd_words(v_dim), kwords = (head_dim + 3) / 4;
   float* qs = smem;                                 // [BQ][kpitch], zeros beyond head_dim
@@ -405,6 +407,7 @@ __global__ void rope_norm_store_kernel(const T* __restrict__ proj, int stride, c
                                        T* __restrict__ v_keep, int write_cache, int pairs, int quads,
                                        const float* __restrict__ q_gain, const float* __restrict__ k_gain, int norm_first,
                                        float temp_coef, int temp_every) {
+  pdl_entry();
   extern __shared__ float rows[];   // per warp: a row of `dim` floats, then cos and sin of the rotated pairs
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int t = blockIdx.x, hh = blockIdx.y * (blockDim.x / 32) + warp;      // grid (tokens, groups of a block's warps)
@@ -533,6 +536,7 @@ __global__ void rope_norm_store_kernel(const T* __restrict__ proj, int stride, c
 template <typename T>
 __global__ void talk_mix_kernel(const float* __restrict__ wide, const float* __restrict__ talk, T* __restrict__ out,
                                 int out_stride, long long total, int heads, int kv_heads, int v_dim) {
+  pdl_entry();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int e = int(i % v_dim), h = int((i / v_dim) % heads);
@@ -550,6 +554,7 @@ __global__ void talk_mix_kernel(const float* __restrict__ wide, const float* __r
 template <typename T>
 __global__ void talk_mix_vec_kernel(const float* __restrict__ wide, const float* __restrict__ talk, T* __restrict__ out,
                                     int out_stride, long long total, int heads, int kv_heads, int v_dim) {
+  pdl_entry();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int quads = v_dim / 4, qpk = heads / kv_heads;
@@ -605,7 +610,7 @@ int launch_attention(const void* q, const void* k_pool, const void* v_pool, void
         return PTB_ERR_LAUNCH;                                                                                                  \
       configured = smem;                                                                                                        \
     }                                                                                                                           \
-    attention_generic_kernel<T, CC><<<grid, THREADS, smem, stream>>>(                                                           \
+    launch_pdl(attention_generic_kernel<T, CC>, grid, THREADS, smem, stream,                                                            \
         (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, sb, tile_seq, tile_q0, slopes, heads, kv_heads, head_dim,     \
         scale, window, v_dim, sinks, (const T*)gate, gate_stride, out_scale, out_stride, keep_first, out_wide, softcap,         \
         gate_wide, async);                                                                                                      \
@@ -624,6 +629,7 @@ int launch_attention(const void* q, const void* k_pool, const void* v_pool, void
 __global__ void rope_table_kernel(const int* __restrict__ tok_pos, const float* __restrict__ inv_freq,
                                   float* __restrict__ cos_out, float* __restrict__ sin_out, int n_tokens, int pairs,
                                   float factor) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_tokens * pairs) return;
   float s, c;
@@ -636,7 +642,7 @@ PTB_API int ptb_rope_table(const int* tok_pos, const float* inv_freq, float* cos
                            int pairs, float factor, cudaStream_t stream) {
   if (n_tokens <= 0 || pairs <= 0) return PTB_OK;
   const int total = n_tokens * pairs;
-  rope_table_kernel<<<(total + 255) / 256, 256, 0, stream>>>(tok_pos, inv_freq, cos_out, sin_out, n_tokens, pairs, factor);
+  launch_pdl(rope_table_kernel, (total + 255) / 256, 256, 0, stream, tok_pos, inv_freq, cos_out, sin_out, n_tokens, pairs, factor);
   return launch_status();
 }
 
@@ -651,11 +657,11 @@ PTB_API int ptb_split_rotate_store(int dtype, const void* fused, void* q_out, vo
   if ((rope_cos == nullptr) != (rope_sin == nullptr)) return PTB_ERR_SIZE;
   const int threads = 256;
   if (dtype == PTB_F32)
-    split_rotate_store_kernel<float><<<sb->n_tokens, threads, 0, stream>>>(
+    launch_pdl(split_rotate_store_kernel<float>, sb->n_tokens, threads, 0, stream, 
         (const float*)fused, (float*)q_out, (float*)k_pool, (float*)v_pool, *sb, inv_freq, rope_cos, rope_sin,
         rot_pairs, kv_heads, q_per_kv, head_dim, write_cache, interleaved);
   else if (dtype == PTB_BF16)
-    split_rotate_store_kernel<__nv_bfloat16><<<sb->n_tokens, threads, 0, stream>>>(
+    launch_pdl(split_rotate_store_kernel<__nv_bfloat16>, sb->n_tokens, threads, 0, stream, 
         (const __nv_bfloat16*)fused, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, *sb,
         inv_freq, rope_cos, rope_sin, rot_pairs, kv_heads, q_per_kv, head_dim, write_cache, interleaved);
   else
@@ -733,12 +739,12 @@ PTB_API int ptb_qk_prepare_store(int dtype, const void* proj, int stride, const 
                      (rot_pairs == 0 || (aligned16(rope_cos) && aligned16(rope_sin))))
                         ? 1 : 0;
   if (dtype == PTB_F32)
-    rope_norm_store_kernel<float><<<blocks, threads, smem, stream>>>(
+    launch_pdl(rope_norm_store_kernel<float>, blocks, threads, smem, stream, 
         (const float*)proj, stride, bias, (float*)q_out, (float*)k_pool, (float*)v_pool, *sb, rope_cos, rope_sin, rot_pairs,
         heads, kv_heads, dim, v_dim, eps, unit_norm, (const float*)v_first, v_first_stride, lam, (float*)v_keep, write_cache,
         pairs, quads, q_gain, k_gain, norm_first, temp_coef, temp_every);
   else if (dtype == PTB_BF16)
-    rope_norm_store_kernel<__nv_bfloat16><<<blocks, threads, smem, stream>>>(
+    launch_pdl(rope_norm_store_kernel<__nv_bfloat16>, blocks, threads, smem, stream, 
         (const __nv_bfloat16*)proj, stride, bias, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, *sb,
         rope_cos, rope_sin, rot_pairs, heads, kv_heads, dim, v_dim, eps, unit_norm, (const __nv_bfloat16*)v_first,
         v_first_stride, lam, (__nv_bfloat16*)v_keep, write_cache, pairs, quads, q_gain, k_gain, norm_first, temp_coef,
@@ -767,9 +773,9 @@ PTB_API int ptb_talk_mix(int dtype, const float* wide, const float* talk, void* 
     const long long total = (long long)n_tokens * kv_heads * (v_dim / 4);
     const unsigned blocks = unsigned((total + 127) / 128);
     if (dtype == PTB_F32)
-      talk_mix_vec_kernel<float><<<blocks, 128, 0, stream>>>(wide, talk, (float*)out, out_stride, total, heads, kv_heads, v_dim);
+      launch_pdl(talk_mix_vec_kernel<float>, blocks, 128, 0, stream, wide, talk, (float*)out, out_stride, total, heads, kv_heads, v_dim);
     else if (dtype == PTB_BF16)
-      talk_mix_vec_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(wide, talk, (__nv_bfloat16*)out, out_stride, total, heads,
+      launch_pdl(talk_mix_vec_kernel<__nv_bfloat16>, blocks, 128, 0, stream, wide, talk, (__nv_bfloat16*)out, out_stride, total, heads,
                                                                      kv_heads, v_dim);
     else
       return PTB_ERR_DTYPE;
@@ -778,9 +784,9 @@ PTB_API int ptb_talk_mix(int dtype, const float* wide, const float* talk, void* 
   const long long total = (long long)n_tokens * heads * v_dim;
   const unsigned blocks = unsigned((total + 255) / 256);
   if (dtype == PTB_F32)
-    talk_mix_kernel<float><<<blocks, 256, 0, stream>>>(wide, talk, (float*)out, out_stride, total, heads, kv_heads, v_dim);
+    launch_pdl(talk_mix_kernel<float>, blocks, 256, 0, stream, wide, talk, (float*)out, out_stride, total, heads, kv_heads, v_dim);
   else if (dtype == PTB_BF16)
-    talk_mix_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(wide, talk, (__nv_bfloat16*)out, out_stride, total, heads,
+    launch_pdl(talk_mix_kernel<__nv_bfloat16>, blocks, 256, 0, stream, wide, talk, (__nv_bfloat16*)out, out_stride, total, heads,
                                                                kv_heads, v_dim);
   else
     return PTB_ERR_DTYPE;

@@ -158,6 +158,39 @@ __device__ __forceinline__ void rotate_pair(float a, float b, float c, float s, 
   out_b = __fadd_rn(__fmul_rn(b, c), __fmul_rn(a, s));
 }
 
+// Programmatic dependent launch. A kernel launched by launch_pdl may get its blocks onto the SMs while the kernel before it in
+// the stream still runs (once all of that one's blocks have begun): the launch and the start of the blocks, one to
+// two microseconds that every kernel of a chain would pay, lie under its predecessor. pdl_entry, the first thing such a kernel does,
+// waits until the kernels before it have completed and their writes are seen, and only then lets the next one's blocks
+// in. Every block of every such kernel waits, so a kernel that has completed says that all before it have: the order of a
+// stream stays what it was, and a kernel launched the ordinary way begins after the completion of what is before it. Before
+// the wait nothing of memory is read or written.
+// Not under stream capture: the edges that a captured launch of this kind becomes made replayed steps slower (52 kernels a
+// step: 270 -> 291 us), where launches one after the other gain (mixture of experts, 8 tokens, 6 kernels: 131 -> 113 us;
+// matrix memory, 9 kernels: 168 -> 157; gated recurrence, 8: 166 -> 158).
+__device__ __forceinline__ void pdl_entry() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  bool captured = true;
+  if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess) captured = capture != cudaStreamCaptureStatusNone;
+  else (void)cudaGetLastError();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = captured ? 0 : 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // the status of the launch just made; a failure is said on stderr with the runtime's own words
 inline int launch_status() {
   const cudaError_t e = cudaGetLastError();

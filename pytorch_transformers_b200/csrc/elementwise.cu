@@ -15,6 +15,7 @@ static int grid_for(size_t total, int threads) {
 template <typename T>
 __global__ void gather_rows_kernel(const int* __restrict__ ids, const T* __restrict__ table, T* __restrict__ out,
                                    int width, int rows, int* status) {
+  pdl_entry();
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= rows) {
@@ -39,9 +40,9 @@ PTB_API int ptb_gather_rows(int dtype, const int* ids, const void* table, void* 
   if (n <= 0) return PTB_OK;
   if (width <= 0 || rows <= 0) return PTB_ERR_SIZE;
   if (dtype == PTB_F32)
-    gather_rows_kernel<float><<<n, 256, 0, stream>>>(ids, (const float*)table, (float*)out, width, rows, status);
+    launch_pdl(gather_rows_kernel<float>, n, 256, 0, stream, ids, (const float*)table, (float*)out, width, rows, status);
   else if (dtype == PTB_BF16)
-    gather_rows_kernel<__nv_bfloat16><<<n, 256, 0, stream>>>(ids, (const __nv_bfloat16*)table, (__nv_bfloat16*)out,
+    launch_pdl(gather_rows_kernel<__nv_bfloat16>, n, 256, 0, stream, ids, (const __nv_bfloat16*)table, (__nv_bfloat16*)out,
                                                              width, rows, status);
   else
     return PTB_ERR_DTYPE;
@@ -53,6 +54,7 @@ PTB_API int ptb_gather_rows(int dtype, const int* ids, const void* table, void* 
 template <typename T>
 __global__ void embed_rows_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out,
                                   int width, int rows, float scale, int* status) {
+  pdl_entry();
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= rows) {
@@ -84,9 +86,9 @@ PTB_API int ptb_embed_rows(int dtype, const int* ids, const void* table, float* 
   if (n <= 0) return PTB_OK;
   if (width <= 0 || rows <= 0) return PTB_ERR_SIZE;
   if (dtype == PTB_F32)
-    embed_rows_kernel<float><<<n, 256, 0, stream>>>(ids, (const float*)table, out, width, rows, scale, status);
+    launch_pdl(embed_rows_kernel<float>, n, 256, 0, stream, ids, (const float*)table, out, width, rows, scale, status);
   else if (dtype == PTB_BF16)
-    embed_rows_kernel<__nv_bfloat16><<<n, 256, 0, stream>>>(ids, (const __nv_bfloat16*)table, out, width, rows, scale, status);
+    launch_pdl(embed_rows_kernel<__nv_bfloat16>, n, 256, 0, stream, ids, (const __nv_bfloat16*)table, out, width, rows, scale, status);
   else
     return PTB_ERR_DTYPE;
   return launch_status();
@@ -106,6 +108,7 @@ __global__ void norm_kernel(const T* __restrict__ x, const T* __restrict__ adden
                             const float* __restrict__ gain1, const float* __restrict__ bias1,
                             T* __restrict__ y1, const float* __restrict__ gain2, const float* __restrict__ bias2,
                             T* __restrict__ y2, int width, float eps, int kind) {
+  pdl_entry();
   extern __shared__ float row[];
   __shared__ float scratch[32];
   const size_t base = size_t(blockIdx.x) * width;
@@ -208,6 +211,7 @@ norm_bf16_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
                      const float* __restrict__ bias1, __nv_bfloat16* __restrict__ y1,
                      const float* __restrict__ gain2, const float* __restrict__ bias2,
                      __nv_bfloat16* __restrict__ y2, int width, float eps, int kind) {
+  pdl_entry();
   __shared__ float scratch[32];
   const size_t base = size_t(blockIdx.x) * width;
   const int nvec = width / 8;
@@ -290,7 +294,7 @@ template <int VPT>
 void launch_norm_reg(const void* x, const void* addend, void* sum_out, const float* gain1, const float* bias1, void* y1,
                      const float* gain2, const float* bias2, void* y2, int n, int width, float eps, int kind,
                      cudaStream_t stream) {
-  norm_bf16_reg_kernel<VPT><<<n, NORM_REG_THREADS, 0, stream>>>(
+  launch_pdl(norm_bf16_reg_kernel<VPT>, n, NORM_REG_THREADS, 0, stream, 
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)addend, (__nv_bfloat16*)sum_out, gain1, bias1,
       (__nv_bfloat16*)y1, gain2, bias2, (__nv_bfloat16*)y2, width, eps, kind);
 }
@@ -323,7 +327,7 @@ PTB_API int ptb_norm(int dtype, const void* x, const void* addend, void* sum_out
       configured_f32 = smem;
     }
     if (e != cudaSuccess) return PTB_ERR_LAUNCH;
-    norm_kernel<float><<<n, threads, smem, stream>>>((const float*)x, (const float*)addend, (float*)sum_out, gain1,
+    launch_pdl(norm_kernel<float>, n, threads, smem, stream, (const float*)x, (const float*)addend, (float*)sum_out, gain1,
                                                      bias1, (float*)y1, gain2, bias2, (float*)y2, width, eps, kind);
   } else if (dtype == PTB_BF16) {
     if (smem > configured_bf16) {
@@ -331,7 +335,7 @@ PTB_API int ptb_norm(int dtype, const void* x, const void* addend, void* sum_out
       configured_bf16 = smem;
     }
     if (e != cudaSuccess) return PTB_ERR_LAUNCH;
-    norm_kernel<__nv_bfloat16><<<n, threads, smem, stream>>>(
+    launch_pdl(norm_kernel<__nv_bfloat16>, n, threads, smem, stream, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)addend, (__nv_bfloat16*)sum_out, gain1, bias1,
         (__nv_bfloat16*)y1, gain2, bias2, (__nv_bfloat16*)y2, width, eps, kind);
   } else {
@@ -346,6 +350,7 @@ PTB_API int ptb_norm(int dtype, const void* x, const void* addend, void* sum_out
 // y[r, c] = act(y[r, c] + bias[c]) in place (bias may be null).
 template <typename T>
 __global__ void bias_act_kernel(T* __restrict__ y, const float* __restrict__ bias, size_t total, int width, int act) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
     float v = to_f(y[i]);
@@ -434,6 +439,7 @@ template <bool FAST_GELU, bool BIAS>
 __global__ void __launch_bounds__(256)
 bias_act_bf16x8_kernel(uint4* __restrict__ y, const float* __restrict__ bias, size_t total8, unsigned words_per_row,
                        int act) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   for (; i + stride < total8; i += 2 * stride) {
@@ -447,8 +453,8 @@ template <bool FAST_GELU>
 void launch_bias_act_x8(void* y, const float* bias, size_t total8, int width, int act, cudaStream_t stream) {
   const int grid = grid_for(total8, 256);
   const unsigned words = unsigned(width / 8);
-  if (bias) bias_act_bf16x8_kernel<FAST_GELU, true><<<grid, 256, 0, stream>>>((uint4*)y, bias, total8, words, act);
-  else bias_act_bf16x8_kernel<FAST_GELU, false><<<grid, 256, 0, stream>>>((uint4*)y, bias, total8, words, act);
+  if (bias) launch_pdl(bias_act_bf16x8_kernel<FAST_GELU, true>, grid, 256, 0, stream, (uint4*)y, bias, total8, words, act);
+  else launch_pdl(bias_act_bf16x8_kernel<FAST_GELU, false>, grid, 256, 0, stream, (uint4*)y, bias, total8, words, act);
 }
 
 PTB_API int ptb_bias_act(int dtype, void* y, const float* bias, int rows, int width, int act, cudaStream_t stream) {
@@ -463,9 +469,9 @@ PTB_API int ptb_bias_act(int dtype, void* y, const float* bias, int rows, int wi
   const int threads = 256;
   const int blocks = grid_for(total, threads);
   if (dtype == PTB_F32)
-    bias_act_kernel<float><<<blocks, threads, 0, stream>>>((float*)y, bias, total, width, act);
+    launch_pdl(bias_act_kernel<float>, blocks, threads, 0, stream, (float*)y, bias, total, width, act);
   else if (dtype == PTB_BF16)
-    bias_act_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>((__nv_bfloat16*)y, bias, total, width, act);
+    launch_pdl(bias_act_kernel<__nv_bfloat16>, blocks, threads, 0, stream, (__nv_bfloat16*)y, bias, total, width, act);
   else
     return PTB_ERR_DTYPE;
   return launch_status();
@@ -475,6 +481,7 @@ PTB_API int ptb_bias_act(int dtype, void* y, const float* bias, int rows, int wi
 template <typename T>
 __global__ void residual_kernel(const T* __restrict__ x, const T* __restrict__ a, const T* __restrict__ b,
                                 T* __restrict__ out, size_t total) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
     float s = to_f(a[i]);
@@ -485,6 +492,7 @@ __global__ void residual_kernel(const T* __restrict__ x, const T* __restrict__ a
 
 __global__ void residual_bf16x8_kernel(const uint4* __restrict__ x, const uint4* __restrict__ a,
                                        const uint4* __restrict__ b, uint4* __restrict__ out, size_t total8) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total8; i += stride) {
     float fx[8], fa[8], fb[8];
@@ -505,17 +513,17 @@ PTB_API int ptb_residual(int dtype, const void* x, const void* a, const void* b,
                          cudaStream_t stream) {
   if (total <= 0) return PTB_OK;
   if (dtype == PTB_BF16 && total % 8 == 0 && aligned16(x) && aligned16(a) && aligned16(b) && aligned16(out)) {
-    residual_bf16x8_kernel<<<grid_for(size_t(total) / 8, 256), 256, 0, stream>>>(
+    launch_pdl(residual_bf16x8_kernel, grid_for(size_t(total) / 8, 256), 256, 0, stream, 
         (const uint4*)x, (const uint4*)a, (const uint4*)b, (uint4*)out, size_t(total) / 8);
     return launch_status();
   }
   const int threads = 256;
   const int blocks = grid_for(size_t(total), threads);
   if (dtype == PTB_F32)
-    residual_kernel<float><<<blocks, threads, 0, stream>>>((const float*)x, (const float*)a, (const float*)b,
+    launch_pdl(residual_kernel<float>, blocks, threads, 0, stream, (const float*)x, (const float*)a, (const float*)b,
                                                            (float*)out, size_t(total));
   else if (dtype == PTB_BF16)
-    residual_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)a,
+    launch_pdl(residual_kernel<__nv_bfloat16>, blocks, threads, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)a,
                                                                    (const __nv_bfloat16*)b, (__nv_bfloat16*)out,
                                                                    size_t(total));
   else
@@ -527,6 +535,7 @@ PTB_API int ptb_residual(int dtype, const void* x, const void* a, const void* b,
 // the logits, where an architecture has one)
 template <typename T>
 __global__ void scale_kernel(T* __restrict__ x, float factor, size_t total) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
     x[i] = from_f<T>(__fmul_rn(to_f(x[i]), factor));
@@ -536,9 +545,9 @@ PTB_API int ptb_scale(int dtype, void* x, float factor, long long total, cudaStr
   if (total <= 0) return PTB_OK;
   const int threads = 256;
   const int blocks = grid_for(size_t(total), threads);
-  if (dtype == PTB_F32) scale_kernel<float><<<blocks, threads, 0, stream>>>((float*)x, factor, size_t(total));
+  if (dtype == PTB_F32) launch_pdl(scale_kernel<float>, blocks, threads, 0, stream, (float*)x, factor, size_t(total));
   else if (dtype == PTB_BF16)
-    scale_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>((__nv_bfloat16*)x, factor, size_t(total));
+    launch_pdl(scale_kernel<__nv_bfloat16>, blocks, threads, 0, stream, (__nv_bfloat16*)x, factor, size_t(total));
   else return PTB_ERR_DTYPE;
   return launch_status();
 }
@@ -546,6 +555,7 @@ PTB_API int ptb_scale(int dtype, void* x, float factor, long long total, cudaStr
 // float32 copy of rows of any dtype: out[r, :] = float(x[r, :]) (logits of a bfloat16 head)
 template <typename T>
 __global__ void to_float_kernel(const T* __restrict__ x, float* __restrict__ out, size_t total) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) out[i] = to_f(x[i]);
 }
@@ -555,9 +565,9 @@ PTB_API int ptb_to_float(int dtype, const void* x, float* out, long long total, 
   const int threads = 256;
   const int blocks = grid_for(size_t(total), threads);
   if (dtype == PTB_F32)
-    to_float_kernel<float><<<blocks, threads, 0, stream>>>((const float*)x, out, size_t(total));
+    launch_pdl(to_float_kernel<float>, blocks, threads, 0, stream, (const float*)x, out, size_t(total));
   else if (dtype == PTB_BF16)
-    to_float_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>((const __nv_bfloat16*)x, out, size_t(total));
+    launch_pdl(to_float_kernel<__nv_bfloat16>, blocks, threads, 0, stream, (const __nv_bfloat16*)x, out, size_t(total));
   else
     return PTB_ERR_DTYPE;
   return launch_status();
@@ -565,6 +575,7 @@ PTB_API int ptb_to_float(int dtype, const void* x, float* out, long long total, 
 
 // x <- cap * tanh(x / cap), in place on float32 values (a soft limit on the logits)
 __global__ void softcap_kernel(float* __restrict__ x, float cap, size_t total) {
+  pdl_entry();
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) x[i] = cap * tanhf(x[i] / cap);
 }
@@ -572,7 +583,7 @@ __global__ void softcap_kernel(float* __restrict__ x, float cap, size_t total) {
 PTB_API int ptb_softcap(float* x, float cap, long long total, cudaStream_t stream) {
   if (total <= 0) return PTB_OK;
   if (!(cap > 0.f)) return PTB_ERR_SIZE;
-  softcap_kernel<<<grid_for(size_t(total), 256), 256, 0, stream>>>(x, cap, size_t(total));
+  launch_pdl(softcap_kernel, grid_for(size_t(total), 256), 256, 0, stream, x, cap, size_t(total));
   return launch_status();
 }
 
@@ -582,6 +593,7 @@ PTB_API int ptb_softcap(float* x, float cap, long long total, cudaStream_t strea
 template <typename T>
 __global__ void glu_clamp_kernel(const T* __restrict__ in, T* __restrict__ out, int rows, int f, float limit,
                                  float alpha) {
+  pdl_entry();
   const size_t total = size_t(rows) * f, stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
     const size_t r = i / f, c = i % f;
@@ -594,6 +606,7 @@ __global__ void glu_clamp_kernel(const T* __restrict__ in, T* __restrict__ out, 
 // the same for bfloat16 rows of whole 16-byte words: eight values a thread
 __global__ void glu_clamp_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int rows,
                                         int f, float limit, float alpha) {
+  pdl_entry();
   const int f8 = f / 8;
   const size_t total = size_t(rows) * f8, stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -615,15 +628,15 @@ PTB_API int ptb_glu_clamp(int dtype, const void* in, void* out, int rows, int f,
   if (rows <= 0) return PTB_OK;
   if (f <= 0) return PTB_ERR_SIZE;
   if (dtype == PTB_BF16 && f % 8 == 0 && aligned16(in) && aligned16(out)) {
-    glu_clamp_bf16x8_kernel<<<grid_for(size_t(rows) * (f / 8), 256), 256, 0, stream>>>(
+    launch_pdl(glu_clamp_bf16x8_kernel, grid_for(size_t(rows) * (f / 8), 256), 256, 0, stream, 
         (const __nv_bfloat16*)in, (__nv_bfloat16*)out, rows, f, limit, alpha);
     return launch_status();
   }
   const int blocks = grid_for(size_t(rows) * f, 256);
   if (dtype == PTB_F32)
-    glu_clamp_kernel<float><<<blocks, 256, 0, stream>>>((const float*)in, (float*)out, rows, f, limit, alpha);
+    launch_pdl(glu_clamp_kernel<float>, blocks, 256, 0, stream, (const float*)in, (float*)out, rows, f, limit, alpha);
   else if (dtype == PTB_BF16)
-    glu_clamp_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, rows, f,
+    launch_pdl(glu_clamp_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)in, (__nv_bfloat16*)out, rows, f,
                                                                 limit, alpha);
   else
     return PTB_ERR_DTYPE;
@@ -634,6 +647,7 @@ PTB_API int ptb_glu_clamp(int dtype, const void* in, void* out, int rows, int f,
 // out = act(gate) * up [rows, F], float32 arithmetic, rounded once.
 template <typename T>
 __global__ void glu_act_kernel(const T* __restrict__ in, T* __restrict__ out, int rows, int f, int act) {
+  pdl_entry();
   const size_t total = size_t(rows) * f, stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
     const size_t r = i / f, c = i % f;
@@ -644,6 +658,7 @@ __global__ void glu_act_kernel(const T* __restrict__ in, T* __restrict__ out, in
 // the same for bfloat16 rows of whole 16-byte words: eight values a thread
 __global__ void glu_act_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int rows, int f,
                                       int act) {
+  pdl_entry();
   const int f8 = f / 8;
   const size_t total = size_t(rows) * f8, stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -661,15 +676,15 @@ PTB_API int ptb_glu_act(int dtype, const void* in, void* out, int rows, int f, i
   if (rows <= 0) return PTB_OK;
   if (f <= 0 || !activation_known(act)) return PTB_ERR_SIZE;
   if (dtype == PTB_BF16 && f % 8 == 0 && aligned16(in) && aligned16(out)) {
-    glu_act_bf16x8_kernel<<<grid_for(size_t(rows) * (f / 8), 256), 256, 0, stream>>>((const __nv_bfloat16*)in,
+    launch_pdl(glu_act_bf16x8_kernel, grid_for(size_t(rows) * (f / 8), 256), 256, 0, stream, (const __nv_bfloat16*)in,
                                                                                       (__nv_bfloat16*)out, rows, f, act);
     return launch_status();
   }
   const int blocks = grid_for(size_t(rows) * f, 256);
   if (dtype == PTB_F32)
-    glu_act_kernel<float><<<blocks, 256, 0, stream>>>((const float*)in, (float*)out, rows, f, act);
+    launch_pdl(glu_act_kernel<float>, blocks, 256, 0, stream, (const float*)in, (float*)out, rows, f, act);
   else if (dtype == PTB_BF16)
-    glu_act_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, rows, f, act);
+    launch_pdl(glu_act_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)in, (__nv_bfloat16*)out, rows, f, act);
   else
     return PTB_ERR_DTYPE;
   return launch_status();

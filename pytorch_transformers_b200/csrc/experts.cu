@@ -36,6 +36,7 @@ template <typename T, int TPB, int EPW, bool VEC>
 __global__ void __launch_bounds__(32 * ROUTE_WARPS)
 route_logits_kernel(const T* __restrict__ h, const float* __restrict__ w_router, const float* __restrict__ bias,
                     float* __restrict__ z, int n_tokens, int width, int n, int n_bias) {
+  pdl_entry();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int t0 = blockIdx.x * TPB, e0 = (blockIdx.y * ROUTE_WARPS + warp) * EPW;
   if (e0 >= n) return;
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(32 * ROUTE_WARPS)
 route_select_kernel(const float* __restrict__ zs_all, const float* __restrict__ correction, int* __restrict__ ids,
                     float* __restrict__ gates, int n_tokens, int n, int n_groups, int keep, int top,
                     float route_scale, int score_kind, int z_stride, int group_top, int normalize) {
+  pdl_entry();
   extern __shared__ float sm[];   // per warp: n choice scores, n_groups group scores
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int t = blockIdx.x * ROUTE_WARPS + warp;
@@ -228,6 +230,7 @@ route_select_kernel(const float* __restrict__ zs_all, const float* __restrict__ 
 __global__ void __launch_bounds__(1024)
 expert_plan_kernel(const int* __restrict__ ids, int* __restrict__ plan, int pairs, int n_experts, int tile_rows,
                    int max_tiles) {
+  pdl_entry();
   extern __shared__ int si[];   // counts [n_experts], offsets [n_experts]
   int* count = si;
   int* offset = count + n_experts;
@@ -293,6 +296,7 @@ __global__ void __launch_bounds__(256)
 expert_linear_kernel(const T* __restrict__ x, const T* __restrict__ w, TO* __restrict__ out,
                      const int* __restrict__ plan, int pairs, int max_tiles, int top, int N, int K,
                      const float* __restrict__ row_scale, int act, float glu_limit, float glu_alpha) {
+  pdl_entry();
   constexpr int EBM = TM * 16;
   const int tile = blockIdx.y;
   if (tile >= plan[0]) return;
@@ -380,6 +384,7 @@ __global__ void expert_combine_kernel(const TB* __restrict__ base, const T* __re
                                       const float* __restrict__ gates, const int* __restrict__ row_of_pair,
                                       TB* __restrict__ out, int width, int top, const float* __restrict__ shared,
                                       const float* __restrict__ shared_gate, int shared_gate_stride) {
+  pdl_entry();
   const int t = blockIdx.x;
   // an expert that every token uses: its float32 rows times sigmoid(one logit per token), added last
   const float sg = shared ? (shared_gate ? 1.f / (1.f + expf(-shared_gate[size_t(t) * shared_gate_stride])) : 1.f) : 0.f;
@@ -411,6 +416,7 @@ __global__ void expert_combine_vec_kernel(const TB* __restrict__ base, const T* 
                                           const float* __restrict__ gates, const int* __restrict__ row_of_pair,
                                           TB* __restrict__ out, int width, int top, const float* __restrict__ shared,
                                           const float* __restrict__ shared_gate, int shared_gate_stride) {
+  pdl_entry();
   const int t = blockIdx.x;
   const float sg = shared ? (shared_gate ? 1.f / (1.f + expf(-shared_gate[size_t(t) * shared_gate_stride])) : 1.f) : 0.f;
   const size_t at0 = size_t(t) * width;
@@ -446,10 +452,10 @@ int launch_expert_linear(const void* x, const void* w, void* out, const int* pla
                          int N, int K, int tile_rows, const float* row_scale, int act, float glu_limit, float glu_alpha, cudaStream_t stream) {
   dim3 grid((N + EBN - 1) / EBN, max_tiles);
   if (tile_rows == 16)
-    expert_linear_kernel<T, TO, MODE, 1><<<grid, 256, 0, stream>>>((const T*)x, (const T*)w, (TO*)out, plan, pairs,
+    launch_pdl(expert_linear_kernel<T, TO, MODE, 1>, grid, 256, 0, stream, (const T*)x, (const T*)w, (TO*)out, plan, pairs,
                                                                    max_tiles, top, N, K, row_scale, act, glu_limit, glu_alpha);
   else if (tile_rows == 64)
-    expert_linear_kernel<T, TO, MODE, 4><<<grid, 256, 0, stream>>>((const T*)x, (const T*)w, (TO*)out, plan, pairs,
+    launch_pdl(expert_linear_kernel<T, TO, MODE, 4>, grid, 256, 0, stream, (const T*)x, (const T*)w, (TO*)out, plan, pairs,
                                                                    max_tiles, top, N, K, row_scale, act, glu_limit, glu_alpha);
   else
     return PTB_ERR_SIZE;
@@ -476,7 +482,7 @@ PTB_API int ptb_route_biased(int dtype, const void* h, const float* w_router, co
   dim3 grid((n_tokens + tpb - 1) / tpb, (n + extra + ROUTE_WARPS * epw - 1) / (ROUTE_WARPS * epw));
   const bool vec = width % 4 == 0 && aligned16(h) && aligned16(w_router);
 #define PTB_ROUTE2(TT, NTOK, NOUT, V)                                                                               \
-  route_logits_kernel<TT, NTOK, NOUT, V><<<grid, 32 * ROUTE_WARPS, 0, stream>>>((const TT*)h, w_router, bias, logits, \
+  launch_pdl(route_logits_kernel<TT, NTOK, NOUT, V>, grid, 32 * ROUTE_WARPS, 0, stream, (const TT*)h, w_router, bias, logits, \
                                                                                 n_tokens, width, n + extra, n)
 #define PTB_ROUTE(TT)                                              \
   do {                                                             \
@@ -493,7 +499,7 @@ PTB_API int ptb_route_biased(int dtype, const void* h, const float* w_router, co
   if (launch_status() != PTB_OK) return PTB_ERR_LAUNCH;
   const size_t smem = size_t(ROUTE_WARPS) * (n + n_groups) * sizeof(float);
 #define PTB_RS(VV)                                                                                                            \
-  route_select_kernel<VV><<<(n_tokens + ROUTE_WARPS - 1) / ROUTE_WARPS, 32 * ROUTE_WARPS, smem, stream>>>(                     \
+  launch_pdl(route_select_kernel<VV>, (n_tokens + ROUTE_WARPS - 1) / ROUTE_WARPS, 32 * ROUTE_WARPS, smem, stream,                      \
       logits, correction, ids, gates, n_tokens, n, n_groups, keep, top, route_scale, score_kind, n + extra, group_top, normalize)
   if (n <= 32) PTB_RS(1);
   else if (n <= 64) PTB_RS(2);
@@ -526,7 +532,7 @@ PTB_API int ptb_expert_plan(const int* ids, int* plan, int pairs, int n_experts,
   if (n_experts <= 0 || n_experts > 4000 || tile_rows <= 0 || max_tiles < pairs / tile_rows + (pairs < n_experts ? pairs : n_experts))
     return PTB_ERR_SIZE;
   const size_t smem = 2 * size_t(n_experts) * sizeof(int);
-  expert_plan_kernel<<<1, 1024, smem, stream>>>(ids, plan, pairs, n_experts, tile_rows, max_tiles);
+  launch_pdl(expert_plan_kernel, 1, 1024, smem, stream, ids, plan, pairs, n_experts, tile_rows, max_tiles);
   return launch_status();
 }
 
@@ -562,11 +568,11 @@ PTB_API int ptb_expert_combine_shared(int dtype, int out_dtype, const void* base
 #define PTB_EC(TT, TTB)                                                                                                         \
   do {                                                                                                                          \
     if (vec)                                                                                                                    \
-      expert_combine_vec_kernel<TT, TTB><<<grid, threads, 0, stream>>>((const TTB*)base, (const TT*)h, y, ids, gates,           \
+      launch_pdl(expert_combine_vec_kernel<TT, TTB>, grid, threads, 0, stream, (const TTB*)base, (const TT*)h, y, ids, gates,           \
                                                                        row_of_pair, (TTB*)out, width, top, shared, shared_gate, \
                                                                        shared_gate_stride);                                     \
     else                                                                                                                        \
-      expert_combine_kernel<TT, TTB><<<grid, threads, 0, stream>>>((const TTB*)base, (const TT*)h, y, ids, gates, row_of_pair,  \
+      launch_pdl(expert_combine_kernel<TT, TTB>, grid, threads, 0, stream, (const TTB*)base, (const TT*)h, y, ids, gates, row_of_pair,  \
                                                                    (TTB*)out, width, top, shared, shared_gate,                  \
                                                                    shared_gate_stride);                                         \
   } while (0)

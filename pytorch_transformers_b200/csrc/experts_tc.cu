@@ -74,6 +74,7 @@ struct ExpertTcParams {
 template <int MODE>
 __global__ void __launch_bounds__(64 + X_GATHER)
 expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertTcParams p) {
+  pdl_entry();
   const int tile = blockIdx.y;
   if (tile >= p.plan[0]) return;
   constexpr int BOXES = MODE == 0 ? 2 : 1;
@@ -261,7 +262,7 @@ int launch_expert_tc(const CUtensorMap& map, ExpertTcParams p, cudaStream_t stre
       return PTB_ERR_LAUNCH;
     configured = smem;
   }
-  expert_linear_tc_kernel<MODE><<<dim3((p.N + XM - 1) / XM, p.max_tiles), 64 + X_GATHER, smem, stream>>>(map, p);
+  launch_pdl(expert_linear_tc_kernel<MODE>, dim3((p.N + XM - 1) / XM, p.max_tiles), 64 + X_GATHER, smem, stream, map, p);
   return launch_status();
 }
 

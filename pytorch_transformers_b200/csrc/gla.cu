@@ -46,6 +46,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // z <- logsigmoid(z + bias) / tau: the logarithm of sigmoid(z + bias)^(1 / tau)
 __global__ void gla_decay_kernel(float* __restrict__ z, const float* __restrict__ bias, long long total, int width,
                                  float inv_tau) {
+  pdl_entry();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const float v = z[i] + (bias ? bias[i % width] : 0.f);
@@ -55,6 +56,7 @@ __global__ void gla_decay_kernel(float* __restrict__ z, const float* __restrict_
 // The same, four neighbouring values a thread (width a multiple of 4, rows at whole words): 2,900 x 2,048 values 12 us against 21
 __global__ void gla_decay_quad_kernel(float* __restrict__ z, const float* __restrict__ bias, long long quads, int width,
                                       float inv_tau) {
+  pdl_entry();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= quads) return;
   float4 v = reinterpret_cast<float4*>(z)[i];
@@ -85,6 +87,7 @@ gla_walk_kernel(const T* __restrict__ proj, int stride, const float* __restrict_
                 int state_stride, const int* __restrict__ slots, StepBatch sb, const int* __restrict__ chunk_seq,
                 const int* __restrict__ chunk_q0, float* __restrict__ sums, float* __restrict__ chunk_decay,
                 float* __restrict__ out, int heads, int dim_any, int v_dim, float q_scale, int role) {
+  pdl_entry();
   const int dim = DIMC > 0 ? DIMC : dim_any;
   constexpr int SB = walk_batch(ROWS, COLS);   // tokens of a batch
   constexpr int IT = SB * ROWS / 32;           // (token, channel) pairs a thread stages of each of q, k and the decays
@@ -337,6 +340,7 @@ template <int V>
 __global__ void gla_chunk_join_kernel(float* __restrict__ sums, const float* __restrict__ chunk_decay,
                                       float* __restrict__ state, int state_stride, const int* __restrict__ slots,
                                       StepBatch sb, const int* __restrict__ seq_chunk0, int heads, int dim, int v_dim) {
+  pdl_entry();
   const int seq = blockIdx.y;
   const size_t per_head = size_t(dim) * v_dim, per = per_head * heads;
   const size_t e = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * V;
@@ -381,7 +385,7 @@ int launch_walk(const void* proj, int stride, const float* log_decay, float* sta
   const int batch = walk_batch(rows, cols), pitch = (dim + 3) & ~3;
   const size_t smem = sizeof(float) * (size_t(3) * batch * pitch + size_t(batch) * VB * cols + size_t(batch) * warps * VB * cols);
 #define PTB_GLA(ROWS, COLS, DIMC)                                                                                        \
-  gla_walk_kernel<T, ROWS, COLS, DIMC><<<grid, 32 * warps, smem, stream>>>((const T*)proj, stride, log_decay, state,      \
+  launch_pdl(gla_walk_kernel<T, ROWS, COLS, DIMC>, grid, 32 * warps, smem, stream, (const T*)proj, stride, log_decay, state,      \
                                                                            state_stride, slots, sb, chunk_seq, chunk_q0,  \
                                                                            sums, chunk_decay, out, heads, dim, v_dim,     \
                                                                            q_scale, role)
@@ -422,9 +426,9 @@ PTB_API int ptb_gla_decay(float* z, const float* bias, int n, int width, float t
   if (width <= 0 || !(tau > 0.f)) return PTB_ERR_SIZE;
   const long long total = (long long)n * width;
   if (width % 4 == 0 && aligned16(z) && aligned16(bias))
-    gla_decay_quad_kernel<<<unsigned((total / 4 + 255) / 256), 256, 0, stream>>>(z, bias, total / 4, width, 1.f / tau);
+    launch_pdl(gla_decay_quad_kernel, unsigned((total / 4 + 255) / 256), 256, 0, stream, z, bias, total / 4, width, 1.f / tau);
   else
-    gla_decay_kernel<<<unsigned((total + 255) / 256), 256, 0, stream>>>(z, bias, total, width, 1.f / tau);
+    launch_pdl(gla_decay_kernel, unsigned((total + 255) / 256), 256, 0, stream, z, bias, total, width, 1.f / tau);
   return launch_status();
 }
 
@@ -476,10 +480,10 @@ PTB_API int ptb_gla_chunks(int dtype, const void* proj, int stride, const float*
     if (role == GLA_CHUNK_SUM) {
       const size_t per = size_t(heads) * dim * v_dim;
       if (v_dim % 4 == 0 && state_stride % 4 == 0 && aligned16(state) && aligned16(sums))
-        gla_chunk_join_kernel<4><<<dim3(unsigned((per / 4 + 127) / 128), sb->n_seqs), 128, 0, stream>>>(
+        launch_pdl(gla_chunk_join_kernel<4>, dim3(unsigned((per / 4 + 127) / 128), sb->n_seqs), 128, 0, stream, 
             sums, chunk_decay, state, state_stride, slots, *sb, seq_chunk0, heads, dim, v_dim);
       else
-        gla_chunk_join_kernel<1><<<dim3(unsigned((per + 255) / 256), sb->n_seqs), 256, 0, stream>>>(
+        launch_pdl(gla_chunk_join_kernel<1>, dim3(unsigned((per + 255) / 256), sb->n_seqs), 256, 0, stream, 
             sums, chunk_decay, state, state_stride, slots, *sb, seq_chunk0, heads, dim, v_dim);
       if (launch_status() != PTB_OK) return PTB_ERR_LAUNCH;
     }

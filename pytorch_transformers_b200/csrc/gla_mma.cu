@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(DK * 2)
 gla_chunk_sum_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, const float* __restrict__ log_decay, StepBatch sb,
                          const int* __restrict__ chunk_seq, const int* __restrict__ chunk_q0, float* __restrict__ sums,
                          float* __restrict__ chunk_decay, int heads) {
+  pdl_entry();
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* k_hi = sm;                       // [CH][DK] weighted keys, hi
   unsigned char* k_lo = k_hi + CH * DK * 2;       // lo
@@ -122,7 +123,7 @@ int launch_sum(const void* proj, int stride, const float* log_decay, const StepB
       return PTB_ERR_LAUNCH;
     configured = true;
   }
-  gla_chunk_sum_mma_kernel<DK, DV><<<dim3(n_chunks, heads), DK * 2, smem, stream>>>((const __nv_bfloat16*)proj, stride, log_decay, sb,
+  launch_pdl(gla_chunk_sum_mma_kernel<DK, DV>, dim3(n_chunks, heads), DK * 2, smem, stream, (const __nv_bfloat16*)proj, stride, log_decay, sb,
                                                                                    chunk_seq, chunk_q0, sums, chunk_decay, heads);
   return launch_status();
 }
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(256, 2)
 gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, const float* __restrict__ log_decay, StepBatch sb,
                          const int* __restrict__ chunk_seq, const int* __restrict__ chunk_q0, const float* __restrict__ before,
                          float* __restrict__ out, int heads, float q_scale) {
+  pdl_entry();
   using Shape = OutShape<DK, DV>;
   constexpr int LP = Shape::LP, NT = DV / 16;      // NT: n-tiles of 8 value columns that a warp owns
   extern __shared__ __align__(128) unsigned char sm[];
@@ -432,7 +434,7 @@ int launch_out(const void* proj, int stride, const float* log_decay, const StepB
       return PTB_ERR_LAUNCH;
     configured = true;
   }
-  gla_chunk_out_mma_kernel<DK, DV><<<dim3(n_chunks, heads), 256, smem, stream>>>((const __nv_bfloat16*)proj, stride, log_decay, sb,
+  launch_pdl(gla_chunk_out_mma_kernel<DK, DV>, dim3(n_chunks, heads), 256, smem, stream, (const __nv_bfloat16*)proj, stride, log_decay, sb,
                                                                                 chunk_seq, chunk_q0, before, out, heads, q_scale);
   return launch_status();
 }

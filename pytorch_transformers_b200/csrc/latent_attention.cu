@@ -28,6 +28,7 @@ __global__ void latent_store_kernel(const T* __restrict__ src, long long src_str
                                     float eps, T* __restrict__ pool, StepBatch sb, const float* __restrict__ rope_cos,
                                     const float* __restrict__ rope_sin, int rot_pairs, int interleaved, int rank,
                                     int rot_dim) {
+  pdl_entry();
   __shared__ float scratch[32];
   const int t = blockIdx.x;
   const int pos = sb.tok_pos[t], seq = sb.tok_seq[t];
@@ -74,6 +75,7 @@ latent_attention_kernel(const float* __restrict__ q_abs, const T* __restrict__ q
                         const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int rot_pairs,
                         int interleaved, int heads, int rank, int rot_dim, int tile_tokens, int heads_per_block,
                         float scale, int n_splits) {
+  pdl_entry();
   extern __shared__ float smem[];
   const int dk = rank + rot_dim, qstride = dk + 1, kstride = dk + 1;
   float* qs = smem;                       // [ROWS][dk + 1]
@@ -234,6 +236,7 @@ __global__ void __launch_bounds__(128)
 latent_join_kernel(const float* __restrict__ part, T* __restrict__ out, StepBatch sb,
                    const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, int heads,
                    int rank, int tile_tokens, int heads_per_block, int n_splits) {
+  pdl_entry();
   extern __shared__ float jw[];   // the splits' weights exp(m_s - m) / l
   const int tile = blockIdx.x, h0 = blockIdx.y * heads_per_block, r = blockIdx.z;
   const int seq = tile_seq[tile], q0 = tile_q0[tile];
@@ -311,12 +314,12 @@ int launch_latent(const float* q_abs, const void* q, long long q_stride, int q_d
   }
   const int chunks = (heads + heads_per_block - 1) / heads_per_block;
   dim3 grid(n_tiles, chunks, n_splits);
-  latent_attention_kernel<T, DPT><<<grid, THREADS, smem, stream>>>(
+  launch_pdl(latent_attention_kernel<T, DPT>, grid, THREADS, smem, stream, 
       q_abs, (const T*)q, q_stride, q_dim, q_rot_off, (const T*)pool, part, (T*)out, sb, tile_seq, tile_q0, rope_cos, rope_sin,
       rot_pairs, interleaved, heads, rank, rot_dim, tile_tokens, heads_per_block, scale, n_splits);
   int rc = launch_status();
   if (rc != PTB_OK || n_splits <= 1) return rc;
-  latent_join_kernel<T><<<dim3(n_tiles, chunks, ROWS), 128, n_splits * sizeof(float), stream>>>(
+  launch_pdl(latent_join_kernel<T>, dim3(n_tiles, chunks, ROWS), 128, n_splits * sizeof(float), stream, 
       part, (T*)out, sb, tile_seq, tile_q0, heads, rank, tile_tokens, heads_per_block, n_splits);
   return launch_status();
 }
@@ -356,11 +359,11 @@ PTB_API int ptb_latent_store(int dtype, const void* src, long long src_stride, c
   if (rank <= 0 || rot_dim < 0 || rot_pairs < 0 || 2 * rot_pairs > rot_dim) return PTB_ERR_SIZE;
   if (rot_pairs > 0 && (rope_cos == nullptr || rope_sin == nullptr)) return PTB_ERR_SIZE;
   if (dtype == PTB_F32)
-    latent_store_kernel<float><<<sb->n_tokens, 128, 0, stream>>>((const float*)src, src_stride, norm_w, eps,
+    launch_pdl(latent_store_kernel<float>, sb->n_tokens, 128, 0, stream, (const float*)src, src_stride, norm_w, eps,
                                                                  (float*)pool, *sb, rope_cos, rope_sin, rot_pairs,
                                                                  interleaved, rank, rot_dim);
   else if (dtype == PTB_BF16)
-    latent_store_kernel<__nv_bfloat16><<<sb->n_tokens, 128, 0, stream>>>(
+    launch_pdl(latent_store_kernel<__nv_bfloat16>, sb->n_tokens, 128, 0, stream, 
         (const __nv_bfloat16*)src, src_stride, norm_w, eps, (__nv_bfloat16*)pool, *sb, rope_cos, rope_sin, rot_pairs,
         interleaved, rank, rot_dim);
   else
@@ -421,6 +424,7 @@ latent_attention_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16
                             const int* __restrict__ tile_q0, const float* __restrict__ rope_cos,
                             const float* __restrict__ rope_sin, int rot_pairs, int interleaved, int heads, int rank,
                             int rot_dim, int tile_tokens, int heads_per_block, float scale, int n_splits) {
+  pdl_entry();
   extern __shared__ __align__(128) unsigned char msm[];
   constexpr int NT = MTHREADS * TG, QROWS = ROWS * TG;
   const int dk = rank + rot_dim;
@@ -679,13 +683,13 @@ int launch_latent_mma_tg(const float* q_abs, const void* q, long long q_stride, 
     configured = smem;
   }
   const int chunks = (heads + heads_per_block - 1) / heads_per_block;
-  latent_attention_mma_kernel<NF, TG, WIDE><<<dim3(n_tiles, chunks, n_splits), MTHREADS * TG, smem, stream>>>(
+  launch_pdl(latent_attention_mma_kernel<NF, TG, WIDE>, dim3(n_tiles, chunks, n_splits), MTHREADS * TG, smem, stream, 
       q_abs, (const __nv_bfloat16*)q, q_stride, q_dim, q_rot_off, (const __nv_bfloat16*)pool, part, (__nv_bfloat16*)out, sb,
       tile_seq, tile_q0, rope_cos, rope_sin, rot_pairs, interleaved, heads, rank, rot_dim, tile_tokens, heads_per_block,
       scale, n_splits);
   int rc = launch_status();
   if (rc != PTB_OK || n_splits <= 1) return rc;
-  latent_join_kernel<__nv_bfloat16><<<dim3(n_tiles, chunks, ROWS), 128, n_splits * sizeof(float), stream>>>(
+  launch_pdl(latent_join_kernel<__nv_bfloat16>, dim3(n_tiles, chunks, ROWS), 128, n_splits * sizeof(float), stream, 
       part, (__nv_bfloat16*)out, sb, tile_seq, tile_q0, heads, rank, tile_tokens, heads_per_block, n_splits);
   return launch_status();
 }
@@ -764,6 +768,7 @@ __global__ void latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, Ste
                                      const int* __restrict__ ctx_seq, const int* __restrict__ ctx_pos,
                                      __nv_bfloat16* __restrict__ c_rows, __nv_bfloat16* __restrict__ kr_rows, int rank,
                                      int rot_dim) {
+  pdl_entry();
   const int i = blockIdx.x, seq = ctx_seq[i], pos = ctx_pos[i];
   const int page = sb.pages[size_t(seq) * sb.pages_stride + pos / PTB_PAGE];
   const __nv_bfloat16* src = pool + kv_offset(page, 0, pos % PTB_PAGE, 1, rank + rot_dim);
@@ -782,6 +787,7 @@ __global__ void latent_unfold_kernel(const __nv_bfloat16* __restrict__ kv, const
                                      StepBatch sb, const int* __restrict__ ctx_seq, const int* __restrict__ ctx_pos,
                                      __nv_bfloat16* __restrict__ k_tmp, __nv_bfloat16* __restrict__ v_tmp, int heads,
                                      int dim, int rot_dim, int vdim, int hd, int hd_v) {
+  pdl_entry();
   typedef typename Word<V>::type W;
   const int i = blockIdx.x, seq = ctx_seq[i], pos = ctx_pos[i];
   const int page = sb.pages[size_t(seq) * sb.pages_stride + pos / PTB_PAGE], slot = pos % PTB_PAGE;
@@ -804,6 +810,7 @@ template <int V>
 __global__ void latent_q_unfold_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, const float* __restrict__ rope_cos,
                                        const float* __restrict__ rope_sin, int rot_pairs, int interleaved,
                                        __nv_bfloat16* __restrict__ out, int heads, int dim, int rot_dim, int hd) {
+  pdl_entry();
   typedef typename Word<V>::type W;
   const size_t t = blockIdx.x;
   const int dq = dim + rot_dim;
@@ -839,6 +846,7 @@ template <int V>
 __global__ void gate_heads_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ gate,
                                   long long gate_t, __nv_bfloat16* __restrict__ out, long long words, int heads, int vdim,
                                   int hd, int per_head) {
+  pdl_entry();
   typedef typename Word<V>::type W;
   const size_t stride = size_t(gridDim.x) * blockDim.x;
   const unsigned dv = unsigned(vdim / V);
@@ -863,7 +871,7 @@ PTB_API int ptb_latent_gather(const void* pool, const StepBatch* sb, const int* 
                               void* c_rows, void* kr_rows, int rank, int rot_dim, cudaStream_t stream) {
   if (n_ctx <= 0) return PTB_OK;
   if (rank <= 0 || rot_dim < 0) return PTB_ERR_SIZE;
-  latent_gather_kernel<<<n_ctx, 128, 0, stream>>>((const __nv_bfloat16*)pool, *sb, ctx_seq, ctx_pos, (__nv_bfloat16*)c_rows,
+  launch_pdl(latent_gather_kernel, n_ctx, 128, 0, stream, (const __nv_bfloat16*)pool, *sb, ctx_seq, ctx_pos, (__nv_bfloat16*)c_rows,
                                                   (__nv_bfloat16*)kr_rows, rank, rot_dim);
   return launch_status();
 }
@@ -876,7 +884,7 @@ PTB_API int ptb_latent_unfold(const void* kv, const void* kr_rows, const StepBat
   const bool words = dim % 8 == 0 && rot_dim % 8 == 0 && vdim % 8 == 0 && hd % 8 == 0 && hd_v % 8 == 0 && aligned16(kv) &&
                      aligned16(kr_rows) && aligned16(k_tmp) && aligned16(v_tmp);
 #define PTB_UNFOLD(V)                                                                                                  \
-  latent_unfold_kernel<V><<<n_ctx, 256, 0, stream>>>((const __nv_bfloat16*)kv, (const __nv_bfloat16*)kr_rows, *sb, ctx_seq, \
+  launch_pdl(latent_unfold_kernel<V>, n_ctx, 256, 0, stream, (const __nv_bfloat16*)kv, (const __nv_bfloat16*)kr_rows, *sb, ctx_seq, \
                                                      ctx_pos, (__nv_bfloat16*)k_tmp, (__nv_bfloat16*)v_tmp, heads, dim,    \
                                                      rot_dim, vdim, hd, hd_v)
   if (words) PTB_UNFOLD(8);
@@ -893,7 +901,7 @@ PTB_API int ptb_latent_q_unfold(const void* q, long long q_stride, const float* 
   if (rot_pairs > 0 && (rope_cos == nullptr || rope_sin == nullptr)) return PTB_ERR_SIZE;
   const bool words = dim % 8 == 0 && rot_dim % 8 == 0 && hd % 8 == 0 && q_stride % 8 == 0 && aligned16(q) && aligned16(out);
 #define PTB_QUNFOLD(V)                                                                                                   \
-  latent_q_unfold_kernel<V><<<n_tokens, 256, 0, stream>>>((const __nv_bfloat16*)q, q_stride, rope_cos, rope_sin, rot_pairs, \
+  launch_pdl(latent_q_unfold_kernel<V>, n_tokens, 256, 0, stream, (const __nv_bfloat16*)q, q_stride, rope_cos, rope_sin, rot_pairs, \
                                                           interleaved, (__nv_bfloat16*)out, heads, dim, rot_dim, hd)
   if (words) PTB_QUNFOLD(8);
   else PTB_QUNFOLD(1);
@@ -910,7 +918,7 @@ PTB_API int ptb_gate_heads(const void* o, const void* gate, long long gate_t, vo
   const size_t want = (size_t(n) + 255) / 256, most = size_t(sm_count()) * 16;
   const int blocks = int(want < most ? want : most);
 #define PTB_GATE(V)                                                                                                     \
-  gate_heads_kernel<V><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)gate, gate_t,          \
+  launch_pdl(gate_heads_kernel<V>, blocks, 256, 0, stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)gate, gate_t,          \
                                                    (__nv_bfloat16*)out, n, heads, vdim, hd, per_head)
   if (words) PTB_GATE(8);
   else PTB_GATE(1);

@@ -24,6 +24,7 @@ __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - l
 // logarithms of the input and forget gates of every (token, head): float32 [n, 2 heads] in place of the sums
 __global__ void mlstm_gates_kernel(float* __restrict__ gates, const float* __restrict__ bias_i, const float* __restrict__ bias_f,
                                    int n, int heads, float cap) {
+  pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * 2 * heads) return;
   const int col = i % (2 * heads);
@@ -43,6 +44,7 @@ mlstm_scan_kernel(const T* __restrict__ proj, int stride, const float* __restric
                   const float* __restrict__ bias_f, float cap, float* __restrict__ state,
                   int state_stride, const int* __restrict__ slots, StepBatch sb, float* __restrict__ out, int heads, int dim,
                   int v_dim, float q_scale) {
+  pdl_entry();
   __shared__ float qs[2][MAX_DIM], ks[2][MAX_DIM], vs[2][VB], red_o[2][WARPS][VB], red_n[2][WARPS];
   const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * VB;
   const int w = threadIdx.x / 32, lane = threadIdx.x % 32, tid = threadIdx.x;
@@ -141,6 +143,7 @@ template <typename T, typename TG>
 __global__ void head_norm_gate_kernel(const float* __restrict__ x, const float* __restrict__ gain, const TG* __restrict__ gate,
                                       int gate_stride, T* __restrict__ out, int out_stride, int n, int heads, int v_dim,
                                       float eps, int gate_silu) {
+  pdl_entry();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
   if (warp >= n * heads) return;
   const int t = warp / heads, h = warp % heads;
@@ -163,7 +166,7 @@ int launch_scan(const void* proj, int stride, const float* gates, const float* b
                 const StepBatch& sb, float* out, int heads, int dim, int v_dim, float q_scale, cudaStream_t stream) {
   dim3 grid(sb.n_seqs, heads, (v_dim + VB - 1) / VB);
 #define PTB_SCAN(ROWS)                                                                                                       \
-  mlstm_scan_kernel<T, ROWS><<<grid, VB * WARPS, 0, stream>>>((const T*)proj, stride, gates, bias_i, bias_f, cap, state, state_stride, slots, sb, \
+  launch_pdl(mlstm_scan_kernel<T, ROWS>, grid, VB * WARPS, 0, stream, (const T*)proj, stride, gates, bias_i, bias_f, cap, state, state_stride, slots, sb, \
                                                               out, heads, dim, v_dim, q_scale)
   if (dim <= 8 * WARPS)
     PTB_SCAN(8);
@@ -184,7 +187,7 @@ PTB_API int ptb_mlstm_gates(float* gates, const float* bias_i, const float* bias
   if (n <= 0) return PTB_OK;
   if (heads <= 0) return PTB_ERR_SIZE;
   const int total = n * 2 * heads;
-  mlstm_gates_kernel<<<(total + 255) / 256, 256, 0, stream>>>(gates, bias_i, bias_f, n, heads, cap);
+  launch_pdl(mlstm_gates_kernel, (total + 255) / 256, 256, 0, stream, gates, bias_i, bias_f, n, heads, cap);
   return launch_status();
 }
 
@@ -232,6 +235,7 @@ template <typename T, typename TG, int LANES>
 __global__ void head_norm_gate_vec_kernel(const float* __restrict__ x, const float* __restrict__ gain, const TG* __restrict__ gate,
                                           int gate_stride, T* __restrict__ out, int out_stride, int n, int heads, int v_dim,
                                           float eps, int gate_silu) {
+  pdl_entry();
   const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / LANES, e = threadIdx.x % LANES * 4;
   const bool on = unit < n * heads && e < v_dim;
   const int t = on ? unit / heads : 0, h = on ? unit % heads : 0, at = h * v_dim + e;
@@ -272,13 +276,13 @@ PTB_API int ptb_head_norm_gate_act(const float* x, const float* gain, int dtype,
 #define PTB_HNG(TT, TG)                                                                                                        \
   do {                                                                                                                         \
     if (vec && lanes == 32)                                                                                                    \
-      head_norm_gate_vec_kernel<TT, TG, 32><<<vec_blocks, threads, 0, stream>>>(x, gain, (const TG*)gate, gate_stride, (TT*)out, \
+      launch_pdl(head_norm_gate_vec_kernel<TT, TG, 32>, vec_blocks, threads, 0, stream, x, gain, (const TG*)gate, gate_stride, (TT*)out, \
                                                                                 out_stride, n, heads, v_dim, eps, gate_silu);  \
     else if (vec)                                                                                                              \
-      head_norm_gate_vec_kernel<TT, TG, 16><<<vec_blocks, threads, 0, stream>>>(x, gain, (const TG*)gate, gate_stride, (TT*)out, \
+      launch_pdl(head_norm_gate_vec_kernel<TT, TG, 16>, vec_blocks, threads, 0, stream, x, gain, (const TG*)gate, gate_stride, (TT*)out, \
                                                                                 out_stride, n, heads, v_dim, eps, gate_silu);  \
     else                                                                                                                       \
-      head_norm_gate_kernel<TT, TG><<<blocks, threads, 0, stream>>>(x, gain, (const TG*)gate, gate_stride, (TT*)out, out_stride, \
+      launch_pdl(head_norm_gate_kernel<TT, TG>, blocks, threads, 0, stream, x, gain, (const TG*)gate, gate_stride, (TT*)out, out_stride, \
                                                                     n, heads, v_dim, eps, gate_silu);                          \
   } while (0)
   if (dtype == PTB_F32 && gate_dtype == PTB_F32) PTB_HNG(float, float);

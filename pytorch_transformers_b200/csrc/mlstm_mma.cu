@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(DK * 2)
 mlstm_chunk_sum_kernel(const __nv_bfloat16* __restrict__ proj, int stride, const float* __restrict__ gates, StepBatch sb,
                        const int* __restrict__ chunk_seq, const int* __restrict__ chunk_q0, float* __restrict__ sums,
                        float* __restrict__ nsums, float* __restrict__ meta, int heads) {
+  pdl_entry();
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* k_hi = sm;                       // [CH][DK] weighted keys, hi
   unsigned char* k_lo = k_hi + CH * DK * 2;       // lo
@@ -151,6 +152,7 @@ mlstm_chunk_sum_kernel(const __nv_bfloat16* __restrict__ proj, int stride, const
 __global__ void mlstm_chunk_decay_kernel(float* __restrict__ meta, float* __restrict__ m_before, float* __restrict__ m_after,
                                          const float* __restrict__ state, int state_stride, const int* __restrict__ slots,
                                          StepBatch sb, const int* __restrict__ seq_chunk0, int heads, int dim, int v_dim) {
+  pdl_entry();
   const unsigned full = 0xffffffffu;
   const int seq = blockIdx.y, lane = threadIdx.x & 31;
   const int h = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -194,6 +196,7 @@ mlstm_chunk_join_kernel(float* __restrict__ sums, float* __restrict__ nsums, con
                         const float* __restrict__ m_after, float* __restrict__ state, int state_stride,
                         const int* __restrict__ slots, StepBatch sb, const int* __restrict__ seq_chunk0, int heads, int dim,
                         int v_dim) {
+  pdl_entry();
   const int seq = blockIdx.y;
   const size_t per_S = size_t(dim) * v_dim, per_head = per_S + dim;      // both multiples of 4
   const size_t e = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
@@ -258,6 +261,7 @@ mlstm_chunk_out_kernel(const __nv_bfloat16* __restrict__ proj, int stride, const
                        const int* __restrict__ chunk_seq, const int* __restrict__ chunk_q0, const float* __restrict__ before,
                        const float* __restrict__ n_before, const float* __restrict__ m_before, float* __restrict__ out,
                        int heads, float q_scale) {
+  pdl_entry();
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* q_s = sm;                          // [CH][DK]
   unsigned char* k_s = q_s + CH * DK * 2;           // [CH][DK]
@@ -437,7 +441,7 @@ int launch_sum(const void* proj, int stride, const float* gates, const StepBatch
       return PTB_ERR_LAUNCH;
     configured = true;
   }
-  mlstm_chunk_sum_kernel<DK, DV><<<dim3(n_chunks, heads), DK * 2, smem, stream>>>((const __nv_bfloat16*)proj, stride, gates, sb,
+  launch_pdl(mlstm_chunk_sum_kernel<DK, DV>, dim3(n_chunks, heads), DK * 2, smem, stream, (const __nv_bfloat16*)proj, stride, gates, sb,
                                                                                  chunk_seq, chunk_q0, sums, nsums, meta, heads);
   return launch_status();
 }
@@ -453,7 +457,7 @@ int launch_out(const void* proj, int stride, const float* gates, const StepBatch
       return PTB_ERR_LAUNCH;
     configured = true;
   }
-  mlstm_chunk_out_kernel<DK, DV><<<dim3(n_chunks, heads), 256, smem, stream>>>((const __nv_bfloat16*)proj, stride, gates, sb, chunk_seq,
+  launch_pdl(mlstm_chunk_out_kernel<DK, DV>, dim3(n_chunks, heads), 256, smem, stream, (const __nv_bfloat16*)proj, stride, gates, sb, chunk_seq,
                                                                               chunk_q0, sums, nsums, m_before, out, heads, q_scale);
   return launch_status();
 }
@@ -494,12 +498,12 @@ PTB_API int ptb_mlstm_chunks(const void* proj, int stride, const float* gates, f
   do {                                                                                                                          \
     rc = launch_sum<DK, DV>(proj, stride, gates, *sb, chunk_seq, chunk_q0, n_chunks, sums, nsums, meta, heads, stream);         \
     if (rc != PTB_OK) return rc;                                                                                                \
-    mlstm_chunk_decay_kernel<<<dim3(unsigned((heads + 3) / 4), sb->n_seqs), 128, 0, stream>>>(                                  \
+    launch_pdl(mlstm_chunk_decay_kernel, dim3(unsigned((heads + 3) / 4), sb->n_seqs), 128, 0, stream,                                   \
         meta, m_before, m_after, state, state_stride, slots, *sb, seq_chunk0, heads, DK, DV);                                   \
     rc = launch_status();                                                                                                       \
     if (rc != PTB_OK) return rc;                                                                                                \
     const size_t per = size_t(heads) * (size_t(DK) * DV + DK) / 4;                                                              \
-    mlstm_chunk_join_kernel<<<dim3(unsigned((per + 127) / 128), sb->n_seqs), 128, 0, stream>>>(                                 \
+    launch_pdl(mlstm_chunk_join_kernel, dim3(unsigned((per + 127) / 128), sb->n_seqs), 128, 0, stream,                                  \
         sums, nsums, meta, m_after, state, state_stride, slots, *sb, seq_chunk0, heads, DK, DV);                                \
     rc = launch_status();                                                                                                       \
     if (rc != PTB_OK) return rc;                                                                                                \

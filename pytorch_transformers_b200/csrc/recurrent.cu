@@ -22,6 +22,7 @@ __global__ void rglru_conv_kernel(const T* __restrict__ proj, const float* __res
                                   const float* __restrict__ conv_b, const float* __restrict__ state,
                                   long long state_stride, const int* __restrict__ slots, StepBatch sb,
                                   T* __restrict__ y_act, T* __restrict__ u, int R, int taps) {
+  pdl_entry();
   const size_t total = size_t(sb.n_tokens) * R, stride = size_t(gridDim.x) * blockDim.x;
   for (size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += stride) {
     const int t = int(idx / R), c = int(idx % R);
@@ -76,6 +77,7 @@ __global__ void rglru_conv_run_kernel(const T* __restrict__ proj, const float* _
                                       const float* __restrict__ conv_w, const float* __restrict__ conv_b,
                                       const float* __restrict__ state, long long state_stride, const int* __restrict__ slots,
                                       StepBatch sb, T* __restrict__ y_act, T* __restrict__ u, int R, int taps) {
+  pdl_entry();
   const int quads = R / 4;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int c = int(idx % quads) * 4;
@@ -151,6 +153,7 @@ __global__ void rglru_scan_kernel(const float* __restrict__ gates, const T* __re
                                   const T* __restrict__ proj, const float* __restrict__ bx, float* __restrict__ state,
                                   long long state_stride, const int* __restrict__ slots, StepBatch sb,
                                   T* __restrict__ out, int R, int bw, int taps, float c_decay) {
+  pdl_entry();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= sb.n_seqs * R) return;
   const int seq = idx / R, c = idx % R;
@@ -202,6 +205,7 @@ __global__ void rglru_chunk_kernel(float* __restrict__ gates, const float* __res
                                    int chunk_len, float* __restrict__ agg_a, float* __restrict__ agg_b,
                                    float* __restrict__ s_start, T* __restrict__ out, int R, int bw, int taps,
                                    float c_decay) {
+  pdl_entry();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= R) return;
   const int len = (chunk_len + SPLIT - 1) / SPLIT;
@@ -285,7 +289,7 @@ int launch_rglru_chunks(float* gates, const float* gates_b, const void* u, const
   float *agg_a = work, *agg_b = work + per, *s_start = work + 2 * per;
   const int threads = 128, gx = (R + threads - 1) / threads;
 #define PTB_CHUNK_PASS(P, GY)                                                                                       \
-  rglru_chunk_kernel<T, P, RAW><<<dim3(gx, GY), threads, 0, stream>>>(                                               \
+  launch_pdl(rglru_chunk_kernel<T, P, RAW>, dim3(gx, GY), threads, 0, stream,                                                \
       gates, gates_b, (const T*)u, (const T*)y_act, lam, (const T*)proj, bx, state, state_stride, slots, sb, chunk_seq, chunk_q0, \
       seq_chunk0, n_chunks, chunk_len, agg_a, agg_b, s_start, (T*)out, R, bw, taps, c_decay)
   PTB_CHUNK_PASS(1, n_chunks * SPLIT);
@@ -307,6 +311,7 @@ __global__ void __launch_bounds__(256)
 block_linear_kernel(const T* __restrict__ x, long long xt, long long xg, const T* __restrict__ w,
                     const float* __restrict__ bias, TO* __restrict__ y, const T* __restrict__ gate, long long gate_t,
                     int gate_g, int gate_n, int M, int G, int N, int K, int act) {
+  pdl_entry();
   __shared__ float xs[BK][BM + 4];
   __shared__ float ws[BK][BN + 4];
   const int tid = threadIdx.x, g = blockIdx.z;
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(SKINNY_THREADS)
 block_linear_skinny_kernel(const T* __restrict__ x, long long xt, long long xg, const T* __restrict__ w,
                            const float* __restrict__ bias, TO* __restrict__ y, const T* __restrict__ gate,
                            long long gate_t, int gate_g, int gate_n, int M, int G, int N, int K, int act, int vec) {
+  pdl_entry();
   const int lane = threadIdx.x % LANES;
   const int per_group = (N + SKINNY_R - 1) / SKINNY_R;
   const long long item = ((long long)blockIdx.x * SKINNY_THREADS + threadIdx.x) / LANES;
@@ -465,6 +471,7 @@ __global__ void __launch_bounds__(128)
 block_linear_mma_kernel(const __nv_bfloat16* __restrict__ x, long long xt, long long xg, const __nv_bfloat16* __restrict__ w,
                         const float* __restrict__ bias, TO* __restrict__ y, const __nv_bfloat16* __restrict__ gate,
                         long long gate_t, int gate_g, int gate_n, int M, int G, int N, int K, int act) {
+  pdl_entry();
   const int lane = threadIdx.x % 32, quad = lane % 4;
   const int tiles = (N + 7) / 8;
   const long long item = (long long)blockIdx.x * 4 + threadIdx.x / 32;
@@ -505,8 +512,8 @@ int launch_block_skinny(const void* x, long long xt, long long xg, const void* w
                         cudaStream_t stream) {
   const long long items = (long long)G * ((N + SKINNY_R - 1) / SKINNY_R);
 #define PTB_BLS(LANES)                                                                                                     \
-  block_linear_skinny_kernel<T, TO, LANES, MT><<<int((items * LANES + SKINNY_THREADS - 1) / SKINNY_THREADS), SKINNY_THREADS, \
-                                                 0, stream>>>((const T*)x, xt, xg, (const T*)w, bias, (TO*)y, (const T*)gate, \
+  launch_pdl(block_linear_skinny_kernel<T, TO, LANES, MT>, int((items * LANES + SKINNY_THREADS - 1) / SKINNY_THREADS), SKINNY_THREADS, \
+                                                 0, stream, (const T*)x, xt, xg, (const T*)w, bias, (TO*)y, (const T*)gate, \
                                                               gate_t, gate_g, gate_n, M, G, N, K, act, vec)
   if (K <= 128) PTB_BLS(4);
   else if (K <= 256) PTB_BLS(8);
@@ -520,6 +527,7 @@ int launch_block_skinny(const void* x, long long xt, long long xg, const void* w
 template <typename TI, typename TO, typename TG>
 __global__ void block_epilogue_kernel(const TI* __restrict__ z, const float* __restrict__ bias, const TG* __restrict__ gate,
                                       long long gate_t, int gate_g, int gate_n, TO* __restrict__ y, int M, int G, int N, int act) {
+  pdl_entry();
   const size_t total = size_t(M) * G * N, stride = size_t(gridDim.x) * blockDim.x;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
     const int n = int(i % N), g = int((i / N) % G), m = int(i / (size_t(N) * G));
@@ -536,6 +544,7 @@ __global__ void block_epilogue_kernel(const TI* __restrict__ z, const float* __r
 template <typename TI, typename TO>
 __global__ void block_epilogue_quad_kernel(const TI* __restrict__ z, const float* __restrict__ bias, TO* __restrict__ y, int M, int G,
                                            int N, int act) {
+  pdl_entry();
   const int quads = N / 4;
   const size_t total = size_t(M) * G * quads, i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -559,7 +568,7 @@ PTB_API int ptb_block_epilogue(int in_dtype, int out_dtype, const void* z, const
   typedef __nv_bfloat16 bf;
   if (gate == nullptr && N % 4 == 0 && aligned16(z) && aligned16(y) && aligned16(bias)) {
     const unsigned quad_blocks = unsigned((total / 4 + 255) / 256);
-#define PTB_BEQ(TI, TO) block_epilogue_quad_kernel<TI, TO><<<quad_blocks, 256, 0, stream>>>((const TI*)z, bias, (TO*)y, M, G, N, act)
+#define PTB_BEQ(TI, TO) launch_pdl(block_epilogue_quad_kernel<TI, TO>, quad_blocks, 256, 0, stream, (const TI*)z, bias, (TO*)y, M, G, N, act)
     if (in_dtype == PTB_F32 && out_dtype == PTB_F32) PTB_BEQ(float, float);
     else if (in_dtype == PTB_F32 && out_dtype == PTB_BF16) PTB_BEQ(float, bf);
     else if (in_dtype == PTB_BF16 && out_dtype == PTB_BF16) PTB_BEQ(bf, bf);
@@ -569,13 +578,13 @@ PTB_API int ptb_block_epilogue(int in_dtype, int out_dtype, const void* z, const
     return launch_status();
   }
   if (in_dtype == PTB_F32 && out_dtype == PTB_F32)
-    block_epilogue_kernel<float, float, bf><<<blocks, 256, 0, stream>>>((const float*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (float*)y, M, G, N, act);
+    launch_pdl(block_epilogue_kernel<float, float, bf>, blocks, 256, 0, stream, (const float*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (float*)y, M, G, N, act);
   else if (in_dtype == PTB_F32 && out_dtype == PTB_BF16)
-    block_epilogue_kernel<float, bf, bf><<<blocks, 256, 0, stream>>>((const float*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (bf*)y, M, G, N, act);
+    launch_pdl(block_epilogue_kernel<float, bf, bf>, blocks, 256, 0, stream, (const float*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (bf*)y, M, G, N, act);
   else if (in_dtype == PTB_BF16 && out_dtype == PTB_BF16)
-    block_epilogue_kernel<bf, bf, bf><<<blocks, 256, 0, stream>>>((const bf*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (bf*)y, M, G, N, act);
+    launch_pdl(block_epilogue_kernel<bf, bf, bf>, blocks, 256, 0, stream, (const bf*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (bf*)y, M, G, N, act);
   else if (in_dtype == PTB_BF16 && out_dtype == PTB_F32)
-    block_epilogue_kernel<bf, float, bf><<<blocks, 256, 0, stream>>>((const bf*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (float*)y, M, G, N, act);
+    launch_pdl(block_epilogue_kernel<bf, float, bf>, blocks, 256, 0, stream, (const bf*)z, bias, (const bf*)gate, gate_t, gate_g, gate_n, (float*)y, M, G, N, act);
   else
     return PTB_ERR_DTYPE;
   return launch_status();
@@ -593,7 +602,7 @@ PTB_API int ptb_rglru_conv(int dtype, const void* proj, const float* by, const f
     const long long runs = (sb->n_tokens + CONV_RUN - 1) / CONV_RUN;
     const unsigned run_blocks = unsigned((runs * (R / 4) + 127) / 128);
 #define PTB_RC(TT, MM)                                                                                                          \
-  rglru_conv_run_kernel<TT, MM><<<run_blocks, 128, 0, stream>>>((const TT*)proj, by, bx, conv_w, conv_b, state, state_stride, slots, \
+  launch_pdl(rglru_conv_run_kernel<TT, MM>, run_blocks, 128, 0, stream, (const TT*)proj, by, bx, conv_w, conv_b, state, state_stride, slots, \
                                                                 *sb, (TT*)y_act, (TT*)u, R, taps)
     if (dtype == PTB_F32) { if (taps <= 4) PTB_RC(float, 4); else PTB_RC(float, MAX_TAPS); }
     else if (dtype == PTB_BF16) { if (taps <= 4) PTB_RC(__nv_bfloat16, 4); else PTB_RC(__nv_bfloat16, MAX_TAPS); }
@@ -602,10 +611,10 @@ PTB_API int ptb_rglru_conv(int dtype, const void* proj, const float* by, const f
     return launch_status();
   }
   if (dtype == PTB_F32)
-    rglru_conv_kernel<float><<<blocks, 256, 0, stream>>>((const float*)proj, by, bx, conv_w, conv_b, state,
+    launch_pdl(rglru_conv_kernel<float>, blocks, 256, 0, stream, (const float*)proj, by, bx, conv_w, conv_b, state,
                                                          state_stride, slots, *sb, (float*)y_act, (float*)u, R, taps);
   else if (dtype == PTB_BF16)
-    rglru_conv_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)proj, by, bx, conv_w, conv_b,
+    launch_pdl(rglru_conv_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)proj, by, bx, conv_w, conv_b,
                                                                  state, state_stride, slots, *sb,
                                                                  (__nv_bfloat16*)y_act, (__nv_bfloat16*)u, R, taps);
   else
@@ -623,11 +632,11 @@ PTB_API int ptb_rglru_scan(int dtype, const float* gates, const void* u, const v
   const int total = sb->n_seqs * R;
   const int threads = 128, grid = (total + threads - 1) / threads;
   if (dtype == PTB_F32)
-    rglru_scan_kernel<float><<<grid, threads, 0, stream>>>(gates, (const float*)u, (const float*)y_act, lam,
+    launch_pdl(rglru_scan_kernel<float>, grid, threads, 0, stream, gates, (const float*)u, (const float*)y_act, lam,
                                                            (const float*)proj, bx, state, state_stride, slots, *sb,
                                                            (float*)out, R, bw, taps, c_decay);
   else if (dtype == PTB_BF16)
-    rglru_scan_kernel<__nv_bfloat16><<<grid, threads, 0, stream>>>(
+    launch_pdl(rglru_scan_kernel<__nv_bfloat16>, grid, threads, 0, stream, 
         gates, (const __nv_bfloat16*)u, (const __nv_bfloat16*)y_act, lam, (const __nv_bfloat16*)proj, bx, state,
         state_stride, slots, *sb, (__nv_bfloat16*)out, R, bw, taps, c_decay);
   else
@@ -672,9 +681,9 @@ PTB_API int ptb_block_linear(int dtype, int out_dtype, const void* x, long long 
     const dim3 mgrid(unsigned(((long long)G * ((N + 7) / 8) + 3) / 4), (M + 15) / 16);
     if (mgrid.y > 65535) return PTB_ERR_SIZE;
     if (out_dtype == PTB_F32)
-      block_linear_mma_kernel<float><<<mgrid, 128, 0, stream>>>((const bf*)x, xt, xg, (const bf*)w, bias, (float*)y, (const bf*)gate, gate_t, gate_g, gate_n, M, G, N, K, act);
+      launch_pdl(block_linear_mma_kernel<float>, mgrid, 128, 0, stream, (const bf*)x, xt, xg, (const bf*)w, bias, (float*)y, (const bf*)gate, gate_t, gate_g, gate_n, M, G, N, K, act);
     else if (out_dtype == PTB_BF16)
-      block_linear_mma_kernel<bf><<<mgrid, 128, 0, stream>>>((const bf*)x, xt, xg, (const bf*)w, bias, (bf*)y, (const bf*)gate, gate_t, gate_g, gate_n, M, G, N, K, act);
+      launch_pdl(block_linear_mma_kernel<bf>, mgrid, 128, 0, stream, (const bf*)x, xt, xg, (const bf*)w, bias, (bf*)y, (const bf*)gate, gate_t, gate_g, gate_n, M, G, N, K, act);
     else
       return PTB_ERR_DTYPE;
     return launch_status();
@@ -691,14 +700,14 @@ PTB_API int ptb_block_linear(int dtype, int out_dtype, const void* x, long long 
     return PTB_ERR_DTYPE;
   }
   if (dtype == PTB_F32 && out_dtype == PTB_F32)
-    block_linear_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)x, xt, xg, (const float*)w, bias,
+    launch_pdl(block_linear_kernel<float, float>, grid, 256, 0, stream, (const float*)x, xt, xg, (const float*)w, bias,
                                                                 (float*)y, (const float*)gate, gate_t, gate_g, gate_n, M, G, N, K, act);
   else if (dtype == PTB_BF16 && out_dtype == PTB_F32)
-    block_linear_kernel<__nv_bfloat16, float><<<grid, 256, 0, stream>>>(
+    launch_pdl(block_linear_kernel<__nv_bfloat16, float>, grid, 256, 0, stream, 
         (const __nv_bfloat16*)x, xt, xg, (const __nv_bfloat16*)w, bias, (float*)y, (const __nv_bfloat16*)gate, gate_t,
         gate_g, gate_n, M, G, N, K, act);
   else if (dtype == PTB_BF16 && out_dtype == PTB_BF16)
-    block_linear_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(
+    launch_pdl(block_linear_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, stream, 
         (const __nv_bfloat16*)x, xt, xg, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)y, (const __nv_bfloat16*)gate,
         gate_t, gate_g, gate_n, M, G, N, K, act);
   else

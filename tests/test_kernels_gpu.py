@@ -379,3 +379,41 @@ def test_talk_mix(K, tokens, heads, kv, v_dim):
     ref = torch.einsum("hg,tghv->thv", talk.double(), per)
     bound = heads * 2.0 ** -24 * torch.einsum("hg,tghv->thv", talk.double().abs(), per.abs()) + 1e-30
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("width", [8, 1000, 4544])
+def test_chain_of_launches_keeps_the_streams_order(K, width):
+    """Kernels that may be placed while their predecessor still runs, one after the other on two buffers, each reading
+    what the last one wrote and writing what it read, with a copy and an ordinary launch between: the same bits as with a
+    synchronisation after each, as on the default stream, and as a replayed graph. Rows enough for several waves."""
+    n, rounds = 3000, 6
+    x0, gain, other = rnd(n, width, seed=1), 1 + rnd(width, scale=0.1, seed=2), rnd(n, width, seed=3)
+
+    def chain(x, wait):
+        for i in range(rounds):
+            y = K.norm(x, gain, None, 1e-6, "rmsnorm")
+            wait()
+            K.scale_(x, 0.5)                # x after its reader
+            wait()
+            x.copy_(K.residual(x, y, other))
+            wait()
+            z = K.bias_act_(y, gain, "gelu")    # y after its readers
+            wait()
+            x.add_(z)                       # an ordinary launch
+            wait()
+        return K.to_float(x)
+
+    want = chain(x0.clone(), torch.cuda.synchronize)
+    assert torch.equal(chain(x0.clone(), lambda: None), want)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert torch.equal(chain(x0.clone(), lambda: None), want)
+    torch.cuda.current_stream().wait_stream(side)
+    x, graph = x0.clone(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(x, lambda: None)
+    for _ in range(2):
+        x.copy_(x0)
+        graph.replay()
+        assert torch.equal(got, want)
