@@ -953,26 +953,29 @@ PTB_API int ptb_attention_tc(const void* q, const void* k_pool, const void* v_po
                                 head_dim, head_dim, scale, 0, error_flag, stream);
 }
 
-// The same with what some designs put around the softmax (TcParams), head sizes 64 and 128, weights of two terms. out: rows
+// The same with what some designs put around the softmax (TcParams), the same sizes; wide_weights as above. out: rows
 // out_stride apart and a gate per entry's rows at whole 16-byte words.
 PTB_API int ptb_attention_tc_extras(const void* q, const void* k_pool, const void* v_pool, int pool_pages, void* out,
                                     const StepBatch* sb, const int* tile_seq, const int* tile_q0, int n_tiles, int heads,
-                                    int kv_heads, int head_dim, float scale, int window, int keep_first, float softcap,
+                                    int kv_heads, int head_dim, int v_dim, float scale, int wide_weights, int window, int keep_first, float softcap,
                                     const float* sinks, const void* gate, int gate_stride, int gate_wide, float out_scale,
                                     int out_stride, int* error_flag, cudaStream_t stream) {
   if (n_tiles <= 0) return PTB_OK;
   if (pool_pages <= 0 || !aligned16(k_pool) || !aligned16(v_pool) || !aligned16(q) || !aligned16(out) || out_stride % 8 != 0 ||
       (gate != nullptr && gate_wide && (!aligned16(gate) || gate_stride % 8 != 0)))
     return PTB_ERR_ALIGN;
-  if (!ptb_attention_tc_supports(head_dim) || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || n_tiles > 65535 ||
-      error_flag == nullptr || window < 0 || keep_first < 0 || softcap < 0.f || out_stride < heads * head_dim ||
-      (gate != nullptr && gate_stride < (gate_wide ? heads * head_dim : heads)))
+  if (!ptb_attention_tc_supports_sizes(head_dim, v_dim) || heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || n_tiles > 65535 ||
+      error_flag == nullptr || window < 0 || keep_first < 0 || softcap < 0.f || out_stride < heads * v_dim ||
+      (gate != nullptr && gate_stride < (gate_wide ? heads * v_dim : heads)))
     return PTB_ERR_SIZE;
   TcParams p = {};
   p.heads = heads; p.kv_heads = kv_heads; p.scale = scale; p.window = window; p.keep_first = keep_first; p.softcap = softcap;
   p.sinks = sinks; p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride; p.gate_wide = gate_wide;
   p.out_scale = out_scale; p.out_stride = out_stride;
-  return head_dim == 64
-             ? launch_tc<64, 64, false, true, true>(q, k_pool, v_pool, pool_pages, out, *sb, tile_seq, tile_q0, n_tiles, p, error_flag, stream)
-             : launch_tc<128, 128, false, true, true>(q, k_pool, v_pool, pool_pages, out, *sb, tile_seq, tile_q0, n_tiles, p, error_flag, stream);
+#define PTB_TCX(DK, DV, W) \
+  launch_tc<DK, DV, false, W, true>(q, k_pool, v_pool, pool_pages, out, *sb, tile_seq, tile_q0, n_tiles, p, error_flag, stream)
+  if (head_dim == 64) return wide_weights ? PTB_TCX(64, 64, true) : PTB_TCX(64, 64, false);
+  if (head_dim == 128) return wide_weights ? PTB_TCX(128, 128, true) : PTB_TCX(128, 128, false);
+  return wide_weights ? PTB_TCX(192, 128, true) : PTB_TCX(192, 128, false);
+#undef PTB_TCX
 }

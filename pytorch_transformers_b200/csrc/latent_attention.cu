@@ -27,7 +27,7 @@ template <typename T>
 __global__ void latent_store_kernel(const T* __restrict__ src, long long src_stride, const float* __restrict__ norm_w,
                                     float eps, T* __restrict__ pool, StepBatch sb, const float* __restrict__ rope_cos,
                                     const float* __restrict__ rope_sin, int rot_pairs, int interleaved, int rank,
-                                    int rot_dim) {
+                                    int rot_dim, T* __restrict__ c_rows, T* __restrict__ kr_rows) {
   pdl_entry();
   __shared__ float scratch[32];
   const int t = blockIdx.x;
@@ -41,7 +41,12 @@ __global__ void latent_store_kernel(const T* __restrict__ src, long long src_str
     q += v * v;
   }
   const float rstd = 1.0f / sqrtf(block_sum(q, scratch) / float(rank) + eps);
-  for (int i = threadIdx.x; i < rank; i += blockDim.x) dst[i] = from_f<T>(to_f(row[i]) * rstd * norm_w[i]);
+  for (int i = threadIdx.x; i < rank; i += blockDim.x) {
+    const T v = from_f<T>(to_f(row[i]) * rstd * norm_w[i]);
+    dst[i] = v;
+    if (c_rows) c_rows[size_t(t) * rank + i] = v;
+  }
+  T* kr = kr_rows ? kr_rows + size_t(t) * rot_dim : nullptr;
   const int items = rot_pairs + (rot_dim - 2 * rot_pairs);
   for (int e = threadIdx.x; e < items; e += blockDim.x) {
     if (e < rot_pairs) {
@@ -51,9 +56,11 @@ __global__ void latent_store_kernel(const T* __restrict__ src, long long src_str
                   rope_sin[size_t(t) * rot_pairs + e], a, b);
       dst[rank + ia] = from_f<T>(a);
       dst[rank + ib] = from_f<T>(b);
+      if (kr) kr[ia] = from_f<T>(a), kr[ib] = from_f<T>(b);
     } else {
       const int i = 2 * rot_pairs + (e - rot_pairs);
       dst[rank + i] = row[rank + i];
+      if (kr) kr[i] = row[rank + i];
     }
   }
 }
@@ -352,20 +359,21 @@ PTB_API long long ptb_latent_part_floats(int n_tiles, int heads, int heads_per_b
   return (long long)n_tiles * chunks * n_splits * ROWS * part_row(rank);
 }
 
+// c_rows [tokens, rank], kr_rows [tokens, rot_dim] or null: the rows' two parts once more, side by side in the order of the tokens
 PTB_API int ptb_latent_store(int dtype, const void* src, long long src_stride, const float* norm_w, float eps,
                              void* pool, const StepBatch* sb, const float* rope_cos, const float* rope_sin,
-                             int rot_pairs, int interleaved, int rank, int rot_dim, cudaStream_t stream) {
+                             int rot_pairs, int interleaved, int rank, int rot_dim, void* c_rows, void* kr_rows, cudaStream_t stream) {
   if (sb->n_tokens <= 0) return PTB_OK;
   if (rank <= 0 || rot_dim < 0 || rot_pairs < 0 || 2 * rot_pairs > rot_dim) return PTB_ERR_SIZE;
   if (rot_pairs > 0 && (rope_cos == nullptr || rope_sin == nullptr)) return PTB_ERR_SIZE;
   if (dtype == PTB_F32)
     launch_pdl(latent_store_kernel<float>, sb->n_tokens, 128, 0, stream, (const float*)src, src_stride, norm_w, eps,
                                                                  (float*)pool, *sb, rope_cos, rope_sin, rot_pairs,
-                                                                 interleaved, rank, rot_dim);
+                                                                 interleaved, rank, rot_dim, (float*)c_rows, (float*)kr_rows);
   else if (dtype == PTB_BF16)
     launch_pdl(latent_store_kernel<__nv_bfloat16>, sb->n_tokens, 128, 0, stream, 
         (const __nv_bfloat16*)src, src_stride, norm_w, eps, (__nv_bfloat16*)pool, *sb, rope_cos, rope_sin, rot_pairs,
-        interleaved, rank, rot_dim);
+        interleaved, rank, rot_dim, (__nv_bfloat16*)c_rows, (__nv_bfloat16*)kr_rows);
   else
     return PTB_ERR_DTYPE;
   return launch_status();

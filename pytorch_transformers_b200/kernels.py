@@ -557,30 +557,33 @@ def attention_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, ba
     return out
 
 
-def attention_tc_extras_take(out: torch.Tensor, gate: Optional[torch.Tensor] = None, gate_wide: bool = False) -> bool:
+def attention_tc_extras_take(out: Optional[torch.Tensor], gate: Optional[torch.Tensor] = None, gate_wide: bool = False) -> bool:
     """Whether ``attention_tc_extras`` can write into ``out`` and read ``gate``: whole 16-byte words (a gate per head is read
     number by number)."""
     def words(t):
         return t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0
-    return words(out) and (gate is None or not gate_wide or words(gate))
+    return (out is None or words(out)) and (gate is None or not gate_wide or words(gate))
 
 
 def attention_tc_extras(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, batch: StepBatchC, tile_seq: torch.Tensor,
                         tile_q0: torch.Tensor, n_tiles: int, kv_heads: int, scale: float, window: int = 0, keep_first: int = 0,
                         softcap: float = 0.0, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
-                        gate_wide: bool = False, out_scale: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                        gate_wide: bool = False, out_scale: float = 1.0, out: Optional[torch.Tensor] = None,
+                        wide_weights: bool = True) -> torch.Tensor:
     """Prompt attention on tcgen05 in tiles of 128 tokens with what ``attention_generic`` takes around the softmax; the softmax
-    weights meet the values as two bfloat16 terms. bfloat16, head sizes 64 and 128, values of the keys' size."""
+    weights meet the values as two bfloat16 terms (not with ``wide_weights=False``). bfloat16, the head sizes that ``attention_tc``
+    takes."""
     _need_cuda(q, k_pool, v_pool, tile_seq, tile_q0, sinks)
     n, heads, head_dim = q.shape
+    v_dim = v_pool.shape[-1]
     if out is None:
-        out = torch.empty((n, heads * head_dim), dtype=q.dtype, device=q.device)
-    _check_rows(out, (n, heads * head_dim), q.dtype, "attention_tc_extras: out")
+        out = torch.empty((n, heads * v_dim), dtype=q.dtype, device=q.device)
+    _check_rows(out, (n, heads * v_dim), q.dtype, "attention_tc_extras: out")
     if gate is not None:
-        _check_rows(gate, (n, heads * head_dim if gate_wide else heads), q.dtype, "attention_tc_extras: gate")
+        _check_rows(gate, (n, heads * v_dim if gate_wide else heads), q.dtype, "attention_tc_extras: gate")
     _check(lib().ptb_attention_tc_extras(_ptr(q), _ptr(k_pool), _ptr(v_pool), k_pool.shape[0], _ptr(out), ctypes.byref(batch),
-                                         _ptr(tile_seq), _ptr(tile_q0), n_tiles, heads, kv_heads, head_dim, ctypes.c_float(scale),
-                                         int(window), int(keep_first), ctypes.c_float(softcap), _ptr(sinks), _ptr(gate),
+                                         _ptr(tile_seq), _ptr(tile_q0), n_tiles, heads, kv_heads, head_dim, v_dim, ctypes.c_float(scale),
+                                         1 if wide_weights else 0, int(window), int(keep_first), ctypes.c_float(softcap), _ptr(sinks), _ptr(gate),
                                          0 if gate is None else gate.stride(0), 1 if gate_wide else 0, ctypes.c_float(out_scale),
                                          out.stride(0), _ptr(error_flag(q.device)), _stream(q)), "attention_tc_extras")
     return out
@@ -881,18 +884,23 @@ LATENT_ROWS = 16   # ptb_latent_rows(): (token, head) rows of a tile
 
 
 def latent_store(src: torch.Tensor, norm_w: torch.Tensor, eps: float, pool: torch.Tensor, batch: StepBatchC, rope,
-                 rank: int, rot_dim: int, interleaved: bool = True) -> None:
+                 rank: int, rot_dim: int, interleaved: bool = True, rows: bool = False):
     """Rows ``src`` [tokens, rank + rot_dim] (a view whose rows may be wider apart) of the latent
     down-projection become cache rows: the first ``rank`` RMS-normed with ``norm_w``, the rest rotated by
-    the tokens' positions (``rope`` = (cos, sin) [tokens, pairs])."""
+    the tokens' positions (``rope`` = (cos, sin) [tokens, pairs]). ``rows``: returns both parts once more in the order of the
+    tokens ([tokens, rank], [tokens, rot_dim]), what ``latent_unfolded_attention`` would gather for sequences without a past."""
     _need_cuda(norm_w, pool)
     if src.stride(1) != 1 or src.shape[1] != rank + rot_dim or pool.shape[-1] != rank + rot_dim or pool.dtype != src.dtype:
         raise KernelError("latent_store: the rows or the pool do not fit rank + rot_dim")
     cos, sin = rope if rope is not None else (None, None)
     pairs = 0 if cos is None else cos.shape[1]
+    c_rows = torch.empty((src.shape[0], rank), dtype=src.dtype, device=src.device) if rows else None
+    kr_rows = torch.empty((src.shape[0], max(rot_dim, 1)), dtype=src.dtype, device=src.device) if rows else None
     _check(lib().ptb_latent_store(_dtype_code(src), _ptr(src), ctypes.c_longlong(src.stride(0)), _ptr(norm_w),
                                   ctypes.c_float(eps), _ptr(pool), ctypes.byref(batch), _ptr(cos), _ptr(sin), pairs,
-                                  1 if interleaved else 0, rank, rot_dim, _stream(pool)), "latent_store")
+                                  1 if interleaved else 0, rank, rot_dim, _ptr(c_rows), _ptr(kr_rows if rot_dim else None),
+                                  _stream(pool)), "latent_store")
+    return (c_rows, kr_rows) if rows else None
 
 
 def latent_attention_mma_supports(rank: int, rot_dim: int) -> bool:
@@ -952,14 +960,15 @@ def latent_unfolded_attention(q: torch.Tensor, pool: torch.Tensor, k_tmp: torch.
                               ctx_pos: torch.Tensor, n_ctx: int, mtile_seq: torch.Tensor, mtile_q0: torch.Tensor,
                               n_mma_tiles: int, rope, dim: int, rot_dim: int, vdim: int, rank: int, scale: float,
                               interleaved: bool = True, gate_per_head: bool = False,
-                              wide_weights: bool = False) -> torch.Tensor:
+                              wide_weights: bool = False, rows=None) -> torch.Tensor:
     """Latent attention of prompts through the tcgen05 prompt kernel (bfloat16): the ``n_ctx`` cached rows
     (``ctx_seq``, ``ctx_pos``: sequence and position of each) of the step's sequences are unfolded with
     ``w_ukv`` = [W_uk; W_uv] into per-head keys and values in the scratch pools ``k_tmp`` / ``v_tmp``
     ([pages, heads, 64, hd], zero outside what is written here; hd may differ between the two), the queries (a view
     whose tokens may lie wider apart) are laid out to match, and ``attention_tc`` runs on them. Returns the heads'
     outputs times sigmoid(gate): [tokens, heads * vdim]; ``gate`` [tokens, heads * vdim], or [tokens, heads] with
-    ``gate_per_head``. ``wide_weights``: as attention_tc takes it."""
+    ``gate_per_head``. ``wide_weights``: as attention_tc takes it. ``rows``: the cached rows' two parts in that order, where they are
+    at hand already (``latent_store``)."""
     _need_cuda(pool, k_tmp, v_tmp, w_ukv, ctx_seq, ctx_pos)
     _check_heads(q, "latent_unfolded_attention")
     n, heads, dq = q.shape
@@ -970,16 +979,25 @@ def latent_unfolded_attention(q: torch.Tensor, pool: torch.Tensor, k_tmp: torch.
     cos, sin = rope if rope is not None else (None, None)
     pairs = 0 if cos is None else cos.shape[1]
     stream = _stream(q)
-    c_rows = torch.empty((n_ctx, rank), dtype=q.dtype, device=q.device)
-    kr_rows = torch.empty((n_ctx, max(rot_dim, 1)), dtype=q.dtype, device=q.device)
-    _check(lib().ptb_latent_gather(_ptr(pool), ctypes.byref(batch), _ptr(ctx_seq), _ptr(ctx_pos), n_ctx, _ptr(c_rows),
-                                   _ptr(kr_rows), rank, rot_dim, stream), "latent_gather")
+    if rows is not None:
+        c_rows, kr_rows = rows
+        if tuple(c_rows.shape) != (n_ctx, rank) or kr_rows.shape[0] != n_ctx or c_rows.dtype != q.dtype:
+            raise KernelError("latent_unfolded_attention: the rows at hand are not the step's cached rows")
+    else:
+        c_rows = torch.empty((n_ctx, rank), dtype=q.dtype, device=q.device)
+        kr_rows = torch.empty((n_ctx, max(rot_dim, 1)), dtype=q.dtype, device=q.device)
+        _check(lib().ptb_latent_gather(_ptr(pool), ctypes.byref(batch), _ptr(ctx_seq), _ptr(ctx_pos), n_ctx, _ptr(c_rows),
+                                       _ptr(kr_rows), rank, rot_dim, stream), "latent_gather")
     kv = matmul_nt(c_rows, w_ukv)
     _check(lib().ptb_latent_unfold(_ptr(kv), _ptr(kr_rows), ctypes.byref(batch), _ptr(ctx_seq), _ptr(ctx_pos), n_ctx,
                                    _ptr(k_tmp), _ptr(v_tmp), heads, dim, rot_dim, vdim, hd, hd_v, stream), "latent_unfold")
     q_tc = torch.empty((n, heads, hd), dtype=q.dtype, device=q.device)
     _check(lib().ptb_latent_q_unfold(_ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(cos), _ptr(sin), pairs, 1 if interleaved else 0, _ptr(q_tc), n, heads,
                                      dim, rot_dim, hd, stream), "latent_q_unfold")
+    if vdim == hd_v and attention_tc_extras_take(None, gate, not gate_per_head):
+        # the gate in the attention's own last step (its rows and the gate's at whole 16-byte words)
+        return attention_tc_extras(q_tc, k_tmp, v_tmp, batch, mtile_seq, mtile_q0, n_mma_tiles, heads, scale, gate=gate,
+                                   gate_wide=not gate_per_head, wide_weights=wide_weights)
     o = attention_tc(q_tc, k_tmp, v_tmp, batch, mtile_seq, mtile_q0, n_mma_tiles, heads, scale, wide_weights=wide_weights)
     out = torch.empty((n, heads * vdim), dtype=q.dtype, device=q.device)
     _check(lib().ptb_gate_heads(_ptr(o), _ptr(gate), ctypes.c_longlong(gate.stride(0)), _ptr(out), n, heads, vdim, hd_v,

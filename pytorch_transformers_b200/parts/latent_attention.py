@@ -187,25 +187,28 @@ class LatentAttention(Part):
         pool, _, group = ctx.cache.entry_storage(entry.cache_entry)
         batch = ctx.batch_c[group]
         rope = ctx.rope(self.position)
+        tiles = ctx.plan(AttentionTiles.plan_key)
+        plan = ctx.plan(LatentContext.plan_key)
+        sizes, pools = self._unfold_size(), None
+        if sizes and plan.facts["n_ctx"] and tiles.facts["mma_tokens"] == k.TC_TILE_TOKENS:
+            pools = self._unfold_pools(ctx.cache, group, *sizes)
+        rows = None
         if entry.writes_cache:
             if not self.own_kv:
                 raise ValueError("a latent attention layer without a key/value projection cannot write a cache entry")
-            k.latent_store(down, self.p_dkv_norm, self.eps, pool, batch, rope, self.kv_rank,
-                           self.rot_dim, self.interleaved)
-        tiles = ctx.plan(AttentionTiles.plan_key)
-        rows = ctx.plan(LatentContext.plan_key)
-        sizes = self._unfold_size()
-        if sizes and rows.facts["n_ctx"] and tiles.facts["mma_tokens"] == k.TC_TILE_TOKENS:
-            pools = self._unfold_pools(ctx.cache, group, *sizes)
-            if pools is not None:
-                # long prompts in bfloat16: per-head keys and values unfolded from the cached latents, and the
-                # tcgen05 prompt kernel on them
-                o = k.latent_unfolded_attention(q, pool, pools[0], pools[1], self.p_ukv, gate, batch, rows.dev["ctx_seq"],
-                                                rows.dev["ctx_pos"], rows.facts["n_ctx"], tiles.dev["mtile_seq"],
-                                                tiles.dev["mtile_q0"], tiles.facts["n_mma_tiles"], rope, self.dim,
-                                                self.rot_dim, self.vdim, self.kv_rank, self.scale, self.interleaved,
-                                                gate_per_head=self.gate_per_head, wide_weights=self.wide_weights)
-                return self._out(o, add)
+            # sequences without a past: the rows that the unfolded path reads are the ones being stored
+            fresh = pools is not None and plan.facts["n_ctx"] == down.shape[0] and not any(ctx.past)
+            rows = k.latent_store(down, self.p_dkv_norm, self.eps, pool, batch, rope, self.kv_rank,
+                                  self.rot_dim, self.interleaved, rows=fresh)
+        if pools is not None:
+            # long prompts in bfloat16: per-head keys and values unfolded from the cached latents, and the
+            # tcgen05 prompt kernel on them
+            o = k.latent_unfolded_attention(q, pool, pools[0], pools[1], self.p_ukv, gate, batch, plan.dev["ctx_seq"],
+                                            plan.dev["ctx_pos"], plan.facts["n_ctx"], tiles.dev["mtile_seq"],
+                                            tiles.dev["mtile_q0"], tiles.facts["n_mma_tiles"], rope, self.dim,
+                                            self.rot_dim, self.vdim, self.kv_rank, self.scale, self.interleaved,
+                                            gate_per_head=self.gate_per_head, wide_weights=self.wide_weights, rows=rows)
+            return self._out(o, add)
         q_abs = k.block_linear(q[:, :, :self.dim], self.p_uk_t, out_dtype=torch.float32)
         if tiles.facts["mma_tokens"] == 1:     # a step of single tokens: a tile is one token's heads
             o_lat = k.latent_attention(q_abs, q, self.dim, pool, batch, tiles.dev["mtile_seq"], tiles.dev["mtile_q0"],

@@ -612,3 +612,98 @@ def test_trace_runner_as_a_child_process(tmp_path, dtype):
         got.append(torch.from_numpy(arr.copy()))
         want += [refs[i][p] for i, p in rows]
     close(torch.cat(got), torch.stack(want), dtype, "trace runner")
+
+
+@pytest.mark.parametrize("dim,rot,vdim,per_head,wide,pasts", [
+    (96, 32, 128, False, True, (0, 0, 0)),       # the gate in the attention's last step, rows at hand
+    (48, 16, 64, True, False, (0, 0, 0)),
+    (128, 64, 128, False, False, (0, 0, 0)),     # keys wider than values
+    (128, 64, 128, True, True, (0, 70, 0)),      # a sequence with a past: rows gathered
+    (64, 32, 96, False, True, (0, 0, 0)),        # values narrower than the kernel's: the gate apart
+    (64, 0, 64, False, True, (0, 0, 0)),         # nothing rotated
+])
+def test_unfolded_attention_gated(dim, rot, vdim, per_head, wide, pasts):
+    """Stored rows, unfolded prompt attention and gate against float64 on the cached rows, and the rows that the store hands
+    on against the gathered ones (the same bits). bfloat16 is met five times on a result's way (q, keys, values, weights
+    unless wide, result): rows within 5 * 2^-9 of their norm."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.attention import AttentionTiles
+    from pytorch_transformers_b200.parts.base import CacheNeed
+    from pytorch_transformers_b200.parts.latent_attention import LatentContext
+    k, dt, heads, rank, scale = K(), torch.bfloat16, 3, 72, 0.1
+    news = (130, 1, 257)
+    g = torch.Generator().manual_seed(dim + vdim)
+    totals = [p + n for p, n in zip(pasts, news)]
+    rows = [torch.randn(t, rank + rot, generator=g).to(dt) for t in totals]
+    n = sum(news)
+    q = torch.randn(n, heads, dim + rot, generator=g).to(dt)
+    wide_gate = torch.randn(n, 8 + (heads if per_head else heads * vdim), generator=g).to(dt).cuda()
+    gate = wide_gate[:, 8:]
+    w_ukv = (torch.randn(heads * (dim + vdim), rank, generator=g) / math.sqrt(rank)).to(dt).cuda()
+    norm_w = (1 + 0.2 * torch.randn(rank, generator=g)).cuda()
+    inv_freq = (1.0 / (1e4 ** (torch.arange(0, rot, 2).float() / rot))).cuda() if rot else None
+    cache = Cache([(0, CacheNeed("full", 1, rank + rot, 0, v_head_dim=0), None)], sum((t + 63) // 64 * 64 for t in totals), dt, "cuda")
+    slots = [cache.open() for _ in totals]
+    pool, _, gi = cache.entry_storage(0)
+
+    def begin(ranges):
+        live = [i for i, (a, b) in enumerate(ranges) if b > a]
+        ctx = StepContext(cache, [slots[i] for i in live], [[0] * (ranges[i][1] - ranges[i][0]) for i in live], 1,
+                          [[] for _ in live], [AttentionTiles(k), LatentContext(k)])
+        rope = k.rope_table(ctx.dev["tok_pos"], inv_freq) if rot else None
+        src = torch.cat([rows[i][ranges[i][0]:ranges[i][1]] for i in live]).cuda()
+        return ctx, rope, k.latent_store(src, norm_w, 1e-6, pool, ctx.batch_c[gi], rope, rank, rot, True, rows=True)
+
+    if any(pasts):
+        begin([(0, p) for p in pasts])[0].commit()
+    ctx, rope, at_hand = begin([(p, t) for p, t in zip(pasts, totals)])
+    tiles, plan = ctx.plan(AttentionTiles.plan_key), ctx.plan(LatentContext.plan_key)
+    hd, hd_v = next(s for s in ((64, 64), (128, 128), (192, 128)) if dim + rot <= s[0] and vdim <= s[1])
+    pages = pool.shape[0]
+
+    def run(rows):
+        k_tmp = torch.zeros((pages, heads, 64, hd), dtype=dt, device="cuda")
+        v_tmp = torch.zeros((pages, heads, 64, hd_v), dtype=dt, device="cuda")
+        return k.latent_unfolded_attention(q.cuda(), pool, k_tmp, v_tmp, w_ukv, gate, ctx.batch_c[gi], plan.dev["ctx_seq"],
+                                           plan.dev["ctx_pos"], plan.facts["n_ctx"], tiles.dev["mtile_seq"],
+                                           tiles.dev["mtile_q0"], tiles.facts["n_mma_tiles"], rope, dim, rot, vdim, rank, scale,
+                                           True, gate_per_head=per_head, wide_weights=wide, rows=rows)
+
+    got = run(None)
+    if any(pasts):
+        with pytest.raises(Exception, match="not the step's cached rows"):
+            run(at_hand)
+    else:
+        assert torch.equal(run(at_hand), got)
+    k.check_device_errors(got.device)
+
+    def turned(x, pos):      # pairs side by side
+        if not rot:
+            return x
+        a = torch.outer(pos.double(), inv_freq.double().cpu())
+        c, s = a.cos(), a.sin()
+        while c.dim() < x.dim():
+            c, s = c.unsqueeze(1), s.unsqueeze(1)
+        e, o = x[..., 0::2], x[..., 1::2]
+        return torch.stack([e * c - o * s, o * c + e * s], -1).flatten(-2)
+
+    ref, at = [], 0
+    wk = w_ukv[:heads * dim].double().cpu().view(heads, dim, rank)
+    wv = w_ukv[heads * dim:].double().cpu().view(heads, vdim, rank)
+    for b, (p, t) in enumerate(zip(pasts, totals)):
+        raw = rows[b].double()
+        c = raw[:, :rank]
+        c = (c * (c.square().mean(1, keepdim=True) + 1e-6).rsqrt() * norm_w.double().cpu()).to(dt).double()
+        kr = turned(raw[:, rank:], torch.arange(t)).to(dt).double()
+        keys = torch.cat([torch.einsum("hdr,tr->thd", wk, c), kr[:, None].expand(t, heads, rot)], -1)
+        qs = q[at:at + t - p].double()
+        qs = torch.cat([qs[..., :dim], turned(qs[..., dim:], torch.arange(p, t))], -1)
+        s = torch.einsum("qhd,khd->hqk", qs, keys) * scale
+        s = s.masked_fill(torch.arange(t)[None, None] > torch.arange(p, t)[None, :, None], -math.inf)
+        ref.append(torch.einsum("hqk,khv->qhv", s.softmax(-1), torch.einsum("hvr,tr->thv", wv, c)))
+        at += t - p
+    ref = torch.cat(ref)
+    gd = torch.sigmoid(gate.double().cpu())
+    ref = ref * (gd[:, :, None] if per_head else gd.view(n, heads, vdim))
+    assert row_errors(got, ref.reshape(n, -1)).max() < 5 * 2.0 ** -9
