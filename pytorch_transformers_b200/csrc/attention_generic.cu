@@ -379,11 +379,6 @@ __device__ __forceinline__ void store_quad(__nv_bfloat16* p, float4 v) {
   u.y = *reinterpret_cast<const uint32_t*>(&b);
   *reinterpret_cast<uint2*>(p) = u;
 }
-// one half of rotate_pair: the entry `own` of a pair whose other entry is `other` (first: own c - other s; second:
-// own c + other s), with rotate_pair's roundings
-__device__ __forceinline__ float rotate_own(float own, float other, float c, float s, bool first) {
-  return first ? __fsub_rn(__fmul_rn(own, c), __fmul_rn(other, s)) : __fadd_rn(__fmul_rn(own, c), __fmul_rn(other, s));
-}
 
 // ------------------------------------------------------------------------------------------------
 // Separate projections q | k | v side by side in a row of `proj` (rows `stride` apart), an optional bias on all of
@@ -397,14 +392,14 @@ __device__ __forceinline__ float rotate_own(float own, float other, float c, flo
 // gains (`q_gain`, `k_gain` [dim] float32, null: none). With temp_every > 0 a query at position p is multiplied by
 // 1 + temp_coef ln(floor((p + 1) / temp_every) + 1) at the end, in float32. A warp per (token, head): query heads, then key heads, then the
 // K/V heads' values; the warps of a block share nothing, so a head's chain of loads, rotation, sum and stores waits
-// for no other.
+// for no other. What rope_norm_store_vec_kernel (below) does not take.
 template <typename T>
 __global__ void rope_norm_store_kernel(const T* __restrict__ proj, int stride, const float* __restrict__ bias,
                                        T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool, StepBatch sb,
                                        const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int rot_pairs,
                                        int heads, int kv_heads, int dim, int v_dim, float eps, int unit_norm,
                                        const T* __restrict__ v_first, int v_first_stride, const float* __restrict__ lam,
-                                       T* __restrict__ v_keep, int write_cache, int pairs, int quads,
+                                       T* __restrict__ v_keep, int write_cache, int pairs,
                                        const float* __restrict__ q_gain, const float* __restrict__ k_gain, int norm_first,
                                        float temp_coef, int temp_every) {
   pdl_entry();
@@ -449,46 +444,6 @@ __global__ void rope_norm_store_kernel(const T* __restrict__ proj, int stride, c
     const int page = sb.pages[size_t(seq) * sb.pages_stride + pos / PTB_PAGE];
     dst = k_pool + kv_offset(page, hh - heads, pos % PTB_PAGE, kv_heads, dim);
   }
-  if (quads) {
-    // heads of up to 128 entries whose rotated part is a multiple of 8: four entries a lane in registers, the other
-    // entry of a rotated pair from the lane rot_pairs / 4 further (or back) by shuffle; no shared memory
-    const unsigned full = 0xffffffffu;
-    const int e = 4 * lane, P = rot_pairs / 4;
-    const bool on = e < dim;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 x = on ? load_quad(src + e) : zero;
-    if (bsrc && on) {
-      const float4 b = *reinterpret_cast<const float4*>(bsrc + e);
-      x = make_float4(x.x + b.x, x.y + b.y, x.z + b.z, x.w + b.w);
-    }
-    if (unit_norm && norm_first) {      // the norm (with its gains) comes before the rotation
-      const float ss = fmaf(x.w, x.w, fmaf(x.z, x.z, fmaf(x.y, x.y, x.x * x.x)));
-      const float r = 1.0f / sqrtf(warp_sum(ss) / float(dim) + eps);
-      const float4 g = (gain && on) ? *reinterpret_cast<const float4*>(gain + e) : make_float4(1.f, 1.f, 1.f, 1.f);
-      x = make_float4(x.x * r * g.x, x.y * r * g.y, x.z * r * g.z, x.w * r * g.w);
-    }
-    if (P > 0) {
-      const bool first = lane < P, rotated = lane < 2 * P;
-      const int other = first ? lane + P : (rotated ? lane - P : lane);
-      float4 c = zero, sn = zero;
-      if (rotated) {
-        c = *reinterpret_cast<const float4*>(rope_cos + size_t(t) * rot_pairs + 4 * (first ? lane : lane - P));
-        sn = *reinterpret_cast<const float4*>(rope_sin + size_t(t) * rot_pairs + 4 * (first ? lane : lane - P));
-      }
-      const float4 y = make_float4(__shfl_sync(full, x.x, other), __shfl_sync(full, x.y, other), __shfl_sync(full, x.z, other),
-                                   __shfl_sync(full, x.w, other));
-      if (rotated)
-        x = make_float4(rotate_own(x.x, y.x, c.x, sn.x, first), rotate_own(x.y, y.y, c.y, sn.y, first),
-                        rotate_own(x.z, y.z, c.z, sn.z, first), rotate_own(x.w, y.w, c.w, sn.w, first));
-    }
-    float rstd = last;
-    if (unit_norm && !norm_first) {
-      const float ss = fmaf(x.w, x.w, fmaf(x.z, x.z, fmaf(x.y, x.y, x.x * x.x)));
-      rstd = last / sqrtf(warp_sum(ss) / float(dim) + eps);
-    }
-    if (on) store_quad(dst + e, make_float4(x.x * rstd, x.y * rstd, x.z * rstd, x.w * rstd));
-    return;
-  }
   for (int i = lane; i < rot_pairs; i += 32) {       // issued with the row's loads
     cs[i] = rope_cos[size_t(t) * rot_pairs + i];
     cs[rot_pairs + i] = rope_sin[size_t(t) * rot_pairs + i];
@@ -528,6 +483,121 @@ __global__ void rope_norm_store_kernel(const T* __restrict__ proj, int stride, c
   } else {
     for (int e = lane; e < dim; e += 32) dst[e] = from_f<T>(buf[e] * rstd);
   }
+}
+
+// The same for heads of whole quads (sizes and rotated parts multiples of 4, heads of up to 8 GROUP entries): GROUP lanes a
+// (token, head), each with eight entries in registers. What bounds the work is instructions, not bytes (a warp a head and
+// four entries a lane issued 110 instructions a head: 17.0 us for 2,048 tokens of 24 heads of 128, a fifth of the copy
+// rate), so a lane holds both entries of four rotated pairs: no shuffles for the rotation, one read of the angles for both
+// halves, two to four heads a warp for every address, root and division; blocks of `per` heads of one token, of at most 256
+// threads (blocks of 384 at 48 registers left half of an SM's warps unused: 12.3 us; as here 10.2 us). Sums run over a lane's
+// eight entries, then a tree over the group's lanes.
+template <typename T, int GROUP>
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 6 : 5) rope_norm_store_vec_kernel(const T* __restrict__ proj, int stride, const float* __restrict__ bias,
+                                           T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool, StepBatch sb,
+                                           const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int rot_pairs,
+                                           int heads, int kv_heads, int dim, int v_dim, float eps, int unit_norm,
+                                           const T* __restrict__ v_first, int v_first_stride, const float* __restrict__ lam,
+                                           T* __restrict__ v_keep, int write_cache, int v_quads,
+                                           const float* __restrict__ q_gain, const float* __restrict__ k_gain, int norm_first,
+                                           float temp_coef, int temp_every, int per) {
+  pdl_entry();
+  const int lane = threadIdx.x % GROUP, t = blockIdx.x;
+  const unsigned mask = (GROUP == 32 ? 0xffffffffu : ((1u << (GROUP % 32)) - 1u)) << (threadIdx.x % 32 / GROUP * GROUP);
+  const T* row = proj + size_t(t) * stride;
+  const int hh = blockIdx.y * per + threadIdx.x / GROUP;      // one path for all lanes of a group
+  if (threadIdx.x / GROUP >= per || hh >= heads + 2 * kv_heads) return;
+  const bool is_q = hh < heads, is_v = hh >= heads + kv_heads;
+  if (!is_q && !write_cache && !(is_v && v_keep)) return;
+  T* dst = nullptr;
+  const int g = is_v ? hh - heads - kv_heads : hh - heads;
+  if (is_q) {
+    dst = q_out + (size_t(t) * heads + hh) * dim;
+  } else if (write_cache) {
+    const int pos = sb.tok_pos[t], seq = sb.tok_seq[t];
+    const int page = sb.pages[size_t(seq) * sb.pages_stride + pos / PTB_PAGE];
+    dst = is_v ? v_pool + kv_offset(page, g, pos % PTB_PAGE, kv_heads, v_dim) : k_pool + kv_offset(page, g, pos % PTB_PAGE, kv_heads, dim);
+  }
+  if (is_v) {
+    const size_t at = size_t(heads + kv_heads) * dim + size_t(g) * v_dim;
+    const float l = (v_first != nullptr) ? lam[0] : 0.f;
+    T* keep = v_keep ? v_keep + (size_t(t) * kv_heads + g) * v_dim : nullptr;
+    const T* vf = v_first ? v_first + size_t(t) * v_first_stride + size_t(g) * v_dim : nullptr;
+    auto mixed = [&](float v, float f) { return (1.f - l) * round_store<T>(v) + l * f; };
+    if (v_quads) {
+      for (int e = 4 * lane; e < v_dim; e += 4 * GROUP) {
+        float4 v = load_quad(row + at + e);
+        if (bias) {
+          const float4 b = *reinterpret_cast<const float4*>(bias + at + e);
+          v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+        }
+        if (keep) store_quad(keep + e, v);
+        if (vf) {
+          const float4 f = load_quad(vf + e);
+          v = make_float4(mixed(v.x, f.x), mixed(v.y, f.y), mixed(v.z, f.z), mixed(v.w, f.w));
+        }
+        if (dst) store_quad(dst + e, v);
+      }
+    } else {
+      for (int e = lane; e < v_dim; e += GROUP) {
+        float v = to_f(row[at + e]) + (bias ? bias[at + e] : 0.f);
+        if (keep) keep[e] = from_f<T>(v);
+        if (vf) v = mixed(v, to_f(vf[e]));
+        if (dst) dst[e] = from_f<T>(v);
+      }
+    }
+    return;
+  }
+  // lanes below P: the pairs (4 lane + i, rot_pairs + 4 lane + i); the others: eight entries behind the rotated part
+  const int P = rot_pairs / 4;
+  const bool rotated = lane < P;
+  const int ea = rotated ? 4 * lane : 2 * rot_pairs + 8 * (lane - P), eb = rotated ? rot_pairs + ea : ea + 4;
+  const bool on_a = ea < dim, on_b = eb < dim;
+  const T* src = row + size_t(hh) * dim;
+  float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  float4 c = make_float4(0.f, 0.f, 0.f, 0.f), sn = c;
+  if (rotated) {
+    c = *reinterpret_cast<const float4*>(rope_cos + size_t(t) * rot_pairs + 4 * lane);
+    sn = *reinterpret_cast<const float4*>(rope_sin + size_t(t) * rot_pairs + 4 * lane);
+  }
+  auto put = [](float* d, float4 v) { d[0] = v.x, d[1] = v.y, d[2] = v.z, d[3] = v.w; };
+  if (on_a) put(x, load_quad(src + ea));
+  if (on_b) put(x + 4, load_quad(src + eb));
+  auto each = [&](const float* w, auto op) {      // op(x, w) with a row of float32 as long as the head
+    float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (on_a) put(y, *reinterpret_cast<const float4*>(w + ea));
+    if (on_b) put(y + 4, *reinterpret_cast<const float4*>(w + eb));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = op(x[i], y[i]);
+  };
+  auto root = [&](float over) {      // over / the head's root mean square
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss = fmaf(x[i], x[i], ss);
+#pragma unroll
+    for (int o = GROUP / 2; o > 0; o /= 2) ss += __shfl_xor_sync(mask, ss, o);
+    return over / sqrtf(ss / float(dim) + eps);
+  };
+  if (bias) each(bias + size_t(hh) * dim, [](float a, float b) { return a + b; });
+  if (unit_norm && norm_first) {      // the norm (with its gains) comes before the rotation
+    const float r = root(1.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] *= r;
+    const float* gain = is_q ? q_gain : k_gain;
+    if (gain) each(gain, [](float a, float b) { return a * b; });
+  }
+  if (rotated) {
+    rotate_pair(x[0], x[4], c.x, sn.x, x[0], x[4]);
+    rotate_pair(x[1], x[5], c.y, sn.y, x[1], x[5]);
+    rotate_pair(x[2], x[6], c.z, sn.z, x[2], x[6]);
+    rotate_pair(x[3], x[7], c.w, sn.w, x[3], x[7]);
+  }
+  // what the finished row is multiplied by: the query temperature of the token's position, the norm
+  float last = 1.f;
+  if (is_q && temp_every > 0) last = 1.f + temp_coef * logf(float((sb.tok_pos[t] + 1) / temp_every) + 1.f);
+  if (unit_norm && !norm_first) last = root(last);
+  if (on_a) store_quad(dst + ea, make_float4(x[0] * last, x[1] * last, x[2] * last, x[3] * last));
+  if (on_b) store_quad(dst + eb, make_float4(x[4] * last, x[5] * last, x[6] * last, x[7] * last));
 }
 
 // out[t][h][:] = sum_g talk[h][g] * wide[t][g][kv head of h][:]: the heads' softmax weights mixed after the softmax,
@@ -731,23 +801,36 @@ PTB_API int ptb_qk_prepare_store(int dtype, const void* proj, int stride, const 
   const int pairs = (dim % 2 == 0 && stride % 2 == 0 && reinterpret_cast<uintptr_t>(proj) % pair_bytes == 0 &&
                      reinterpret_cast<uintptr_t>(q_out) % pair_bytes == 0 && reinterpret_cast<uintptr_t>(k_pool) % pair_bytes == 0)
                         ? 1 : 0;
+  // whole quads at aligned rows; heads of more than 256 entries would leave a warp too few registers' worth of entries
   const size_t quad_bytes = 2 * pair_bytes;
-  const int quads = (dim % 4 == 0 && dim <= 128 && rot_pairs % 4 == 0 && stride % 4 == 0 &&
-                     reinterpret_cast<uintptr_t>(proj) % quad_bytes == 0 && reinterpret_cast<uintptr_t>(q_out) % quad_bytes == 0 &&
-                     reinterpret_cast<uintptr_t>(k_pool) % quad_bytes == 0 && (bias == nullptr || aligned16(bias)) && (q_gain == nullptr || aligned16(q_gain)) &&
-                     (k_gain == nullptr || aligned16(k_gain)) &&
-                     (rot_pairs == 0 || (aligned16(rope_cos) && aligned16(rope_sin))))
-                        ? 1 : 0;
+  auto quads = [&](const void* p) { return reinterpret_cast<uintptr_t>(p) % quad_bytes == 0; };
+  if (dim % 4 == 0 && dim <= 256 && rot_pairs % 4 == 0 && stride % 4 == 0 && quads(proj) && quads(q_out) && quads(k_pool) &&
+      aligned16(bias) && aligned16(q_gain) && aligned16(k_gain) && (rot_pairs == 0 || (aligned16(rope_cos) && aligned16(rope_sin)))) {
+    const int v_quads = v_dim % 4 == 0 && quads(v_pool) && quads(v_first) && v_first_stride % 4 == 0 && quads(v_keep) ? 1 : 0;
+    const int group = dim <= 64 ? 8 : dim <= 128 ? 16 : 32;
+    const int rows = (units * group + 255) / 256, per = (units + rows - 1) / rows;      // blocks of a token; alike, of at most 256 threads
+    const int wide = (per * group + 31) / 32 * 32;
+#define PTB_RNS(T, G)                                                                                                        \
+  launch_pdl(rope_norm_store_vec_kernel<T, G>, dim3(sb->n_tokens, rows), wide, 0, stream, (const T*)proj, stride, bias, (T*)q_out, (T*)k_pool, \
+             (T*)v_pool, *sb, rope_cos, rope_sin, rot_pairs, heads, kv_heads, dim, v_dim, eps, unit_norm, (const T*)v_first,  \
+             v_first_stride, lam, (T*)v_keep, write_cache, v_quads, q_gain, k_gain, norm_first, temp_coef, temp_every, per)
+    if (dtype != PTB_F32 && dtype != PTB_BF16) return PTB_ERR_DTYPE;
+    if (group == 8) dtype == PTB_F32 ? PTB_RNS(float, 8) : PTB_RNS(__nv_bfloat16, 8);
+    else if (group == 16) dtype == PTB_F32 ? PTB_RNS(float, 16) : PTB_RNS(__nv_bfloat16, 16);
+    else dtype == PTB_F32 ? PTB_RNS(float, 32) : PTB_RNS(__nv_bfloat16, 32);
+#undef PTB_RNS
+    return launch_status();
+  }
   if (dtype == PTB_F32)
     launch_pdl(rope_norm_store_kernel<float>, blocks, threads, smem, stream, 
         (const float*)proj, stride, bias, (float*)q_out, (float*)k_pool, (float*)v_pool, *sb, rope_cos, rope_sin, rot_pairs,
         heads, kv_heads, dim, v_dim, eps, unit_norm, (const float*)v_first, v_first_stride, lam, (float*)v_keep, write_cache,
-        pairs, quads, q_gain, k_gain, norm_first, temp_coef, temp_every);
+        pairs, q_gain, k_gain, norm_first, temp_coef, temp_every);
   else if (dtype == PTB_BF16)
     launch_pdl(rope_norm_store_kernel<__nv_bfloat16>, blocks, threads, smem, stream, 
         (const __nv_bfloat16*)proj, stride, bias, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, *sb,
         rope_cos, rope_sin, rot_pairs, heads, kv_heads, dim, v_dim, eps, unit_norm, (const __nv_bfloat16*)v_first,
-        v_first_stride, lam, (__nv_bfloat16*)v_keep, write_cache, pairs, quads, q_gain, k_gain, norm_first, temp_coef,
+        v_first_stride, lam, (__nv_bfloat16*)v_keep, write_cache, pairs, q_gain, k_gain, norm_first, temp_coef,
         temp_every);
   else
     return PTB_ERR_DTYPE;

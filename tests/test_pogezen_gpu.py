@@ -634,3 +634,61 @@ def test_trace_runner_as_a_child_process(tmp_path, dtype):
         got.append(torch.from_numpy(arr.copy()))
         want += [refs[i][p] for i, p in rows]
     close(torch.cat(got), torch.stack(want), dtype, "trace")
+
+
+@pytest.mark.parametrize("d,pairs,vd,H,G,norm_first", [
+    (64, 32, 64, 5, 1, False),       # a quarter of a warp a head
+    (128, 64, 128, 16, 4, True),     # half a warp
+    (128, 16, 96, 3, 3, False),      # entries behind the rotated part, in whole eights
+    (100, 4, 20, 70, 2, True),       # ... with four left over; more heads than a block's groups
+    (36, 0, 7, 2, 1, False),         # nothing rotated; values that are no quads
+    (256, 128, 256, 33, 1, False),   # a warp a head
+    (60, 6, 12, 2, 2, True),         # a rotated part that is no quads: the general kernel
+])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_prepared_queries_and_keys_over_head_sizes(dtype, d, pairs, vd, H, G, norm_first):
+    """Every way that the kernel deals a head's entries to lanes, with bias, norm, gains, temperature and mixed values, against
+    float64 on the same inputs. float32: a sum of d squares and four roundings, below 2e-6 of an entry's scale; bfloat16: one
+    rounding (2^-8 of the entry) of results, two of mixed values."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.base import CacheNeed
+    k, dt, T, eps = K(), tdtype(dtype), 67, 1e-5
+    g = torch.Generator().manual_seed(d + pairs)
+    width = (H + G) * d + G * vd
+    proj = torch.randn(T, width + (4 if d != 36 else 1), generator=g).to(dt)
+    bias, first = 0.3 * torch.randn(width, generator=g), torch.randn(T, G * vd, generator=g).to(dt)
+    gains = [1 + 0.2 * torch.randn(d, generator=g) for _ in range(2)]
+    angle = 6 * torch.rand(T, max(pairs, 1), generator=g, dtype=torch.float64)
+    cos, sin = angle.cos().float(), angle.sin().float()
+    cache = Cache([(0, CacheNeed("full", G, d, v_head_dim=vd), None)], 128, dt, "cuda")
+    s = cache.open()
+    ctx = StepContext(cache, [s], [[0] * T], 1, [[]])
+    k_pool, v_pool, _ = cache.entry_storage(0)
+    q, kept = k.rope_norm_store(proj.cuda(), bias.cuda(), k_pool, v_pool, ctx.batch_c[0], (cos.cuda(), sin.cuda()) if pairs else None,
+                                H, G, d, vd, eps, unit_norm=True, v_first=first.cuda(), lam=torch.tensor(0.35, device="cuda"),
+                                keep_values=True, norm_first=norm_first, q_temp=(0.1, 16),
+                                **(dict(q_gain=gains[0].cuda(), k_gain=gains[1].cuda()) if norm_first else {}))
+    x = proj[:, :width].double() + bias.double()
+    qk = x[:, :(H + G) * d].view(T, H + G, d)
+
+    def rms(y):
+        return y / (y.square().mean(-1, keepdim=True) + eps).sqrt()
+
+    if norm_first:
+        qk = rms(qk) * torch.cat([gains[0].double().expand(H, d), gains[1].double().expand(G, d)])
+    if pairs:
+        c, sn = cos.double()[:, None], sin.double()[:, None]
+        a, b = qk[..., :pairs], qk[..., pairs:2 * pairs]
+        qk = torch.cat([a * c - b * sn, b * c + a * sn, qk[..., 2 * pairs:]], -1)
+    if not norm_first:
+        qk = rms(qk)
+    temp = 1 + 0.1 * torch.log(torch.floor((torch.arange(T).double() + 1) / 16) + 1)
+    pages = cache.pages(s, 0)
+    rows = lambda pool: torch.cat([pool[p].transpose(0, 1) for p in pages])[:T]
+    v = x[:, (H + G) * d:].view(T, G, vd)
+    rtol = dict(rtol=2e-6, atol=4e-6) if dtype == "float32" else dict(rtol=2.0 ** -8, atol=2.0 ** -14)
+    mixed = dict(rtol=2e-6, atol=4e-6) if dtype == "float32" else dict(rtol=2.0 ** -8, atol=2.0 ** -8 * 0.65 * float(v.abs().max()))
+    for got, want, t in ((q, qk[:, :H] * temp[:, None, None], rtol), (rows(k_pool), qk[:, H:], rtol), (kept.view(T, G, vd), v, rtol),
+                         (rows(v_pool), 0.65 * v + 0.35 * first.double().view(T, G, vd), mixed)):
+        torch.testing.assert_close(got.double().cpu(), want, **t)
