@@ -567,10 +567,10 @@ def falcon_beside(size):
 class KernelTimes:
     """Times every call of the kernel module's entry points with a pair of CUDA events while it is on."""
     NAMES = ("gather_rows", "norm", "norm_stream", "add_stream", "residual", "bias_act_", "to_float", "matmul_nt",
-             "skinny_linear", "linear_f32", "rope_table", "split_rotate_store", "attention_tc", "attention_mma",
+             "skinny_linear", "linear_f32", "rope_table", "split_rotate_store", "attention_tc", "attention_tc_extras", "attention_mma",
              "attention_generic", "attention_decode", "attention_decode_tc", "latent_store", "latent_attention",
              "latent_unfolded_attention",
-             "latent_expand", "block_linear", "rglru_conv", "rglru_scan", "rglru_scan_chunks", "route", "routed_experts", "scale_",
+             "latent_expand", "block_linear", "block_product", "skinny_linear_split", "rglru_conv", "rglru_scan", "rglru_scan_chunks", "route", "routed_experts", "scale_",
              "embed_sum", "post_norm_add", "qk_norm_store", "linear_attention", "norm_gate", "glu_clamp", "softcap_",
              "dyt", "mlstm", "head_norm_gate", "rope_norm_store", "talk_mix", "embed_rows", "gla", "gla_decay_", "glu_act",
              "delta_prepare", "delta_rule", "expert_rows", "post_norm", "post_norm_pair", "post_norm_experts", "norm_add", "token_gate",
@@ -793,7 +793,7 @@ def run_zalunex(args):
 
     roof = {}
     seen = sum(min(t + 1, l["mask"]["size"]) for t in range(tokens))        # (query, key) pairs inside the window
-    for key in ("attention_generic", "attention_mma"):
+    for key in ("attention_generic", "attention_mma", "attention_tc_extras"):
         t = per_call(Z["prefill_kernels_ms"], key)
         if t:
             roof[f"sink_{key}_prefill_TFLOPs"] = round(l["heads"] * seen * 2 * (l["dim"] + l["vdim"]) / t / 1e9, 1)
@@ -895,7 +895,7 @@ def run_pogezen(args):
     keep, size = att["mask"]["keep_first"], att["mask"]["size"]
     seen = sum(min(t + 1, size) + max(0, min(keep, t + 1 - size)) for t in range(tokens))     # visible (query, key) pairs
     # the attention with mixed weights: scores of every head, then every head's weights on every K/V head's values
-    for key in ("attention_generic", "attention_mma"):
+    for key in ("attention_generic", "attention_mma", "attention_tc_extras"):
         t = per_call(G["prefill_kernels_ms"], key)
         if t:
             roof[f"talk_{key}_prefill_TFLOPs_as_run"] = round(H * seen * 2 * (d + K * vd) / t / 1e9, 1)
@@ -1010,7 +1010,7 @@ def run_figudra(args):
     full = tokens * (tokens + 1) // 2                                                         # pairs the full layer sees
     zl, zr = zalunex_config(args.size)["layers"][0]["mixer"]["left"], zalunex_config(args.size)["layers"][0]["mixer"]["right"]
     zseen = sum(min(t_ + 1, zl["mask"]["size"]) for t_ in range(tokens))
-    for key in ("attention_generic", "attention_mma"):
+    for key in ("attention_generic", "attention_mma", "attention_tc_extras"):
         t = F["prefill_kernels_ms"].get(key)
         if t:   # one windowed layer and one full layer share the kernel and the table's row
             roof[f"{key}_prefill_TFLOPs"] = round(H * (seen + full) * 2 * (d + vd) / t["ms"] / 1e9, 1)
@@ -1235,9 +1235,9 @@ def run_vabedra(args):
     keep, size = left["mask"]["keep_first"], left["mask"]["size"]
     seen = sum(min(t + 1, size) + max(0, min(keep, t + 1 - size)) for t in range(tokens))
     full = tokens * (tokens + 1) // 2
-    rate("attention_prefill", per_call(V, "attention_mma"), flops=H * seen * 2 * (d + vd))
-    if "attention_mma" in F:    # one windowed and one full layer share the table's row
-        rate("figudra_attention_prefill", F["attention_mma"]["ms"], flops=H * (seen + full) * 2 * (d + vd))
+    rate("attention_prefill", per_call(V, "attention_tc_extras"), flops=H * seen * 2 * (d + vd))
+    if "attention_tc_extras" in F:    # one windowed and one full layer share the table's row
+        rate("figudra_attention_prefill", F["attention_tc_extras"]["ms"], flops=H * (seen + full) * 2 * (d + vd))
     # the delta rule: queries, keys and values in, decays in (per channel in two layers, per head in two), float32 rows out;
     # what it needs a token and head: the read at the key, the write and the read at the query, 3 dim vdim multiply-adds
     lh, ld, lv = right["heads"], right["dim"], right["vdim"]
