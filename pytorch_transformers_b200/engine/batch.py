@@ -144,7 +144,7 @@ class StepContext:
                 logits_at.append(int(seq_start[b]) + int(i))
         self.n_wanted = len(logits_at)
         # every token's row in order (a step of single tokens, say): the last rows need not be gathered
-        self.all_wanted = logits_at == list(range(self.n_tokens))
+        self.all_wanted = self.n_wanted == self.n_tokens and logits_at == list(range(self.n_tokens))
 
         # what the mixers' planners add (parts that share a plan_key share one plan); they see the
         # counts and positions above, and run before anything is reserved
