@@ -19,6 +19,14 @@ __device__ __forceinline__ void split_pack(float x, float y, uint32_t& hi, uint3
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
+// the same in three terms, which hold all 24 bits of a float32 value
+__device__ __forceinline__ void split3_pack(float x, float y, uint32_t& first, uint32_t& second, uint32_t& third) {
+  const __nv_bfloat16 xh = __float2bfloat16_rn(x), yh = __float2bfloat16_rn(y);
+  const __nv_bfloat162 h = __halves2bfloat162(xh, yh);
+  first = *reinterpret_cast<const uint32_t*>(&h);
+  split_pack(x - __bfloat162float(xh), y - __bfloat162float(yh), second, third);
+}
+
 // 8 values of a projection row (one 16-byte word) activated: float32 values rounded to bfloat16
 __device__ __forceinline__ void act8(const uint4& w, int act_silu, float (&f)[8]) {
   unpack_bf16x8(w, f);

@@ -12,9 +12,10 @@
 // ahead, and the warps' partial outputs meet there in a fixed order. It runs in three roles: over a sequence's new
 // tokens from and to the state area (steps of any length); over one chunk of 64 tokens from zero, leaving the
 // chunk's own sum and its total decay (pass 1 of the chunked form); over one chunk from the state before it, with
-// outputs (pass 3). Pass 2 joins the chunks of a sequence in order. The chunked form differs from the plain walk by
-// the order of float32 operations only. With bfloat16 projections and keys and values of 64 or 128 entries passes 1
-// and 3 run on the tensor cores instead (csrc/gla_mma.cu: float32 operands enter a product as two bfloat16 terms).
+// outputs (pass 3). Pass 2 joins the chunks of a sequence in order. In these roles the chunked form differs from the plain
+// walk by the order of float32 operations only. With bfloat16 projections and keys and values of 64 or 128 entries passes 1
+// and 3 run on the tensor cores instead (csrc/gla_mma.cu): there float32 operands enter a product as bfloat16 terms, two
+// in pass 1 (the decayed keys, 16 bits) and three in pass 3 (24 bits).
 #include "common.cuh"
 
 namespace {

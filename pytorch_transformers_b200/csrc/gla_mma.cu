@@ -138,12 +138,16 @@ int launch_sum(const void* proj, int stride, const float* log_decay, const StepB
 // most 1, nothing is subtracted, and the scores are a product. Inside a sub-block every (t, i, channel) has an exponent of its
 // own: a warp walks t from i on with its lanes' channels' sums in registers. That is what bounds the kernel: 136 (t, i) pairs a sub-block and
 // channel, 70,000 exponentials a block against 16 a clock and SM, and the instructions around them. 2,900 tokens of
-// 16 heads of 128 x 128: 94 us, where the walk on the CUDA cores took 175.
-// Operands of a product that are float32 (scaled queries and keys, scores, the state) enter it as two bfloat16 terms (the product
-// of two such operands leaves out lo x lo, 2^-18 of it).
-// One block = one chunk x one head, 8 warps; 101 KB of shared memory, two blocks an SM:
-//     tiles of q, k (then the keys' hi terms, then the state's quarters), the keys' lo terms (then v), the logarithms (then
-//     their sums inside a sub-block up to t), the scores.
+// 16 heads of 128 x 128: 117 us (94 with operands of two terms), where the walk on the CUDA cores took 175.
+// Operands of a product that are float32 (scaled queries and keys, scores, the state) enter it as three bfloat16 terms, 24 bits: what
+// a product leaves out (second x third, third x third) is 2^-26 of it, below the rounding of its float32 sum. A matrix instruction
+// cuts its sum off instead of rounding it, so the six products of 16 entries are summed from zero, the small ones first, and
+// join the running sum by a rounded addition. With two terms the outputs of one chunk from a given state were 4e-6 off 64
+// bits, with three into one running sum 1e-6, where the walk in float32 is 2e-7 off.
+// One block = one chunk x one head, 8 warps; 112.5 KB of shared memory, two blocks an SM:
+//     tiles of q, k (then the keys' first terms, then two terms of the state's quarters), the keys' second terms (then v), the
+//     third terms of the keys of the first three sub-blocks (nothing reads the last one's scaled; then the state's), the
+//     logarithms (then their sums inside a sub-block up to t), the scores.
 constexpr int SUB = 16, SUBS = CH / SUB, SPITCH = CH + 4;     // tokens of a sub-block; pitch of the scores' rows
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -151,7 +155,9 @@ template <int DK, int DV>
 struct OutShape {
   static constexpr int LP = DK + 8;                            // floats from one token's logarithms to the next's
   static constexpr int A_BYTES = CH * (DK > DV ? DK : DV) * 2; // a tile, also of v or of a quarter of the state (two terms)
-  static constexpr size_t SMEM = size_t(CH) * DK * 2 + 2 * size_t(A_BYTES) + size_t(CH) * LP * 4 + size_t(SUBS) * DK * 4 + size_t(CH) * SPITCH * 4;
+  static constexpr int C_BYTES = (CH - SUB) * DK * 2;          // third terms: of 48 keys, or of a quarter of the state
+  static constexpr size_t SMEM =
+      size_t(CH) * DK * 2 + 2 * size_t(A_BYTES) + C_BYTES + size_t(CH) * LP * 4 + size_t(SUBS - 1) * DK * 4 + size_t(CH) * SPITCH * 4;
 };
 
 __device__ __forceinline__ float2 pair_f(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
@@ -167,10 +173,11 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* q_s = sm;                                  // [CH][DK]
   unsigned char* k_s = q_s + CH * DK * 2;                   // [CH][DK] k, then the scaled keys' hi terms, then quarters of the state
-  unsigned char* b_s = k_s + Shape::A_BYTES;                // [CH][DK] the scaled keys' lo terms, then [CH][DV] v
-  float* l_s = reinterpret_cast<float*>(b_s + Shape::A_BYTES);   // [CH][LP] logarithms (powers of two), then sums up to t
-  float* t_s = l_s + CH * LP;                               // [SUBS][DK] a sub-block's sum
-  float* s_s = t_s + SUBS * DK;                             // [CH][SPITCH] scores
+  unsigned char* b_s = k_s + Shape::A_BYTES;                // [CH][DK] the scaled keys' second terms, then [CH][DV] v
+  unsigned char* c_s = b_s + Shape::A_BYTES;                // [CH - SUB][DK] their third terms, then a quarter of the state's
+  float* l_s = reinterpret_cast<float*>(c_s + Shape::C_BYTES);   // [CH][LP] logarithms (powers of two), then sums up to t
+  float* t_s = l_s + CH * LP;                               // [SUBS - 1][DK] a sub-block's sum (nothing follows the last)
+  float* s_s = t_s + (SUBS - 1) * DK;                             // [CH][SPITCH] scores
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp8 = tid >> 5, warp = warp8 & 3, half = warp8 >> 2;
   const int seq = chunk_seq[c], q0 = chunk_q0[c];
   const int start = sb.seq_start[seq] + q0, n = min(CH, sb.seq_new[seq] - q0);
@@ -250,7 +257,8 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
     }
   }
   __syncthreads();
-  // the sums inside sub-blocks: up to t in place of the logarithms, and what follows i into the keys (two terms)
+  // the sums inside sub-blocks: up to t in place of the logarithms, and what follows i into the keys (three terms; no later
+  // sub-block meets the last one's keys)
   for (int u = tid; u < SUBS * DK; u += 256) {
     const int sub = u / DK, ch = u % DK;
     float l[SUB], up = 0.f;
@@ -261,28 +269,32 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
       up += l[t];
       l_s[(sub * SUB + t) * LP + ch] = up;
     }
+    if (sub == SUBS - 1) continue;
     t_s[sub * DK + ch] = up;
     float rest = 0.f;
 #pragma unroll
     for (int t = SUB - 1; t >= 0; --t) {
       const uint32_t at = swz<DK>(sub * SUB + t, ch / 8) + (ch % 8) * 2;
       const float k = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(k_s + at)) * fast_exp2(rest);
-      const __nv_bfloat16 hi = __float2bfloat16_rn(k);
-      *reinterpret_cast<__nv_bfloat16*>(k_s + at) = hi;
-      *reinterpret_cast<__nv_bfloat16*>(b_s + at) = __float2bfloat16_rn(k - __bfloat162float(hi));
+      const __nv_bfloat16 first = __float2bfloat16_rn(k);
+      const float left = k - __bfloat162float(first);
+      const __nv_bfloat16 second = __float2bfloat16_rn(left);
+      *reinterpret_cast<__nv_bfloat16*>(k_s + at) = first;
+      *reinterpret_cast<__nv_bfloat16*>(b_s + at) = second;
+      *reinterpret_cast<__nv_bfloat16*>(c_s + at) = __float2bfloat16_rn(left - __bfloat162float(second));
       rest += l[t];
     }
   }
   StagedWords<DV, 256> vw;      // on their way under the scores between sub-blocks
   vw.load(row0 + 2 * heads * DK + h * DV, stride, n, tid);
   __syncthreads();
-  const uint32_t ks = smem_u32(k_s), bs = smem_u32(b_s);
+  const uint32_t ks = smem_u32(k_s), bs = smem_u32(b_s), cs = smem_u32(c_s);
   const int g4 = lane >> 2, t4 = lane & 3, m = lane >> 3;
   // two neighbouring channels (ch, ch + 1) of query row r, times exp2(sum up to r in its sub-block + extra)
-  auto scaled_q = [&](int r, int ch, float2 extra, uint32_t& hi, uint32_t& lo) {
+  auto scaled_q = [&](int r, int ch, float2 extra, uint32_t& q1, uint32_t& q2, uint32_t& q3) {
     const float2 q = pair_f(*reinterpret_cast<const uint32_t*>(q_s + swz<DK>(r, ch / 8) + (ch % 8) * 2));
     const float2 e = *reinterpret_cast<const float2*>(l_s + r * LP + ch);
-    split_pack(q.x * fast_exp2(e.x + extra.x), q.y * fast_exp2(e.y + extra.y), hi, lo);
+    split3_pack(q.x * fast_exp2(e.x + extra.x), q.y * fast_exp2(e.y + extra.y), q1, q2, q3);
   };
   if (warp8 < 6) {      // scores of sub-block w with the keys of sub-block u < w: a pair a warp
     const int w = warp8 == 0 ? 1 : warp8 < 3 ? 2 : 3, u = warp8 == 0 ? 0 : warp8 < 3 ? warp8 - 1 : warp8 - 3;
@@ -291,7 +303,7 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
 #pragma unroll
     for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
     for (int kk = 0; kk < DK / 16; ++kk) {
-      uint32_t qh[4], ql[4];
+      uint32_t q1[4], q2[4], q3[4];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         const int ch = kk * 16 + 8 * x + 2 * t4;
@@ -301,19 +313,29 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
           mid.x += t.x;
           mid.y += t.y;
         }
-        scaled_q(r_lo, ch, mid, qh[2 * x], ql[2 * x]);
-        scaled_q(r_hi, ch, mid, qh[2 * x + 1], ql[2 * x + 1]);
+        scaled_q(r_lo, ch, mid, q1[2 * x], q2[2 * x], q3[2 * x]);
+        scaled_q(r_hi, ch, mid, q1[2 * x + 1], q2[2 * x + 1], q3[2 * x + 1]);
       }
-      uint32_t h0, h1, h2, h3, l0, l1, l2, l3;      // keys 0..7 and 8..15 of the sub-block, 16 channels each
+      uint32_t b0, b1, b2, b3, d0, d1, d2, d3;      // keys 0..7 and 8..15 of the sub-block, 16 channels each
       const uint32_t off = swz<DK>(u * SUB + (m >> 1) * 8 + (lane & 7), kk * 2 + (m & 1));
-      ldmatrix_x4(h0, h1, h2, h3, ks + off);
-      ldmatrix_x4(l0, l1, l2, l3, bs + off);
-      mma_bf16(s[0], qh, h0, h1);
-      mma_bf16(s[1], qh, h2, h3);
-      mma_bf16(s[0], qh, l0, l1);
-      mma_bf16(s[1], qh, l2, l3);
-      mma_bf16(s[0], ql, h0, h1);
-      mma_bf16(s[1], ql, h2, h3);
+      float x0[4] = {0.f, 0.f, 0.f, 0.f}, x1[4] = {0.f, 0.f, 0.f, 0.f};
+      ldmatrix_x4(b0, b1, b2, b3, cs + off);
+      mma_bf16(x0, q1, b0, b1);
+      mma_bf16(x1, q1, b2, b3);
+      ldmatrix_x4(b0, b1, b2, b3, bs + off);
+      mma_bf16(x0, q2, b0, b1);
+      mma_bf16(x1, q2, b2, b3);
+      ldmatrix_x4(d0, d1, d2, d3, ks + off);
+      mma_bf16(x0, q3, d0, d1);
+      mma_bf16(x1, q3, d2, d3);
+      mma_bf16(x0, q1, b0, b1);
+      mma_bf16(x1, q1, b2, b3);
+      mma_bf16(x0, q2, d0, d1);
+      mma_bf16(x1, q2, d2, d3);
+      mma_bf16(x0, q1, d0, d1);
+      mma_bf16(x1, q1, d2, d3);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[0][e] += x0[e], s[1][e] += x1[e];
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -342,29 +364,31 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
 #pragma unroll
   for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
   const int r_lo = warp * SUB + g4, r_hi = r_lo + 8, j0 = half * NT;      // this thread's two tokens; the warp's first n-tile
-  unsigned char* s_hi = k_s;                      // [QR][DV]
-  unsigned char* s_lo = k_s + QR * DV * 2;
-  const uint32_t shi = smem_u32(s_hi), slo = smem_u32(s_lo);
+  unsigned char* s_1 = k_s;                       // [QR][DV], the three terms
+  unsigned char* s_2 = k_s + QR * DV * 2;
+  unsigned char* s_3 = c_s;
+  const uint32_t ss1 = smem_u32(s_1), ss2 = smem_u32(s_2), ss3 = smem_u32(s_3);
 #pragma unroll 1
   for (int quarter = 0; quarter < 4; ++quarter) {
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       const int i = tid + u * 256, row = i / CHUNKS, cc = i % CHUNKS;
       if (i < QR * CHUNKS) {
-        uint4 hi, lo;
-        split_pack(sx[u].x, sx[u].y, hi.x, lo.x);
-        split_pack(sx[u].z, sx[u].w, hi.y, lo.y);
-        split_pack(sy[u].x, sy[u].y, hi.z, lo.z);
-        split_pack(sy[u].z, sy[u].w, hi.w, lo.w);
-        *reinterpret_cast<uint4*>(s_hi + swz<DV>(row, cc)) = hi;
-        *reinterpret_cast<uint4*>(s_lo + swz<DV>(row, cc)) = lo;
+        uint4 a, b, d;
+        split3_pack(sx[u].x, sx[u].y, a.x, b.x, d.x);
+        split3_pack(sx[u].z, sx[u].w, a.y, b.y, d.y);
+        split3_pack(sy[u].x, sy[u].y, a.z, b.z, d.z);
+        split3_pack(sy[u].z, sy[u].w, a.w, b.w, d.w);
+        *reinterpret_cast<uint4*>(s_1 + swz<DV>(row, cc)) = a;
+        *reinterpret_cast<uint4*>(s_2 + swz<DV>(row, cc)) = b;
+        *reinterpret_cast<uint4*>(s_3 + swz<DV>(row, cc)) = d;
       }
     }
     __syncthreads();      // this quarter (and v) is staged
     if (quarter < 3) load_state(quarter + 1);
 #pragma unroll
     for (int kk = 0; kk < QR / 16; ++kk) {
-      uint32_t qh[4], ql[4];
+      uint32_t q1[4], q2[4], q3[4];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         const int ch = quarter * QR + kk * 16 + 8 * x + 2 * t4;
@@ -374,21 +398,31 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
           front.x += t.x;
           front.y += t.y;
         }
-        scaled_q(r_lo, ch, front, qh[2 * x], ql[2 * x]);
-        scaled_q(r_hi, ch, front, qh[2 * x + 1], ql[2 * x + 1]);
+        scaled_q(r_lo, ch, front, q1[2 * x], q2[2 * x], q3[2 * x]);
+        scaled_q(r_hi, ch, front, q1[2 * x + 1], q2[2 * x + 1], q3[2 * x + 1]);
       }
 #pragma unroll
       for (int j = 0; j < NT; j += 2) {
-        uint32_t b0, b1, b2, b3;
+        uint32_t b0, b1, b2, b3, d0, d1, d2, d3;
+        float x0[4] = {0.f, 0.f, 0.f, 0.f}, x1[4] = {0.f, 0.f, 0.f, 0.f};
         const uint32_t off = swz<DV>(kk * 16 + (m & 1) * 8 + (lane & 7), j0 + j + (m >> 1));
-        ldmatrix_x4_trans(b0, b1, b2, b3, shi + off);
-        mma_bf16(o[j], qh, b0, b1);
-        mma_bf16(o[j + 1], qh, b2, b3);
-        mma_bf16(o[j], ql, b0, b1);
-        mma_bf16(o[j + 1], ql, b2, b3);
-        ldmatrix_x4_trans(b0, b1, b2, b3, slo + off);
-        mma_bf16(o[j], qh, b0, b1);
-        mma_bf16(o[j + 1], qh, b2, b3);
+        ldmatrix_x4_trans(b0, b1, b2, b3, ss3 + off);
+        mma_bf16(x0, q1, b0, b1);
+        mma_bf16(x1, q1, b2, b3);
+        ldmatrix_x4_trans(b0, b1, b2, b3, ss2 + off);
+        mma_bf16(x0, q2, b0, b1);
+        mma_bf16(x1, q2, b2, b3);
+        ldmatrix_x4_trans(d0, d1, d2, d3, ss1 + off);
+        mma_bf16(x0, q3, d0, d1);
+        mma_bf16(x1, q3, d2, d3);
+        mma_bf16(x0, q1, b0, b1);
+        mma_bf16(x1, q1, b2, b3);
+        mma_bf16(x0, q2, d0, d1);
+        mma_bf16(x1, q2, d2, d3);
+        mma_bf16(x0, q1, d0, d1);
+        mma_bf16(x1, q1, d2, d3);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] += x0[e], o[j + 1][e] += x1[e];
       }
     }
     __syncthreads();      // the quarter is no longer read
@@ -396,22 +430,27 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
 #pragma unroll
   for (int kb = 0; kb < SUBS; ++kb) {
     if (kb > warp) break;
-    uint32_t ph[4], pl[4];
+    uint32_t p1[4], p2[4], p3[4];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
       const float2 a = *reinterpret_cast<const float2*>(s_s + r_lo * SPITCH + kb * 16 + 8 * x + 2 * t4);
       const float2 b = *reinterpret_cast<const float2*>(s_s + r_hi * SPITCH + kb * 16 + 8 * x + 2 * t4);
-      split_pack(a.x, a.y, ph[2 * x], pl[2 * x]);
-      split_pack(b.x, b.y, ph[2 * x + 1], pl[2 * x + 1]);
+      split3_pack(a.x, a.y, p1[2 * x], p2[2 * x], p3[2 * x]);
+      split3_pack(b.x, b.y, p1[2 * x + 1], p2[2 * x + 1], p3[2 * x + 1]);
     }
 #pragma unroll
     for (int j = 0; j < NT; j += 2) {
       uint32_t b0, b1, b2, b3;
       ldmatrix_x4_trans(b0, b1, b2, b3, bs + swz<DV>(kb * 16 + (m & 1) * 8 + (lane & 7), j0 + j + (m >> 1)));
-      mma_bf16(o[j], ph, b0, b1);
-      mma_bf16(o[j], pl, b0, b1);
-      mma_bf16(o[j + 1], ph, b2, b3);
-      mma_bf16(o[j + 1], pl, b2, b3);
+      float x0[4] = {0.f, 0.f, 0.f, 0.f}, x1[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_bf16(x0, p3, b0, b1);
+      mma_bf16(x1, p3, b2, b3);
+      mma_bf16(x0, p2, b0, b1);
+      mma_bf16(x1, p2, b2, b3);
+      mma_bf16(x0, p1, b0, b1);
+      mma_bf16(x1, p1, b2, b3);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] += x0[e], o[j + 1][e] += x1[e];
     }
   }
 #pragma unroll

@@ -302,6 +302,44 @@ def test_chunk_sums_on_the_tensor_cores(d, vd):
         assert (left - refs[i][1]).norm() < 1e-5 * refs[i][1].norm()
 
 
+@pytest.mark.parametrize("d,vd", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_outputs_of_one_chunk_in_32_bits(d, vd):
+    """Kernel alone: sequences of one chunk each (1 to 64 tokens, the edges of its sub-blocks of 16) after a state of earlier
+    tokens, so that only the pass of the outputs rounds. Its products take their float32 operands whole: what is left is
+    the exponentials' 2^-22 and the float32 sums' few roundings of 2^-24, together below 2^-20 of a row; with operands cut
+    to 16 bits a row is off by more than three times that."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.base import StateNeed
+    k = K()
+    H, lengths = 2, [64, 1, 15, 16, 17, 33, 48, 49, 63]
+    g = torch.Generator().manual_seed(d + 3 * vd)
+    n = sum(lengths)
+    q, kk, v = (bf16_exact(torch.randn(n, H, x, generator=g)).float() for x in (d, d, vd))
+    la = -torch.rand(n, H, d, generator=g) * 0.05
+    la[:, :, 0] = 0.0                   # never decays
+    la[:, :, 1] = -6.0                  # all but gone after one token
+    before = torch.randn(len(lengths), H, d, vd, generator=g) * 3.0
+    cache = Cache([(0, None, StateNeed(H * d * vd))], 64 * len(lengths), torch.bfloat16, "cuda", max_slots=len(lengths))
+    slots = [cache.open() for _ in lengths]
+    ctx = StepContext(cache, slots, [[0] * L for L in lengths], 1, [[]] * len(lengths), [])
+    state = torch.zeros(cache.state.shape[0], H * d * vd, device="cuda")
+    for i, slot in enumerate(slots):
+        state[slot] = before[i].reshape(-1).cuda()
+    index = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    chunks = (index(range(len(lengths))), index([0] * len(lengths)), index(range(len(lengths))), len(lengths))
+    proj = torch.cat([q.reshape(n, -1), kk.reshape(n, -1), v.reshape(n, -1)], 1).bfloat16().cuda()
+    got = k.gla(proj, la.reshape(n, -1).cuda().contiguous(), state, ctx.dev["slots"], ctx.batch_c[0], H, d, vd, d ** -0.5, chunks)
+    refs, lo = [], 0
+    for i, L in enumerate(lengths):
+        S = before[i].double()
+        for t in range(lo, lo + L):
+            S = la[t].double().exp()[:, :, None] * S + kk[t].double()[:, :, None] * v[t].double()[:, None, :]
+            refs.append(torch.einsum("hd,hdv->hv", q[t].double() * d ** -0.5, S).reshape(-1))
+        lo += L
+    assert row_errors(got, torch.stack(refs)).max() < 2.0 ** -20, row_errors(got, torch.stack(refs)).max()
+
+
 # ------------------------------------------------------------------------------------------------ the attentions
 def capped_spec(m, width, p="mix."):
     from pytorch_transformers_b200.parts.base import PartSpec
