@@ -49,15 +49,6 @@ __device__ __forceinline__ void arrive_when_copied(uint32_t bar) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// gated_unit with the fast exponential and division (relative error about 1e-6, under a result rounded to 2^-9)
-__device__ __forceinline__ float gated_unit_fast(float gate, float up, float limit, float alpha) {
-  if (limit > 0.f) {
-    const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-    return __fdividef(g, 1.f + __expf(-alpha * g)) * (u + 1.f);
-  }
-  return __fdividef(gate, 1.f + __expf(-gate)) * up;
-}
-
 struct ExpertTcParams {
   const __nv_bfloat16* x;
   void* out;
@@ -200,7 +191,7 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
         float u[8];
         tmem_ld8(lane_addr + p.acc2 + g * 8, u);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = gated_unit_fast(v[j], u[j], p.glu_limit, p.glu_alpha);
+        for (int j = 0; j < 8; ++j) v[j] = gated_unit(v[j], u[j], p.glu_limit, p.glu_alpha);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {

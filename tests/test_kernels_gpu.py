@@ -417,3 +417,30 @@ def test_chain_of_launches_keeps_the_streams_order(K, width):
         x.copy_(x0)
         graph.replay()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("clamp", [None, (7.0, 1.702)])
+def test_expert_units_at_large_gates(K, clamp):
+    """Gates of either sign beyond where the exponential leaves float32 (results stay finite: an infinite one would meet the
+    zeros of the second matrix), among them those whose 1 + exp(-gate) lies
+    between 2^126 and 2^128: the unit is the float32 formula with a true division, rounded once to bfloat16 (2^-8 of
+    itself beside the exponential's few units of 2^-24)."""
+    g = torch.tensor([0.0, 1e-3, 0.5, 1.0, 3.0, 20.0, 50.0, 80.0, 86.0, 87.0, 87.5, 88.0, 88.5, 100.0, 1e4, 1e6])
+    g = torch.cat([g, -g]).repeat_interleave(3).bfloat16()
+    u = torch.tensor([1.0, 1e30, -3e4]).repeat(g.numel() // 3).bfloat16()
+    h = torch.zeros(g.numel(), 8, dtype=torch.bfloat16)
+    h[:, 0], h[:, 1] = g, u
+    w = torch.zeros(1, 16, 8, dtype=torch.bfloat16)
+    w[0, :8, 0], w[0, 8:, 1] = 1.0, 1.0
+    down = torch.eye(8, dtype=torch.bfloat16)[None].contiguous()
+    y, rows = K.expert_rows(h.cuda(), torch.zeros(g.numel(), 1, dtype=torch.int32, device="cuda"), w.cuda(), down.cuda(), clamp=clamp)
+    got = y[rows.long()].cpu()
+    g, u = g.float(), u.float()
+    if clamp is not None:
+        g, u, alpha = g.clamp(max=clamp[0]), u.clamp(-clamp[0], clamp[0]) + 1.0, clamp[1]
+    else:
+        alpha = 1.0
+    ref = g / (1.0 + torch.exp(-alpha * g)) * u
+    # what is smaller than float32's normal numbers may be flushed to zero
+    for f in range(8):
+        torch.testing.assert_close(got[:, f], ref.bfloat16().float(), rtol=2.0 ** -8, atol=2.0 ** -126, equal_nan=True)
