@@ -417,13 +417,8 @@ int launch_decode(const void* fused, void* k_pool, void* v_pool, void* out, cons
   size_t smem = ring + size_t(p.hpk + 2) * D * 2 + size_t(D) * sizeof(float);
   const size_t join = size_t(KS) * warps * 16 * (D + 2) * sizeof(float);  // partial results reuse the ring
   if (join > smem) smem = join;
-  static size_t configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(attention_decode_kernel<D, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-        cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(attention_decode_kernel<D, KS>, smem)) return PTB_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(sb.n_seqs, p.kv_heads * chunks, p.n_splits * p.n_teams);
   cfg.blockDim = dim3(warps * KS * 32);

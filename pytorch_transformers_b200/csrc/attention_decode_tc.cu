@@ -538,14 +538,8 @@ static size_t decode_tc_smem() {
   return 1024 + TILE_Q + 2 * STAGES_D * TILE_KV + size_t(ROWS + 2) * DD * 2 + DD * sizeof(float) + 256;
 }
 static bool decode_tc_configure() {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_decode_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(decode_tc_smem())) != cudaSuccess)
-      return false;
-    configured = true;
-  }
-  return true;
+  static SharedLimit limit;
+  return limit.allows(attention_decode_tc_kernel, decode_tc_smem());
 }
 
 // Every sequence of the step brings exactly one token. fused [n_seqs, kv_heads * (q_per_kv + 2) * 64]

@@ -673,13 +673,8 @@ int launch_attention(const void* q, const void* k_pool, const void* v_pool, void
   dim3 grid(n_tiles, heads, out_wide ? kv_heads : 1);
 #define PTB_AG(CC)                                                                                                              \
   do {                                                                                                                          \
-    static size_t configured = 48 * 1024; /* per instance: raised when a larger head size first comes */                       \
-    if (smem > configured) {                                                                                                    \
-      if (cudaFuncSetAttribute(attention_generic_kernel<T, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=      \
-          cudaSuccess)                                                                                                          \
-        return PTB_ERR_LAUNCH;                                                                                                  \
-      configured = smem;                                                                                                        \
-    }                                                                                                                           \
+    static SharedLimit limit;                                                                                                   \
+    if (!limit.allows(attention_generic_kernel<T, CC>, smem)) return PTB_ERR_LAUNCH;                                            \
     launch_pdl(attention_generic_kernel<T, CC>, grid, THREADS, smem, stream,                                                            \
         (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, sb, tile_seq, tile_q0, slopes, heads, kv_heads, head_dim,     \
         scale, window, v_dim, sinks, (const T*)gate, gate_stride, out_scale, out_stride, keep_first, out_wide, softcap,         \

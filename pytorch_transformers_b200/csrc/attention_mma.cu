@@ -8,7 +8,6 @@
 // page), double-buffered through shared memory with cp.async into a 16-byte XOR swizzle that makes
 // the ldmatrix reads conflict-free. With n_splits > 1 the pages of a sequence are divided among
 // gridDim.z blocks which write unnormalised partial results; attention_mma_reduce joins them.
-#include <mutex>
 #include "mma_common.cuh"
 
 namespace {
@@ -394,21 +393,8 @@ int launch_mma(const void* q, const void* k_pool, const void* v_pool, void* out,
   const int qpk = p.heads / p.kv_heads;
   const int chunks = (qpk + p.hpk - 1) / p.hpk;
   const size_t smem = size_t(2) * 2 * KEYS * D * 2;  // two stages of (K, V)
-  // the kernel's limit of dynamic shared memory is raised once per device and head size (a function
-  // attribute belongs to the device's context), by whichever thread comes first
-  {
-    static std::mutex mutex;
-    static bool configured[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return PTB_ERR_LAUNCH;
-    std::lock_guard<std::mutex> lock(mutex);
-    if (smem > 48 * 1024 && !configured[dev]) {
-      if (cudaFuncSetAttribute(attention_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-          cudaSuccess)
-        return PTB_ERR_LAUNCH;
-      configured[dev] = true;
-    }
-  }
+  static SharedLimit limit;
+  if (!limit.allows(attention_mma_kernel<D>, smem)) return PTB_ERR_LAUNCH;
   const int y_blocks = p.kv_heads * chunks * (p.out_wide ? p.kv_heads : 1);
   dim3 grid(n_tiles, y_blocks, p.n_splits);
   const bool partial = p.n_splits > 1;

@@ -852,12 +852,8 @@ int launch_tc_pair(const void* q, const void* k_pool, const void* v_pool, int po
   const CUtensorMap* vm = pool_map(v_pool, pool_pages, p.kv_heads, D);
   if (km == nullptr || vm == nullptr) return PTB_ERR_LAUNCH;
   constexpr size_t smem = PairShape<D>::SMEM;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_tc_pair_kernel<D, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(attention_tc_pair_kernel<D, BIAS>, smem)) return PTB_ERR_LAUNCH;
   const int qpk = p.heads / p.kv_heads;
   dim3 grid(p.kv_heads * ((qpk + 1) / 2), n_tiles);
   attention_tc_pair_kernel<D, BIAS><<<grid, PAIR_THREADS, smem, stream>>>(
@@ -892,12 +888,8 @@ int launch_tc(const void* q, const void* k_pool, const void* v_pool, int pool_pa
   const CUtensorMap* vm = pool_map(v_pool, pool_pages, p.kv_heads, DV);
   if (km == nullptr || vm == nullptr) return PTB_ERR_LAUNCH;
   const size_t smem = 1024 + TQ * DK * 2 + TcShape<TWO>::STAGES * KEYS * (DK + DV) * 2 + 192;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO>, smem)) return PTB_ERR_LAUNCH;
   dim3 grid(p.heads, n_tiles);
   attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO><<<grid, BLOCK_THREADS, smem, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, sb,

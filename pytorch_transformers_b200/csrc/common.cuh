@@ -1,9 +1,11 @@
 // Shared helpers of the sm_100a kernels: element access in float32 and bfloat16, reductions,
 // the step's batch description and the paged cache's addressing.
 #pragma once
+#include <atomic>
 #include <cstdio>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <mutex>
 #include <stdint.h>
 
 #define PTB_API extern "C" __attribute__((visibility("default")))
@@ -190,6 +192,39 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cfg.numAttrs = captured ? 0 : 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+
+// How much dynamic shared memory a kernel may use is an attribute of the kernel on one device, asked for before its first launch
+// there that needs more than any before. A launching function keeps one of these for each kernel (a static beside the
+// launch); several threads may launch at a time, and the limit never falls.
+class SharedLimit {
+ public:
+  template <typename Kernel>
+  bool allows(Kernel* kernel, size_t bytes) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    return allows_on(device, bytes, [&] {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) == cudaSuccess) return true;
+      (void)cudaGetLastError();
+      return false;
+    });
+  }
+  // `ask`: raises the limit on `device` to `bytes`
+  template <typename Ask>
+  bool allows_on(int device, size_t bytes, Ask ask) {
+    if (device < 0 || device >= DEVICES) return false;
+    if (bytes <= granted_[device].load(std::memory_order_acquire)) return true;
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (bytes <= granted_[device].load(std::memory_order_relaxed)) return true;
+    if (!ask()) return false;
+    granted_[device].store(bytes, std::memory_order_release);
+    return true;
+  }
+
+ private:
+  static constexpr int DEVICES = 64;
+  std::mutex mutex_;
+  std::atomic<size_t> granted_[DEVICES] = {};
+};
 
 // the status of the launch just made; a failure is said on stderr with the runtime's own words
 inline int launch_status() {

@@ -636,12 +636,8 @@ int launch_local(const void* act, const float* inv, const float* logd, const flo
                  const int* chunk_seq, const int* chunk_q0, int n_chunks, void* mq, void* bo, float* dec, int heads, int kv_heads,
                  cudaStream_t stream) {
   constexpr int smem = LocalSmem<DK, DV, PER_HEAD>::bytes;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(delta_chunk_local_kernel<DK, DV, PER_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(delta_chunk_local_kernel<DK, DV, PER_HEAD>, smem)) return PTB_ERR_LAUNCH;
   delta_chunk_local_kernel<DK, DV, PER_HEAD><<<dim3(n_chunks, heads), DK * 4, smem, stream>>>(
       (const __nv_bfloat16*)act, inv, logd, beta, sb, chunk_seq, chunk_q0, (uint4*)mq, (float4*)bo, dec, heads, kv_heads);
   return launch_status();

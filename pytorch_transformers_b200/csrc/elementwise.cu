@@ -319,22 +319,13 @@ PTB_API int ptb_norm(int dtype, const void* x, const void* addend, void* sum_out
   const size_t smem = size_t(width) * sizeof(float);
   if (smem > 200 * 1024) return PTB_ERR_SIZE;
   const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
-  cudaError_t e = cudaSuccess;
-  static size_t configured_f32 = 48 * 1024, configured_bf16 = 48 * 1024;
+  static SharedLimit limit_f32, limit_bf16;
   if (dtype == PTB_F32) {
-    if (smem > configured_f32) {
-      e = cudaFuncSetAttribute(norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-      configured_f32 = smem;
-    }
-    if (e != cudaSuccess) return PTB_ERR_LAUNCH;
+    if (!limit_f32.allows(norm_kernel<float>, smem)) return PTB_ERR_LAUNCH;
     launch_pdl(norm_kernel<float>, n, threads, smem, stream, (const float*)x, (const float*)addend, (float*)sum_out, gain1,
                                                      bias1, (float*)y1, gain2, bias2, (float*)y2, width, eps, kind);
   } else if (dtype == PTB_BF16) {
-    if (smem > configured_bf16) {
-      e = cudaFuncSetAttribute(norm_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-      configured_bf16 = smem;
-    }
-    if (e != cudaSuccess) return PTB_ERR_LAUNCH;
+    if (!limit_bf16.allows(norm_kernel<__nv_bfloat16>, smem)) return PTB_ERR_LAUNCH;
     launch_pdl(norm_kernel<__nv_bfloat16>, n, threads, smem, stream, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)addend, (__nv_bfloat16*)sum_out, gain1, bias1,
         (__nv_bfloat16*)y1, gain2, bias2, (__nv_bfloat16*)y2, width, eps, kind);

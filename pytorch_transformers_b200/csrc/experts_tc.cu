@@ -247,12 +247,8 @@ int launch_expert_tc(const CUtensorMap& map, ExpertTcParams p, cudaStream_t stre
   // epilogue under the other's products: down, tiles of 256, 142 -> 114 us), else one block with what the SM has
   p.ring_bytes = (p.tmem_cols <= 256 && 2 * most <= 110 * 1024) ? 110 * 1024 : 222 * 1024;
   const size_t smem = 1024 + size_t(p.ring_bytes);
-  static size_t configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(expert_linear_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(expert_linear_tc_kernel<MODE>, smem)) return PTB_ERR_LAUNCH;
   launch_pdl(expert_linear_tc_kernel<MODE>, dim3((p.N + XM - 1) / XM, p.max_tiles), 64 + X_GATHER, smem, stream, map, p);
   return launch_status();
 }

@@ -117,12 +117,8 @@ template <int DK, int DV>
 int launch_sum(const void* proj, int stride, const float* log_decay, const StepBatch& sb, const int* chunk_seq,
                const int* chunk_q0, int n_chunks, float* sums, float* chunk_decay, int heads, cudaStream_t stream) {
   const size_t smem = size_t(2) * CH * DK * 2 + size_t(CH) * DV * 2 + size_t(CH) * DK * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gla_chunk_sum_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(gla_chunk_sum_mma_kernel<DK, DV>, smem)) return PTB_ERR_LAUNCH;
   launch_pdl(gla_chunk_sum_mma_kernel<DK, DV>, dim3(n_chunks, heads), DK * 2, smem, stream, (const __nv_bfloat16*)proj, stride, log_decay, sb,
                                                                                    chunk_seq, chunk_q0, sums, chunk_decay, heads);
   return launch_status();
@@ -467,12 +463,8 @@ template <int DK, int DV>
 int launch_out(const void* proj, int stride, const float* log_decay, const StepBatch& sb, const int* chunk_seq, const int* chunk_q0,
                int n_chunks, const float* before, float* out, int heads, float q_scale, cudaStream_t stream) {
   constexpr size_t smem = OutShape<DK, DV>::SMEM;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gla_chunk_out_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(gla_chunk_out_mma_kernel<DK, DV>, smem)) return PTB_ERR_LAUNCH;
   launch_pdl(gla_chunk_out_mma_kernel<DK, DV>, dim3(n_chunks, heads), 256, smem, stream, (const __nv_bfloat16*)proj, stride, log_decay, sb,
                                                                                 chunk_seq, chunk_q0, before, out, heads, q_scale);
   return launch_status();

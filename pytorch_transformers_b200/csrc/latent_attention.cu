@@ -315,13 +315,8 @@ int launch_latent(const float* q_abs, const void* q, long long q_stride, int q_d
   const int dk = rank + rot_dim;
   const size_t smem = sizeof(float) * (size_t(ROWS) * (dk + 1) + size_t(PTB_PAGE) * (dk + 1) + ROWS * PTB_PAGE);
   if (smem > 220 * 1024) return PTB_ERR_SIZE;
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(latent_attention_kernel<T, DPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(latent_attention_kernel<T, DPT>, smem)) return PTB_ERR_LAUNCH;
   const int chunks = (heads + heads_per_block - 1) / heads_per_block;
   dim3 grid(n_tiles, chunks, n_splits);
   launch_pdl(latent_attention_kernel<T, DPT>, grid, THREADS, smem, stream, 
@@ -686,13 +681,8 @@ int launch_latent_mma_tg(const float* q_abs, const void* q, long long q_stride, 
   const int rowb = (rank + rot_dim) * 2 + 16;
   const size_t smem = size_t(16 * TG + PTB_PAGE) * rowb + TG * ((WIDE ? 2 : 1) * 16 * 144 + 2 * 64 * sizeof(float));
   if (smem > 220 * 1024) return PTB_ERR_SIZE;
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(latent_attention_mma_kernel<NF, TG, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-        cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(latent_attention_mma_kernel<NF, TG, WIDE>, smem)) return PTB_ERR_LAUNCH;
   const int chunks = (heads + heads_per_block - 1) / heads_per_block;
   launch_pdl(latent_attention_mma_kernel<NF, TG, WIDE>, dim3(n_tiles, chunks, n_splits), MTHREADS * TG, smem, stream, 
       q_abs, (const __nv_bfloat16*)q, q_stride, q_dim, q_rot_off, (const __nv_bfloat16*)pool, part, (__nv_bfloat16*)out, sb,

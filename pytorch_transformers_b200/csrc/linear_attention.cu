@@ -332,14 +332,6 @@ __global__ void qk_norm_store_kernel(const T* __restrict__ proj, int stride, T* 
   }
 }
 
-size_t raise_smem(const void* fn, size_t smem, size_t& configured) {
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
-    configured = smem;
-  }
-  return smem;
-}
-
 constexpr size_t SMEM_MOST = 200 * 1024;
 
 // value columns of a block of the scan and chunk-sum kernels: 64, or 32 where values are that short or
@@ -363,13 +355,13 @@ PTB_API int ptb_linear_attention_scan(int dtype, const void* proj, int stride, f
   if (smem > SMEM_MOST) return PTB_ERR_SIZE;
   dim3 grid(sb->n_seqs, heads, (v_dim + vb - 1) / vb);
   if (dtype == PTB_F32) {
-    static size_t configured = 48 * 1024;
-    if (!raise_smem((const void*)linear_attention_scan_kernel<float>, smem, configured)) return PTB_ERR_LAUNCH;
+    static SharedLimit limit;
+    if (!limit.allows(linear_attention_scan_kernel<float>, smem)) return PTB_ERR_LAUNCH;
     linear_attention_scan_kernel<float><<<grid, vb, smem, stream>>>((const float*)proj, stride, state, state_stride, slots,
                                                                     *sb, decay, out, heads, dim, v_dim, act);
   } else if (dtype == PTB_BF16) {
-    static size_t configured = 48 * 1024;
-    if (!raise_smem((const void*)linear_attention_scan_kernel<__nv_bfloat16>, smem, configured)) return PTB_ERR_LAUNCH;
+    static SharedLimit limit;
+    if (!limit.allows(linear_attention_scan_kernel<__nv_bfloat16>, smem)) return PTB_ERR_LAUNCH;
     linear_attention_scan_kernel<__nv_bfloat16><<<grid, vb, smem, stream>>>(
         (const __nv_bfloat16*)proj, stride, state, state_stride, slots, *sb, decay, out, heads, dim, v_dim, act);
   } else {
@@ -427,9 +419,9 @@ PTB_API int ptb_linear_attention_chunks(int dtype, const void* proj, int stride,
   dim3 grid2(unsigned((per + 255) / 256), sb->n_seqs);
 #define PTB_LA_CHUNKS(TT)                                                                                              \
   {                                                                                                                    \
-    static size_t c1 = 48 * 1024, c3 = 48 * 1024;                                                                      \
-    if (!raise_smem((const void*)linear_attention_chunk_sum_kernel<TT>, smem1, c1)) return PTB_ERR_LAUNCH;             \
-    if (!raise_smem((const void*)linear_attention_chunk_out_kernel<TT>, smem3, c3)) return PTB_ERR_LAUNCH;             \
+    static SharedLimit limit1, limit3;                                                                                 \
+    if (!limit1.allows(linear_attention_chunk_sum_kernel<TT>, smem1)) return PTB_ERR_LAUNCH;                           \
+    if (!limit3.allows(linear_attention_chunk_out_kernel<TT>, smem3)) return PTB_ERR_LAUNCH;                           \
     linear_attention_chunk_sum_kernel<TT><<<grid1, vb, smem1, stream>>>((const TT*)proj, stride, *sb, chunk_seq,        \
                                                                         chunk_q0, decay, sums, heads, dim, v_dim, act); \
     if (launch_status() != PTB_OK) return PTB_ERR_LAUNCH;                                                              \

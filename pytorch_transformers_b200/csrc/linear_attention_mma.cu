@@ -244,12 +244,8 @@ template <int DK, int DV>
 int launch_sum(const void* proj, int stride, const StepBatch& sb, const int* chunk_seq, const int* chunk_q0, int n_chunks,
                const float* decay, float* sums, int heads, int act, cudaStream_t stream) {
   const size_t smem = size_t(2) * CH * DK * 2 + size_t(CH) * DV * 2 + (CH + 1) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(la_chunk_sum_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(la_chunk_sum_mma_kernel<DK, DV>, smem)) return PTB_ERR_LAUNCH;
   la_chunk_sum_mma_kernel<DK, DV><<<dim3(n_chunks, heads), DK * 2, smem, stream>>>((const __nv_bfloat16*)proj, stride, sb, chunk_seq,
                                                                                   chunk_q0, decay, sums, heads, act);
   return launch_status();
@@ -259,12 +255,8 @@ template <int DK, int DV>
 int launch_out(const void* proj, int stride, const StepBatch& sb, const int* chunk_seq, const int* chunk_q0, int n_chunks,
                const float* decay, const float* before, float* out, int heads, int act, cudaStream_t stream) {
   const size_t smem = size_t(2) * CH * DK * 2 + size_t(CH) * DV * 2 + size_t(2) * DK * DV * 2 + (CH + 1) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(la_chunk_out_mma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(la_chunk_out_mma_kernel<DK, DV>, smem)) return PTB_ERR_LAUNCH;
   la_chunk_out_mma_kernel<DK, DV><<<dim3(n_chunks, heads), 256, smem, stream>>>((const __nv_bfloat16*)proj, stride, sb, chunk_seq,
                                                                                chunk_q0, decay, before, out, heads, act);
   return launch_status();

@@ -151,12 +151,8 @@ template <int TM, bool VEC>
 int launch_linear_f32(const float* x, const float* w, const float* bias, float* y, int M, int N, int K, int ldx, int act,
                       int ranks, cudaStream_t stream) {
   const size_t smem = size_t(LSTAGES) * (8 * TM + LBN) * LPITCH * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(linear_f32_kernel<TM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(linear_f32_kernel<TM, VEC>, smem)) return PTB_ERR_LAUNCH;
   const int steps = (K + LBK - 1) / LBK, stretch = (steps + ranks - 1) / ranks * LBK;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((N + LBN - 1) / LBN, (M + 8 * TM - 1) / (8 * TM), ranks);

@@ -435,12 +435,8 @@ template <int DK, int DV>
 int launch_sum(const void* proj, int stride, const float* gates, const StepBatch& sb, const int* chunk_seq, const int* chunk_q0,
                int n_chunks, float* sums, float* nsums, float* meta, int heads, cudaStream_t stream) {
   const size_t smem = size_t(2) * CH * DK * 2 + size_t(CH) * DV * 2 + 3 * CH * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(mlstm_chunk_sum_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(mlstm_chunk_sum_kernel<DK, DV>, smem)) return PTB_ERR_LAUNCH;
   launch_pdl(mlstm_chunk_sum_kernel<DK, DV>, dim3(n_chunks, heads), DK * 2, smem, stream, (const __nv_bfloat16*)proj, stride, gates, sb,
                                                                                  chunk_seq, chunk_q0, sums, nsums, meta, heads);
   return launch_status();
@@ -451,12 +447,8 @@ int launch_out(const void* proj, int stride, const float* gates, const StepBatch
                int n_chunks, const float* sums, const float* nsums, const float* m_before, float* out, int heads, float q_scale,
                cudaStream_t stream) {
   const size_t smem = size_t(2) * CH * DK * 2 + size_t(CH) * DV * 2 + size_t(2) * DK * DV * 2 + (4 * CH + DK) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(mlstm_chunk_out_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(mlstm_chunk_out_kernel<DK, DV>, smem)) return PTB_ERR_LAUNCH;
   launch_pdl(mlstm_chunk_out_kernel<DK, DV>, dim3(n_chunks, heads), 256, smem, stream, (const __nv_bfloat16*)proj, stride, gates, sb, chunk_seq,
                                                                               chunk_q0, sums, nsums, m_before, out, heads, q_scale);
   return launch_status();

@@ -145,12 +145,8 @@ __global__ void post_norm_kernel(PostNormArgs p) {
 template <typename TA, typename TO, int KIND, int V>
 int launch_post_norm_v(const PostNormArgs& p, int n, cudaStream_t stream) {
   const size_t smem = size_t(p.width) * sizeof(float) * (KIND == PN_PAIR ? 2 : 1);
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(post_norm_kernel<TA, TO, KIND, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(post_norm_kernel<TA, TO, KIND, V>, smem)) return PTB_ERR_LAUNCH;
   const int units = (p.width + V - 1) / V;
   const int threads = units >= 512 ? 512 : (units >= 256 ? 256 : (units >= 128 ? 128 : 64));
   post_norm_kernel<TA, TO, KIND, V><<<n, threads, smem, stream>>>(p);

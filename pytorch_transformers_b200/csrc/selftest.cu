@@ -22,6 +22,21 @@ __global__ void bounded_wait_kernel(int* error_flag, uint32_t tries, int* gave_u
 }  // namespace
 
 // tries: 1 .. 100,000 (each try may park the thread for up to two microseconds)
+// A SharedLimit on `n` launches that need bytes[i] on devices[i], without a device: asked[i] says whether launch i raised the
+// limit, and it cannot where bytes[i] is above `most`. Returns how many launches were allowed.
+PTB_API int ptb_selftest_shared_limit(const int* devices, const long long* bytes, int n, long long most, int* asked) {
+  SharedLimit limit;
+  int allowed = 0;
+  for (int i = 0; i < n; ++i) {
+    asked[i] = 0;
+    allowed += limit.allows_on(devices[i], size_t(bytes[i]), [&] {
+      asked[i] = 1;
+      return bytes[i] <= most;
+    });
+  }
+  return allowed;
+}
+
 PTB_API int ptb_selftest_bounded_wait(int tries, int* error_flag, int* gave_up, cudaStream_t stream) {
   if (tries < 1 || tries > 100000 || error_flag == nullptr) return PTB_ERR_SIZE;
   bounded_wait_kernel<<<1, 32, 0, stream>>>(error_flag, uint32_t(tries), gave_up);
@@ -86,12 +101,8 @@ PTB_API int ptb_selftest_mma_cadence(int n, int reps, int a_in_tmem, int blocks,
       (a_in_tmem && n > 128))
     return PTB_ERR_SIZE;
   const int smem = 1024 + (128 + 256) * 128;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(mma_cadence_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = true;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(mma_cadence_kernel, smem)) return PTB_ERR_LAUNCH;
   mma_cadence_kernel<<<blocks, 128, smem, stream>>>(n, reps, a_in_tmem, clocks, error_flag);
   return launch_status();
 }

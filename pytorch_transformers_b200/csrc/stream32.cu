@@ -103,13 +103,8 @@ template <typename TA, typename TO>
 int launch_norm_stream(const float* x, const void* addend, float* sum_out, const float* gain, const float* bias,
                        void* y, int n, int width, float eps, int kind, cudaStream_t stream) {
   const size_t smem = size_t(width) * sizeof(float);
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(norm_stream_kernel<TA, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-        cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(norm_stream_kernel<TA, TO>, smem)) return PTB_ERR_LAUNCH;
   const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
   norm_stream_kernel<TA, TO><<<n, threads, smem, stream>>>(x, (const TA*)addend, sum_out, gain, bias, (TO*)y, width,
                                                            eps, kind);
@@ -163,13 +158,8 @@ PTB_API int ptb_post_norm_add(const float* x, int y_dtype, const void* y, const 
   const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
 #define PTB_PNA(TA, TO)                                                                                              \
   {                                                                                                                  \
-    static size_t configured = 48 * 1024;                                                                            \
-    if (smem > configured) {                                                                                         \
-      if (cudaFuncSetAttribute(post_norm_add_kernel<TA, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                               int(smem)) != cudaSuccess)                                                            \
-        return PTB_ERR_LAUNCH;                                                                                       \
-      configured = smem;                                                                                             \
-    }                                                                                                                \
+    static SharedLimit limit;                                                                                        \
+    if (!limit.allows(post_norm_add_kernel<TA, TO>, smem)) return PTB_ERR_LAUNCH;                                    \
     post_norm_add_kernel<TA, TO><<<n, threads, smem, stream>>>(x, (const TA*)y, gain, eps, mult, out, gain_next,     \
                                                                eps_next, (TO*)next, width);                          \
   }

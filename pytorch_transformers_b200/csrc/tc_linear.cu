@@ -329,12 +329,8 @@ PTB_API int ptb_tc_linear(const void* x, const void* w, const float* bias, const
   if (stages < 2 || size_t(stages) * stage_bytes < recv_bytes) return PTB_ERR_SIZE;
   p.stages = stages;
   const size_t smem = 1024 + size_t(stages) * stage_bytes;
-  static size_t configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(tc_linear_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return PTB_ERR_LAUNCH;
-    configured = smem;
-  }
+  static SharedLimit limit;
+  if (!limit.allows(tc_linear_kernel, smem)) return PTB_ERR_LAUNCH;
   const CUtensorMap* wm = weight_map_sw128(w, N, K);
   CUtensorMap xm;
   if (wm == nullptr || !make_map_sw128(&xm, x, M, K, p.n_tok)) return PTB_ERR_LAUNCH;

@@ -192,3 +192,28 @@ def test_activation_names_match_the_kernels_table():
     for name in os.listdir(os.path.join(os.path.dirname(kernels.__file__), "csrc")):
         if name.endswith(".cu"):
             assert "erff(" not in open(os.path.join(os.path.dirname(kernels.__file__), "csrc", name)).read(), name
+
+
+def test_the_limit_of_shared_memory_is_kept_per_kernel_and_device():
+    """A launch asks for its dynamic shared memory where no earlier one on the same device asked for as much; a refusal
+    changes nothing, and a device that is no device is refused."""
+    import ctypes
+    from pytorch_transformers_b200 import native
+    lib = native.library()
+    launches = [(0, 55), (0, 55), (1, 55), (0, 40), (0, 90), (1, 55), (1, 500), (1, 60), (63, 55), (64, 55), (-1, 55)]
+    n = len(launches)
+    asked = (ctypes.c_int * n)()
+    allowed = lib.ptb_selftest_shared_limit((ctypes.c_int * n)(*[d for d, _ in launches]), (ctypes.c_longlong * n)(*[b for _, b in launches]),
+                                            n, ctypes.c_longlong(227), asked)
+    assert list(asked) == [1, 0, 1, 0, 1, 0, 1, 1, 1, 0, 0]
+    assert allowed == n - 3
+
+
+def test_every_kernel_asks_for_shared_memory_through_the_per_device_limit():
+    import os
+    from pytorch_transformers_b200 import native
+    for path in native._sources() + native._headers():
+        with open(path) as f:
+            text = f.read()
+        calls = text.count("cudaFuncAttributeMaxDynamicSharedMemorySize")
+        assert calls == (1 if os.path.basename(path) == "common.cuh" else 0), path
