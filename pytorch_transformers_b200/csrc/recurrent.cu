@@ -590,6 +590,18 @@ PTB_API int ptb_block_epilogue(int in_dtype, int out_dtype, const void* z, const
   return launch_status();
 }
 
+// Whether the filter runs eight tokens a thread (rglru_conv_run_kernel) or an output a thread (rglru_conv_kernel). A run costs 4.6 us
+// however little there is to do, and up to 8.8 us where each of its tokens begins a sequence (a chain of loads each: the
+// sequence, its slot, its history); an output a thread costs 2.5 us until its threads are a wave of the device (2,048 an
+// SM) and grows with them from there. So a run takes steps of more than a wave, and of up to three waves more the more of their
+// tokens begin a sequence. us, run against output a thread, 2,560 channels in bfloat16: 8 sequences of one token 8.8 against 2.6,
+// 256 of one 9.8 / 8.1, 512 of one 10.9 / 14.1, 64 of four 6.3 / 8.2, one of 64 4.7 / 3.6, one of 192 4.8 / 6.6, one of 2,048
+// 18 / 50.
+PTB_API int ptb_rglru_conv_runs(int n_tokens, int n_seqs, int R) {
+  const double wave = 2048.0 * sm_count();
+  return double(n_tokens) * R >= wave * (1.0 + 3.0 * n_seqs / n_tokens) ? 1 : 0;
+}
+
 PTB_API int ptb_rglru_conv(int dtype, const void* proj, const float* by, const float* bx, const float* conv_w,
                            const float* conv_b, const float* state, long long state_stride, const int* slots,
                            const StepBatch* sb, void* y_act, void* u, int R, int taps, cudaStream_t stream) {
@@ -598,7 +610,7 @@ PTB_API int ptb_rglru_conv(int dtype, const void* proj, const float* by, const f
   const size_t total = size_t(sb->n_tokens) * R;
   const size_t want = (total + 255) / 256, most = size_t(sm_count()) * 16;
   const int blocks = int(want < most ? want : most);
-  if (R % 4 == 0 && aligned16(proj) && aligned16(by) && aligned16(bx) && aligned16(conv_b) && aligned16(y_act) && aligned16(u)) {
+  if (R % 4 == 0 && ptb_rglru_conv_runs(sb->n_tokens, sb->n_seqs, R) && aligned16(proj) && aligned16(by) && aligned16(bx) && aligned16(conv_b) && aligned16(y_act) && aligned16(u)) {
     const long long runs = (sb->n_tokens + CONV_RUN - 1) / CONV_RUN;
     const unsigned run_blocks = unsigned((runs * (R / 4) + 127) / 128);
 #define PTB_RC(TT, MM)                                                                                                          \

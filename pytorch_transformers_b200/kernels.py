@@ -97,7 +97,7 @@ def lib():
                      "ptb_tc_linear_k_multiple", "ptb_attention_decode_tc", "ptb_attention_decode_tc_supports",
                      "ptb_fill_normal", "ptb_selftest_bounded_wait", "ptb_scale", "ptb_selftest_mma_cadence",
                      "ptb_norm_stream", "ptb_add_stream", "ptb_latent_store", "ptb_latent_attention", "ptb_latent_rows",
-                     "ptb_rglru_conv", "ptb_rglru_scan", "ptb_block_linear", "ptb_route", "ptb_expert_plan",
+                     "ptb_rglru_conv", "ptb_rglru_conv_runs", "ptb_rglru_scan", "ptb_block_linear", "ptb_route", "ptb_expert_plan",
                      "ptb_expert_linear", "ptb_expert_combine", "ptb_expert_linear_tc", "ptb_latent_attention_mma",
                      "ptb_latent_attention_mma_supports", "ptb_rglru_scan_chunks", "ptb_block_epilogue", "ptb_latent_gather",
                      "ptb_latent_unfold", "ptb_latent_q_unfold", "ptb_gate_heads", "ptb_linear_attention_scan",
@@ -1063,6 +1063,12 @@ def rglru_conv(proj: torch.Tensor, by: torch.Tensor, bx: torch.Tensor, conv_w: t
                                 _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(slots), ctypes.byref(batch),
                                 _ptr(y_act), _ptr(u), r, taps, _stream(proj)), "rglru_conv")
     return y_act, u
+
+
+def rglru_conv_runs(n_tokens: int, n_seqs: int, r: int) -> bool:
+    """Whether ``rglru_conv`` slides its filter over eight tokens a thread in a step of ``n_tokens`` of ``n_seqs`` sequences
+    (prompts), instead of forming an output a thread (steps of few tokens). Both give the same bits."""
+    return bool(lib().ptb_rglru_conv_runs(int(n_tokens), int(n_seqs), int(r)))
 
 
 def rglru_scan(gates: torch.Tensor, u: torch.Tensor, y_act: torch.Tensor, lam: torch.Tensor, proj: torch.Tensor,

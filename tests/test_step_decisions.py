@@ -217,3 +217,18 @@ def test_every_kernel_asks_for_shared_memory_through_the_per_device_limit():
             text = f.read()
         calls = text.count("cudaFuncAttributeMaxDynamicSharedMemorySize")
         assert calls == (1 if os.path.basename(path) == "common.cuh" else 0), path
+
+
+@pytest.mark.parametrize("r", [320, 1280, 2560, 5120])
+def test_the_recurrences_filter_takes_runs_of_tokens_on_prompts_only(r):
+    """Steps of few tokens form an output a thread, long prompts slide the filter over runs; more tokens, or fewer sequences
+    among as many, never take the rule back."""
+    runs = kernels.rglru_conv_runs
+    assert not any(runs(n, n, r) for n in (1, 4, 8, 16, 64))          # decoding
+    assert not any(runs(per * n, n, r) for n in (1, 8) for per in (2, 3, 5, 7))
+    assert runs(2048, 1, r) and runs(8 * 2048, 8, r)
+    for seqs in (1, 8, 64, 300):
+        sizes = [runs(n, seqs, r) for n in range(seqs, 6000, 37)]
+        assert sizes == sorted(sizes)
+    for n in (64, 256, 1000, 3000):
+        assert all(runs(n, s, r) >= runs(n, s + 1, r) for s in range(1, n, 13))
