@@ -19,12 +19,27 @@ constexpr int PPITCH = PTB_PAGE + 4;
 // floats from one row of `n` values to the next: whole 16-byte words, an odd number of them
 __host__ __device__ constexpr int odd_words(int n) { return 4 * ((n + 3) / 4 + ((n + 3) / 4 % 2 == 0 ? 1 : 0)); }
 
-// a page's rows of `d` values into shared rows `pitch` apart, zeros in rows from `valid` on and beyond d; `async`: by cp.async
-// (float32 rows of whole 16-byte words)
+// a page's rows of `d` values into shared rows `pitch` apart, zeros in rows from `valid` on and beyond d; `whole`: the rows are
+// whole 16-byte words, which go by cp.async in float32 and through registers, a word a load, in bfloat16. (A value a load, a
+// head size of 256 in bfloat16 was slower than the kernel before this one where sequences are many, an SM holding one block:
+// 64 sequences of 1,000 keys 3,198 us against 2,940; a word a load 1,667 us.)
 template <typename T>
-__device__ __forceinline__ void load_rows(float* dst, const T* src, int d, int pitch, int valid, int async) {
+__device__ __forceinline__ void load_rows(float* dst, const T* src, int d, int pitch, int valid, int whole) {
   const int words = (d + 3) / 4;
-  if (sizeof(T) == 4 && async) {
+  if (sizeof(T) == 2 && whole) {
+    const int per_row = d / 8;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < PTB_PAGE * per_row; i += THREADS) {
+      const int j = i / per_row, c = (i - j * per_row) * 8;
+      const uint4 w = j < valid ? *reinterpret_cast<const uint4*>(src + size_t(j) * d + c) : make_uint4(0, 0, 0, 0);
+      float f[8];
+      unpack_bf16x8(w, f);
+      *reinterpret_cast<float4*>(dst + j * pitch + c) = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float4*>(dst + j * pitch + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+    return;
+  }
+  if (sizeof(T) == 4 && whole) {
     for (int i = threadIdx.x; i < PTB_PAGE * words; i += THREADS) {
       const int j = i / words, c = (i - j * words) * 4;
       if (j < valid) cp_async16(smem_u32(dst + j * pitch + c), src + size_t(j) * d + c);
@@ -177,7 +192,7 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, 
                          const int* __restrict__ tile_q0, const float* __restrict__ alibi_slopes, int heads,
                          int kv_heads, int head_dim, float scale, int window, int v_dim,
                          const float* __restrict__ sinks, const T* __restrict__ gate, int gate_stride, float out_scale,
-                         int out_stride, int keep_first, float* __restrict__ out_wide, float softcap, int gate_wide, int async) {
+                         int out_stride, int keep_first, float* __restrict__ out_wide, float softcap, int gate_wide, int whole) {
   pdl_entry();
   extern __shared__ __align__(16) float smem[];
   const int kpitch = odd_words(head_dim), vpitch = odd_words(v_dim), kwords = (head_dim + 3) / 4;
@@ -220,7 +235,7 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, 
   auto after = [&](int kb) { return (kb + 1 == kept_pages && kb + 1 < kb_lo) ? kb_lo : kb + 1; };
   auto load_keys = [&](int kb) {
     const T* src = k_pool + kv_offset(pages[kb], g, 0, kv_heads, head_dim);
-    load_rows(ks, src, head_dim, kpitch, min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE), async);
+    load_rows(ks, src, head_dim, kpitch, min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE), whole);
   };
 
   int kb = kept_pages > 0 ? 0 : kb_lo;
@@ -229,7 +244,7 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, 
   while (kb <= kb_hi) {
     const int next = after(kb);
     load_rows(vs, v_pool + kv_offset(pages[kb], gv, 0, kv_heads, v_dim), v_dim, vpitch,
-              min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE), async);
+              min(PTB_PAGE, last_pos + 1 - kb * PTB_PAGE), whole);
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();  // this page's keys are here
@@ -669,7 +684,8 @@ int launch_attention(const void* q, const void* k_pool, const void* v_pool, void
                      int gate_stride, float out_scale, int out_stride, int keep_first, float* out_wide, float softcap,
                      int gate_wide, cudaStream_t stream) {
   const size_t smem = sizeof(float) * (size_t(BQ + PTB_PAGE) * odd_words(head_dim) + size_t(PTB_PAGE) * odd_words(v_dim) + BQ * PPITCH);
-  const int async = sizeof(T) == 4 && head_dim % 4 == 0 && v_dim % 4 == 0 && aligned16(k_pool) && aligned16(v_pool);
+  constexpr int PER = 16 / sizeof(T);
+  const int whole = head_dim % PER == 0 && v_dim % PER == 0 && aligned16(k_pool) && aligned16(v_pool);
   dim3 grid(n_tiles, heads, out_wide ? kv_heads : 1);
 #define PTB_AG(CC)                                                                                                              \
   do {                                                                                                                          \
@@ -678,7 +694,7 @@ int launch_attention(const void* q, const void* k_pool, const void* v_pool, void
     launch_pdl(attention_generic_kernel<T, CC>, grid, THREADS, smem, stream,                                                            \
         (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, sb, tile_seq, tile_q0, slopes, heads, kv_heads, head_dim,     \
         scale, window, v_dim, sinks, (const T*)gate, gate_stride, out_scale, out_stride, keep_first, out_wide, softcap,         \
-        gate_wide, async);                                                                                                      \
+        gate_wide, whole);                                                                                                      \
   } while (0)
   if (v_dim <= 64) PTB_AG(1);
   else if (v_dim <= 128) PTB_AG(2);

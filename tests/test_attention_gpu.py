@@ -458,3 +458,36 @@ def test_tc_extras(K, heads, kv, d, window, keep, softcap, sinks, gate, strided)
     assert K.attention_tc_extras_take(q.view(n, -1), gates, gate == "entry")
     assert ((got - ref).abs() <= 2.0 ** -7 * ref.abs() + 2e-4).all(), (got - ref).abs().max()
     K.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,vd", [(8, 8), (8, 16), (16, 12), (72, 136), (128, 64), (256, 256), (250, 256)])
+def test_general_attention_reads_words_and_values_alike(K, dtype, d, vd):
+    """Pools whose rows are whole 16-byte words against the same pools one value further on, which are read a value at a time:
+    the same bits, for single tokens and portions, whole pages and short ones."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.attention import AttentionTiles
+    from pytorch_transformers_b200.parts.base import CacheNeed
+    heads, kv = 4, 2
+    g = torch.Generator(device="cuda").manual_seed(d + vd)
+    for pasts, news in (([63, 64, 200], [1, 1, 1]), ([0, 60, 130], [150, 70, 3])):
+        cache = Cache([(0, CacheNeed("full", kv, d, 0, v_head_dim=vd), None)], 1024, dtype, "cuda", max_slots=3)
+        slots = [cache.open() for _ in pasts]
+        live = [(s, p) for s, p in zip(slots, pasts) if p]
+        StepContext(cache, [s for s, _ in live], [[0] * p for _, p in live], 1, [[]] * len(live), []).commit()
+        ctx = StepContext(cache, slots, [[0] * m for m in news], 1, [[]] * 3, [AttentionTiles(K)])
+        tiles = ctx.plan(AttentionTiles.plan_key)
+        k_pool, v_pool, group = cache.entry_storage(0)
+        q = torch.randn(sum(news), heads, d, generator=g, device="cuda").to(dtype)
+        out = []
+        for off in (0, 1):
+            flat = [torch.empty(p.numel() + 8, dtype=dtype, device="cuda") for p in (k_pool, v_pool)]
+            moved = [f[off:off + p.numel()].view(p.shape) for f, p in zip(flat, (k_pool, v_pool))]
+            if not out:
+                src = [torch.randn(p.shape, generator=g, device="cuda").to(dtype) for p in (k_pool, v_pool)]
+            for m, s in zip(moved, src):
+                m.copy_(s)
+            out.append(K.attention_generic(q, moved[0], moved[1], ctx.batch_c[group], tiles.dev["tile_seq"], tiles.dev["tile_q0"],
+                                           tiles.facts["n_tiles"], None, kv, d ** -0.5))
+        assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
