@@ -857,13 +857,21 @@ PTB_API int ptb_rope_norm_store(int dtype, const void* proj, int stride, const f
                               nullptr, 0, 0.f, 0, stream);
 }
 
+// Whether talk_mix takes the form that reads `wide` once (talk_mix_vec_kernel: a thread has four columns and a K/V group's heads,
+// eight of them at a time) or a thread an output. The first costs the same whatever the tokens until its threads fill the
+// device; the second is shorter while its threads are few, so the line lies at 768 outputs an SM for every eight heads
+// of a group. us, once against an output a thread: 16 heads of 128 on 4: 8 tokens 5.7 / 4.1, 48 5.7 / 4.8, 80 5.8 / 5.8, 148
+// 5.8 / 8.5, 256 6.5 / 12.2; 8 on 4: 64 3.8 / 3.2, 128 3.9 / 4.0; 32 heads of 128 on one: 96 22.1 / 14.4, 192 22.1 / 25.4.
+PTB_API int ptb_talk_mix_reads_once(int n_tokens, int heads, int kv_heads, int v_dim) {
+  const long long passes = (heads / kv_heads + 7) / 8;
+  return v_dim % 4 == 0 && (long long)n_tokens * heads * v_dim >= 768LL * sm_count() * passes ? 1 : 0;
+}
+
 PTB_API int ptb_talk_mix(int dtype, const float* wide, const float* talk, void* out, int out_stride, int n_tokens, int heads,
                          int kv_heads, int v_dim, cudaStream_t stream) {
   if (n_tokens <= 0) return PTB_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0 || v_dim <= 0 || out_stride < heads * v_dim) return PTB_ERR_SIZE;
-  // the form that reads `wide` once, where its threads (four columns and a K/V group's heads each) fill the device; steps of few
-  // tokens take a thread an output: 4 tokens of 16 heads on 4 are 512 threads in one form and 8,192 in the other (6.3 against 5.4 us)
-  if (v_dim % 4 == 0 && aligned16(wide) && (long long)n_tokens * kv_heads * (v_dim / 4) >= 256LL * sm_count()) {
+  if (aligned16(wide) && ptb_talk_mix_reads_once(n_tokens, heads, kv_heads, v_dim)) {
     const long long total = (long long)n_tokens * kv_heads * (v_dim / 4);
     const unsigned blocks = unsigned((total + 127) / 128);
     if (dtype == PTB_F32)

@@ -232,3 +232,15 @@ def test_the_recurrences_filter_takes_runs_of_tokens_on_prompts_only(r):
         assert sizes == sorted(sizes)
     for n in (64, 256, 1000, 3000):
         assert all(runs(n, s, r) >= runs(n, s + 1, r) for s in range(1, n, 13))
+
+
+def test_mixed_weights_read_the_heads_results_once_where_outputs_are_many():
+    """The rule follows the outputs: steps of few tokens take a thread an output; at twice the outputs where that form was
+    measured slower the other one is taken."""
+    once = lambda *a: bool(kernels.lib().ptb_talk_mix_reads_once(*a))
+    assert not once(1, 16, 4, 128) and not once(32, 16, 4, 128) and not once(64, 8, 4, 128) and not once(64, 32, 1, 128)
+    assert once(148, 16, 4, 128) and once(128, 32, 8, 64) and once(200, 8, 4, 128) and once(200, 32, 1, 128)
+    assert not once(5000, 16, 4, 126)           # rows that are no whole words
+    for shape in ((16, 4, 128), (8, 8, 64), (32, 1, 128)):
+        got = [once(n, *shape) for n in range(1, 3000, 7)]
+        assert got == sorted(got)
