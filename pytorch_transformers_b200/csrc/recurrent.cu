@@ -236,8 +236,8 @@ __global__ void rglru_chunk_kernel(float* __restrict__ gates, const float* __res
     for (int k = 0; k < taps - 1; ++k) st[R + size_t(k) * R + c] = keep[k];
     return;
   }
-  const int chunk = blockIdx.y, part = chunk % SPLIT;
-  const int seq = chunk_seq[chunk / SPLIT], q0 = chunk_q0[chunk / SPLIT] + part * len;
+  const int part = blockIdx.z, chunk = blockIdx.y * SPLIT + part;
+  const int seq = chunk_seq[blockIdx.y], q0 = chunk_q0[blockIdx.y] + part * len;
   const int first = sb.seq_start[seq] + q0, count = min(min(len, chunk_len - part * len), sb.seq_new[seq] - q0);
   const float l = lam[c];
   const float sp = (l > 20.f) ? l : log1pf(expf(l));
@@ -288,13 +288,13 @@ int launch_rglru_chunks(float* gates, const float* gates_b, const void* u, const
   const size_t per = size_t(n_chunks) * SPLIT * R;
   float *agg_a = work, *agg_b = work + per, *s_start = work + 2 * per;
   const int threads = 128, gx = (R + threads - 1) / threads;
-#define PTB_CHUNK_PASS(P, GY)                                                                                       \
-  launch_pdl(rglru_chunk_kernel<T, P, RAW>, dim3(gx, GY), threads, 0, stream,                                                \
+#define PTB_CHUNK_PASS(P, GY, GZ)                                                                                       \
+  launch_pdl(rglru_chunk_kernel<T, P, RAW>, dim3(gx, GY, GZ), threads, 0, stream,                                                \
       gates, gates_b, (const T*)u, (const T*)y_act, lam, (const T*)proj, bx, state, state_stride, slots, sb, chunk_seq, chunk_q0, \
       seq_chunk0, n_chunks, chunk_len, agg_a, agg_b, s_start, (T*)out, R, bw, taps, c_decay)
-  PTB_CHUNK_PASS(1, n_chunks * SPLIT);
-  PTB_CHUNK_PASS(2, sb.n_seqs);
-  PTB_CHUNK_PASS(3, n_chunks * SPLIT);
+  PTB_CHUNK_PASS(1, n_chunks, SPLIT);
+  PTB_CHUNK_PASS(2, sb.n_seqs, 1);
+  PTB_CHUNK_PASS(3, n_chunks, SPLIT);
 #undef PTB_CHUNK_PASS
   return launch_status();
 }
@@ -668,7 +668,7 @@ PTB_API int ptb_rglru_scan_chunks(int dtype, float* gates, const float* gates_b,
                                   int blocks_n, int taps, float c_decay, cudaStream_t stream) {
   if (sb->n_tokens <= 0 || n_chunks <= 0) return PTB_OK;
   if (R <= 0 || blocks_n <= 0 || R % blocks_n != 0 || taps < 1 || taps > MAX_TAPS || chunk_len <= 0 ||
-      n_chunks > 65535 / SPLIT || sb->n_seqs > 65535)
+      n_chunks > 65535 || sb->n_seqs > 65535)
     return PTB_ERR_SIZE;
 #define PTB_RSC(TT, RAW)                                                                                                     \
   launch_rglru_chunks<TT, RAW>(gates, gates_b, u, y_act, lam, proj, bx, state, state_stride, slots, *sb, chunk_seq, chunk_q0, \

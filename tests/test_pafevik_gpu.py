@@ -707,3 +707,32 @@ def test_unfolded_attention_gated(dim, rot, vdim, per_head, wide, pasts):
     gd = torch.sigmoid(gate.double().cpu())
     ref = ref * (gd[:, :, None] if per_head else gd.view(n, heads, vdim))
     assert row_errors(got, ref.reshape(n, -1)).max() < 5 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("raw", [False, True])
+def test_scan_of_as_many_chunks_as_a_grid_has_rows(raw):
+    """40,000 chunks of two tokens: a step is taken up to 65,535 chunks, however a chunk is divided among blocks. Against the
+    walk; a chunk's start is joined from its predecessors' sums of logarithms, 2^-24 of the state a chunk at most, and decays
+    near 0.5 forget all but the last few of them."""
+    k = __import__("pytorch_transformers_b200.kernels", fromlist=["kernels"])
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.base import StateNeed
+    n, R, blocks, taps, chunk = 80000, 8, 2, 2, 2
+    g = torch.Generator().manual_seed(3)
+    rn = lambda *s: torch.randn(*s, generator=g).cuda()
+    cache = Cache([(0, None, StateNeed(R * taps))], 64, torch.bfloat16, "cuda", max_slots=1)
+    slots = [cache.open()]
+    ctx = StepContext(cache, slots, [[0] * n], 1, [[]], [])
+    product, bias, u, y = rn(blocks, n, 2 * R // blocks), rn(blocks, 2 * R // blocks), rn(n, R).bfloat16(), rn(n, R).bfloat16()
+    proj, bx, lam = rn(n, 2 * R).bfloat16(), rn(R), torch.zeros(R, device="cuda")
+    gates = torch.sigmoid(product + bias[:, None]).transpose(0, 1).contiguous()
+    n_chunks = n // chunk
+    index = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    tiles = (index([0] * n_chunks), index(list(range(0, n, chunk))), index([0]), n_chunks, chunk)
+    walked, joined = (torch.zeros(cache.state.shape[0], R * taps, device="cuda") for _ in range(2))
+    ref = k.rglru_scan(gates, u, y, lam, proj, bx, walked, ctx.dev["slots"], ctx.batch_c[0], blocks, taps, 8.0)
+    got = k.rglru_scan_chunks(product.clone() if raw else gates, u, y, lam, proj, bx, joined, ctx.dev["slots"], ctx.batch_c[0], blocks, taps,
+                              8.0, *tiles, gates_bias=bias if raw else None)
+    torch.testing.assert_close(got.float(), ref.float(), rtol=2.0 ** -7, atol=1e-4)      # one unit of bfloat16
+    torch.testing.assert_close(joined, walked, rtol=1e-5, atol=1e-6)
