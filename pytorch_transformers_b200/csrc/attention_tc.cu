@@ -434,8 +434,8 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
     if (EXTRAS) {
       if (p.sinks) {
         const float m2 = m_run * sl2, sink2 = p.sinks[h] * 1.4426950408889634f, m_all = fmaxf(m2, sink2);
-        const float keep = (m_run == -INFINITY) ? 0.f : fast_exp2(m2 - m_all);
-        const float l = l_run * keep + fast_exp2(sink2 - m_all);
+        const float keep = (m_run == -INFINITY) ? 0.f : exp2f(m2 - m_all);
+        const float l = l_run * keep + exp2f(sink2 - m_all);
         inv = (l > 0.f ? 1.f / l : 0.f) * keep;
       }
       inv *= p.out_scale;
