@@ -660,7 +660,7 @@ PTB_API int ptb_rglru_scan(int dtype, const float* gates, const void* u, const v
 PTB_API long long ptb_rglru_chunks_work_floats(int n_chunks, int R) { return 3LL * n_chunks * SPLIT * R; }
 
 // gates_b null: `gates` [tokens, blocks, 2 bw] after their sigmoid. gates_b [blocks][2 bw]: `gates` [blocks][tokens][2 bw] is the
-// gates' product without bias and sigmoid, which the scan writes over.
+// gates' product without bias and sigmoid, which the scan writes over (bfloat16 only: float32 prompts have no such product).
 PTB_API int ptb_rglru_scan_chunks(int dtype, float* gates, const float* gates_b, const void* u, const void* y_act, const float* lam,
                                   const void* proj, const float* bx, float* state, long long state_stride,
                                   const int* slots, const StepBatch* sb, const int* chunk_seq, const int* chunk_q0,
@@ -673,7 +673,7 @@ PTB_API int ptb_rglru_scan_chunks(int dtype, float* gates, const float* gates_b,
 #define PTB_RSC(TT, RAW)                                                                                                     \
   launch_rglru_chunks<TT, RAW>(gates, gates_b, u, y_act, lam, proj, bx, state, state_stride, slots, *sb, chunk_seq, chunk_q0, \
                                seq_chunk0, n_chunks, chunk_len, work, out, R, R / blocks_n, taps, c_decay, stream)
-  if (dtype == PTB_F32) return gates_b ? PTB_RSC(float, true) : PTB_RSC(float, false);
+  if (dtype == PTB_F32) return gates_b ? PTB_ERR_DTYPE : PTB_RSC(float, false);
   if (dtype == PTB_BF16) return gates_b ? PTB_RSC(__nv_bfloat16, true) : PTB_RSC(__nv_bfloat16, false);
 #undef PTB_RSC
   return PTB_ERR_DTYPE;

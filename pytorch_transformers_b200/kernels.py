@@ -1108,6 +1108,8 @@ def rglru_scan_chunks(gates: torch.Tensor, u: torch.Tensor, y_act: torch.Tensor,
     n, r = u.shape
     if gates.dtype != torch.float32 or gates.numel() != n * 2 * r or state.stride(1) != 1 or state.shape[1] != r * taps:
         raise KernelError("rglru_scan_chunks: gates or state do not fit")
+    if gates_bias is not None and u.dtype != torch.bfloat16:
+        raise KernelError("rglru_scan_chunks: the gates' bare product is for bfloat16")
     if gates_bias is not None and (gates_bias.dtype != torch.float32 or gates_bias.numel() != 2 * r or gates.shape[0] != blocks):
         raise KernelError("rglru_scan_chunks: the gates' product is [blocks, tokens, 2 R / blocks] and their bias float32")
     out = torch.empty_like(u)

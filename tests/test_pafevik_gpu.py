@@ -736,3 +736,13 @@ def test_scan_of_as_many_chunks_as_a_grid_has_rows(raw):
                               8.0, *tiles, gates_bias=bias if raw else None)
     torch.testing.assert_close(got.float(), ref.float(), rtol=2.0 ** -7, atol=1e-4)      # one unit of bfloat16
     torch.testing.assert_close(joined, walked, rtol=1e-5, atol=1e-6)
+
+
+def test_scan_refuses_the_gates_product_in_float32():
+    """float32 prompts have no bare product; the form is refused before any pointer is read."""
+    from pytorch_transformers_b200 import kernels as k
+    z = lambda *s: torch.zeros(*s, device="cuda")
+    ints = torch.zeros(4, dtype=torch.int32, device="cuda")
+    with pytest.raises(k.KernelError, match="bfloat16"):
+        k.rglru_scan_chunks(z(2, 64, 8), z(64, 8), z(64, 8), z(8), z(64, 16), z(8), z(1, 16), ints, k.StepBatchC(), 2, 2, 8.0, ints,
+                            ints, ints, 1, 64, gates_bias=z(2, 8))
