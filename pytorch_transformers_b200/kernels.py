@@ -574,8 +574,12 @@ def attention_tc_extras(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Ten
     weights meet the values as two bfloat16 terms (not with ``wide_weights=False``). bfloat16, the head sizes that ``attention_tc``
     takes."""
     _need_cuda(q, k_pool, v_pool, tile_seq, tile_q0, sinks)
+    if not q.dtype == k_pool.dtype == v_pool.dtype == torch.bfloat16:
+        raise KernelError("attention_tc_extras takes bfloat16 tensors")
     n, heads, head_dim = q.shape
     v_dim = v_pool.shape[-1]
+    if k_pool.shape[:-1] != v_pool.shape[:-1] or k_pool.shape[-1] != head_dim:
+        raise KernelError("attention_tc_extras takes the K and V pools of one cache entry")
     if out is None:
         out = torch.empty((n, heads * v_dim), dtype=q.dtype, device=q.device)
     _check_rows(out, (n, heads * v_dim), q.dtype, "attention_tc_extras: out")

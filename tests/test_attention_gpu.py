@@ -491,3 +491,17 @@ def test_general_attention_reads_words_and_values_alike(K, dtype, d, vd):
             out.append(K.attention_generic(q, moved[0], moved[1], ctx.batch_c[group], tiles.dev["tile_seq"], tiles.dev["tile_q0"],
                                            tiles.facts["n_tiles"], None, kv, d ** -0.5))
         assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
+
+
+def test_prompt_attention_with_extras_refuses_other_types_and_pools(K):
+    """What the plain prompt attention refuses: other element types, pools that do not belong together."""
+    ints = torch.zeros(1, dtype=torch.int32, device="cuda")
+    def call(q, k_pool, v_pool):
+        return K.attention_tc_extras(q, k_pool, v_pool, K.StepBatchC(), ints, ints, 0, 1, 1.0)
+    z = lambda *s, dt=torch.bfloat16: torch.zeros(*s, dtype=dt, device="cuda")
+    call(z(4, 2, 64), z(2, 1, 64, 64), z(2, 1, 64, 64))         # no tiles: nothing runs
+    for bad in ((z(4, 2, 64, dt=torch.float32), z(2, 1, 64, 64), z(2, 1, 64, 64)),
+                (z(4, 2, 64), z(2, 1, 64, 64, dt=torch.float32), z(2, 1, 64, 64)),
+                (z(4, 2, 64), z(2, 1, 64, 128), z(2, 1, 64, 128)), (z(4, 2, 64), z(2, 1, 64, 64), z(3, 1, 64, 64))):
+        with pytest.raises(K.KernelError):
+            call(*bad)
