@@ -119,10 +119,14 @@ constexpr int BLOCK_THREADS = SOFTMAX_THREADS + 64;
 // exponential and a reciprocal a score): 16 heads of 128 on 4 K/V heads, 2,048 tokens, window 1,024: 39 us, where
 // the mma.sync kernel took 175; prompts of 500, 1,000 and 1,501 tokens, cap and a gate per entry: 75 us against 261.
 // TWO (head size 128 with weights of two terms): two S buffers and two page stages instead of three and four, 97 KB and 256
-// columns of tensor memory a block, so that two blocks fit on an SM and one's softmax runs under the other's waits. Worth it
-// where the blocks make more than two waves (384 blocks, capped: 104 -> 75 us) or the walks of a window are alike long (256
-// blocks: 41 -> 39 us); with fewer blocks and the triangle of a full context the longest chain counts, and a
-// block with an SM of its own runs it faster (256 blocks: 41 us alone, 52 us two an SM).
+// columns of tensor memory a block, so that two blocks fit on an SM and one's softmax runs under the other's waits. Taken where
+// the blocks make more than two waves, or more than one with a window, whose walks are alike long; with fewer blocks and the
+// triangle of a full context the longest chain counts, and a block with an SM of its own runs it faster. us, one an SM
+// against two: full context 256 blocks 39 / 47, 288 47 / 54, 320 59 / 60, 384 (one prompt) 81 / 72, 512 126 / 116, 640 110 /
+// 88; capped 256 55 / 55, 288 66 / 63, 320 85 / 71, 384 (three prompts) 56 / 46; window of 300: 160 18 / 16, 256 24 / 19, 512
+// 45 / 34; of 1,024: 256 (2,048 tokens) 38 / 32, 288 44 / 38, 512 72 / 68. Where most of a prompt fits into its window the walks are
+// a triangle again and one an SM would be the faster: 160 blocks of 1,024 in 2,560 tokens 24 / 30, four prompts of 640 15 / 19 (the
+// rule does not look at lengths).
 template <bool TWO> struct TcShape {
   static constexpr int BUFS = TWO ? 2 : 3;                 // S buffers
   static constexpr int STAGES = TWO ? 2 : STAGES_TC;       // page stages

@@ -20,10 +20,10 @@
 // Every wait on a barrier is bounded: when one runs out, the error flag is raised and the block carries on to its end without
 // waiting again.
 //
-// One B200, 64 experts of 1,408, width 2,048: 12,288 rows (about 192 an expert, tiles of 256) gate and up 491 -> 182 us
-// (780 TFLOP/s), down 263 -> 114 us; 48 rows (tiles of 16) 88 -> 67 and 45 -> 35 us (5.9 TB/s of the matrices of the experts
-// in use); before, 64 x 128 tiles on mma.sync. With many rows nothing is saturated (tensor pipe 38 %, memory 52 %): the ring's three or
-// four stages of 56 KB hold too little of the way from memory. Boxes asked into L2 eight stages ahead changed nothing there
+// One B200, 64 experts of 1,408, width 2,048: 12,288 rows (about 192 an expert, tiles of 256) gate and up 491 -> 204 us
+// (695 TFLOP/s), down 263 -> 114 us; 48 rows (tiles of 16) 88 -> 70 and 45 -> 35 us (5.7 TB/s of the matrices of the experts
+// in use); before, 64 x 128 tiles on mma.sync. With many rows nothing is saturated (tensor pipe 38 %, memory 52 %): the rings hold too
+// little of the way from memory (192 rows: three stages of 56 KB for gate and up; two of 40 KB in each of two blocks for down). Boxes asked into L2 eight stages ahead changed nothing there
 // and cost a third with few rows (67 -> 90 us).
 #include <cudaTypedefs.h>
 

@@ -2,16 +2,16 @@
 // No tensor cores and no reduced-precision mode: every product and sum is an IEEE float32 FMA.
 //
 // The sums of one output element: the k of a step of 32 are summed in two chains (even and odd k, 16 products each, ascending),
-// the two chains join and go into a running total; a K of 1,024 or more is cut into 2 or 4 stretches whose totals are added
-// in order. All of this follows from N and K alone, so a row's result depends neither on how many other rows are in the
+// the two chains join and go into a running total; a K of 2,048 or more is cut into four stretches whose totals are added in
+// order, a K of 1,024 to 2,047 beside fewer than 2,048 outputs into two, any other into none. All of this follows from N and K alone, so a row's result depends neither on how many other rows are in the
 // launch nor on the tile, and the rounding error stays small for K in the tens of thousands.
 //
 // What bounds it is the FMA pipe (128 lanes an SM). A block owns 8 TM rows x 64 outputs, a thread TM x 4 of them: of every
 // 16 bytes that it reads from shared memory (operands stay in [row][k] order, so cp.async brings them without a
 // transposition, and rows lie 36 floats apart, which lets eight rows' 16-byte words meet no bank twice) it makes
 // 2 TM x 4 / (TM + 4) two-wide FMAs (fma.rn.f32x2: the two k chains in one 64-bit register). A three-stage ring keeps two
-// steps of copies in flight. Matrices with few outputs would leave SMs idle: their K is cut among a thread-block cluster
-// whose blocks join their tiles through distributed shared memory.
+// steps of copies in flight. Few rows or few outputs would leave SMs idle: K is cut among a thread-block cluster whose blocks
+// join their tiles through distributed shared memory.
 // One B200: the four products of a block of width 1,024 on 700 rows 1,057 -> 517 us (700 x 1,024 x 4,096: 152 us, 39 TFLOP/s of
 // 72; 2,048 rows: 43), 20 rows of 1,024 x 4,096 30 us; before, 64 x 64 tiles with two scalar loads a product and no copies in
 // flight. Now the two-wide FMAs of three blocks an SM leave half of the issue slots empty: registers (168 a thread) allow no more
@@ -177,8 +177,12 @@ PTB_API int ptb_linear_f32(const float* x, const float* w, const float* bias, fl
   if (M <= 0 || N <= 0) return PTB_OK;
   if (K <= 0 || ldx < K || !activation_known(act)) return PTB_ERR_SIZE;
   if ((long(M) + 63) / 64 > 65535) return PTB_ERR_SIZE;
-  // stretches of K, by N and K alone (the order of a row's sums must not follow the number of rows): a matrix of 1,024
-  // outputs and 700 rows has 176 tiles, little more than an SM each, which two or four stretches even out
+  // stretches of K, by N and K alone (the order of a row's sums must not follow the number of rows). A matrix of 1,024 outputs
+  // and 700 rows has 176 tiles, little more than an SM each, which stretches even out; with one row it has 16. us for one,
+  // two and four stretches: 1 row, N 1,024 K 4,096: 73, 39, 21; 4,096 x 2,048: 38, 22, 17; 18,176 x 4,544: 120, 119, 120. 700
+  // rows, 1,024 x 1,024: 67, 55, 52; 1,024 x 4,096: 256, 189, 181; 2,048 x 2,048: 184, 158, 170; 4,096 x 2,048: 295, 301, 316;
+  // 4,544 x 18,176: 3,047, 2,747, 2,835; 18,176 x 4,544: 2,701, 2,674, 2,852. So long K gains most where rows or outputs are
+  // few, and from some 8,192 outputs on the join costs 3 to 10 % on many rows and gives nothing back on few.
   const int ranks = K >= 2048 ? 4 : (K >= 1024 && N < 2048) ? 2 : 1;
   // 16-byte copies where every row starts at a whole word
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && aligned16(x) && aligned16(w);
