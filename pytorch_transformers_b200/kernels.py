@@ -46,7 +46,8 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream(t: torch.Tensor):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    # the current stream's handle as torch keeps it: 0.1 us, where current_stream(device) makes an object in 2.5
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(t.get_device()))
 
 
 launches = 0  # entry points called so far (every one launches one kernel of this library)
