@@ -21,6 +21,30 @@ namespace {
 
 constexpr float LOG2E_F = 1.4426950408889634f;
 
+// two float32 values in a 64-bit register: the two-wide multiply-adds
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ float2 halves2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ unsigned long long wide2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long minus2(unsigned long long a, unsigned long long b) { return fma2(b, 0xbf800000bf800000ull, a); }
+
 // hi and lo terms of two neighbouring values of a row of a swizzled [rows][D] tile
 template <int D>
 __device__ __forceinline__ void put_split(unsigned char* hi_tile, unsigned char* lo_tile, int row, int col, float x, float y) {
@@ -31,26 +55,40 @@ __device__ __forceinline__ void put_split(unsigned char* hi_tile, unsigned char*
   *reinterpret_cast<uint32_t*>(lo_tile + off) = lo;
 }
 
+template <int N>
+struct Count {       // a number that an unrolled loop knows
+  __device__ constexpr operator int() const { return N; }
+};
+
 template <int DK, int DV, bool PER_HEAD>
 struct LocalSmem {
-  static constexpr int KP = DK + 8, CP = PER_HEAD ? 1 : DK + 8, TP = CH + 1;
+  static constexpr int KP = DK + 8, CP = PER_HEAD ? 1 : DK + 8, TP = CH + 4;
   static constexpr int cb = 0;                                   // [CH][CP] float: sums of logarithms from the sub-block's start
   static constexpr int tot = cb + (CH * CP * 4 + 127) / 128 * 128;   // [4][DK] float: the sub-blocks' totals
-  static constexpr int q = tot + (PER_HEAD ? 128 : 4 * DK * 4);  // [CH][KP] bfloat16
+  static constexpr int fr = tot + (PER_HEAD ? 128 : 4 * DK * 4); // [4][DK] float: the totals of the sub-blocks before each, summed
+  static constexpr int bk = fr + (PER_HEAD ? 128 : 4 * DK * 4);  // [4][DK] float: of those after
+  static constexpr int q = bk + (PER_HEAD ? 128 : 4 * DK * 4);   // [CH][KP] bfloat16
   static constexpr int k = q + CH * KP * 2;
   static constexpr int v = k + CH * KP * 2;                      // [CH][DV] swizzled: values, then U_0's hi
   static constexpr int a = v + CH * DV * 2;                      // [CH][TP] float: L, then T diag(beta) hi and lo [CH][CH]
   static constexpr int p = a + CH * TP * 4;                      // P hi and lo [CH][CH]
   static constexpr int t = p + 2 * CH * CH * 2;                  // [CH][TP] float: (I + L)^-1
-  static constexpr int x = t + CH * TP * 4;                      // [3][16][16] float
-  static constexpr int kw = x + 3 * 256 * 4;                     // Kc hi and lo [CH][DK], then W
+  static constexpr int x = t + CH * TP * 4;                      // [32][32] float, or two of [16][16]
+  static constexpr int kw = x + 4 * 256 * 4;                     // Kc hi and lo [CH][DK], then W
   static constexpr int ulo = kw + 2 * CH * DK * 2;               // [CH][DV]: U_0's lo
   static constexpr int kd = ulo + CH * DV * 2;                   // Kd hi and lo [CH][DK]
   static constexpr int small = kd + 2 * CH * DK * 2;             // rq, rk, beta [CH] float each
   static constexpr int bytes = small + 3 * CH * 4;
 };
 
-// One block = one chunk x one head; DK / 8 warps.
+// One block = one chunk x one head; DK / 8 warps. What bounds it: a block takes 225 KB of shared memory, so an SM holds one, and its
+// phases are short chains between barriers (decay per channel, 128 x 128: 42,000 clocks a block, of them scores 12,000, products 14,000,
+// loads 5,400, the inverse with the decayed keys 5,000 and its join 4,000; 79,400 before). So the scores' work is divided by count of
+// instructions over all warps: a pair of sub-blocks' keys and queries take the same exponentials and the same decayed keys, halves of a sub-block
+// meet by a product too, which leaves 288 pairs of tokens with exponents of their own of 544; totals before and after a sub-block are
+// kept instead of summed at every use; decayed keys are formed four channels a lane (one channel's neighbours in a lane met the
+// same bank eight times); the inverse joins 16 below 16, then 32 below 32, from rows in 16-byte words. 2,048 tokens of 16 heads of
+// 128 x 128, both passes 222 -> 171 us (this one 153 -> 102).
 // mq [chunk][head][DK / 16 + 4 row tiles][DK / 16][hi, lo][32 lanes] 16-byte words: M's rows, then Q's, as mma A fragments.
 // bo [chunk][head][DK / 16 + 4 row tiles][DV / 8][32 lanes] float4: B's rows, then O_0's, as mma C fragments.
 // dec [chunk][head][DK]: exp(c_n).
@@ -64,7 +102,7 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
   extern __shared__ __align__(128) unsigned char sm[];
   constexpr int NW = DK / 8, NT = NW * 32, KP = L::KP, CP = L::CP, TP = L::TP, MT = DK / 16 + 4;
   float* cb = reinterpret_cast<float*>(sm + L::cb);
-  float* tot = reinterpret_cast<float*>(sm + L::tot);
+  float *tot = reinterpret_cast<float*>(sm + L::tot), *fr = reinterpret_cast<float*>(sm + L::fr), *bk = reinterpret_cast<float*>(sm + L::bk);
   __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(sm + L::q);
   __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(sm + L::k);
   float* As = reinterpret_cast<float*>(sm + L::a);
@@ -134,129 +172,220 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
     }
   }
   __syncthreads();
-  auto cb_at = [&](int row, int d) { return PER_HEAD ? cb[row] : cb[row * CP + d]; };
-  auto tot_at = [&](int b, int d) { return PER_HEAD ? tot[b] : tot[b * DK + d]; };
-  // exponents (base 2): from the chunk's start to the token, and from the token to the chunk's end
-  auto from_start = [&](int row, int d) {
-    float s = 0.f;
-    for (int b = 0; b < row / 16; ++b) s += tot_at(b, d);
-    return s + cb_at(row, d);
-  };
-  auto to_end = [&](int row, int d) {
-    float s = tot_at(row / 16, d) - cb_at(row, d);
-    for (int b = row / 16 + 1; b < 4; ++b) s += tot_at(b, d);
-    return s;
-  };
-
-  // ---- L and P between sub-blocks, a warp per (later, earlier, L or P); with one decay per head also inside them
-  constexpr int PAIRS = PER_HEAD ? 10 : 6;
-  for (int task = warp; task < 2 * PAIRS; task += NW) {
-    const int pair = task >> 1;
-    const bool is_p = task & 1;
-    int i, j;
-    if (PER_HEAD) {     // (0,0) (1,0) (1,1) (2,0) ...
-      i = pair < 1 ? 0 : (pair < 3 ? 1 : (pair < 6 ? 2 : 3));
-      j = pair - i * (i + 1) / 2;
-    } else {            // (1,0) (2,0) (2,1) (3,0) ...
-      i = pair < 1 ? 1 : (pair < 3 ? 2 : 3);
-      j = pair - i * (i - 1) / 2;
+  // the totals before and after every sub-block (read after the next barrier)
+  constexpr int LD = PER_HEAD ? 1 : DK;
+  for (int i = tid; i < 4 * LD; i += NT) {
+    const int b = i / LD, d = i % LD;
+    float f = 0.f, e = 0.f;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      const float t = tot[o * LD + d];
+      if (o < b) f += t;
+      if (o > b) e += t;
     }
-    const __nv_bfloat16* left = is_p ? qs : ks;
-    float acc[2][4] = {};
+    fr[i] = f;
+    bk[i] = e;
+  }
+  // exponents (base 2) of two neighbouring channels from the chunk's start to the token
+  auto from_start = [&](int row, int d) {
+    if constexpr (PER_HEAD) {
+      const float x = fr[row / 16] + cb[row];
+      return make_float2(x, x);
+    } else {
+      const float2 f = *reinterpret_cast<const float2*>(fr + row / 16 * DK + d), c2 = *reinterpret_cast<const float2*>(cb + row * CP + d);
+      return make_float2(f.x + c2.x, f.y + c2.y);
+    }
+  };
+  // ---- L and P
+  auto put_scores = [&](int i, int j, int nt, const float (&l)[4], const float (&q)[4], auto factor) {
 #pragma unroll
-    for (int kk = 0; kk < DK / 16; ++kk) {
-      uint32_t ah[4], al[4];
+    for (int half = 0; half < 2; ++half) {
+      const int row = i * 16 + g4 + half * 8, col = j * 16 + nt * 8 + t4 * 2;
+      float f[2];
 #pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        const int row = i * 16 + g4 + (f & 1) * 8, d = kk * 16 + t4 * 2 + (f >> 1) * 8;
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(left + row * KP + d);
-        if constexpr (PER_HEAD) {
-          ah[f] = w;
-        } else {
-          const float2 e = *reinterpret_cast<const float2*>(cb + row * CP + d);
-          split_pack(__uint_as_float(w << 16) * fast_exp2(e.x), __uint_as_float(w & 0xffff0000u) * fast_exp2(e.y), ah[f], al[f]);
+      for (int e = 0; e < 2; ++e) f[e] = rk[col + e] * factor(row, col + e);
+      const float b = rk[row] * bt[row];
+      As[row * TP + col] = l[half * 2] * f[0] * b;
+      As[row * TP + col + 1] = l[half * 2 + 1] * f[1] * b;
+      put_split<CH>(p_hi, p_lo, row, col, q[half * 2] * f[0] * rq[row], q[half * 2 + 1] * f[1] * rq[row]);
+    }
+  };
+  if constexpr (PER_HEAD) {
+    // one decay per head: a factor of the product's result, also inside sub-blocks; a warp per (later, earlier)
+    for (int pair = warp; pair < 10; pair += NW) {       // (0,0) (1,0) (1,1) (2,0) ...
+      const int i = pair < 1 ? 0 : (pair < 3 ? 1 : (pair < 6 ? 2 : 3)), j = pair - i * (i + 1) / 2;
+      float l[2][4] = {}, q[2][4] = {};
+#pragma unroll
+      for (int kk = 0; kk < DK / 16; ++kk) {
+        uint32_t ak[4], aq[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const int at = (i * 16 + g4 + (f & 1) * 8) * KP + kk * 16 + t4 * 2 + (f >> 1) * 8;
+          ak[f] = *reinterpret_cast<const uint32_t*>(ks + at);
+          aq[f] = *reinterpret_cast<const uint32_t*>(qs + at);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const __nv_bfloat16* b = ks + (j * 16 + nt * 8 + g4) * KP + kk * 16 + t4 * 2;
+          const uint32_t b0 = *reinterpret_cast<const uint32_t*>(b), b1 = *reinterpret_cast<const uint32_t*>(b + 8);
+          mma_bf16(l[nt], ak, b0, b1);
+          mma_bf16(q[nt], aq, b0, b1);
         }
       }
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        uint32_t bh[2], bl[2];
+      for (int nt = 0; nt < 2; ++nt)
+        put_scores(i, j, nt, l[nt], q[nt], [&](int row, int col) {
+          float x = i == j ? cb[row] - cb[col] : tot[j] - cb[col] + cb[row];
+          for (int b = j + 1; b < i; ++b) x += tot[b];
+          return col <= row ? fast_exp2(x) : 0.f;       // what comes later takes no part
+        });
+    }
+  } else {
+    // Between sub-blocks a warp a pair (later, earlier): keys and queries of the later one take the same exponentials, and L and P the
+    // same decayed keys of the earlier one. Inside a sub-block the later half meets the earlier one in the same way, with the sums from
+    // the halves' border: keys and queries are the two halves of the matrix instruction's rows. Inside a half every pair of tokens has
+    // exponents of its own, four lanes along the channels, eight pairs a warp at a time.
+    // KSPLIT warps share a pair's channels; the second one's sums wait where the decayed keys will stand.
+    constexpr int KSPLIT = NW == 16 ? 2 : 1;
+    if (warp < 6 * KSPLIT) {
+      const int pair = warp / KSPLIT, part = warp % KSPLIT;          // (1,0) (2,0) (2,1) (3,0) ...
+      const int i = pair < 1 ? 1 : (pair < 3 ? 2 : 3), j = pair - i * (i - 1) / 2;
+      float l[2][4] = {}, q[2][4] = {};
+#pragma unroll 2
+      for (int kk = part * (DK / 16 / KSPLIT); kk < (part + 1) * (DK / 16 / KSPLIT); ++kk) {
+        uint32_t kh[4], kl[4], qh[4], ql[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const int row = i * 16 + g4 + (f & 1) * 8, d = kk * 16 + t4 * 2 + (f >> 1) * 8;
+          const uint32_t wk = *reinterpret_cast<const uint32_t*>(ks + row * KP + d), wq = *reinterpret_cast<const uint32_t*>(qs + row * KP + d);
+          float2 e = *reinterpret_cast<const float2*>(cb + row * CP + d);
+          e.x = fast_exp2(e.x), e.y = fast_exp2(e.y);
+          split_pack(__uint_as_float(wk << 16) * e.x, __uint_as_float(wk & 0xffff0000u) * e.y, kh[f], kl[f]);
+          split_pack(__uint_as_float(wq << 16) * e.x, __uint_as_float(wq & 0xffff0000u) * e.y, qh[f], ql[f]);
+        }
+        float2 mid[2];      // the whole sub-blocks between
 #pragma unroll
         for (int f = 0; f < 2; ++f) {
-          const int row = j * 16 + nt * 8 + g4, d = kk * 16 + t4 * 2 + f * 8;
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(ks + row * KP + d);
-          if constexpr (PER_HEAD) {
-            bh[f] = w;
-          } else {
-            const float2 e = *reinterpret_cast<const float2*>(cb + row * CP + d);
-            float2 r = *reinterpret_cast<const float2*>(tot + j * DK + d);
-            r.x -= e.x;
-            r.y -= e.y;
-            for (int b = j + 1; b < i; ++b) {
-              const float2 o = *reinterpret_cast<const float2*>(tot + b * DK + d);
-              r.x += o.x;
-              r.y += o.y;
-            }
-            split_pack(__uint_as_float(w << 16) * fast_exp2(r.x), __uint_as_float(w & 0xffff0000u) * fast_exp2(r.y), bh[f], bl[f]);
+          const int d = kk * 16 + t4 * 2 + f * 8;
+          mid[f] = *reinterpret_cast<const float2*>(tot + j * DK + d);
+#pragma unroll
+          for (int b = 1; b < 3; ++b) {
+            if (b <= j || b >= i) continue;
+            const float2 o = *reinterpret_cast<const float2*>(tot + b * DK + d);
+            mid[f].x += o.x;
+            mid[f].y += o.y;
           }
         }
-        mma_bf16(acc[nt], ah, bh[0], bh[1]);
-        if constexpr (!PER_HEAD) {
-          mma_bf16(acc[nt], ah, bl[0], bl[1]);
-          mma_bf16(acc[nt], al, bh[0], bh[1]);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          uint32_t bh[2], bl[2];
+#pragma unroll
+          for (int f = 0; f < 2; ++f) {
+            const int row = j * 16 + nt * 8 + g4, d = kk * 16 + t4 * 2 + f * 8;
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(ks + row * KP + d);
+            const float2 e = *reinterpret_cast<const float2*>(cb + row * CP + d);
+            split_pack(__uint_as_float(w << 16) * fast_exp2(mid[f].x - e.x), __uint_as_float(w & 0xffff0000u) * fast_exp2(mid[f].y - e.y), bh[f], bl[f]);
+          }
+          mma_bf16(l[nt], kh, bh[0], bh[1]);
+          mma_bf16(q[nt], qh, bh[0], bh[1]);
+          mma_bf16(l[nt], kh, bl[0], bl[1]);
+          mma_bf16(q[nt], qh, bl[0], bl[1]);
+          mma_bf16(l[nt], kl, bh[0], bh[1]);
+          mma_bf16(q[nt], ql, bh[0], bh[1]);
         }
+      }
+      if constexpr (KSPLIT == 2) {
+        float4* wait = reinterpret_cast<float4*>(kd_hi) + pair * 4 * 32 + lane;
+        if (part == 1) {
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            wait[nt * 32] = make_float4(l[nt][0], l[nt][1], l[nt][2], l[nt][3]);
+            wait[(2 + nt) * 32] = make_float4(q[nt][0], q[nt][1], q[nt][2], q[nt][3]);
+          }
+        }
+        asm volatile("bar.sync %0, 64;\n" ::"r"(pair + 1) : "memory");      // the pair's two warps
+        if (part == 0) {
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            const float4 x = wait[nt * 32], y = wait[(2 + nt) * 32];
+            l[nt][0] += x.x, l[nt][1] += x.y, l[nt][2] += x.z, l[nt][3] += x.w;
+            q[nt][0] += y.x, q[nt][1] += y.y, q[nt][2] += y.z, q[nt][3] += y.w;
+          }
+        }
+      }
+      if (part == 0) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) put_scores(i, j, nt, l[nt], q[nt], [](int, int) { return 1.f; });
       }
     }
+    auto halves_meet = [&](int b) {
+      float acc[4] = {};      // rows 0 - 7: L, rows 8 - 15: P
+      const int row = b * 16 + 8 + g4, col = b * 16 + g4, edge = b * 16 + 7;
+#pragma unroll 2
+      for (int kk = 0; kk < DK / 16; ++kk) {
+        uint32_t ah[4], al[4], bh[2], bl[2];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int row = i * 16 + g4 + half * 8, col = j * 16 + nt * 8 + t4 * 2;
-        float v[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float f = rk[col + e] * (is_p ? rq[row] : rk[row] * bt[row]);
-          if constexpr (PER_HEAD) {
-            float x = i == j ? cb[row] - cb[col + e] : tot[j] - cb[col + e] + cb[row];
-            for (int b = j + 1; b < i; ++b) x += tot[b];
-            f = col + e <= row ? f * fast_exp2(x) : 0.f;       // what comes later takes no part
-          }
-          v[e] = acc[nt][half * 2 + e] * f;
+        for (int f = 0; f < 2; ++f) {
+          const int d = kk * 16 + t4 * 2 + f * 8;
+          const float2 m = *reinterpret_cast<const float2*>(cb + edge * CP + d);
+          float2 e = *reinterpret_cast<const float2*>(cb + row * CP + d);
+          e.x = fast_exp2(e.x - m.x), e.y = fast_exp2(e.y - m.y);
+          const uint32_t wk = *reinterpret_cast<const uint32_t*>(ks + row * KP + d), wq = *reinterpret_cast<const uint32_t*>(qs + row * KP + d);
+          split_pack(__uint_as_float(wk << 16) * e.x, __uint_as_float(wk & 0xffff0000u) * e.y, ah[2 * f], al[2 * f]);
+          split_pack(__uint_as_float(wq << 16) * e.x, __uint_as_float(wq & 0xffff0000u) * e.y, ah[2 * f + 1], al[2 * f + 1]);
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(ks + col * KP + d);
+          const float2 o = *reinterpret_cast<const float2*>(cb + col * CP + d);
+          split_pack(__uint_as_float(w << 16) * fast_exp2(m.x - o.x), __uint_as_float(w & 0xffff0000u) * fast_exp2(m.y - o.y), bh[f], bl[f]);
         }
-        if (is_p) {
-          put_split<CH>(p_hi, p_lo, row, col, v[0], v[1]);
-        } else {
-          As[row * TP + col] = v[0];
-          As[row * TP + col + 1] = v[1];
-        }
+        mma_bf16(acc, ah, bh[0], bh[1]);
+        mma_bf16(acc, ah, bl[0], bl[1]);
+        mma_bf16(acc, al, bh[0], bh[1]);
       }
-  }
-  if constexpr (!PER_HEAD) {
-    // ---- inside a sub-block: every pair of tokens with exponents of its own, four lanes along the channels
-    const int sub = tid & 3;
-    for (int task = tid >> 2; task < 4 * 136; task += NT / 4) {
-      const int b = task / 136, pr = task % 136, ra = pr / 17, rb = pr % 17;
-      const int r = rb <= ra ? ra : 15 - ra, s = rb <= ra ? rb : rb - ra - 1;     // s <= r
-      const int row = b * 16 + r, col = b * 16 + s;
-      float a = 0.f, p = 0.f;
+      const int c0 = b * 16 + t4 * 2;
+      const float w = rk[row] * bt[row];
+      As[row * TP + c0] = acc[0] * rk[c0] * w;
+      As[row * TP + c0 + 1] = acc[1] * rk[c0 + 1] * w;
+      put_split<CH>(p_hi, p_lo, row, c0, acc[2] * rk[c0] * rq[row], acc[3] * rk[c0 + 1] * rq[row]);
+    };
+    // shares by count of instructions: a pair's half of the channels costs what two halves of a sub-block do, or two and a half eights
+    constexpr int EIGHTS = 8 * 36 / 8;
+    int eight, step, last;
+    if constexpr (NW == 16) {
+      if (warp >= 12) halves_meet(warp - 12);
+      eight = warp < 12 ? warp : 24 + warp - 12;
+      step = warp < 12 ? 12 : 4;
+      last = warp < 12 ? 24 : EIGHTS;
+    } else {
+      if (warp >= 6) {
+        halves_meet(2 * (warp - 6));
+        halves_meet(2 * (warp - 6) + 1);
+      }
+      eight = warp < 6 ? 8 + warp : warp - 6;
+      step = warp < 6 ? 6 : 2;
+      last = warp < 6 ? EIGHTS : 8;
+    }
+    const int sub = lane & 3;
+    for (; eight < last; eight += step) {
+      const int task = eight * 8 + (lane >> 2), b = task / 36, pr = task % 36, ra = pr / 9, rb = pr % 9;
+      const int r = rb <= ra ? ra : 7 - ra, s = rb <= ra ? rb : rb - ra - 1;     // s <= r
+      const int row = b * 8 + r, col = b * 8 + s;
+      unsigned long long a2 = 0ull, p2 = 0ull;      // the even and the odd channels' sums
 #pragma unroll 4
       for (int d = sub * 4; d < DK; d += 16) {
-        const float4 ct = *reinterpret_cast<const float4*>(cb + row * CP + d);
-        const float4 cs = *reinterpret_cast<const float4*>(cb + col * CP + d);
+        const ulonglong2 ct = *reinterpret_cast<const ulonglong2*>(cb + row * CP + d);
+        const ulonglong2 cs = *reinterpret_cast<const ulonglong2*>(cb + col * CP + d);
         const uint2 kt = *reinterpret_cast<const uint2*>(ks + row * KP + d);
         const uint2 k2 = *reinterpret_cast<const uint2*>(ks + col * KP + d);
         const uint2 qt = *reinterpret_cast<const uint2*>(qs + row * KP + d);
-        const float e0 = __uint_as_float(k2.x << 16) * fast_exp2(ct.x - cs.x), e1 = __uint_as_float(k2.x & 0xffff0000u) * fast_exp2(ct.y - cs.y);
-        const float e2 = __uint_as_float(k2.y << 16) * fast_exp2(ct.z - cs.z), e3 = __uint_as_float(k2.y & 0xffff0000u) * fast_exp2(ct.w - cs.w);
-        a = fmaf(__uint_as_float(kt.x << 16), e0, a);
-        a = fmaf(__uint_as_float(kt.x & 0xffff0000u), e1, a);
-        a = fmaf(__uint_as_float(kt.y << 16), e2, a);
-        a = fmaf(__uint_as_float(kt.y & 0xffff0000u), e3, a);
-        p = fmaf(__uint_as_float(qt.x << 16), e0, p);
-        p = fmaf(__uint_as_float(qt.x & 0xffff0000u), e1, p);
-        p = fmaf(__uint_as_float(qt.y << 16), e2, p);
-        p = fmaf(__uint_as_float(qt.y & 0xffff0000u), e3, p);
+        const float2 x = halves2(minus2(ct.x, cs.x)), y = halves2(minus2(ct.y, cs.y));
+        const unsigned long long e0 = mul2(wide2(k2.x), pack2(fast_exp2(x.x), fast_exp2(x.y)));
+        const unsigned long long e1 = mul2(wide2(k2.y), pack2(fast_exp2(y.x), fast_exp2(y.y)));
+        a2 = fma2(wide2(kt.x), e0, a2);
+        a2 = fma2(wide2(kt.y), e1, a2);
+        p2 = fma2(wide2(qt.x), e0, p2);
+        p2 = fma2(wide2(qt.y), e1, p2);
       }
-      // 4 * 136 tasks are whole warps of 8 tasks: all lanes of a warp are here together
+      float a = halves2(a2).x + halves2(a2).y, p = halves2(p2).x + halves2(p2).y;
       a += __shfl_xor_sync(0xffffffffu, a, 1);
       p += __shfl_xor_sync(0xffffffffu, p, 1);
       a += __shfl_xor_sync(0xffffffffu, a, 2);
@@ -273,7 +402,7 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
   }
   __syncthreads();
 
-  // ---- (I + L)^-1 by sub-blocks: the four on the diagonal by substitution, a thread per column
+  // ---- (I + L)^-1 by sub-blocks: the four on the diagonal by substitution, a thread per column of the first two warps
   if (tid < 64) {
     const int b = tid / 16, cc = tid % 16;
     const float* Lb = As + b * 16 * TP + b * 16;
@@ -282,51 +411,96 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
     for (int r = 0; r < 16; ++r) {
       float s = r == cc ? 1.f : 0.f;
 #pragma unroll
-      for (int i = 0; i < r; ++i) s = fmaf(-Lb[r * TP + i], x[i], s);
-      x[r] = s;
-      Ts[(b * 16 + r) * TP + b * 16 + cc] = s;
-    }
-  }
-  // decayed keys meanwhile: both as they stand at the token and as they reach the chunk's end
-  for (int i = tid; i < CH * (DK / 8); i += NT) {
-    const int row = i / (DK / 8), cc = i % (DK / 8);
-    float f[8];
-    unpack_bf16x8(*reinterpret_cast<const uint4*>(ks + row * KP + cc * 8), f);
-    uint4 hi, lo, hi2, lo2;
-    uint32_t *H = &hi.x, *Lo = &lo.x, *H2 = &hi2.x, *Lo2 = &lo2.x;
-    const float r = rk[row];
+      for (int i = 0; i < r; i += 4) {
+        const float4 l = *reinterpret_cast<const float4*>(Lb + r * TP + i);
+        const float lv[4] = {l.x, l.y, l.z, l.w};
 #pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      const int d = cc * 8 + e;
-      const float x = f[e] * r, y = f[e + 1] * r;
-      split_pack(x * fast_exp2(from_start(row, d)), y * fast_exp2(from_start(row, d + 1)), H[e / 2], Lo[e / 2]);
-      split_pack(x * fast_exp2(to_end(row, d)), y * fast_exp2(to_end(row, d + 1)), H2[e / 2], Lo2[e / 2]);
+        for (int e = 0; e < 4; ++e)
+          if (i + e < r) s = fmaf(-lv[e], x[i + e], s);
+      }
+      x[r] = s;
     }
-    const uint32_t off = swz<DK>(row, cc);
-    *reinterpret_cast<uint4*>(w_hi + off) = hi;
-    *reinterpret_cast<uint4*>(w_lo + off) = lo;
-    *reinterpret_cast<uint4*>(kd_hi + off) = hi2;
-    *reinterpret_cast<uint4*>(kd_lo + off) = lo2;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) Ts[(b * 16 + r) * TP + b * 16 + cc] = x[r];
+  }
+  // decayed keys meanwhile, four channels a thread (neighbouring lanes' words then meet no bank twice): both as they stand at the
+  // token and as they reach the chunk's end
+  for (int i = tid - 64; i >= 0 && i < CH * (DK / 4); i += NT - 64) {
+    const int row = i / (DK / 4), d = i % (DK / 4) * 4;
+    const uint2 w = *reinterpret_cast<const uint2*>(ks + row * KP + d);
+    const float r = rk[row];
+    const float x[4] = {__uint_as_float(w.x << 16) * r, __uint_as_float(w.x & 0xffff0000u) * r, __uint_as_float(w.y << 16) * r,
+                        __uint_as_float(w.y & 0xffff0000u) * r};
+    float up[4], down[4];
+    if constexpr (PER_HEAD) {
+      const float u = fast_exp2(fr[row / 16] + cb[row]), v = fast_exp2((tot[row / 16] - cb[row]) + bk[row / 16]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) up[e] = u, down[e] = v;
+    } else {
+      const float4 f = *reinterpret_cast<const float4*>(fr + row / 16 * DK + d), t = *reinterpret_cast<const float4*>(tot + row / 16 * DK + d);
+      const float4 z = *reinterpret_cast<const float4*>(bk + row / 16 * DK + d), y = *reinterpret_cast<const float4*>(cb + row * CP + d);
+      up[0] = fast_exp2(f.x + y.x), up[1] = fast_exp2(f.y + y.y), up[2] = fast_exp2(f.z + y.z), up[3] = fast_exp2(f.w + y.w);
+      down[0] = fast_exp2((t.x - y.x) + z.x), down[1] = fast_exp2((t.y - y.y) + z.y);
+      down[2] = fast_exp2((t.z - y.z) + z.z), down[3] = fast_exp2((t.w - y.w) + z.w);
+    }
+    uint2 hi, lo, hi2, lo2;
+    split_pack(x[0] * up[0], x[1] * up[1], hi.x, lo.x);
+    split_pack(x[2] * up[2], x[3] * up[3], hi.y, lo.y);
+    split_pack(x[0] * down[0], x[1] * down[1], hi2.x, lo2.x);
+    split_pack(x[2] * down[2], x[3] * down[3], hi2.y, lo2.y);
+    const uint32_t off = swz<DK>(row, d >> 3) + (d & 4) * 2;
+    *reinterpret_cast<uint2*>(w_hi + off) = hi;
+    *reinterpret_cast<uint2*>(w_lo + off) = lo;
+    *reinterpret_cast<uint2*>(kd_hi + off) = hi2;
+    *reinterpret_cast<uint2*>(kd_lo + off) = lo2;
   }
   for (int d = tid; d < DK; d += NT)
-    dec[(size_t(c) * heads + h) * DK + d] = fast_exp2(tot_at(0, d) + tot_at(1, d) + tot_at(2, d) + tot_at(3, d));
+    dec[(size_t(c) * heads + h) * DK + d] = fast_exp2(fr[3 * LD + (PER_HEAD ? 0 : d)] + tot[3 * LD + (PER_HEAD ? 0 : d)]);
   __syncthreads();
-  // ... and the others: T_ij = -T_ii sum_k L_ik T_kj, one distance from the diagonal after the other
-#pragma unroll 1
-  for (int lev = 1; lev < 4; ++lev) {
-    for (int e = tid; e < (4 - lev) * 256; e += NT) {
-      const int i = e / 256 + lev, j = i - lev, r = e % 256 / 16, cc = e % 16;
-      float s = 0.f;
-      for (int x = j * 16; x < i * 16; ++x) s = fmaf(As[(i * 16 + r) * TP + x], Ts[x * TP + j * 16 + cc], s);
-      Xs[e] = s;
+  // ... and the others, T_21 = -T_22 (L_21 T_11): first of 16 rows below 16, then of 32 below 32; four columns a thread
+  auto row_times = [&](const float* left, const float* right, int pitch, int from, auto to, float4& s) {     // += sum_x left[x] right[x][0..3]
+#pragma unroll
+    for (int x = 0; x < to; x += 4) {
+      if (x < from) continue;
+      const float4 l = *reinterpret_cast<const float4*>(left + x);
+      const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 t = *reinterpret_cast<const float4*>(right + (x + e) * pitch);
+        s.x = fmaf(lv[e], t.x, s.x), s.y = fmaf(lv[e], t.y, s.y), s.z = fmaf(lv[e], t.z, s.z), s.w = fmaf(lv[e], t.w, s.w);
+      }
+    }
+  };
+  {
+    const int i = tid / 64 * 2 + 1, j = i - 1, r = tid % 64 / 4, cc = tid % 4 * 4;
+    const bool on = tid < 128;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (on) {
+      row_times(As + (i * 16 + r) * TP + j * 16, Ts + j * 16 * TP + j * 16 + cc, TP, 0, Count<16>(), s);
+      *reinterpret_cast<float4*>(Xs + (tid / 64) * 256 + r * 16 + cc) = s;
     }
     __syncthreads();
-    for (int e = tid; e < (4 - lev) * 256; e += NT) {
-      const int i = e / 256 + lev, j = i - lev, r = e % 256 / 16, cc = e % 16;
-      float s = 0.f;
-#pragma unroll
-      for (int x = 0; x < 16; ++x) s = fmaf(-Ts[(i * 16 + r) * TP + i * 16 + x], Xs[(e / 256) * 256 + x * 16 + cc], s);
-      Ts[(i * 16 + r) * TP + j * 16 + cc] = s;
+    if (on) {
+      s = make_float4(0.f, 0.f, 0.f, 0.f);
+      row_times(Ts + (i * 16 + r) * TP + i * 16, Xs + (tid / 64) * 256 + cc, 16, 0, Count<16>(), s);
+      *reinterpret_cast<float4*>(Ts + (i * 16 + r) * TP + j * 16 + cc) = make_float4(-s.x, -s.y, -s.z, -s.w);
+    }
+    __syncthreads();
+  }
+  {
+    const int r = tid / 8, cc = tid % 8 * 4;      // a row and four columns of 32 x 32
+    const bool on = tid < 256;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (on) {
+      row_times(As + (32 + r) * TP, Ts + cc, TP, cc & 16, Count<32>(), s);      // above the diagonal T_11 is zero
+      *reinterpret_cast<float4*>(Xs + r * 32 + cc) = s;
+    }
+    __syncthreads();
+    if (on) {
+      s = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < 16) row_times(Ts + (32 + r) * TP + 32, Xs + cc, 32, 0, Count<16>(), s);
+      else row_times(Ts + (32 + r) * TP + 32, Xs + cc, 32, 0, Count<32>(), s);
+      *reinterpret_cast<float4*>(Ts + (32 + r) * TP + cc) = make_float4(-s.x, -s.y, -s.z, -s.w);
     }
     __syncthreads();
   }
@@ -436,8 +610,9 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
       for (int f = 0; f < 4; ++f) {
         const int row = mi * 16 + g4 + (f & 1) * 8, d = (ng * WN + j + (f >> 1)) * 8 + t4 * 2;
         const uint32_t w = *reinterpret_cast<const uint32_t*>(qs + row * KP + d);
-        const float x = __uint_as_float(w << 16) * rq[row] * fast_exp2(from_start(row, d));
-        const float y = __uint_as_float(w & 0xffff0000u) * rq[row] * fast_exp2(from_start(row, d + 1));
+        const float2 e = from_start(row, d);
+        const float x = __uint_as_float(w << 16) * rq[row] * fast_exp2(e.x);
+        const float y = __uint_as_float(w & 0xffff0000u) * rq[row] * fast_exp2(e.y);
         split_pack(x - wa[j + (f >> 1)][(f & 1) * 2], y - wa[j + (f >> 1)][(f & 1) * 2 + 1], H[f], Lo[f]);
       }
       uint4* dst = mq_c + ((size_t(DK / 16 + mi) * (DK / 16) + (ng * WN + j) / 2) * 2) * 32 + lane;
