@@ -1,5 +1,5 @@
-// True float32 linear layer on the CUDA cores: y[m, n] = act(sum_k x[m, k] * w[n, k] + bias[n]).
-// No tensor cores and no reduced-precision mode: every product and sum is an IEEE float32 FMA.
+// Float32 linear layer: y[m, n] = act(sum_k x[m, k] * w[n, k] + bias[n]). Matrices of some size go to linear_f32_tc.cu; here what is
+// small or laid out oddly, on the CUDA cores: every product and sum is an IEEE float32 FMA.
 //
 // The sums of one output element: the k of a step of 32 are summed in two chains (even and odd k, 16 products each, ascending),
 // the two chains join and go into a running total; a K of 2,048 or more is cut into four stretches whose totals are added in
@@ -18,6 +18,7 @@
 // warps, and tiles of 8 x 8 a thread, which read less, were as fast (43) at 2,048 rows and slower below.
 #include <cooperative_groups.h>
 
+#include "linear_f32.cuh"
 #include "mma_common.cuh"
 
 namespace {
@@ -173,10 +174,15 @@ int launch_linear_f32(const float* x, const float* w, const float* bias, float* 
 
 // x [M, K] with rows ldx apart
 PTB_API int ptb_linear_f32(const float* x, const float* w, const float* bias, float* y, int M, int N, int K, int ldx, int act,
-                           cudaStream_t stream) {
+                           int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return PTB_OK;
-  if (K <= 0 || ldx < K || !activation_known(act)) return PTB_ERR_SIZE;
+  if (K <= 0 || ldx < K || !activation_known(act) || error_flag == nullptr) return PTB_ERR_SIZE;
   if ((long(M) + 63) / 64 > 65535) return PTB_ERR_SIZE;
+  // The tensor cores (linear_f32_tc.cu) take matrices whose rows are whole 16-byte words, of half a tile's outputs and two stages of k at
+  // least: by the matrix alone, so that a row's bits do not follow the batch. us, FMAs against tensor cores, of 64 x 128: 9 and 11 for one row,
+  // 14 and 17 for 700; 64 x 1,024: 16 and 12, 33 and 23; 256 x 256: 10 and 12, 18 and 23; 512 x 512: 16 and 13, 29 and 27.
+  if (K % 4 == 0 && aligned16(w) && ((N >= 64 && K >= 1024) || (N >= 512 && K >= 256)))
+    return linear_f32_tensor(x, w, bias, y, M, N, K, ldx, act, error_flag, stream);
   // stretches of K, by N and K alone (the order of a row's sums must not follow the number of rows). A matrix of 1,024 outputs
   // and 700 rows has 176 tiles, little more than an SM each, which stretches even out; with one row it has 16. us for one,
   // two and four stretches: 1 row, N 1,024 K 4,096: 73, 39, 21; 4,096 x 2,048: 38, 22, 17; 18,176 x 4,544: 120, 119, 120. 700

@@ -212,7 +212,8 @@ def fill_normal(out: torch.Tensor, key: int, std: float, offset: float = 0.0, fi
 
 
 def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none"):
-    """act(x @ w.T + bias) in true float32 on the CUDA cores (the rows of x may lie wider apart)."""
+    """act(x @ w.T + bias) to float32 (the rows of x may lie wider apart): on the tensor cores with operands of three bfloat16 terms
+    and sums in float32 registers, small and oddly laid out matrices in FMAs; which one follows from w alone."""
     _need_cuda(w, bias)
     _check_rows(x, x.shape, torch.float32, "linear_f32: x")
     if x.dtype != torch.float32 or w.dtype != torch.float32:
@@ -223,8 +224,7 @@ def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
         raise KernelError(f"linear_f32: x is [{m}, {k}] but w is {list(w.shape)}")
     y = torch.empty((m, n), dtype=torch.float32, device=x.device)
     _check(lib().ptb_linear_f32(_ptr(x), _ptr(w), _ptr(bias), _ptr(y), m, n, k, x.stride(0) if m > 1 else k, ACTIVATIONS[act],
-                               _stream(x)),
-           "linear_f32")
+                                _ptr(error_flag(x.device)), _stream(x)), "linear_f32")
     return y
 
 

@@ -1,7 +1,7 @@
 """The linear layer that mixers and feed-forwards share: y = act(x @ W.T + b) [+ add].
 
-float32 models run the library's own true-float32 kernel (CUDA-core FMAs, bias and activation
-in its epilogue). bfloat16 models with a few rows (decode steps) run the hand-written
+float32 models run the library's own float32 kernel (operands in three bfloat16 terms on the tensor cores with
+float32 sums, small matrices in FMAs; bias and activation in its epilogue). bfloat16 models with a few rows (decode steps) run the hand-written
 weight-streaming kernel, which also takes the bias, the activation and a tensor to add (a
 residual) in its float32 epilogue. bfloat16 models with many rows (prompts) use the library
 matrix product that the reference's engine uses too (cuBLAS; ``FalconLinear``,

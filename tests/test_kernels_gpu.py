@@ -148,6 +148,45 @@ def test_linear_f32_tiles_and_stretches(K, m, n, k):
     assert torch.equal(K.linear_f32(wide[-1:, :k], w, b), K.linear_f32(wide[:, :k], w, b)[-1:])
 
 
+@pytest.mark.parametrize("n,k", [(64, 1024), (65, 1028), (512, 256), (1000, 1028), (129, 2052), (4096, 2048), (4300, 1024), (9000, 300), (96, 33000)])
+def test_linear_f32_on_tensor_cores(K, n, k):
+    """Matrices that the tensor-core form takes, around its tiles of 128 outputs and 16 to 128 rows, with K in one to four stretches and
+    an end inside a stage of 64; rows at odd words and apart; rows alone and in every size of tile the same bits. A product of
+    three-term operands is off by 2^-26 of itself at most, 32 of them are summed cut off (12 sums of 16, 2^-23 each), and k / 32
+    such sums are rounded additions."""
+    wide, w = rnd(300, k + 3, seed=1), rnd(n, k, seed=2, scale=0.1)
+    b = rnd(n, seed=3)
+    ref = wide[:, :k].double() @ w.double().T
+    size = wide[:, :k].double().abs() @ w.double().abs().T
+    for m in (1, 15, 16, 17, 33, 64, 65, 128, 129, 300):
+        for x in (wide[:m, :k], wide[:m, :k].contiguous()):
+            out = K.linear_f32(x, w)
+            assert ((out.double() - ref[:m]).abs() <= (k / 32 + 26) * 2.0 ** -24 * size[:m]).all()
+            full = out if m == 1 else full
+            assert torch.equal(out[:1], full[:1]) and torch.equal(K.linear_f32(x[-1:], w), out[-1:])
+    out = K.linear_f32(wide[:40, :k], w, b, "gelu")
+    torch.testing.assert_close(out.double().cpu(), plain.activation((ref[:40] + b.double()).cpu(), "gelu"), atol=1e-5, rtol=1e-5)
+
+
+def test_linear_f32_of_values_without_three_terms(K):
+    """Infinities, NaN, values that round to an infinity in bfloat16 and products beyond float32: what float32 multiply-adds give. Small
+    normal numbers keep their bits."""
+    x, w = rnd(20, 1024, seed=1), rnd(70, 1024, seed=2)
+    x[3, 7], x[5, 9], x[6, 1], x[7, 2] = math.inf, math.nan, 3.4e38, -3.4e38
+    w[11, 7], w[12, 1], w[13, 30] = 0.0, 0.5, -math.inf
+    # a product beyond float32 beside an infinity of the other sign has no number in float32 and one in 64 bits: zero times infinity instead
+    x[6:8, 30] = 0.0
+    x[8], w[20] = 1e30, 1e30
+    out, ref = K.linear_f32(x, w), x.double() @ w.double().T
+    inside = ref.abs() < 3.4028e38
+    assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out[~inside & ~ref.isnan()], ref[~inside & ~ref.isnan()].clamp(-math.inf, math.inf).sign() * math.inf)
+    size = x.double().abs() @ w.double().abs().T
+    assert ((out.double() - ref).abs()[inside] <= 80 * 2.0 ** -24 * size[inside]).all()
+    tiny = rnd(20, 1024, seed=4) * 1e-30
+    torch.testing.assert_close(K.linear_f32(tiny, w[:64].nan_to_num(0, 1, -1).clamp(-4, 4)).double() * 1e30,
+                               (tiny.double() @ w[:64].nan_to_num(0, 1, -1).clamp(-4, 4).double().T) * 1e30, atol=1e-5, rtol=1e-5)
+
+
 def test_to_float(K):
     x = rnd(3, 1000, dtype=torch.bfloat16)
     assert torch.equal(K.to_float(x), x.float())
