@@ -227,6 +227,7 @@ route_select_kernel(const float* __restrict__ zs_all, const float* __restrict__ 
 //   then row_of_pair [pairs] (-1 for an identity expert) and pair_of_row [pairs]
 // Pairs of one expert take consecutive rows; their order among themselves is not fixed, and no
 // result depends on it (every row is computed alone and summed per token in the order of the choice).
+constexpr int AHEAD = 8;
 __global__ void __launch_bounds__(1024)
 expert_plan_kernel(const int* __restrict__ ids, int* __restrict__ plan, int pairs, int n_experts, int tile_rows,
                    int max_tiles) {
@@ -241,10 +242,15 @@ expert_plan_kernel(const int* __restrict__ ids, int* __restrict__ plan, int pair
   int* pair_of_row = row_of_pair + pairs;
   for (int e = threadIdx.x; e < n_experts; e += blockDim.x) count[e] = 0;
   __syncthreads();
-  // one pass of atomics: a pair's place among its expert's pairs waits where its row will stand
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int e = ids[p];
-    row_of_pair[p] = e < n_experts ? atomicAdd(&count[e], 1) : -1;
+  // one pass of atomics: a pair's place among its expert's pairs waits where its row will stand. Bound by the way from memory, so the
+  // choices of eight pairs are asked for before the first is used, here and below (12,288 pairs 16 -> 13 us)
+  for (int p0 = threadIdx.x; p0 < pairs; p0 += AHEAD * blockDim.x) {
+    int e[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) e[u] = p0 + u * int(blockDim.x) < pairs ? ids[p0 + u * blockDim.x] : n_experts;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+      if (p0 + u * int(blockDim.x) < pairs) row_of_pair[p0 + u * blockDim.x] = e[u] < n_experts ? atomicAdd(&count[e[u]], 1) : -1;
   }
   __syncthreads();
   if (threadIdx.x < 32) {       // a warp sums rows and tiles over the experts, 32 at a time
@@ -271,12 +277,21 @@ expert_plan_kernel(const int* __restrict__ ids, int* __restrict__ plan, int pair
     if (lane == 0) plan[0] = tiles;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int e = ids[p];
-    if (e >= n_experts) continue;
-    const int row = offset[e] + row_of_pair[p];
-    pair_of_row[row] = p;
-    row_of_pair[p] = row;
+  for (int p0 = threadIdx.x; p0 < pairs; p0 += AHEAD * blockDim.x) {
+    int e[AHEAD], place[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int p = p0 + u * int(blockDim.x);
+      e[u] = p < pairs ? ids[p] : n_experts;
+      place[u] = p < pairs ? row_of_pair[p] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (e[u] >= n_experts) continue;
+      const int p = p0 + u * int(blockDim.x), row = offset[e[u]] + place[u];
+      pair_of_row[row] = p;
+      row_of_pair[p] = row;
+    }
   }
 }
 

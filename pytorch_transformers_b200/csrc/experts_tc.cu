@@ -12,19 +12,26 @@
 // rows of the same columns) are the M side of tcgen05.mma, the tile's x rows, rounded up to 16, are the N side, and a tile
 // holds all rows of an expert where it can: the matrix crosses once, whatever the number of rows, and nothing is
 // computed for padding beyond 15 rows. Accumulators [128 x rows] (two in mode 0) live in tensor memory.
-//   warp 0       one thread: per 64 values of k the boxes of 128 matrix rows by TMA (128-byte swizzle) into a ring of stages
-//   warp 1       one thread: per stage four (mode 0: eight) matrix instructions of 16 k, tcgen05.commit on the "empty" barrier
-//   warps 2 - 9  the x rows: cp.async of 16-byte chunks from rows found through the plan, to their swizzled places, each
-//                thread's arrival at the "full" barrier made by the copies themselves when they have landed. Then the
-//                epilogue: a warp reads its quarter of the lanes (a lane is a matrix row), every other group of eight x rows.
+// A block stays and walks every (blocks)-th tile, matrix columns first, so that the matrix boxes of its next tile are on their way while
+// this one's results leave. What it has in flight is two rings, since the boxes come from memory and the rows from L2:
+//   warp 0       one thread: per 64 values of k the boxes of 128 matrix rows by TMA (128-byte swizzle) into the ring of matrices
+//   warps 1, 2   one thread each, a box and its accumulator: per stage four matrix instructions of 16 k, tcgen05.commit on both rings' "empty"
+//                barriers. (A thread's two waits, two commits and four instructions take 625 clocks, two boxes' 805: a stage of
+//                few rows would wait for it.)
+//   then         the x rows: cp.async of 16-byte chunks from rows found through the plan, to their swizzled places, each
+//                thread's arrival at the "full" barrier made by the copies themselves when they have landed; the next tile's rows are
+//                looked up meanwhile
+//   then         results: a warp reads its quarter of the lanes (a lane is a matrix row), sixteen x rows at a time. Accumulators of two tiles take
+//                turns where tensor memory holds them (tiles of up to 128 rows); in tiles of 256 the matrix instructions wait for the gated
+//                units (17,500 clocks a tile of 192 rows with a true division; the fast one where the divisor lies in [1, 2]).
 // Every wait on a barrier is bounded: when one runs out, the error flag is raised and the block carries on to its end without
 // waiting again.
 //
-// One B200, 64 experts of 1,408, width 2,048: 12,288 rows (about 192 an expert, tiles of 256) gate and up 491 -> 204 us
-// (695 TFLOP/s), down 263 -> 114 us; 48 rows (tiles of 16) 88 -> 70 and 45 -> 35 us (5.7 TB/s of the matrices of the experts
-// in use); before, 64 x 128 tiles on mma.sync. With many rows nothing is saturated (tensor pipe 38 %, memory 52 %): the rings hold too
-// little of the way from memory (192 rows: three stages of 56 KB for gate and up; two of 40 KB in each of two blocks for down). Boxes asked into L2 eight stages ahead changed nothing there
-// and cost a third with few rows (67 -> 90 us).
+// One B200, 64 experts of 1,408, width 2,048, both products: 12,288 rows (about 192 an expert, tiles of 256) 334 -> 289 us (735 TFLOP/s),
+// 21,000 rows 500 -> 438, 4,200 rows 241 -> 220, 48 rows 136 -> 124 (4.9 TB/s of the matrices of the experts in use); before, a block a
+// tile and one ring of three stages. With many rows shared memory's bandwidth bounds it (a stage of 192 rows: 56 KB in, 80 KB
+// read by the matrix instructions, 1,090 of its clocks), then the results of a tile and a last round of few tiles. Boxes asked into L2 eight
+// stages ahead cost a third with few rows (67 -> 90 us).
 #include <cudaTypedefs.h>
 
 #include <mutex>
@@ -37,8 +44,14 @@ namespace {
 constexpr int XM = 128;                    // matrix rows of a box = M of the matrix instruction
 constexpr int XK = 64;                     // k per stage: 128 bytes, one swizzle row
 constexpr int X_BOX_BYTES = XM * XK * 2;   // 16 KB
-constexpr int X_MAX_STAGES = 6;
-constexpr int X_GATHER = 256;              // threads of warps 2 - 9
+constexpr int X_MAX_W = 7, X_MAX_X = 4;   // stages of the rings of matrix boxes and of x rows
+constexpr int MAX_BOXES = 2;               // boxes of a tile, each with an accumulator and a thread that issues for it
+// TWO: two blocks an SM, for tiles of few rows
+template <bool TWO>
+struct ExpertThreads {
+  static constexpr int GATHER = TWO ? 64 : 256, STORE = TWO ? 128 : 256, ALL = 32 * (1 + MAX_BOXES) + GATHER + STORE;
+  static constexpr int RING = (TWO ? 111 : 225) * 1024;
+};
 
 __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0));
@@ -49,6 +62,19 @@ __device__ __forceinline__ void arrive_when_copied(uint32_t bar) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// gated_unit (common.cuh) for results that are rounded to bfloat16. The sigmoid from e^-|g|, which does not overflow and leaves the
+// divisor in [1, 2], where the fast division is off by two units in the last place of 24 bits at most, whatever the gate. Zero where
+// e^-g leaves float32, as there.
+__device__ __forceinline__ float gated_unit_rounded(float gate, float up, float limit, float alpha) {
+  float a = 1.f;
+  if (limit > 0.f) {
+    gate = fminf(gate, limit), up = fminf(fmaxf(up, -limit), limit) + 1.f;
+    a = alpha;
+  }
+  const float x = a * gate, t = expf(-fabsf(x)), s = __fdividef(x < 0.f ? t : 1.f, 1.f + t);
+  return (x < -88.72283f ? 0.f * gate : gate * s) * up;
+}
+
 struct ExpertTcParams {
   const __nv_bfloat16* x;
   void* out;
@@ -56,47 +82,52 @@ struct ExpertTcParams {
   const float* row_scale;
   int* error_flag;
   int pairs, max_tiles, top, N, K, act;
-  int tile_rows;            // most rows of a tile
-  int ring_bytes, acc2;     // shared memory for stages; tensor-memory column of the second accumulator
-  int tmem_cols;
+  int w_stages, x_stages, x_stage_bytes;      // the two rings
+  int acc2, sets;           // tensor-memory columns from one accumulator to the next; tiles whose accumulators fit side by side
   float glu_limit, glu_alpha;
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(64 + X_GATHER)
+template <int MODE, bool TWO>
+__global__ void __launch_bounds__(ExpertThreads<TWO>::ALL, TWO ? 2 : 1)
 expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertTcParams p) {
   pdl_entry();
-  const int tile = blockIdx.y;
-  if (tile >= p.plan[0]) return;
-  constexpr int BOXES = MODE == 0 ? 2 : 1;
-  const int expert = p.plan[1 + tile], row0 = p.plan[1 + p.max_tiles + tile], rows = p.plan[1 + 2 * p.max_tiles + tile];
-  const int* pair_of_row = p.plan + 1 + 3 * p.max_tiles + p.pairs;
-  const int n16 = (rows + 15) / 16 * 16;
+  constexpr int X_GATHER = ExpertThreads<TWO>::GATHER, X_STORE = ExpertThreads<TWO>::STORE;
+  constexpr int TMEM_COLS = TWO ? 256 : 512;
+  constexpr int BOXES = MODE != 0 && TWO ? 1 : 2;
+  constexpr int COLS = MODE == 0 ? XM : BOXES * XM;      // output columns of a tile
+  const int m_tiles = (p.N + COLS - 1) / COLS, total = p.plan[0] * m_tiles;
+  if (int(blockIdx.x) >= total) return;
+  const int *tile_expert = p.plan + 1, *tile_row0 = tile_expert + p.max_tiles, *tile_n = tile_row0 + p.max_tiles;
+  const int* pair_of_row = tile_n + p.max_tiles + p.pairs;
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte alignment: the swizzle pattern is a function of address bits 4..9
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  // the ring is cut by this tile's rows: fewer rows, more stages in flight
-  const int stage_bytes = BOXES * X_BOX_BYTES + n16 * XK * 2;   // a multiple of 1024
-  const int stages = min(X_MAX_STAGES, p.ring_bytes / stage_bytes);
-  __shared__ uint64_t bars[2 * X_MAX_STAGES + 1];   // full[stages], empty[stages], accumulators complete
+  constexpr int W_BYTES = BOXES * X_BOX_BYTES;
+  __shared__ uint64_t bars[2 * X_MAX_W + 2 * X_MAX_X + 4];   // full and empty of both rings; accumulators complete, accumulators read
   __shared__ uint32_t tmem_slot;
-  __shared__ int alive_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * XM;
-  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[X_MAX_STAGES]), bar_done = smem_u32(&bars[2 * X_MAX_STAGES]);
-  const uint32_t ring0 = smem_u32(ring);
+  const uint32_t wfull0 = smem_u32(&bars[0]), wempty0 = smem_u32(&bars[X_MAX_W]);
+  const uint32_t xfull0 = smem_u32(&bars[2 * X_MAX_W]), xempty0 = smem_u32(&bars[2 * X_MAX_W + X_MAX_X]);
+  const uint32_t done0 = smem_u32(&bars[2 * X_MAX_W + 2 * X_MAX_X]), read0 = done0 + 16;
+  const uint32_t wring = smem_u32(ring), xring = wring + p.w_stages * W_BYTES;
   const int n_iter = (p.K + XK - 1) / XK;
   if (tid == 0) {
-    for (int s = 0; s < stages; ++s) {
-      mbar_init(full0 + 8 * s, 1 + X_GATHER);     // the TMA thread's arrival and each gathering thread's
-      mbar_init(empty0 + 8 * s, 1);
+    for (int s = 0; s < p.w_stages; ++s) {
+      mbar_init(wfull0 + 8 * s, 1);
+      mbar_init(wempty0 + 8 * s, BOXES);
     }
-    mbar_init(bar_done, 1);
-    alive_s = 1;
+    for (int s = 0; s < p.x_stages; ++s) {
+      mbar_init(xfull0 + 8 * s, X_GATHER);
+      mbar_init(xempty0 + 8 * s, BOXES);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(done0 + 8 * s, BOXES);
+      mbar_init(read0 + 8 * s, X_STORE / 32);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)), "r"(p.tmem_cols));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)), "n"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   tc_fence_before();
@@ -106,114 +137,164 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
 
   if (warp == 0) {
     if (lane == 0) {
-      const int wrow = expert * BOXES * p.N + m0;      // rows past an expert's own come along and are not stored
       uint32_t st = 0, parity = 1;                     // parity of the round before
-      int i = 0;
-      for (; i < n_iter; ++i) {
-        const uint32_t full = full0 + 8 * st, base = ring0 + st * stage_bytes;
-        if (i >= stages && !mbar_wait(empty0 + 8 * st, parity, p.error_flag, 31)) break;
-        mbar_expect_tx(full, uint32_t(BOXES * X_BOX_BYTES));   // a box delivers all its bytes, zeros where out of range
-        tma_load_2d(base, &w_map, i * XK, wrow, full);
-        if (MODE == 0) tma_load_2d(base + X_BOX_BYTES, &w_map, i * XK, wrow + p.N, full);
-        if (++st == uint32_t(stages)) { st = 0; parity ^= 1; }
-      }
-      // the copies in flight land before the block ends, also where a wait ran out (bounded waits again)
-      for (int j = max(0, i - stages); j < i; ++j) mbar_wait(full0 + 8 * (j % stages), (j / stages) & 1, p.error_flag, 31);
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16(XM, n16, false);
-      const uint64_t desc0 = smem_desc(ring0, 16, 1024);
-      const uint64_t step = uint64_t(stage_bytes >> 4), x_off = uint64_t((BOXES * X_BOX_BYTES) >> 4), up_off = uint64_t(X_BOX_BYTES >> 4);
-      uint32_t st = 0, parity = 0;
+      int filled = 0;
       bool alive = true;
-      for (int i = 0; i < n_iter; ++i) {
-        alive = mbar_wait(full0 + 8 * st, parity, p.error_flag, 32);
-        if (!alive) break;
-        proxy_fence_async();      // the x rows came by ordinary copies; the matrix instructions read them through the other proxy
-        tc_fence_after();
-        const uint64_t d = desc0 + st * step;
-        tc_mma4(tmem_base, d, d + x_off, idesc, i > 0 ? 1u : 0u);
-        if (MODE == 0) tc_mma4(tmem_base + p.acc2, d + up_off, d + x_off, idesc, i > 0 ? 1u : 0u);
-        tc_commit(empty0 + 8 * st);
-        if (++st == uint32_t(stages)) { st = 0; parity ^= 1; }
-      }
-      if (alive) {
-        tc_commit(bar_done);
-        alive = mbar_wait(bar_done, 0, p.error_flag, 33);
-      }
-      if (!alive) alive_s = 0;
-    }
-    __syncwarp();
-  } else {
-    const int gt = tid - 64, c = gt % 8;      // chunk c (8 values) of rows gt / 8 + 32 j
-    const __nv_bfloat16* src[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = gt / 8 + 32 * j;
-      src[j] = nullptr;
-      if (r < rows) src[j] = p.x + size_t(MODE == 1 ? row0 + r : pair_of_row[row0 + r] / p.top) * p.K + c * 8;
-    }
-    const uint32_t dst0 = ring0 + BOXES * X_BOX_BYTES + (gt / 8) * 128 + ((c ^ ((gt / 8) & 7)) << 4);
-    uint32_t st = 0, parity = 1;
-    for (int i = 0; i < n_iter; ++i) {
-      if (i >= stages && !mbar_wait(empty0 + 8 * st, parity, p.error_flag, 34)) break;
-      const bool k_ok = i * XK + c * 8 < p.K;
-      const uint32_t dst = dst0 + st * stage_bytes;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (gt / 8 + 32 * j < n16)
-          copy16_or_zero(dst + j * 4096, src[j] && k_ok ? src[j] + i * XK : p.x, src[j] && k_ok);
-      arrive_when_copied(full0 + 8 * st);
-      if (++st == uint32_t(stages)) { st = 0; parity ^= 1; }
-    }
-    cp_async_wait_all();
-  }
-  __syncthreads();
-  tc_fence_after();
-
-  // -------------------------------------------------------------------- epilogue
-  if (warp >= 2 && alive_s) {
-    const int quarter = warp & 3, half = (warp - 2) >> 2;
-    const int f = m0 + quarter * 32 + lane;      // output column = lane of tensor memory
-    const uint32_t lane_addr = tmem_base + (uint32_t(quarter * 32) << 16);
-    for (int g = half; g * 8 < n16; g += 2) {
-      float v[8];
-      tmem_ld8(lane_addr + g * 8, v);
-      if (MODE == 1) {
-        float* o = reinterpret_cast<float*>(p.out) + size_t(row0 + g * 8) * p.N + f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (g * 8 + j < rows && f < p.N) o[size_t(j) * p.N] = v[j];
-        continue;
-      }
-      if (MODE == 0) {
-        float u[8];
-        tmem_ld8(lane_addr + p.acc2 + g * 8, u);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = gated_unit(v[j], u[j], p.glu_limit, p.glu_alpha);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = g * 8 + j;
-          const float rs = (p.row_scale && r < rows) ? p.row_scale[pair_of_row[row0 + r]] : 1.f;
-          v[j] = apply_activation(v[j] * rs, p.act);
+      int expert = tile_expert[blockIdx.x / m_tiles];
+      for (int t = blockIdx.x; t < total && alive; t += gridDim.x) {
+        const int m0 = t % m_tiles * COLS, wrow = expert * (MODE == 0 ? 2 : 1) * p.N + m0;      // rows past an expert's own come along and are not stored
+        if (t + int(gridDim.x) < total) expert = tile_expert[(t + gridDim.x) / m_tiles];
+        for (int i = 0; i < n_iter; ++i, ++filled) {
+          const uint32_t full = wfull0 + 8 * st, base = wring + st * W_BYTES;
+          if (filled >= p.w_stages && !mbar_wait(wempty0 + 8 * st, parity, p.error_flag, 31)) {
+            alive = false;
+            break;
+          }
+          mbar_expect_tx(full, uint32_t(W_BYTES));     // a box delivers all its bytes, zeros where out of range
+          tma_load_2d(base, &w_map, i * XK, wrow, full);
+          if (BOXES == 2) tma_load_2d(base + X_BOX_BYTES, &w_map, i * XK, wrow + (MODE == 0 ? p.N : XM), full);
+          if (++st == uint32_t(p.w_stages)) { st = 0; parity ^= 1; }
         }
       }
-      // two rows at a time: an even lane stores columns f, f + 1 of the first, the odd lane above it those of the second
-      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(row0 + g * 8 + (lane & 1)) * p.N + (f & ~1);
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        const float other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[j] : v[j + 1], 1);
-        const uint32_t word = (lane & 1) ? pack_bf16(other, v[j + 1]) : pack_bf16(v[j], other);
-        if (g * 8 + j + (lane & 1) < rows && f < p.N) *reinterpret_cast<uint32_t*>(o + size_t(j) * p.N) = word;
+      // the copies in flight land before the block ends, also where a wait ran out (bounded waits again)
+      for (int j = max(0, filled - p.w_stages); j < filled; ++j)
+        mbar_wait(wfull0 + 8 * (j % p.w_stages), (j / p.w_stages) & 1, p.error_flag, 31);
+    }
+  } else if (warp < 1 + MAX_BOXES) {
+    if (lane == 0 && warp < 1 + BOXES) {
+      const uint32_t box = warp - 1;
+      const uint64_t wdesc0 = smem_desc(wring + box * X_BOX_BYTES, 16, 1024), xdesc0 = smem_desc(xring, 16, 1024);
+      uint32_t ws = 0, wpar = 0, xs = 0, xpar = 0, n = 0;      // n: tiles so far
+      bool alive = true;
+      int rows = tile_n[blockIdx.x / m_tiles];
+      for (int t = blockIdx.x; t < total && alive; t += gridDim.x, ++n) {
+        const uint32_t set = p.sets == 2 ? n & 1 : 0, round = p.sets == 2 ? n >> 1 : n;
+        const uint32_t idesc = idesc_bf16(XM, (rows + 15) / 16 * 16, false), acc = tmem_base + (set * BOXES + box) * p.acc2;
+        if (t + int(gridDim.x) < total) rows = tile_n[(t + gridDim.x) / m_tiles];
+        if (round > 0) alive = mbar_wait(read0 + 8 * set, (round - 1) & 1, p.error_flag, 35);
+        tc_fence_after();
+        for (int i = 0; i < n_iter && alive; ++i) {
+          alive = mbar_wait(xfull0 + 8 * xs, xpar, p.error_flag, 32) && mbar_wait(wfull0 + 8 * ws, wpar, p.error_flag, 32);
+          if (!alive) break;
+          proxy_fence_async();      // the x rows came by ordinary copies; the matrix instructions read them through the other proxy
+          tc_fence_after();
+          const uint64_t dw = wdesc0 + uint64_t(ws * (W_BYTES >> 4)), dx = xdesc0 + uint64_t(xs * (uint32_t(p.x_stage_bytes) >> 4));
+          tc_mma4(acc, dw, dx, idesc, i > 0 ? 1u : 0u);
+          tc_commit(xempty0 + 8 * xs);
+          tc_commit(wempty0 + 8 * ws);
+          if (++ws == uint32_t(p.w_stages)) { ws = 0; wpar ^= 1; }
+          if (++xs == uint32_t(p.x_stages)) { xs = 0; xpar ^= 1; }
+        }
+        if (alive) tc_commit(done0 + 8 * set);
       }
+    }
+    __syncwarp();
+  } else if (warp < 1 + MAX_BOXES + X_GATHER / 32) {
+    const int gt = tid - 32 * (1 + MAX_BOXES), c = gt % 8;      // chunk c (8 values) of rows gt / 8 + X_GATHER / 8 j
+    // a tile's rows; those of the block's next tile are looked up while this one's are copied
+    int row[8], next[8], rows = 0, next_rows = 0;
+    auto look_up = [&](int t, int (&to)[8]) {
+      const int tile = t / m_tiles, row0 = tile_row0[tile], n = tile_n[tile];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = gt / 8 + X_GATHER / 8 * j;
+        to[j] = r < n ? (MODE == 1 ? row0 + r : pair_of_row[row0 + r]) : -1;
+      }
+      return n;
+    };
+    rows = look_up(blockIdx.x, row);
+    const uint32_t dst0 = xring + (gt / 8) * 128 + ((c ^ ((gt / 8) & 7)) << 4);
+    uint32_t st = 0, parity = 1;
+    int filled = 0;
+    bool alive = true;
+    for (int t = blockIdx.x; t < total && alive; t += gridDim.x) {
+      const bool more = t + int(gridDim.x) < total;
+      if (more) next_rows = look_up(t + gridDim.x, next);
+      const int n16 = (rows + 15) / 16 * 16;
+      const __nv_bfloat16* src[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) src[j] = row[j] >= 0 ? p.x + size_t(MODE == 1 ? row[j] : row[j] / p.top) * p.K + c * 8 : nullptr;
+      for (int i = 0; i < n_iter; ++i, ++filled) {
+        if (filled >= p.x_stages && !mbar_wait(xempty0 + 8 * st, parity, p.error_flag, 34)) {
+          alive = false;
+          break;
+        }
+        const bool k_ok = i * XK + c * 8 < p.K;
+        const uint32_t dst = dst0 + st * p.x_stage_bytes;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (gt / 8 + X_GATHER / 8 * j < n16)
+            copy16_or_zero(dst + j * (X_GATHER * 16), src[j] && k_ok ? src[j] + i * XK : p.x, src[j] && k_ok);
+        arrive_when_copied(xfull0 + 8 * st);
+        if (++st == uint32_t(p.x_stages)) { st = 0; parity ^= 1; }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) row[j] = next[j];
+      rows = next_rows;
+    }
+    cp_async_wait_all();
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    const int quarter = warp & 3, half = (warp - 1 - MAX_BOXES - X_GATHER / 32) >> 2;
+    const uint32_t lane_addr = tmem_base + (uint32_t(quarter * 32) << 16);
+    uint32_t n = 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, ++n) {
+      const uint32_t set = p.sets == 2 ? n & 1 : 0, round = p.sets == 2 ? n >> 1 : n;
+      const int tile = t / m_tiles, row0 = tile_row0[tile], rows = tile_n[tile];
+      const int f0 = t % m_tiles * COLS + quarter * 32 + lane;      // output column = lane of tensor memory
+      if (!mbar_wait(done0 + 8 * set, round & 1, p.error_flag, 33)) break;
+      tc_fence_after();
+      const uint32_t acc = lane_addr + set * BOXES * p.acc2;
+      for (int g = 2 * half; g * 8 < rows; g += X_STORE / 64) {      // sixteen rows at a time
+        uint32_t r[BOXES][16];
+#pragma unroll
+        for (int b = 0; b < BOXES; ++b) tmem_ld16_nowait(acc + b * p.acc2 + g * 8, r[b]);
+        tmem_ld_wait();
+        if constexpr (MODE == 1) {
+#pragma unroll
+          for (int b = 0; b < BOXES; ++b) {
+            const int f = f0 + b * XM;
+            float* o = reinterpret_cast<float*>(p.out) + size_t(row0 + g * 8) * p.N + f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (g * 8 + j < rows && f < p.N) o[size_t(j) * p.N] = __uint_as_float(r[b][j]);
+          }
+        } else {
+#pragma unroll
+          for (int b = 0; b < (MODE == 0 ? 1 : BOXES); ++b) {
+            const int f = f0 + b * XM;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              v[j] = __uint_as_float(r[b][j]);
+              if (MODE == 0) {
+                v[j] = gated_unit_rounded(v[j], __uint_as_float(r[BOXES - 1][j]), p.glu_limit, p.glu_alpha);
+              } else {
+                const int at = g * 8 + j;
+                const float rs = (p.row_scale && at < rows) ? p.row_scale[pair_of_row[row0 + at]] : 1.f;
+                v[j] = apply_activation(v[j] * rs, p.act);
+              }
+            }
+            // two rows at a time: an even lane stores columns f, f + 1 of the first, the odd lane above it those of the second
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(row0 + g * 8 + (lane & 1)) * p.N + (f & ~1);
+#pragma unroll
+            for (int j = 0; j < 16; j += 2) {
+              const float other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[j] : v[j + 1], 1);
+              const uint32_t word = (lane & 1) ? pack_bf16(other, v[j + 1]) : pack_bf16(v[j], other);
+              if (g * 8 + j + (lane & 1) < rows && f < p.N) *reinterpret_cast<uint32_t*>(o + size_t(j) * p.N) = word;
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(read0 + 8 * set);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(p.tmem_cols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "n"(TMEM_COLS));
 }
 
 // a [rows, K] bfloat16 row-major matrix in boxes of 128 rows x 64 k, written with the 128-byte swizzle
@@ -237,20 +318,30 @@ bool make_expert_map(CUtensorMap* map, const void* base, long long rows, int K) 
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int MODE>
-int launch_expert_tc(const CUtensorMap& map, ExpertTcParams p, cudaStream_t stream) {
-  constexpr int BOXES = MODE == 0 ? 2 : 1;
-  p.acc2 = p.tile_rows < 32 ? 32 : p.tile_rows;
-  p.tmem_cols = BOXES * p.acc2;
-  const int most = BOXES * X_BOX_BYTES + p.tile_rows * XK * 2;     // a stage of the largest tile
-  // two blocks an SM where tensor memory holds both and two stages fit into half of its shared memory (one's start and
-  // epilogue under the other's products: down, tiles of 256, 142 -> 114 us), else one block with what the SM has
-  p.ring_bytes = (p.tmem_cols <= 256 && 2 * most <= 110 * 1024) ? 110 * 1024 : 222 * 1024;
-  const size_t smem = 1024 + size_t(p.ring_bytes);
+template <int MODE, bool TWO>
+int launch_expert_tc(const CUtensorMap& map, ExpertTcParams p, int tile_rows, cudaStream_t stream) {
+  constexpr int RING = ExpertThreads<TWO>::RING, BOXES = MODE != 0 && TWO ? 1 : 2, COLS = MODE == 0 ? XM : BOXES * XM;
+  p.acc2 = tile_rows < 32 ? 32 : tile_rows;
+  p.sets = 2 * BOXES * p.acc2 <= (TWO ? 256 : 512) ? 2 : 1;
+  p.x_stage_bytes = tile_rows * XK * 2;
+  p.x_stages = tile_rows >= 128 ? 3 : TWO && tile_rows == 32 ? 3 : X_MAX_X;
+  p.w_stages = min(X_MAX_W, (RING - p.x_stages * p.x_stage_bytes) / (BOXES * X_BOX_BYTES));
+  const size_t smem = 1024 + size_t(RING);
   static SharedLimit limit;
-  if (!limit.allows(expert_linear_tc_kernel<MODE>, smem)) return PTB_ERR_LAUNCH;
-  launch_pdl(expert_linear_tc_kernel<MODE>, dim3((p.N + XM - 1) / XM, p.max_tiles), 64 + X_GATHER, smem, stream, map, p);
+  if (!limit.allows(expert_linear_tc_kernel<MODE, TWO>, smem)) return PTB_ERR_LAUNCH;
+  const long long most = (long long)p.max_tiles * ((p.N + COLS - 1) / COLS), slots = (long long)sm_count() * (TWO ? 2 : 1);
+  launch_pdl(expert_linear_tc_kernel<MODE, TWO>, int(most < slots ? most : slots), ExpertThreads<TWO>::ALL, smem, stream, map, p);
   return launch_status();
+}
+
+template <int MODE>
+int launch_expert_tc(const CUtensorMap& map, const ExpertTcParams& p, int tile_rows, cudaStream_t stream) {
+  // Two blocks an SM, each with half of its shared memory, for tiles of up to 32 rows, and of 64 where all tiles are resident then: what
+  // counts there is the matrices' stream, which a last round of few tiles on a block an SM each leaves slack in (16 experts of 1,408, 40
+  // tokens of 6 choices: 68 us with one block an SM, 58 with two; 64 experts, 300 tokens, tiles of 64: 187 with one)
+  const long long most = (long long)p.max_tiles * ((p.N + XM - 1) / XM);
+  const bool two = tile_rows <= 32 || (tile_rows == 64 && most <= 2 * sm_count());
+  return two ? launch_expert_tc<MODE, true>(map, p, tile_rows, stream) : launch_expert_tc<MODE, false>(map, p, tile_rows, stream);
 }
 
 }  // namespace
@@ -270,8 +361,8 @@ PTB_API int ptb_expert_linear_tc(int mode, const void* x, const void* w, void* o
   if (!make_expert_map(&map, w, (long long)n_experts * (mode == 0 ? 2 : 1) * N, K)) return PTB_ERR_LAUNCH;
   ExpertTcParams p = {};
   p.x = (const __nv_bfloat16*)x; p.out = out; p.plan = plan; p.row_scale = row_scale; p.error_flag = error_flag;
-  p.pairs = pairs; p.max_tiles = max_tiles; p.top = top; p.N = N; p.K = K; p.act = act; p.tile_rows = tile_rows;
+  p.pairs = pairs; p.max_tiles = max_tiles; p.top = top; p.N = N; p.K = K; p.act = act;
   p.glu_limit = glu_limit; p.glu_alpha = glu_alpha;
-  return mode == 0 ? launch_expert_tc<0>(map, p, stream) : mode == 1 ? launch_expert_tc<1>(map, p, stream)
-                                                                     : launch_expert_tc<2>(map, p, stream);
+  return mode == 0 ? launch_expert_tc<0>(map, p, tile_rows, stream) : mode == 1 ? launch_expert_tc<1>(map, p, tile_rows, stream)
+                                                                                : launch_expert_tc<2>(map, p, tile_rows, stream);
 }

@@ -397,6 +397,29 @@ def test_expert_tiles(K, kind, width, inner, tile_rows):
     K.check_device_errors("cuda:0")
 
 
+@pytest.mark.parametrize("kind", ["gated", "plain"])
+@pytest.mark.parametrize("tile_rows", [16, 32, 64, 128, 256])
+def test_expert_tiles_beyond_the_blocks(K, kind, tile_rows):
+    """More tiles than blocks stay on the device, so that a block walks several: its rings carry on from tile to tile at any
+    stage (9 and 21 stages of k, each with a remainder), and tiles of different rows take turns in tensor memory. The bound
+    is that of test_expert_tiles."""
+    width, inner, n_experts = 520, 1304, 40
+    counts = [(1, 16, 17, 64, 65, 130, 0, 200)[e % 8] for e in range(n_experts)]
+    h = rnd(sum(counts), width, dtype=torch.bfloat16, seed=1)
+    ids = torch.repeat_interleave(torch.arange(n_experts), torch.tensor(counts))[torch.randperm(sum(counts), generator=torch.Generator().manual_seed(5))]
+    up = rnd(n_experts, inner if kind == "plain" else 2 * inner, width, dtype=torch.bfloat16, scale=width ** -0.5, seed=2)
+    down = rnd(n_experts, width, inner, dtype=torch.bfloat16, scale=inner ** -0.5, seed=3)
+    y, rows = K.expert_rows(h, ids.int().reshape(-1, 1).cuda(), up, down, mma_tile_rows=tile_rows, plain_act="relu" if kind == "plain" else None)
+    got = y[rows.long()]
+    for e in range(n_experts):
+        at = (ids == e).nonzero()[:, 0].cuda()
+        z = h[at].double() @ up[e].double().T
+        a = (z.relu() if kind == "plain" else z[:, :inner] * torch.sigmoid(z[:, :inner]) * z[:, inner:]).bfloat16().double()
+        bound = (2.0 ** -8 * a.abs() + 1e-5) @ down[e].double().abs().T + 1e-5
+        assert ((got[at].double() - a @ down[e].double().T).abs() <= bound).all(), (kind, e)
+    K.check_device_errors("cuda:0")
+
+
 @pytest.mark.parametrize("m", [1, 8, 9, 32])
 @pytest.mark.parametrize("n,n_bf16,k", [(40, 8, 64), (8224, 8192, 2048), (50, 49, 4096), (10000, 9000, 256)])
 def test_skinny_linear_split(K, m, n, n_bf16, k):
