@@ -133,6 +133,13 @@ __global__ void rglru_conv_run_kernel(const T* __restrict__ proj, const float* _
   }
 }
 
+// 1 / (1 + e^-x) from e^-|x|: the divisor lies in [1, 2], where the fast division is off by two units of 2^-24 at most. The gates of a
+// token and channel are formed by this one expression wherever they are formed.
+__device__ __forceinline__ float sigmoid_of(float x) {
+  const float t = expf(-fabsf(x));
+  return __fdividef(x < 0.f ? t : 1.f, 1.f + t);
+}
+
 // a S + drive with a = exp(log_a), formed as S + ((a - 1) S + drive) with a - 1 = expm1(log_a): a decay close
 // to 1 rounded to float32 is off by up to 3e-8 of itself, which a channel whose decay hardly changes would
 // carry into every step alike (1,000 steps: 3e-5 of the state); a - 1 keeps its digits, and what is left is
@@ -263,8 +270,8 @@ __global__ void rglru_chunk_kernel(float* __restrict__ gates, const float* __res
         float a1 = r[i], drive = in[i];
         if (!RAW || PASS == 1) {
           if (RAW) {
-            r[i] = 1.f / (1.f + expf(-(r[i] + b_r)));
-            in[i] = 1.f / (1.f + expf(-(in[i] + b_i)));
+            r[i] = sigmoid_of(r[i] + b_r);
+            in[i] = sigmoid_of(in[i] + b_i);
           }
           // a - 1, and 1 - a^2 = -(a - 1)(a + 1) from it, in which nothing cancels: one expm1f a token
           const float log_a = -c_decay * r[i] * sp;
@@ -369,7 +376,7 @@ block_linear_kernel(const T* __restrict__ x, long long xt, long long xg, const T
       if (gn >= N) continue;
       float v = acc[i][j];
       if (bias) v += bias[size_t(g) * N + gn];
-      if (act == 1) v = 1.f / (1.f + expf(-v));
+      if (act == 1) v = sigmoid_of(v);
       if (gate) v *= 1.f / (1.f + expf(-to_f(gate[size_t(gm) * gate_t + size_t(g) * gate_g + size_t(gn) * gate_n])));
       y[(size_t(gm) * G + g) * N + gn] = from_f<TO>(v);
     }
@@ -457,7 +464,7 @@ block_linear_skinny_kernel(const T* __restrict__ x, long long xt, long long xg, 
       const int n = n0 + r;
       if (lane == m % LANES && m < M && mine && n < N) {      // every lane holds the sum: the rows' epilogues are shared out
         if (bias) v += bias[size_t(g) * N + n];
-        if (act == 1) v = 1.f / (1.f + expf(-v));
+        if (act == 1) v = sigmoid_of(v);
         if (gate) v *= 1.f / (1.f + expf(-to_f(gate[size_t(m) * gate_t + size_t(g) * gate_g + size_t(n) * gate_n])));
         y[(size_t(m) * G + g) * N + n] = from_f<TO>(v);
       }
@@ -503,7 +510,7 @@ block_linear_mma_kernel(const __nv_bfloat16* __restrict__ x, long long xt, long 
     if (m >= M || col >= N) continue;
     float v = acc[i];
     if (bias) v += bias[size_t(g) * N + col];
-    if (act == 1) v = 1.f / (1.f + expf(-v));
+    if (act == 1) v = sigmoid_of(v);
     if (gate) v *= 1.f / (1.f + expf(-to_f(gate[size_t(m) * gate_t + size_t(g) * gate_g + size_t(col) * gate_n])));
     y[(size_t(m) * G + g) * N + col] = from_f<TO>(v);
   }
@@ -536,7 +543,7 @@ __global__ void block_epilogue_kernel(const TI* __restrict__ z, const float* __r
     const int n = int(i % N), g = int((i / N) % G), m = int(i / (size_t(N) * G));
     float v = to_f(z[(size_t(g) * M + m) * N + n]);
     if (bias) v += bias[size_t(g) * N + n];
-    if (act == 1) v = 1.f / (1.f + expf(-v));
+    if (act == 1) v = sigmoid_of(v);
     if (gate) v *= 1.f / (1.f + expf(-to_f(gate[size_t(m) * gate_t + size_t(g) * gate_g + size_t(n) * gate_n])));
     y[i] = from_f<TO>(v);
   }
@@ -555,7 +562,7 @@ __global__ void block_epilogue_quad_kernel(const TI* __restrict__ z, const float
   float4 v = Quad<TI>::wide(load_raw(z + (size_t(g) * M + m) * N + n));
   if (bias) v = add4(v, *reinterpret_cast<const float4*>(bias + size_t(g) * N + n));
   if (act == 1)
-    v = make_float4(1.f / (1.f + expf(-v.x)), 1.f / (1.f + expf(-v.y)), 1.f / (1.f + expf(-v.z)), 1.f / (1.f + expf(-v.w)));
+    v = make_float4(sigmoid_of(v.x), sigmoid_of(v.y), sigmoid_of(v.z), sigmoid_of(v.w));
   store_quad(y + (size_t(m) * G + g) * N + n, v);
 }
 
