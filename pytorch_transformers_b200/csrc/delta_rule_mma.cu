@@ -735,7 +735,7 @@ delta_chunk_join_kernel(const uint4* __restrict__ mq, const float4* __restrict__
     }
     // one barrier a chunk: the buffer written next was last read before this barrier
     __syncthreads();
-    float acc[NTILE][4];
+    float acc[NTILE][4], low[NTILE][4] = {};      // the products with a second term apart: half as long a chain of matrix instructions
 #pragma unroll
     for (int nt = 0; nt < NTILE; ++nt) {
       acc[nt][0] = init[nt].x; acc[nt][1] = init[nt].y; acc[nt][2] = init[nt].z; acc[nt][3] = init[nt].w;
@@ -768,12 +768,16 @@ delta_chunk_join_kernel(const uint4* __restrict__ mq, const float4* __restrict__
         ldmatrix_x4_trans(bl[0], bl[1], bl[2], bl[3], lb + row + j * 16);
         mma_bf16(acc[j], ah, b[0], b[1]);
         mma_bf16(acc[j + 1], ah, b[2], b[3]);
-        mma_bf16(acc[j], ah, bl[0], bl[1]);
-        mma_bf16(acc[j + 1], ah, bl[2], bl[3]);
-        mma_bf16(acc[j], al, b[0], b[1]);
-        mma_bf16(acc[j + 1], al, b[2], b[3]);
+        mma_bf16(low[j], ah, bl[0], bl[1]);
+        mma_bf16(low[j + 1], ah, bl[2], bl[3]);
+        mma_bf16(low[j], al, b[0], b[1]);
+        mma_bf16(low[j + 1], al, b[2], b[3]);
       }
     }
+#pragma unroll
+    for (int nt = 0; nt < NTILE; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[nt][e] += low[nt][e];
     if (is_state) {
 #pragma unroll
       for (int nt = 0; nt < NTILE; ++nt)
