@@ -2,7 +2,9 @@
 // memory, for head sizes 64 and 128 (and keys of 192 entries beside values of 128), bfloat16, causal, with or
 // without per-head score slopes (ALiBi), over the paged cache. The description below
 // is for head size 64; with 128 the tiles of Q, K and V are two blocks of 64 dims, S takes two groups
-// of matrix instructions, O two (one per 64 dims of the output), and one block fits on an SM.
+// of matrix instructions, O is 128 columns, and one block fits on an SM (two with TWO, below). Above 64 the matrix
+// instructions of S and of O += P V are issued by a warp each (APART), and extras and weights of two terms have two
+// softmax threads a row.
 //
 // One block = 128 consecutive new tokens of one sequence x one query head. 128 softmax threads, one per
 // query row (tensor-memory lane t = row t). One more warp's first lane issues every matrix
@@ -79,6 +81,26 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return r;
 }
 
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// tanh(x) / x of z = x^2 up to 1: the polynomial of degree 6 whose largest relative error is smallest (5e-8; 1.6e-7 with float32 roundings)
+__device__ __forceinline__ uint64_t tanh_ratio2(uint64_t z) {
+  constexpr float C[7] = {0.99999995024f, -0.33332839152f, 0.13325204069f, -0.053457029272f, 0.020289979855f, -0.0062033786024f, 0.0010410224670f};
+  uint64_t r = pack2(C[6], C[6]);
+#pragma unroll
+  for (int k = 5; k >= 0; --k) r = fma2(r, z, pack2(C[k], C[k]));
+  return r;
+}
+// of a divisor from 1 on (infinity: 0)
+__device__ __forceinline__ float fast_rcp(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
+  return r;
+}
+
 constexpr int TQ = 128;          // query rows per block
 constexpr int STAGES_TC = 4;      // page stages (three are 15 to 30 % slower, five bring nothing)
 // Tiles of D = 64 or 128 dims are kept as D / 64 blocks of [rows][64 dims], one after another, each
@@ -102,11 +124,6 @@ struct TcParams {
   int out_stride;                    // from one token's results to the next's
 };
 
-constexpr int SOFTMAX_THREADS = TQ;                 // one thread per query row
-// one more warp whose first lane issues the matrix instructions, and one whose first lane asks the
-// tensor memory accelerator for the pages
-constexpr int BLOCK_THREADS = SOFTMAX_THREADS + 64;
-
 // DK, DV: entries of a query or key row and of a value row (64 or 128 alike, or 192 beside 128).
 // BIAS: a per-head slope times the key's position is added to the raw scores, formed in bfloat16 as
 // the reference forms it.
@@ -115,30 +132,46 @@ constexpr int BLOCK_THREADS = SOFTMAX_THREADS + 64;
 // groups of matrix instructions on the same V tile.
 // EXTRAS: a window with kept first positions, a soft cap, sinks, an output gate, an output factor and strided results. A walk
 // takes the kept pages, then the window's: page i of the walk is not page i of the sequence, and a row may see nothing of a
-// page. Nothing else of the pipeline changes. What such a prompt costs is the chain of a page as above (a cap adds an
-// exponential and a reciprocal a score): 16 heads of 128 on 4 K/V heads, 2,048 tokens, window 1,024: 39 us, where
-// the mma.sync kernel took 175; prompts of 500, 1,000 and 1,501 tokens, cap and a gate per entry: 75 us against 261.
-// TWO (head size 128 with weights of two terms): two S buffers and two page stages instead of three and four, 97 KB and 256
-// columns of tensor memory a block, so that two blocks fit on an SM and one's softmax runs under the other's waits. Taken where
+// page. Nothing else of the pipeline changes. 16 heads of 128 on 4 K/V heads, 2,048 tokens, window 1,024: 31 us (the mma.sync
+// kernel 175); prompts of 500, 1,000 and 1,501 tokens, cap and a gate per entry: 66 us against 261.
+// Head sizes above 64: what a page costs is a chain of waits and of instructions issued one after another. One thread that issues S and
+// O += P V needs 1,810 clocks a page (weights of two terms): a wait costs a hundred and more also where what it waits for is there, a
+// commit 44, a request for a page some hundreds; the instructions are 900. So each product has a thread, and keys and values of a page
+// have a barrier each. With two threads a softmax row (each takes 32 keys of a page; they exchange their maxima through shared memory
+// and share the work on O by columns) the softmax is no longer the longest part: 1,500. us before and with both: full context
+// of 2,048 tokens, 16 heads 41 -> 38, latent keys of 192 at 3,000 tokens 99 -> 82, 32 heads of 3,400 tokens (TWO) 165 -> 131, window of
+// 1,024 in 2,048 tokens 37 -> 31; two threads a row alone 41 -> 41 and 38 -> 37. A walk of three pages (window of 100) 18 -> 19. Head size
+// 64 is bound by the exponential unit: 3 to 7 % slower with two issuing threads or two barriers a page.
+// TWO (head size 128 with weights of two terms): two S buffers and two page stages instead of three and four, 99 KB and 256
+// columns of tensor memory a block, so that two blocks fit on an SM and one's softmax runs under the other's waits. A stage of keys is
+// asked for again when its S is complete, not only when its O += P V is (before, S waited 1,000 of a page's 2,560 clocks for its keys),
+// and by the thread that issues from it: a third warp would leave 80 registers a thread (2 to 4 % slower). Taken where
 // the blocks make more than two waves, or more than one with a window, whose walks are alike long; with fewer blocks and the
 // triangle of a full context the longest chain counts, and a block with an SM of its own runs it faster. us, one an SM
-// against two: full context 256 blocks 39 / 47, 288 47 / 54, 320 59 / 60, 384 (one prompt) 81 / 72, 512 126 / 116, 640 110 /
-// 88; capped 256 55 / 55, 288 66 / 63, 320 85 / 71, 384 (three prompts) 56 / 46; window of 300: 160 18 / 16, 256 24 / 19, 512
-// 45 / 34; of 1,024: 256 (2,048 tokens) 38 / 32, 288 44 / 38, 512 72 / 68. Where most of a prompt fits into its window the walks are
-// a triangle again and one an SM would be the faster: 160 blocks of 1,024 in 2,560 tokens 24 / 30, four prompts of 640 15 / 19 (the
-// rule does not look at lengths).
+// against two: full context 208 blocks 32 / 36, 256 37 / 42, 288 44 / 47, 320 56 / 49, 864 (32 heads) 167 / 131; capped 240 51 / 54, 304 73 /
+// 71, 864 245 / 187; window of 300: 160 20 / 16; of 1,024: 256 (2,048 tokens) 38 / 31. Where most of a prompt fits into its window the
+// walks are a triangle again and one an SM would be the faster: 160 blocks of 1,024 in 2,560 tokens 23 / 27 (the rule does not
+// look at lengths).
+template <int DK, bool WIDE, bool EXTRAS, bool TWO> struct TcThreads {
+  static constexpr int PER = DK > 64 && (WIDE || EXTRAS) ? 2 : 1, SOFTMAX = TQ * PER;
+  static constexpr bool APART = DK > 64;      // S and O += P V by a thread each; and (not TWO) a third for the pages
+  static constexpr int BLOCK = SOFTMAX + (APART && !TWO ? 96 : 64);
+};
 template <bool TWO> struct TcShape {
   static constexpr int BUFS = TWO ? 2 : 3;                 // S buffers
   static constexpr int STAGES = TWO ? 2 : STAGES_TC;       // page stages
 };
 template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS, bool TWO>
-__global__ void __launch_bounds__(BLOCK_THREADS, DK == 64 || TWO ? 2 : 1)
+__global__ void __launch_bounds__(TcThreads<DK, WIDE, EXTRAS, TWO>::BLOCK, DK == 64 || TWO ? 2 : 1)
 attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_pool,
                     const __nv_bfloat16* __restrict__ v_pool, __nv_bfloat16* __restrict__ out, StepBatch sb,
                     const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, TcParams p,
                     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                     int* __restrict__ error_flag) {
+  constexpr bool APART = TcThreads<DK, WIDE, EXTRAS, TWO>::APART;
   constexpr int BUFS = TcShape<TWO>::BUFS, STAGES = TcShape<TWO>::STAGES;
+  constexpr int PER = TcThreads<DK, WIDE, EXTRAS, TWO>::PER, SOFTMAX_THREADS = TcThreads<DK, WIDE, EXTRAS, TWO>::SOFTMAX, MINE = KEYS / PER;
+  __shared__ float row_words[PER == 2 ? 2 : 1][2][PER == 2 ? TQ : 1];      // what a row's two threads tell each other
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte alignment: the swizzle pattern is a function of address bits 4..9
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
@@ -156,13 +189,14 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   unsigned char* k_ring = q_tile + TILE_Q_BYTES;                      // STAGES pages
   unsigned char* v_ring = k_ring + STAGES * TILE_K_BYTES;          // STAGES pages
   // barriers: [0..2] S buffer written; [3..6] O updated (page % 4); [7..9] P written (page % 3);
-  // then per stage: page landed, stage free again
+  // then per stage: keys landed, values landed
   uint64_t* bars = reinterpret_cast<uint64_t*>(v_ring + STAGES * TILE_V_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10 + 2 * STAGES);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool mma_warp = warp == SOFTMAX_THREADS / 32;
-  const bool copy_warp = warp == SOFTMAX_THREADS / 32 + 1;
+  const bool score_warp = warp == SOFTMAX_THREADS / 32;
+  const bool value_warp = APART && warp == SOFTMAX_THREADS / 32 + 1;
+  const bool copy_warp = !TWO && warp == SOFTMAX_THREADS / 32 + (APART ? 2 : 1);
   const int row = tid & (TQ - 1);        // query row of a softmax thread (= its tensor-memory lane)
   // heads are the fast index of the grid: the blocks of one tile start together (they read the same
   // pages), and tiles come in the order of the list, which the caller sorts by falling key count so that
@@ -185,36 +219,40 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   const int n_blocks = kept_pages + last_pos / KEYS + 1 - kb_lo;
   auto block_of = [&](int i) { return EXTRAS ? (i < kept_pages ? i : kb_lo + i - kept_pages) : i; };   // page i of the walk
 
-  // A warp may be up to three pages ahead of another one (S of page i + 2 is issued before P of page i is
-  // complete, S of page i + 3 only after it): arrivals for pages i + 1 and i + 2 must not count for page
+  // A warp may be up to three pages ahead of another one (S of page i + 3 is issued after the O += P V of page i, that of page i + 2
+  // before P of page i is complete): arrivals for pages i + 1 and i + 2 must not count for page
   // i, hence a "P written" barrier per S buffer. A wait names a barrier's phase by its parity, which is
   // only right if the completion before the awaited one has happened already. A thread that has read S of
-  // page i knows that O += P V of page i - 3 has completed (the tensor pipe runs in order), and so the one
+  // page i knows that O += P V of page i - 3 has completed (S of page i was issued after that), and so the one
   // of page i - 4: hence four "O updated" barriers that take turns. With two, a warp that reached the end
   // of its walk pages ahead of the others could take the completion of page i - 2 for that of page i and
   // read O before the last products were in it. With two S buffers every distance is one page less.
   const uint32_t bar_s = smem_u32(&bars[0]), bar_o = smem_u32(&bars[3]);
   const uint32_t bar_p = smem_u32(&bars[7]);
-  const uint32_t bar_k = smem_u32(&bars[10]), bar_free = smem_u32(&bars[10 + STAGES]);
-  // The copy warp's first lane sets the barriers up and asks for the first pages at once (their numbers
-  // read by the warp's lanes, one each): they are on their way while the other warps fetch Q and tensor
-  // memory is allocated. Nobody else touches a barrier before the block-wide barrier below.
-  constexpr uint32_t PAGE_BYTES = TILE_K_BYTES + TILE_V_BYTES;
-  auto ask_page = [&](int b, int page) {
-    const int st = b % STAGES;
-    const int y = (page * p.kv_heads + g) * KEYS;   // first row of the page in the pool seen as [rows][D]
+  const uint32_t bar_k = smem_u32(&bars[10]), bar_v = smem_u32(&bars[10 + STAGES]);
+  // The keys or values of page b of the walk into stage b % STAGES, as boxes [64 keys x 64 dims] in the swizzled layout; a barrier counts
+  // the bytes, one for both where one thread waits for both.
+  auto ask_keys = [&](int b, int page) {
+    const int st = b % STAGES, y = (page * p.kv_heads + g) * KEYS;   // first row of the page in the pool seen as [rows][D]
     const uint32_t full = bar_k + 8 * st;
-    mbar_expect_tx(full, PAGE_BYTES);
+    mbar_expect_tx(full, TILE_K_BYTES + (APART ? 0 : TILE_V_BYTES));
 #pragma unroll
     for (int blk = 0; blk < DK / 64; ++blk)
       tma_load_2d(smem_u32(k_ring + st * TILE_K_BYTES + blk * (KEYS * 128)), &k_map, blk * 64, y, full);
+  };
+  auto ask_values = [&](int b, int page) {      // after ask_keys of the page
+    const int st = b % STAGES, y = (page * p.kv_heads + g) * KEYS;
+    const uint32_t full = (APART ? bar_v : bar_k) + 8 * st;
+    if (APART) mbar_expect_tx(full, TILE_V_BYTES);
 #pragma unroll
     for (int blk = 0; blk < DV / 64; ++blk)
       tma_load_2d(smem_u32(v_ring + st * TILE_V_BYTES + blk * (KEYS * 128)), &v_map, blk * 64, y, full);
   };
-  int first_pages = 0;   // the copy warp's lanes: the number of page b = lane
-  if (copy_warp) {
-    first_pages = lane < n_blocks ? pages[block_of(lane)] : 0;
+  // The first lane of the copy warp (TWO: of the one that issues S) sets the barriers up and asks for the first pages at once (their numbers
+  // read by the warp's lanes, one each): they are on their way while the other warps fetch Q and tensor
+  // memory is allocated. Nobody else touches a barrier before the block-wide barrier below.
+  if (TWO ? score_warp : copy_warp) {
+    const int first_pages = lane < n_blocks ? pages[block_of(lane)] : 0;   // lane b: the number of page b
     if (lane == 0) {
       for (int b = 0; b < 3; ++b) {
         mbar_init(bar_s + 8 * b, 1);
@@ -222,21 +260,24 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       }
       for (int b = 0; b < 4; ++b) mbar_init(bar_o + 8 * b, 1);
       for (int s = 0; s < STAGES; ++s) {
-        mbar_init(bar_k + 8 * s, 1);      // the copy thread's expect_tx; the bytes complete it
-        mbar_init(bar_free + 8 * s, 1);   // tcgen05.commit after the stage's O += P V
+        mbar_init(bar_k + 8 * s, 1);      // the asking thread's expect_tx; the bytes complete it
+        mbar_init(bar_v + 8 * s, 1);
       }
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     for (int b = 0; b < STAGES && b < n_blocks; ++b) {
       const int page = __shfl_sync(0xffffffffu, first_pages, b);
-      if (lane == 0) ask_page(b, page);
+      if (lane == 0) {
+        ask_keys(b, page);
+        ask_values(b, page);
+      }
     }
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
-  if (!mma_warp && !copy_warp) {
+  if (warp < SOFTMAX_THREADS / 32) {
     // Q tile: rows of the tile, zero beyond the valid tokens
     const uint32_t qs = smem_u32(q_tile);
     for (int i = tid; i < TQ * (DK / 8); i += SOFTMAX_THREADS) {
@@ -257,80 +298,129 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   const uint32_t tmem_o = tmem_base + TMEM_O;
   bool alive = true;  // false after a wait ran out: keep going without waiting, results are void
 
+  // At head sizes above 64 two threads issue matrix instructions, each for its own products: a wait costs a hundred clocks and more
+  // also where what it waits for is there, a commit 44, and one thread's waits and instructions in a row were what a page cost (1,810
+  // clocks at head size 128, of which the instructions are 900). At 64 one thread issues both (900 clocks of the 1,500 that a page
+  // costs; with two threads 3 to 7 % slower).
+  constexpr uint32_t IDESC_S = idesc_bf16(TQ, KEYS, false);
+  // all DV dims of the output in one instruction: an instruction of M = 128, K = 16 takes 51 clocks at
+  // least whatever its N (N / 2 clocks from N = 128 on), so their number is what a page costs
+  constexpr uint32_t IDESC_PV = idesc_bf16(TQ, DV, true);
+  const uint64_t desc_q = smem_desc(smem_u32(q_tile), 16, 1024), desc_k0 = smem_desc(smem_u32(k_ring), 16, 1024);
+  // V is MN-major: blocks of 64 dims lie KEYS * 128 bytes apart (the leading offset), groups of 8 keys
+  // 1024 bytes (the stride offset)
+  const uint64_t desc_v0 = smem_desc(smem_u32(v_ring), KEYS * 128, 1024);
+  constexpr uint64_t K_UNITS = TILE_K_BYTES >> 4, V_UNITS = TILE_V_BYTES >> 4;   // the address field counts 16-byte units
+  constexpr uint64_t Q_BLOCK = (TQ * 128) >> 4, KV_BLOCK = (KEYS * 128) >> 4;   // blocks of 64 dims
+  // S = Q K^T of page i into S buffer `buf`
+  auto issue_s = [&](int i, int buf) {
+    tc_fence_after();
+#pragma unroll
+    for (int blk = 0; blk < DK / 64; ++blk)
+      tc_mma4<2, 2>(tmem_base + buf * 64, desc_q + blk * Q_BLOCK, desc_k0 + (i % STAGES) * K_UNITS + blk * KV_BLOCK, IDESC_S,
+                    blk > 0 ? 1u : 0u);
+    tc_commit(bar_s + buf * 8);
+  };
+  // P of page i is written and O is rescaled: O += P V (16 keys: 32 bytes along P's rows, 2048 bytes down V's rows)
+  auto issue_pv = [&](int i, int buf) {
+    tc_fence_after();
+    const uint64_t desc_v = desc_v0 + (i % STAGES) * V_UNITS;
+    tc_mma4_ts<128>(tmem_o, tmem_base + buf * 64, desc_v, IDESC_PV, i > 0 ? 1u : 0u);
+    if (WIDE) tc_mma4_ts<128>(tmem_o, tmem_base + buf * 64 + KEYS / 2, desc_v, IDESC_PV, 1u);
+    tc_commit(bar_o + 8 * (i & 3));
+  };
   if (copy_warp) {
-    // ------------------------------------------------------------ the thread that asks for the pages
-    // Page b goes into stage b % STAGES as DK / 64 and DV / 64 boxes [64 keys x 64 dims] for K and V, in
-    // the swizzled layout; the stage's barrier counts the bytes. A stage is free again when the
-    // O += P V that read it has completed (S of that page completed before it).
-    // The first pages were asked for above; the rest is the first lane's alone.
+    // ------------------------------------------------------------ the pages
+    // A stage is free again when the O += P V that read it has completed (S of that page completed before it).
     if (lane == 0) {
-      int issued = min(n_blocks, STAGES);
+      int asked = min(n_blocks, STAGES);
       for (int b = STAGES; b < n_blocks; ++b) {
-        if (!mbar_wait(bar_free + 8 * (b % STAGES), ((b / STAGES) - 1) & 1, error_flag, 6)) break;
-        ask_page(b, pages[block_of(b)]);
-        issued = b + 1;
+        const int page = pages[block_of(b)];
+        alive = mbar_wait(bar_o + 8 * ((b - STAGES) & 3), ((b - STAGES) >> 2) & 1, error_flag, 6);
+        if (!alive) break;
+        ask_keys(b, page);
+        ask_values(b, page);
+        asked = b + 1;
       }
-      if (issued < n_blocks) {
-        // a wait ran out: what is in flight lands before the block ends (bounded waits again)
-        for (int b = max(0, issued - STAGES); b < issued; ++b)
+      if (!alive)      // a wait ran out: what is in flight lands before the block ends (bounded waits again)
+        for (int b = max(0, asked - STAGES); b < asked; ++b) {
           mbar_wait(bar_k + 8 * (b % STAGES), (b / STAGES) & 1, error_flag, 6);
+          if (APART) mbar_wait(bar_v + 8 * (b % STAGES), (b / STAGES) & 1, error_flag, 6);
+        }
+    }
+  } else if (score_warp) {
+    // ------------------------------------------------------------ S, and at head size 64 O += P V
+    if (lane == 0) {
+      int buf = 0, phase = 0;   // S buffer of page i (i % BUFS) and the parity of its barriers ((i / BUFS) & 1)
+      if constexpr (APART) {
+        int asked = min(n_blocks, STAGES), next_page = TWO && asked < n_blocks ? pages[block_of(asked)] : 0;
+        for (int i = 0; i < n_blocks; ++i) {
+          if (TWO && i > 0 && asked < n_blocks) {      // the stage of page i - 1 is free again when its S is complete
+            alive = mbar_wait(bar_s + 8 * ((i - 1) % BUFS), ((i - 1) / BUFS) & 1, error_flag, 6);
+            if (!alive) break;
+            ask_keys(asked, next_page);
+            if (++asked < n_blocks) next_page = pages[block_of(asked)];
+          }
+          alive = mbar_wait(bar_k + 8 * (i % STAGES), (i / STAGES) & 1, error_flag, 4);
+          // S goes where S and P of page i - BUFS were: the O += P V that read that P has completed, and every thread had read
+          // that S before it wrote its P
+          if (alive && i >= BUFS) alive = mbar_wait(bar_o + 8 * ((i - BUFS) & 3), ((i - BUFS) >> 2) & 1, error_flag, 4);
+          if (!alive) break;
+          issue_s(i, buf);
+          if (++buf == BUFS) buf = 0;
+        }
+        if (TWO && !alive)      // a wait ran out: what is in flight lands before the block ends (bounded waits again)
+          for (int b = max(0, asked - STAGES); b < asked; ++b) mbar_wait(bar_k + 8 * (b % STAGES), (b / STAGES) & 1, error_flag, 6);
+      } else {
+        for (int b = 0; b < BUFS - 1 && b < n_blocks && alive; ++b) {
+          alive = mbar_wait(bar_k + 8 * b, 0, error_flag, 4);
+          if (alive) issue_s(b, b);
+        }
+        for (int i = 0; i < n_blocks && alive; ++i) {
+          const int ahead = i + BUFS - 1;
+          if (ahead < n_blocks) {
+            // S of page `ahead` goes where S_{i-1} and P_{i-1} were: every thread had read that S before it reported
+            // P_{i-1}, and the O += P_{i-1} V_{i-1} that reads the P was issued before (the tensor pipe runs in order)
+            alive = mbar_wait(bar_k + 8 * (ahead % STAGES), (ahead / STAGES) & 1, error_flag, 4);
+            if (alive) issue_s(ahead, buf == 0 ? BUFS - 1 : buf - 1);
+          }
+          if (alive) alive = mbar_wait(bar_p + buf * 8, phase, error_flag, 5);
+          if (alive) issue_pv(i, buf);
+          if (++buf == BUFS) { buf = 0; phase ^= 1; }
+        }
       }
     }
-  } else if (mma_warp) {
-    // ------------------------------------------------------------ the thread that issues matrix instructions
+  } else if (value_warp) {
+    // ------------------------------------------------------------ O += P V
     if (lane == 0) {
-      constexpr uint32_t IDESC_S = idesc_bf16(TQ, KEYS, false);
-      // all DV dims of the output in one instruction: an instruction of M = 128, K = 16 takes 51 clocks at
-      // least whatever its N (N / 2 clocks from N = 128 on), so their number is what a page costs
-      constexpr uint32_t IDESC_PV = idesc_bf16(TQ, DV, true);
-      const uint64_t desc_q = smem_desc(smem_u32(q_tile), 16, 1024);
-      const uint64_t desc_k0 = smem_desc(smem_u32(k_ring), 16, 1024);
-      // V is MN-major: blocks of 64 dims lie KEYS * 128 bytes apart (the leading offset), groups of 8 keys
-      // 1024 bytes (the stride offset)
-      const uint64_t desc_v0 = smem_desc(smem_u32(v_ring), KEYS * 128, 1024);
-      constexpr uint64_t K_UNITS = TILE_K_BYTES >> 4, V_UNITS = TILE_V_BYTES >> 4;   // the address field counts 16-byte units
-      constexpr uint64_t Q_BLOCK = (TQ * 128) >> 4, KV_BLOCK = (KEYS * 128) >> 4;   // blocks of 64 dims
-      // S_b = Q K_b^T into S buffer `buf`; the page sits in stage b % STAGES
-      auto issue_s = [&](int b, int buf) {
-        const int st = b % STAGES;
-#pragma unroll
-        for (int blk = 0; blk < DK / 64; ++blk)
-          tc_mma4<2, 2>(tmem_base + buf * 64, desc_q + blk * Q_BLOCK, desc_k0 + st * K_UNITS + blk * KV_BLOCK,
-                        IDESC_S, blk > 0 ? 1u : 0u);
-        tc_commit(bar_s + buf * 8);
-      };
-      // S of the first pages
-      for (int b = 0; b < BUFS - 1 && b < n_blocks && alive; ++b) {
-        alive = mbar_wait(bar_k + 8 * b, 0, error_flag, 4);
-        tc_fence_after();
-        if (alive) issue_s(b, b);
-      }
-      int buf = 0, phase = 0;   // S buffer of page i (i % BUFS) and the parity of its barriers ((i / BUFS) & 1)
-      for (int i = 0; i < n_blocks && alive; ++i) {
-        const int ahead = i + BUFS - 1;
-        if (ahead < n_blocks) {
-          // page `ahead` landed; its S goes where S_{i-1} and P_{i-1} were: every thread had read that S
-          // before it reported P_{i-1}, and the O += P_{i-1} V_{i-1} that reads the P was issued before
-          alive = mbar_wait(bar_k + 8 * (ahead % STAGES), (ahead / STAGES) & 1, error_flag, 4);
-          tc_fence_after();
-          issue_s(ahead, buf == 0 ? BUFS - 1 : buf - 1);
-        }
-        // P_i is written and O is rescaled: O += P_i V_i (16 keys: 32 bytes along P's rows, 2048 bytes
-        // down V's rows)
+      int buf = 0, phase = 0, asked = min(n_blocks, STAGES), next_page = TWO && asked < n_blocks ? pages[block_of(asked)] : 0;
+      for (int i = 0; i < n_blocks; ++i) {
+        alive = mbar_wait(bar_v + 8 * (i % STAGES), (i / STAGES) & 1, error_flag, 5);
         if (alive) alive = mbar_wait(bar_p + buf * 8, phase, error_flag, 5);
-        tc_fence_after();
-        const int st = i % STAGES;
-        tc_mma4_ts<128>(tmem_o, tmem_base + buf * 64, desc_v0 + st * V_UNITS, IDESC_PV, i > 0 ? 1u : 0u);
-        if (WIDE) tc_mma4_ts<128>(tmem_o, tmem_base + buf * 64 + KEYS / 2, desc_v0 + st * V_UNITS, IDESC_PV, 1u);
-        tc_commit(bar_o + 8 * (i & 3));
-        tc_commit(bar_free + 8 * st);   // the copy thread may refill this stage
+        if (!alive) break;
+        issue_pv(i, buf);
         if (++buf == BUFS) { buf = 0; phase ^= 1; }
+        if (TWO && i > 0 && asked < n_blocks) {      // the stage of page i - 1 is free again when its O += P V is complete
+          alive = mbar_wait(bar_o + 8 * ((i - 1) & 3), ((i - 1) >> 2) & 1, error_flag, 6);
+          if (!alive) break;
+          ask_values(asked, next_page);
+          if (++asked < n_blocks) next_page = pages[block_of(asked)];
+        }
       }
+      if (TWO && !alive)
+        for (int b = max(0, asked - STAGES); b < asked; ++b) mbar_wait(bar_v + 8 * (b % STAGES), (b / STAGES) & 1, error_flag, 6);
     }
   } else {
     // ------------------------------------------------------------ softmax threads
+    const int part = PER == 2 ? warp >> 2 : 0;      // of the row: keys [MINE part, MINE part + MINE) of a page, DV / PER columns of O
     const uint32_t lane_addr = tmem_base + (uint32_t((warp & 3) * 32) << 16);   // this warp's lanes
-    const uint32_t o_addr = lane_addr + TMEM_O;
+    const uint32_t o_addr = lane_addr + TMEM_O + part * (DV / PER);
+    // what the row's other thread says to `mine`; `turn`: 0 and 1 in turns, so that nothing is overwritten before it is read
+    auto other = [&](float mine, int turn) {
+      row_words[turn][part][row] = mine;
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (warp & 3)) : "memory");
+      return row_words[turn][part ^ 1][row];
+    };
     int buf = 0, phase = 0;   // S buffer of page i (i % BUFS) and the parity of its barriers ((i / BUFS) & 1)
     float m_run = -INFINITY, l_run = 0.f;   // running maximum of the raw scores, the row's sum
     const float slope = BIAS ? p.slopes[h] : 0.f;
@@ -338,42 +428,75 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
     const float sl2 = capped ? 1.f : p.scale * 1.4426950408889634f;      // capped scores are in powers of two already
     const uint64_t sl2_2 = pack2(sl2, sl2);
     for (int i = 0; i < n_blocks; ++i) {
-      const int key0 = block_of(i) * KEYS;
+      const int page0 = block_of(i) * KEYS, key0 = page0 + part * MINE;
       // (1) this thread's row of S_i: both halves asked for, one wait
       if (alive) alive = mbar_wait(bar_s + buf * 8, phase, error_flag, 1);
       tc_fence_after();
-      float s[KEYS];
-      tmem_ld64_once(lane_addr + buf * 64, s);
+      float s[MINE];
+      if constexpr (PER == 2) tmem_ld32(lane_addr + buf * 64 + part * MINE, s);
+      else tmem_ld64_once(lane_addr + buf * 64, s);
       if (BIAS) {
 #pragma unroll
-        for (int j = 0; j < KEYS; ++j) s[j] += alibi_bias(slope, key0 + j);
+        for (int j = 0; j < MINE; ++j) s[j] += alibi_bias(slope, key0 + j);
       }
-      if (capped) {      // tanh(x) = 1 - 2 / (1 + exp(2 x)), times the cap, in powers of two
-        const float in = p.scale * (2.f * 1.4426950408889634f / p.softcap), out2 = p.softcap * 1.4426950408889634f;
+      // only pages that reach past some row's position, or left of some row's window, hide keys: `with` in their places
+      auto hide = [&](float with) {
+        if (page0 + KEYS - 1 > past + q0 || !row_ok) {   // first part is uniform over the block
+          const int visible = row_pos - key0;   // columns j <= visible are seen by this row
 #pragma unroll
-        for (int j = 0; j < KEYS; ++j) s[j] = out2 * (1.f - __fdividef(2.f, fast_exp2(s[j] * in) + 1.f));
-      }
-      // (2) maximum of the visible scores; only pages that reach past some row's position, or left of some row's window,
-      // need the test
-      if (key0 + KEYS - 1 > past + q0 || !row_ok) {   // first part is uniform over the block
-        const int visible = row_pos - key0;   // columns j <= visible are seen by this row
+          for (int j = 0; j < MINE; ++j) s[j] = (j <= visible) ? s[j] : with;
+        }
+        if (EXTRAS && p.window > 0 && page0 <= last_pos - p.window) {   // uniform over the block
+          const int left = row_pos - p.window - key0, kept = p.keep_first - key0;   // columns left < j or j < kept are seen
 #pragma unroll
-        for (int j = 0; j < KEYS; ++j) s[j] = (j <= visible) ? s[j] : -INFINITY;
-      }
-      if (EXTRAS && p.window > 0 && key0 <= last_pos - p.window) {   // uniform over the block
-        const int left = row_pos - p.window - key0, kept = p.keep_first - key0;   // columns left < j or j < kept are seen
+          for (int j = 0; j < MINE; ++j) s[j] = (j > left || j < kept) ? s[j] : with;
+        }
+      };
+      if (capped) {      // cap * tanh(score / cap), in powers of two
+        // Where none of the visible ones reaches the cap, by multiply-adds: the exponential unit, with its exponential and its
+        // reciprocal here beside the softmax's exponential, is 1,536 clocks of a capped page (32 heads of 3,400 tokens, two blocks an SM 202
+        // -> 187 us; one block an SM 49 -> 51 of 1,900 tokens). Else tanh(x) = 1 - 2 / (1 + exp(2 x)). Which one follows from what the
+        // thread's row sees of the page.
+        const float to_x = p.scale / p.softcap, out2 = p.softcap * 1.4426950408889634f;
+        bool inside = false;
+        if constexpr (PER == 2) {
+          hide(0.f);
+          float most = 0.f;
 #pragma unroll
-        for (int j = 0; j < KEYS; ++j) s[j] = (j > left || j < kept) ? s[j] : -INFINITY;
+          for (int j = 0; j < MINE; ++j) most = fmaxf(most, fabsf(s[j]));
+          inside = most * to_x <= 1.f;
+        }
+        if (inside) {
+          const uint64_t to_x2 = pack2(to_x, to_x), to_out2 = pack2(to_x * out2, to_x * out2);
+#pragma unroll
+          for (int j = 0; j < MINE; j += 2) {
+            const uint64_t v = pack2(s[j], s[j + 1]), x = mul2(v, to_x2);
+            unpack2(mul2(mul2(v, to_out2), tanh_ratio2(mul2(x, x))), s[j], s[j + 1]);
+          }
+        } else {
+          const float in = to_x * (2.f * 1.4426950408889634f);
+#pragma unroll
+          for (int j = 0; j < MINE; ++j) s[j] = fmaf(-2.f * out2, fast_rcp(fast_exp2(s[j] * in) + 1.f), out2);
+        }
+        __syncwarp();
       }
+      // (2) maximum of the visible scores
+      hide(-INFINITY);
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int j = 0; j < KEYS; j += 8) {
+      for (int j = 0; j < MINE; j += 8) {
         mx[0] = max3(mx[0], s[j], s[j + 1]);
         mx[1] = max3(mx[1], s[j + 2], s[j + 3]);
         mx[2] = max3(mx[2], s[j + 4], s[j + 5]);
         mx[3] = max3(mx[3], s[j + 6], s[j + 7]);
       }
-      float m_new = fmaxf(m_run, fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]));
+      float m_page = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+      if constexpr (PER == 2) {      // and the other thread has its scores in registers: their places may be written below
+        tc_fence_before();
+        m_page = fmaxf(m_page, other(m_page, i & 1));
+        tc_fence_after();
+      }
+      float m_new = fmaxf(m_run, m_page);
       if ((m_new - m_run) * sl2 <= RESCALE_LOG2) m_new = m_run;   // (false from -inf: the first scores set it)
       const float corr = (m_run == -INFINITY) ? 0.f : fast_exp2((m_run - m_new) * sl2);
       const bool moved = (m_new != m_run) && (m_run != -INFINITY);
@@ -384,8 +507,8 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       if (i > 0 && __any_sync(0xffffffffu, moved)) {
         if (alive) alive = mbar_wait(bar_o + 8 * ((i - 1) & 3), ((i - 1) >> 2) & 1, error_flag, 2);
         tc_fence_after();
-#pragma unroll
-        for (int c0 = 0; c0 < DV; c0 += 32) {
+#pragma unroll (PER == 2 ? 1 : DV / 32)
+        for (int c0 = 0; c0 < DV / PER; c0 += 32) {
           float o[32];
           tmem_ld32(o_addr + c0, o);
 #pragma unroll
@@ -397,9 +520,9 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       // (4) P = exp2(S - max) as bfloat16 pairs, two values per packed multiply-add
       const uint64_t moff_2 = pack2(-m_off, -m_off);
       uint64_t acc2[4] = {0ull, 0ull, 0ull, 0ull};
-      uint32_t w[KEYS / 2];
+      uint32_t w[MINE / 2];
 #pragma unroll
-      for (int e = 0; e < KEYS / 2; ++e) {
+      for (int e = 0; e < MINE / 2; ++e) {
         float x0, x1;
         unpack2(fma2(pack2(s[2 * e], s[2 * e + 1]), sl2_2, moff_2), x0, x1);
         const float a = fast_exp2(x0), b = fast_exp2(x1);
@@ -412,12 +535,12 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       }
       // P in place of this page's S: keys 2c, 2c + 1 in column c of the buffer (this thread's row of S is in
       // registers since the load above)
-      tmem_st_u32<KEYS / 2>(lane_addr + buf * 64, w);
+      tmem_st_u32<MINE / 2>(lane_addr + buf * 64 + part * (MINE / 2), w);
       if (WIDE) {
-        uint32_t lo[KEYS / 2];
+        uint32_t lo[MINE / 2];
 #pragma unroll
-        for (int e = 0; e < KEYS / 2; ++e) lo[e] = pack_bf16(s[2 * e], s[2 * e + 1]);
-        tmem_st_u32<KEYS / 2>(lane_addr + buf * 64 + KEYS / 2, lo);
+        for (int e = 0; e < MINE / 2; ++e) lo[e] = pack_bf16(s[2 * e], s[2 * e + 1]);
+        tmem_st_u32<MINE / 2>(lane_addr + buf * 64 + KEYS / 2 + part * (MINE / 2), lo);
       }
       tmem_st_wait();
       float l0, l1, l2, l3;
@@ -431,9 +554,10 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
     // the walk's last O += P V
     if (alive) alive = mbar_wait(bar_o + 8 * ((n_blocks - 1) & 3), ((n_blocks - 1) >> 2) & 1, error_flag, 3);
     tc_fence_after();
+    if constexpr (PER == 2) l_run += other(l_run, n_blocks & 1);
     float inv = l_run > 0.f ? 1.f / l_run : 0.f;
     const size_t t = size_t(start + q0 + row);
-    __nv_bfloat16* dst = out + (t * p.heads + h) * DV;
+    __nv_bfloat16* dst = out + (t * p.heads + h) * DV + part * (DV / PER);
     const __nv_bfloat16* ge = nullptr;      // a gate per entry
     if (EXTRAS) {
       if (p.sinks) {
@@ -443,12 +567,12 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
         inv = (l > 0.f ? 1.f / l : 0.f) * keep;
       }
       inv *= p.out_scale;
-      dst = out + t * p.out_stride + size_t(h) * DV;
-      if (p.gate && p.gate_wide) ge = p.gate + t * p.gate_stride + size_t(h) * DV;
+      dst = out + t * p.out_stride + size_t(h) * DV + part * (DV / PER);
+      if (p.gate && p.gate_wide) ge = p.gate + t * p.gate_stride + size_t(h) * DV + part * (DV / PER);
       else if (p.gate && row_ok) inv *= 1.f / (1.f + expf(-__bfloat162float(p.gate[t * p.gate_stride + h])));
     }
-#pragma unroll
-    for (int c0 = 0; c0 < DV; c0 += 32) {
+#pragma unroll (PER == 2 ? 1 : DV / 32)
+    for (int c0 = 0; c0 < DV / PER; c0 += 32) {
       float o[32];
       tmem_ld32(o_addr + c0, o);
       if (row_ok) {
@@ -895,7 +1019,7 @@ int launch_tc(const void* q, const void* k_pool, const void* v_pool, int pool_pa
   static SharedLimit limit;
   if (!limit.allows(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO>, smem)) return PTB_ERR_LAUNCH;
   dim3 grid(p.heads, n_tiles);
-  attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO><<<grid, BLOCK_THREADS, smem, stream>>>(
+  attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO><<<grid, TcThreads<DK, WIDE, EXTRAS, TWO>::BLOCK, smem, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, sb,
       tile_seq, tile_q0, p, *km, *vm, error_flag);
   return launch_status();

@@ -460,6 +460,40 @@ def test_tc_extras(K, heads, kv, d, window, keep, softcap, sinks, gate, strided)
     K.check_device_errors("cuda:0")
 
 
+@pytest.mark.parametrize("heads,d", [(4, 64), (4, 128), (60, 128)])
+@pytest.mark.parametrize("window,softcap", [(0, 1.0), (0, 9.0), (100, 9.0)])
+def test_tc_cap_inside_and_beyond(K, heads, d, window, softcap):
+    """Scores of deviation 3 under a cap of 9, which a few rows of a page reach, and of 1, which nearly all do: tanh by its polynomial
+    and by the exponential, in one warp. Against the general kernel, bound as for test_tc_extras (tanh is off by 2e-7 of the cap
+    at most in either form). Which form a row takes does not follow from keys that it does not see: the same bits whatever lies there."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.attention import AttentionTiles
+    from pytorch_transformers_b200.parts.base import CacheNeed
+    kv, news = 2, [300, 129, 500, 50]
+    cache = Cache([(0, CacheNeed("full", kv, d), None)], sum((n + 63) // 64 * 64 for n in news), BF, "cuda")
+    slots = [cache.open() for _ in news]
+    ctx = StepContext(cache, slots, [[0] * n for n in news], 1, [[] for _ in news], [AttentionTiles(K)])
+    g = torch.Generator(device="cuda").manual_seed(window + heads)
+    k_pool, v_pool, gi = cache.entry_storage(0)
+    k_pool.normal_(generator=g), v_pool.normal_(generator=g)
+    q = (3 * torch.randn(sum(news), heads, d, generator=g, device="cuda")).to(BF)
+    tiles, batch = ctx.plan(AttentionTiles.plan_key), ctx.batch_c[gi]
+
+    def result(fn, name_seq, name_q0, count):
+        out = torch.empty(sum(news), heads * d, dtype=BF, device="cuda")
+        fn(q, k_pool, v_pool, batch, tiles.dev[name_seq], tiles.dev[name_q0], tiles.facts[count],
+           *(() if fn is K.attention_tc_extras else (None,)), kv, d ** -0.5, window, softcap=softcap, out=out)
+        return out
+    got = result(K.attention_tc_extras, "mtile_seq", "mtile_q0", "n_mma_tiles")
+    ref = result(K.attention_generic, "tile_seq", "tile_q0", "n_tiles").double()
+    assert ((got.double() - ref).abs() <= 2.0 ** -7 * ref.abs() + 2e-4).all(), (got.double() - ref).abs().max()
+    for s, n in zip(slots, news):      # what lies behind a sequence's last token
+        k_pool[cache.pages(s, gi)[n // 64], :, n % 64:] *= 1000
+    assert torch.equal(result(K.attention_tc_extras, "mtile_seq", "mtile_q0", "n_mma_tiles"), got)
+    K.check_device_errors("cuda:0")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("d,vd", [(8, 8), (8, 16), (16, 12), (72, 136), (128, 64), (256, 256), (250, 256)])
 def test_general_attention_reads_words_and_values_alike(K, dtype, d, vd):
