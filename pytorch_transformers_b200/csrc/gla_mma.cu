@@ -132,9 +132,11 @@ int launch_sum(const void* proj, int stride, const float* log_decay, const StepB
 // 16 tokens. Between sub-blocks u < w the exponent is a sum of three sums of logarithms of one sign, the rest of u after i,
 // the whole sub-blocks between, and w up to t: the first goes into the keys, the others into the queries, all factors are at
 // most 1, nothing is subtracted, and the scores are a product. Inside a sub-block every (t, i, channel) has an exponent of its
-// own: a warp walks t from i on with its lanes' channels' sums in registers. That is what bounds the kernel: 136 (t, i) pairs a sub-block and
-// channel, 70,000 exponentials a block against 16 a clock and SM, and the instructions around them. 2,900 tokens of
-// 16 heads of 128 x 128: 117 us (94 with operands of two terms), where the walk on the CUDA cores took 175.
+// own: a warp takes four keys and walks the tokens, its lanes' channels' sums for each key in registers; no branch on the keys' places, so that
+// the loads run ahead (117 -> 109 us). What bounds this part is the exponential unit: 136 (t, i) pairs a sub-block and channel, 70,000
+// exponentials a block against 16 a clock and SM. Decaying the four keys to their last one's token, and one exponential for all four from there
+// on, took 100 us, but two roundings and an exponential more a term: 1.48e-7 off 64 bits (one chunk, 2-norm) instead of 1.43e-7. 2,900
+// tokens of 16 heads of 128 x 128; with operands of two terms 94 (before), the walk on the CUDA cores 175.
 // Operands of a product that are float32 (scaled queries and keys, scores, the state) enter it as three bfloat16 terms, 24 bits: what
 // a product leaves out (second x third, third x third) is 2^-26 of it, below the rounding of its float32 sum. A matrix instruction
 // cuts its sum off instead of rounding it, so the six products of 16 entries are summed from zero, the small ones first, and
@@ -156,6 +158,30 @@ struct OutShape {
       size_t(CH) * DK * 2 + 2 * size_t(A_BYTES) + C_BYTES + size_t(CH) * LP * 4 + size_t(SUBS - 1) * DK * 4 + size_t(CH) * SPITCH * 4;
 };
 
+// two float32 values in a 64-bit register
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ float2 halves2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ unsigned long long wide2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(c) : "l"(a), "l"(b));
+  return c;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(a) : "l"(b));
+  return a;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  asm("add.rn.f32x2 %0, %0, %1;\n" : "+l"(a) : "l"(b));
+  return a;
+}
 __device__ __forceinline__ float2 pair_f(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
 template <int DK, int DV>
@@ -199,48 +225,44 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
     }
   }
   __syncthreads();
-  {   // scores inside sub-block `warp`: half of its keys (0, 3, 4, 7, .. or 1, 2, 5, 6, ..: 68 pairs each)
-    constexpr int CPL = DK / 32;      // channels of a lane
-    const int c0 = lane * CPL;
-    auto load_row = [&](const unsigned char* tile, int row, float (&f)[CPL]) {
+  {   // scores inside sub-block `warp`, in groups of four keys
+    constexpr int PAIRS = DK / 64;      // a lane's channels, two in a register pair: half the multiply-adds
+    const int c0 = lane * 2 * PAIRS;
+    auto load_row = [&](const unsigned char* tile, int row, unsigned long long (&f)[PAIRS]) {
       const unsigned char* p = tile + swz<DK>(row, c0 / 8) + (c0 % 8) * 2;
-      if (CPL == 4) {
+      if constexpr (PAIRS == 2) {
         const uint2 v = *reinterpret_cast<const uint2*>(p);
-        const float2 a = pair_f(v.x), b = pair_f(v.y);
-        f[0] = a.x; f[1] = a.y; f[CPL - 2] = b.x; f[CPL - 1] = b.y;
+        f[0] = wide2(v.x), f[1] = wide2(v.y);
       } else {
-        const float2 a = pair_f(*reinterpret_cast<const uint32_t*>(p));
-        f[0] = a.x; f[1] = a.y;
+        f[0] = wide2(*reinterpret_cast<const uint32_t*>(p));
       }
     };
-    for (int ii = 0; ii < SUB / 2; ++ii) {
-      const int i = 2 * ii + (half ^ (ii & 1));
-      float k[CPL], e[CPL], p[SUB];
-      load_row(k_s, warp * SUB + i, k);
+    const int r0 = warp * SUB;
+    // a lane's part of sum_c q[c] k[c] exp2(e[c])
+    auto score = [&](const unsigned long long (&q)[PAIRS], const unsigned long long (&k)[PAIRS], const unsigned long long (&e)[PAIRS]) {
+      unsigned long long sum = 0ull;
 #pragma unroll
-      for (int u = 0; u < CPL; ++u) e[u] = 0.f;
-#pragma unroll
-      for (int t = 0; t < SUB; ++t) {
-        p[t] = 0.f;
-        if (t < i) continue;
-        float q[CPL];
-        load_row(q_s, warp * SUB + t, q);
-        if (t > i) {
-          const float* lt = l_s + (warp * SUB + t) * LP + c0;
-          if (CPL == 4) {
-            const float4 l = *reinterpret_cast<const float4*>(lt);
-            e[0] += l.x; e[1] += l.y; e[CPL - 2] += l.z; e[CPL - 1] += l.w;
-          } else {
-            const float2 l = *reinterpret_cast<const float2*>(lt);
-            e[0] += l.x; e[1] += l.y;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < CPL; ++u) p[t] = fmaf(q[u] * k[u], fast_exp2(e[u]), p[t]);
+      for (int u = 0; u < PAIRS; ++u) {
+        const float2 x = halves2(e[u]);
+        sum = fma2(mul2(q[u], k[u]), pack2(fast_exp2(x.x), fast_exp2(x.y)), sum);
       }
-      // sums over the lanes of 16 values at once: at every step a lane hands half of its values on
+      const float2 v = halves2(sum);
+      return v.x + v.y;
+    };
+    auto load_logs = [&](int row, unsigned long long (&l)[PAIRS]) {
+      const unsigned long long* from = reinterpret_cast<const unsigned long long*>(l_s + row * LP + c0);
+      if constexpr (PAIRS == 2) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(from);
+        l[0] = v.x, l[1] = v.y;
+      } else {
+        l[0] = from[0];
+      }
+    };
+    // the lanes' sums of sixteen scores (4 tokens of group T x 4 keys of group g) and their place: at every step a lane hands half of its
+    // values on
+    auto put16 = [&](int T, int g, float (&p)[16]) {
 #pragma unroll
-      for (int w = SUB / 2; w > 0; w >>= 1) {
+      for (int w = 8; w > 0; w >>= 1) {
         const bool up = (lane & (2 * w)) != 0;
 #pragma unroll
         for (int t = 0; t < w; ++t) {
@@ -249,7 +271,37 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
         }
       }
       p[0] += __shfl_xor_sync(0xffffffffu, p[0], 1);
-      if ((lane & 1) == 0) s_s[(warp * SUB + (lane >> 1)) * SPITCH + warp * SUB + i] = p[0];
+      const int v = lane >> 1;
+      if ((lane & 1) == 0) s_s[(r0 + 4 * T + (v >> 2)) * SPITCH + r0 + 4 * g + (v & 3)] = p[0];
+    };
+#pragma unroll 1
+    for (int gi = 0; gi < 2; ++gi) {
+      const int g = half ? 1 + gi : 3 * gi;      // 20 tokens a warp: groups 0 and 3, or 1 and 2
+      unsigned long long k[4][PAIRS], e[4][PAIRS], q[PAIRS], l[PAIRS];      // e: a key's logarithms after it, up to the token
+      float p[16];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) load_row(k_s, r0 + 4 * g + a, k[a]);
+#pragma unroll 1
+      for (int T = g; T < 4; ++T) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          load_row(q_s, r0 + 4 * T + t, q);
+          load_logs(r0 + 4 * T + t, l);
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+#pragma unroll
+            for (int u = 0; u < PAIRS; ++u) e[a][u] = T == g && a >= t ? 0ull : add2(e[a][u], l[u]);
+            p[4 * t + a] = score(q, k[a], e[a]);
+            if (T == g && a > t) p[4 * t + a] = 0.f;      // before the key
+          }
+        }
+        put16(T, g, p);
+      }
+    }
+    // keys of later groups take no part: six squares of four, three a warp
+    for (int x = lane + 48 * half; x < 48 + 48 * half; x += 32) {
+      const int sq = x >> 4, T = sq < 3 ? 0 : sq < 5 ? 1 : 2, g = sq < 3 ? 1 + sq : sq < 5 ? sq - 1 : 3;      // (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
+      s_s[(r0 + 4 * T + ((x >> 2) & 3)) * SPITCH + r0 + 4 * g + (x & 3)] = 0.f;
     }
   }
   __syncthreads();
