@@ -136,7 +136,8 @@ def test_linear_f32_rows_do_not_depend_on_the_batch(K):
 @pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 131])
 @pytest.mark.parametrize("n,k", [(64, 1024), (65, 1056), (2048, 1024), (7, 2048), (130, 2081), (64, 4100)])
 def test_linear_f32_tiles_and_stretches(K, m, n, k):
-    """Tiles of 16, 32 and 64 rows with remainders, K in one, two and four stretches, rows at odd words, rows that lie apart.
+    """Tiles of 16 to 128 rows with remainders, in either form (matrices of 64 outputs and K of 1,024 on in whole 16-byte words go to the
+    tensor cores), K in several stretches, rows at odd words, rows that lie apart.
     An element's error: its chains are 16 products long, then about k / 32 sums, each a rounding of 2^-24 of the partial sum."""
     wide, w = rnd(m, k + 3, seed=1), rnd(n, k, seed=2, scale=0.1)
     b = rnd(n, seed=3)
@@ -166,6 +167,18 @@ def test_linear_f32_on_tensor_cores(K, n, k):
             assert torch.equal(out[:1], full[:1]) and torch.equal(K.linear_f32(x[-1:], w), out[-1:])
     out = K.linear_f32(wide[:40, :k], w, b, "gelu")
     torch.testing.assert_close(out.double().cpu(), plain.activation((ref[:40] + b.double()).cpu(), "gelu"), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 131])
+@pytest.mark.parametrize("n,k", [(40, 1024), (63, 1500), (130, 1027), (300, 2047), (33, 4100), (2100, 1026), (12, 2048)])
+def test_linear_f32_multiply_adds_in_stretches(K, m, n, k):
+    """What stays with the multiply-adds (fewer than 64 outputs, or rows that are no whole 16-byte words), K in one, two and four stretches
+    among a cluster, copies of 4 and of 16 bytes. Bound: test_linear_f32_tiles_and_stretches."""
+    wide, w = rnd(m, k + 4, seed=1), rnd(n, k, seed=2, scale=0.1)
+    for x in (wide[:, :k], wide[:, :k].contiguous()):
+        ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+        assert ((K.linear_f32(x, w).double() - ref).abs() <= (16 + k / 32 + 6) * 2.0 ** -24 * size).all()
+    assert torch.equal(K.linear_f32(wide[-1:, :k], w), K.linear_f32(wide[:, :k], w)[-1:])
 
 
 def test_linear_f32_of_values_without_three_terms(K):
