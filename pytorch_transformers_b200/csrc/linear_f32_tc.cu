@@ -2,10 +2,15 @@
 //
 // Every operand value is three bfloat16 terms that hold all its 24 bits, x = x1 + x2 + x3 (each the rounding of what the ones before
 // leave), and a product is the six products of terms down to 2^-18 of it: x3 w1, x1 w3, x2 w2, x2 w1, x1 w2, x1 w1. What is left
-// out is below 2^-26. The tensor core cuts its running sums off instead of rounding them, so it sums 32 values of k only, from
-// zero, the small products first; these sums are added in float32 registers with rounded additions, a stretch of K after the other. The stretches
-// follow from N and K alone and join in order, whoever forms them: a row's result depends neither on the other rows nor on the
-// tile. Off 64 bits (2-norm, normal values, K 512 to 18,176): 0.85e-7 to 1.9e-7, where float32 FMAs in two chains of 16 are 1.1e-7 to 2.3e-7.
+// out is 2^-27.5 of a product (root mean square) and at most 2^-24. The tensor core cuts its running sums off instead of rounding them, so it
+// sums 32 values of k only, from zero, the small products first; these sums are added in float32 registers with rounded additions, a
+// stretch of K after the other. A sum is 5.1e-8 of itself too small on average, whatever the values (every cut is towards zero), so that share of
+// the result is put back where the stretches' totals join, exactly up to one rounding. The stretches follow from N and K alone and join in order,
+// whoever forms them: a row's result depends neither on the other rows nor on the tile. As many as the multiply-adds of
+// linear_f32.cu take, or more: a stretch is a chain of roundings. 2-norm off 64 bits in 1e-7, multiply-adds in brackets, normal values and ones
+// between 0 and 1: 1,024 x 1,024 0.71 (1.13) and 0.35 (0.53), 9,216 x 4,096 1.14 (1.38) and 0.48 (0.55), 1,536 x 6,144 1.36 (1.56) and 0.57 (0.65),
+// 65,024 x 4,544 1.20 (1.43) and 0.56 (0.62), 4,544 x 18,176 1.83 (2.35) and 0.68 (0.99). Before, with one or two stretches of a wide
+// matrix and nothing put back, 2.13 and 1.59 at 9,216 x 4,096.
 //
 // A block owns 128 outputs (the M side of tcgen05.mma) x BN rows:
 //   8 warps      take the operands apart: 32-byte words of both matrices from global memory into registers, a stage of 64 k (two of them
@@ -34,6 +39,7 @@ constexpr int FM = 128;                       // outputs of a tile: M of the mat
 constexpr int FK = 64;                        // k of a stage: 128 bytes of bfloat16, one swizzle row
 constexpr int FSUB = 32;                      // k that the tensor core sums
 constexpr int F_CONV = 256, F_ISSUE = FK / FSUB;      // threads that take operands apart, warps that issue
+constexpr float F_CUT = 5.1e-8f;              // what a sum of FSUB loses by being cut, of itself, on average (measured: 0.51 to 0.52)
 constexpr int F_TERM = FM * FK * 2;           // bytes of one term of a stage's matrix rows
 
 struct LinearF32Params {
@@ -41,7 +47,7 @@ struct LinearF32Params {
   float* y;
   int* error_flag;
   int M, N, K, ldx, act;
-  int stretches, stretch_steps;               // K in `stretches` stretches of so many stages, divided evenly among a cluster's blocks
+  int stretches;                              // of K, even but for one stage, divided evenly among a cluster's blocks
   int w_vec, x_vec;                           // floats of a load
 };
 
@@ -125,6 +131,13 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
                ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
 }
+// The stretches' totals join exactly, as hi + lo (Knuth's sum of two), and round once, with what their sums have lost by being cut
+__device__ __forceinline__ void join(float& hi, float& lo, float t) {
+  const float s = hi + t, b = s - hi;
+  lo += (hi - (s - b)) + (t - b);
+  hi = s;
+}
+__device__ __forceinline__ float joined(float hi, float lo) { return hi + fmaf(hi, F_CUT, lo); }
 // v[i] += column i of tensor memory, N a multiple of 8
 template <int N>
 __device__ __forceinline__ void tmem_add(uint32_t taddr, float (&v)[N]) {
@@ -139,6 +152,28 @@ __device__ __forceinline__ void tmem_add(uint32_t taddr, float (&v)[N]) {
     for (int j = 0; j < S; ++j) v[g + j] += __uint_as_float(r[j / 8][j % 8]);
   }
 }
+// v joins the totals in columns 0 .. N of tensor memory (hi) and lo_at .. (lo); LAST: v becomes their sum
+template <bool LAST, int N>
+__device__ __forceinline__ void tmem_join(uint32_t taddr, int lo_at, float (&v)[N]) {
+#pragma unroll
+  for (int g = 0; g < N; g += 8) {
+    uint32_t h[8], l[8];
+    tmem_ld8_nowait(taddr + g, h);
+    tmem_ld8_nowait(taddr + lo_at + g, l);
+    tmem_ld_wait();
+    float hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      hi[j] = __uint_as_float(h[j]), lo[j] = __uint_as_float(l[j]);
+      join(hi[j], lo[j], v[g + j]);
+      if (LAST) v[g + j] = joined(hi[j], lo[j]);
+    }
+    if (!LAST) {
+      tmem_st8(taddr + g, hi);
+      tmem_st8(taddr + lo_at + g, lo);
+    }
+  }
+}
 
 template <int BN>
 struct LinearF32Tile {
@@ -146,7 +181,7 @@ struct LinearF32Tile {
   static constexpr int STAGES = BN <= 64 ? 3 : 2;
   static constexpr int SUMS = BN <= 64 ? 128 : 256, THREADS = F_CONV + SUMS + 32 * F_ISSUE;      // up to 16 warps leave 128 registers a thread
   static constexpr int SMEM = 1024 + STAGES * STAGE;
-  static constexpr int COLS = 4 * BN;      // two sums in turn and a total; a power of two
+  static constexpr int COLS = 4 * BN;      // two sums in turn, the stretches' totals in hi and lo
 };
 
 template <int BN, bool WIDE>
@@ -183,7 +218,8 @@ linear_f32_tc_kernel(const LinearF32Params p) {
   const uint32_t tmem_base = tmem_slot;
   // this block's stretches and their stages
   const int total = (p.K + FK - 1) / FK, ranks = int(gridDim.z), rank = int(blockIdx.z), own = p.stretches / ranks;
-  const int first = min(total, rank * own * p.stretch_steps), last = min(total, (rank + 1) * own * p.stretch_steps);
+  auto stretch_at = [&](int j) { return int((long long)j * total / p.stretches); };
+  const int first = stretch_at(rank * own), last = stretch_at((rank + 1) * own);
   const int steps = last - first, whole = p.K / FK;
 
   if (warp < F_CONV / 32) {
@@ -268,25 +304,31 @@ linear_f32_tc_kernel(const LinearF32Params p) {
     for (int j = 0; j < own; ++j) {
 #pragma unroll
       for (int e = 0; e < SC; ++e) acc[e] = 0.f;
-      const int s0 = min(total, (rank * own + j) * p.stretch_steps), s1 = min(total, (rank * own + j + 1) * p.stretch_steps);
+      const int s0 = stretch_at(rank * own + j), s1 = stretch_at(rank * own + j + 1);
       for (int i = s0; i < s1 && alive; ++i, ++n)
 #pragma unroll 1
         for (uint32_t buf = 0; buf < F_ISSUE; ++buf) {
           alive = mbar_wait(done0 + 8 * buf, n & 1, p.error_flag, 44);
           if (!alive) break;
           tc_fence_after();
-          tmem_add<SC>(lane_addr + buf * BN, acc);
+          tmem_add(lane_addr + buf * BN, acc);
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(read0 + 8 * buf);
         }
       // the stretches' totals join in order: in one block as they come, waiting in tensor memory; of a cluster's blocks at the end
-      if (j > 0 && ranks == 1) tmem_add<SC>(lane_addr + 2 * BN, acc);
-      if (j + 1 < own) {
+      const uint32_t totals = lane_addr + 2 * BN;
+      if (j == 0 && own > 1) {
 #pragma unroll
-        for (int e = 0; e < SC; e += 8) tmem_st8(lane_addr + 2 * BN + e, acc + e);
-        tmem_st_wait();
+        for (int e = 0; e < SC; e += 8) tmem_st8(totals + e, acc + e);
+        const float none[8] = {};
+#pragma unroll
+        for (int e = 0; e < SC; e += 8) tmem_st8(totals + BN + e, none);
+      } else if (ranks == 1) {
+        if (j + 1 < own) tmem_join<false>(totals, BN, acc);
+        else tmem_join<true>(totals, BN, acc);
       }
+      tmem_st_wait();
     }
     // the ring is free: the last sums are complete, so its last stage has been read. Results leave through it, in a loop of all threads: the
     // activations written out for every register of a tile would be more code than the instruction cache holds
@@ -297,7 +339,7 @@ linear_f32_tc_kernel(const LinearF32Params p) {
     if (tiles == 2) {
 #pragma unroll
       for (int e = 0; e < SC; ++e) acc[e] = 0.f;
-      tmem_add<SC>(lane_addr + 2 * BN, acc);
+      tmem_add(lane_addr + 2 * BN, acc);
 #pragma unroll
       for (int e = 0; e < SC; ++e) tile[(half * SC + e) * FM + row - BN * FM] = acc[e];
     }
@@ -310,10 +352,15 @@ linear_f32_tc_kernel(const LinearF32Params p) {
     for (int at = rank * T::THREADS + tid; at < BN * FM; at += ranks * T::THREADS) {
       const int m = m0 + at / FM, n = n0 + at % FM;
       if (m >= p.M || n >= p.N) continue;
-      float v = 0.f;
-      if (ranks == 1) v = tile[at];
-      else
-        for (int s = 0; s < p.stretches; ++s) v += *cluster.map_shared_rank(tile + s % own * BN * FM + at, s / own);
+      float v;
+      if (ranks == 1) {
+        v = tile[at];
+      } else {
+        float lo = 0.f;
+        v = 0.f;
+        for (int s = 0; s < p.stretches; ++s) join(v, lo, *cluster.map_shared_rank(tile + s % own * BN * FM + at, s / own));
+        v = joined(v, lo);
+      }
       finish_f32(p, m, n, v);
     }
     cluster.sync();       // no block leaves while its tile is still read
@@ -358,13 +405,15 @@ int linear_f32_tensor(const float* x, const float* w, const float* bias, float* 
   // Stretches of K, by N and K alone: a row's sums must not follow the number of rows. As many as blocks of a cluster may share a
   // matrix of few tiles, each of four stages at least (clusters of four blocks: 33 are resident at a time with a block an SM, of three 44,
   // of two 70 and more; 36 clusters of four are two waves: 4,544 x 18,176 and one row 157 us, in clusters of three 108), and then as many as keep
-  // a stretch at 64 stages or fewer, since each of its 128 additions rounds (one cluster's block holds two at most).
+  // a stretch at 64 stages or fewer, at least two, from K of 2,048 on four, since each of its additions rounds (one cluster's block holds two
+  // at most). A stretch more costs a block its totals' way through tensor memory: 700 rows, one or two and now, 4,096 x 1,024 82 -> 86 us,
+  // 9,216 x 4,096 362 -> 354.
   const int shared = tiles <= 33 ? 4 : tiles <= 44 ? 3 : tiles <= 70 ? 2 : 1;
   int most = shared;
   while (most > 1 && total / most < 4) --most;
-  const int each = (total + 64 * most - 1) / (64 * most);
+  const int least = total >= 32 ? 4 : 2;
+  const int each = max((total + 64 * most - 1) / (64 * most), (least + most - 1) / most);
   p.stretches = most * (most > 1 && each > 2 ? 2 : each);
-  p.stretch_steps = (total + p.stretches - 1) / p.stretches;
   const bool wide = p.w_vec == 8 && p.x_vec == 8 && K % FK == 0;
   // Rows of a tile: as few as hold them all, then 128. Blocks that share a tile: as many as may where all of them are resident, else two
   // (two stretches each) or one. us at 700 rows, one block a tile against what is taken: 1,024 x 4,096 139 and 76, 1,024 x 1,024 67 and 35.
