@@ -2,14 +2,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-// one output from the values themselves: ascending k, IEEE multiply-adds
-__device__ __forceinline__ float linear_f32_plain_dot(const float* x, const float* w, int K) {
-  float s = 0.f;
-#pragma unroll 1
-  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
-  return s;
-}
-
 // arguments as ptb_linear_f32 takes them; rows of w at whole 16-byte words
 int linear_f32_tensor(const float* x, const float* w, const float* bias, float* y, int M, int N, int K, int ldx, int act,
                       int* error_flag, cudaStream_t stream);

@@ -121,11 +121,27 @@ __device__ __forceinline__ void issue_terms(uint32_t acc, uint64_t a, uint32_t i
     }
   }
 }
-// infinities and NaN have no three terms: a sum that is none is formed again from the values themselves
-__device__ __forceinline__ void finish_f32(const LinearF32Params& p, int m, int n, float v) {
-  if (!(fabsf(v) <= 3.402823466e38f)) v = linear_f32_plain_dot(p.x + size_t(m) * p.ldx, p.w + size_t(n) * p.K, p.K);
-  if (p.bias) v += p.bias[n];
-  p.y[size_t(m) * p.N + n] = apply_activation(v, p.act);
+// A warp's 32 results of row m, outputs n .. n + 31, from its sums. Infinities and NaN have no three
+// terms: a sum that is no number is formed again from the values themselves, by the whole warp.
+__device__ __forceinline__ void finish_f32(const LinearF32Params& p, int m, int n, float v, int lane) {
+  uint32_t again = __ballot_sync(0xffffffffu, n + lane < p.N && !(fabsf(v) <= 3.402823466e38f));
+  while (again) {
+    const int from = __ffs(again) - 1;
+    again &= again - 1;
+    const float *x = p.x + size_t(m) * p.ldx, *w = p.w + size_t(n + from) * p.K;
+    float s = 0.f;
+    for (int k0 = lane; k0 < p.K; k0 += 16 * 32) {      // chains of 16
+      float t = 0.f;
+      for (int k = k0; k < min(p.K, k0 + 16 * 32); k += 32) t = fmaf(x[k], w[k], t);
+      s += t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == from) v = s;
+  }
+  if (n + lane >= p.N) return;
+  if (p.bias) v += p.bias[n + lane];
+  p.y[size_t(m) * p.N + n + lane] = apply_activation(v, p.act);
 }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
@@ -350,8 +366,8 @@ linear_f32_tc_kernel(const LinearF32Params p) {
     const float* tile = reinterpret_cast<const float*>(ring);
 #pragma unroll 1
     for (int at = rank * T::THREADS + tid; at < BN * FM; at += ranks * T::THREADS) {
-      const int m = m0 + at / FM, n = n0 + at % FM;
-      if (m >= p.M || n >= p.N) continue;
+      const int m = m0 + at / FM, n = n0 + (at - lane) % FM;      // a warp's are of one row
+      if (m >= p.M) continue;
       float v;
       if (ranks == 1) {
         v = tile[at];
@@ -361,7 +377,7 @@ linear_f32_tc_kernel(const LinearF32Params p) {
         for (int s = 0; s < p.stretches; ++s) join(v, lo, *cluster.map_shared_rank(tile + s % own * BN * FM + at, s / own));
         v = joined(v, lo);
       }
-      finish_f32(p, m, n, v);
+      finish_f32(p, m, n, v, lane);
     }
     cluster.sync();       // no block leaves while its tile is still read
   }
