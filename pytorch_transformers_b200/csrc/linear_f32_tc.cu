@@ -39,6 +39,7 @@ constexpr int FM = 128;                       // outputs of a tile: M of the mat
 constexpr int FK = 64;                        // k of a stage: 128 bytes of bfloat16, one swizzle row
 constexpr int FSUB = 32;                      // k that the tensor core sums
 constexpr int F_CONV = 256, F_ISSUE = FK / FSUB;      // threads that take operands apart, warps that issue
+constexpr float F_SCALE = 131072.f;           // 2^17, of both operands
 constexpr float F_CUT = 5.1e-8f;              // what a sum of FSUB loses by being cut, of itself, on average (measured: 0.51 to 0.52)
 constexpr int F_TERM = FM * FK * 2;           // bytes of one term of a stage's matrix rows
 
@@ -68,7 +69,13 @@ __device__ __forceinline__ void load8(float (&f)[8], const float* p, int vec) {
   }
 }
 
-// the three terms of two values, packed
+// the three terms of two values times F_SCALE, packed
+__device__ __forceinline__ void scale2(float& x, float& y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
+  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(v) : "l"(0x4800000048000000ull));
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v));
+}
 __device__ __forceinline__ void minus2(float& x, float& y, uint32_t pair) {      // x - low half, y - high half
   unsigned long long v, t;
   asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
@@ -77,6 +84,7 @@ __device__ __forceinline__ void minus2(float& x, float& y, uint32_t pair) {     
   asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v));
 }
 __device__ __forceinline__ void three_terms(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
+  scale2(x, y);
   a = pack_bf16(x, y);
   minus2(x, y, a);
   b = pack_bf16(x, y);
@@ -121,10 +129,11 @@ __device__ __forceinline__ void issue_terms(uint32_t acc, uint64_t a, uint32_t i
     }
   }
 }
-// A warp's 32 results of row m, outputs n .. n + 31, from its sums. Infinities and NaN have no three
+// A warp's 32 results of row m, outputs n .. n + 31, from the scaled sums. Infinities, NaN and what leaves float32 by the scale have no three
 // terms: a sum that is no number is formed again from the values themselves, by the whole warp.
 __device__ __forceinline__ void finish_f32(const LinearF32Params& p, int m, int n, float v, int lane) {
   uint32_t again = __ballot_sync(0xffffffffu, n + lane < p.N && !(fabsf(v) <= 3.402823466e38f));
+  v *= 1.f / (F_SCALE * F_SCALE);
   while (again) {
     const int from = __ffs(again) - 1;
     again &= again - 1;

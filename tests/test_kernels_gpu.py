@@ -230,9 +230,19 @@ def test_linear_f32_multiply_adds_in_stretches(K, m, n, k):
     assert torch.equal(K.linear_f32(wide[-1:, :k], w), K.linear_f32(wide[:, :k], w)[-1:])
 
 
+@pytest.mark.parametrize("scale", [1e-30, 1e-33, 1e-36, 1e-38, 1e34])
+@pytest.mark.parametrize("n,k", [(1024, 1024), (640, 4096)])
+def test_linear_f32_of_small_and_large_numbers(K, n, k, scale):
+    """Down to numbers without a leading one (1e-38) and up to where the scale of the terms leaves float32: no further off than
+    multiply-adds. A third term without that scale would lie under bfloat16's smallest number from 1e-33 down."""
+    for x, w in ((rnd(40, k, seed=1) * scale, rnd(n, k, seed=2)), (rnd(40, k, seed=1), rnd(n, k, seed=2) * scale)):
+        ref = x.double() @ w.double().T
+        assert norm_error(K.linear_f32(x, w), ref) <= norm_error(multiply_adds(x, w, n), ref)
+
+
 def test_linear_f32_of_values_without_three_terms(K):
     """Infinities, NaN, values that round to an infinity in bfloat16 and products beyond float32: what float32 multiply-adds give. Small
-    normal numbers keep their bits."""
+    numbers: the test above."""
     x, w = rnd(20, 1024, seed=1), rnd(70, 1024, seed=2)
     x[3, 7], x[5, 9], x[6, 1], x[7, 2] = math.inf, math.nan, 3.4e38, -3.4e38
     w[11, 7], w[12, 1], w[13, 30] = 0.0, 0.5, -math.inf
