@@ -11,10 +11,10 @@
 // the state's float32 values in registers, one product [M; Q] S_0 a chunk, and writes the outputs.
 //
 // No factor can grow: inside a sub-block of 16 tokens sums of logarithms start at the sub-block, the exponent between two
-// sub-blocks is the rest of the earlier one, the whole ones between and the beginning of the later one, and inside a
-// sub-block the exponent of every pair of tokens is formed by itself. Float32 operands (the state, decayed keys and
-// queries, T, P, W, U_0) enter the products split in two bfloat16 terms, hi hi + hi lo + lo hi; projections are bfloat16 as
-// they are, their unit norms factors of the results.
+// sub-blocks is the rest of the earlier one, the whole ones between and the beginning of the later one; a sub-block's halves of 8
+// meet in the same way at their border, and inside a half the exponent of every pair of tokens is formed by itself. Float32 operands (the
+// state, decayed keys and queries, T, P, W, U_0) enter the products split in two bfloat16 terms, hi hi + hi lo + lo hi, but for
+// the scores inside a sub-block, which keep 32 bits; projections are bfloat16 as they are, their unit norms factors of the results.
 #include "chunk_mma.cuh"
 
 namespace {
@@ -85,7 +85,7 @@ struct LocalSmem {
 // phases are short chains between barriers (decay per channel, 128 x 128: 42,000 clocks a block, of them scores 12,000, products 14,000,
 // loads 5,400, the inverse with the decayed keys 5,000 and its join 4,000; 79,400 before). So the scores' work is divided by count of
 // instructions over all warps: a pair of sub-blocks' keys and queries take the same exponentials and the same decayed keys, halves of a sub-block
-// meet by a product too, which leaves 288 pairs of tokens with exponents of their own of 544; totals before and after a sub-block are
+// meet by a product too (in three terms), which leaves 288 pairs of tokens with exponents of their own of 544; totals before and after a sub-block are
 // kept instead of summed at every use; decayed keys are formed four channels a lane (one channel's neighbours in a lane met the
 // same bank eight times); the inverse joins 16 below 16, then 32 below 32, from rows in 16-byte words. 2,048 tokens of 16 heads of
 // 128 x 128, both passes 222 -> 171 us (this one 153 -> 102).
@@ -318,12 +318,15 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
         for (int nt = 0; nt < 2; ++nt) put_scores(i, j, nt, l[nt], q[nt], [](int, int) { return 1.f; });
       }
     }
+    // The nearest tokens' scores keep 32 bits, as inside a half: operands of three terms, the six products of 16 channels from zero, the
+    // small ones first (a matrix instruction cuts its sum off), and rounded additions of these. With two terms a score was 4.5e-6 off 64
+    // bits, and a sub-block's outputs 5.9e-6 where they are 5.2e-6 (the products after the scores); the layer took 296.7 us, now 298.2.
     auto halves_meet = [&](int b) {
       float acc[4] = {};      // rows 0 - 7: L, rows 8 - 15: P
       const int row = b * 16 + 8 + g4, col = b * 16 + g4, edge = b * 16 + 7;
-#pragma unroll 2
+#pragma unroll 1
       for (int kk = 0; kk < DK / 16; ++kk) {
-        uint32_t ah[4], al[4], bh[2], bl[2];
+        uint32_t a1[4], a2[4], a3[4], b1[2], b2[2], b3[2];
 #pragma unroll
         for (int f = 0; f < 2; ++f) {
           const int d = kk * 16 + t4 * 2 + f * 8;
@@ -331,15 +334,21 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
           float2 e = *reinterpret_cast<const float2*>(cb + row * CP + d);
           e.x = fast_exp2(e.x - m.x), e.y = fast_exp2(e.y - m.y);
           const uint32_t wk = *reinterpret_cast<const uint32_t*>(ks + row * KP + d), wq = *reinterpret_cast<const uint32_t*>(qs + row * KP + d);
-          split_pack(__uint_as_float(wk << 16) * e.x, __uint_as_float(wk & 0xffff0000u) * e.y, ah[2 * f], al[2 * f]);
-          split_pack(__uint_as_float(wq << 16) * e.x, __uint_as_float(wq & 0xffff0000u) * e.y, ah[2 * f + 1], al[2 * f + 1]);
+          split3_pack(__uint_as_float(wk << 16) * e.x, __uint_as_float(wk & 0xffff0000u) * e.y, a1[2 * f], a2[2 * f], a3[2 * f]);
+          split3_pack(__uint_as_float(wq << 16) * e.x, __uint_as_float(wq & 0xffff0000u) * e.y, a1[2 * f + 1], a2[2 * f + 1], a3[2 * f + 1]);
           const uint32_t w = *reinterpret_cast<const uint32_t*>(ks + col * KP + d);
           const float2 o = *reinterpret_cast<const float2*>(cb + col * CP + d);
-          split_pack(__uint_as_float(w << 16) * fast_exp2(m.x - o.x), __uint_as_float(w & 0xffff0000u) * fast_exp2(m.y - o.y), bh[f], bl[f]);
+          split3_pack(__uint_as_float(w << 16) * fast_exp2(m.x - o.x), __uint_as_float(w & 0xffff0000u) * fast_exp2(m.y - o.y), b1[f], b2[f], b3[f]);
         }
-        mma_bf16(acc, ah, bh[0], bh[1]);
-        mma_bf16(acc, ah, bl[0], bl[1]);
-        mma_bf16(acc, al, bh[0], bh[1]);
+        float x[4] = {};
+        mma_bf16(x, a3, b1[0], b1[1]);
+        mma_bf16(x, a1, b3[0], b3[1]);
+        mma_bf16(x, a2, b2[0], b2[1]);
+        mma_bf16(x, a2, b1[0], b1[1]);
+        mma_bf16(x, a1, b2[0], b2[1]);
+        mma_bf16(x, a1, b1[0], b1[1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] += x[e];
       }
       const int c0 = b * 16 + t4 * 2;
       const float w = rk[row] * bt[row];

@@ -328,6 +328,27 @@ def test_chunks_on_the_tensor_cores_against_the_walk_and_the_plain_rule(H, G, d,
             assert (rule.left(cache, slot) - S2).norm() < limit * S2.norm()
 
 
+@pytest.mark.parametrize("d,vd", [(128, 128), (64, 64), (64, 128)])
+@pytest.mark.parametrize("strength", [0.01, 0.3])
+def test_scores_between_the_halves_of_a_sub_block_in_32_bits(d, vd, strength):
+    """One token a sequence writes a value, and the eight tokens of the sub-block's later half answer with it times their score alone: off by the
+    two terms that a score is kept in afterwards, not by what terms of its operands leave out. Two terms: the first one's rest is evenly spread up
+    to 2^-8, the second one's up to 2^-8 of that rest's power of two, whose mean square is 1 / 7: 2^-16 / sqrt(7 * 3) = 3.3e-6."""
+    n, seqs, H = 16, 12, 4
+    g = torch.Generator().manual_seed(d + vd)
+    ld = -strength * torch.rand(n * seqs, H * d, generator=g)
+    beta = torch.zeros(n * seqs, H)
+    for i in range(seqs):
+        beta[i * n + i % 8] = 1.0
+    rule = Rule(torch.randn(n * seqs, H, d, generator=g), torch.randn(n * seqs, H, d, generator=g), torch.randn(n * seqs, H, vd, generator=g),
+                ld, beta, "bfloat16")
+    cache = rule.cache(seqs)
+    spans = [(i * n, (i + 1) * n) for i in range(seqs)]
+    got = torch.cat([o[8:] for o in rule.run(cache, [cache.open() for _ in spans], spans, True)])
+    ref = torch.cat([rule.reference(a, b)[0].reshape(n, -1)[8:] for a, b in spans])
+    assert (got - ref).norm() < 2.0 ** -16 / 21 ** 0.5 * ref.norm()
+
+
 @pytest.mark.parametrize("dtype,chunked", [("float32", False), ("bfloat16", False), ("bfloat16", True)])
 @pytest.mark.parametrize("n,back", [(700, 650), (300, 299), (130, 64), (65, 63), (17, 16), (16, 15), (40, 3), (2, 1), (1, 0)])
 def test_a_far_key_on_an_open_channel_and_on_a_closed_one(n, back, dtype, chunked):
