@@ -3,8 +3,8 @@
 //
 // The sums of one output element: the k of a step of 32 are summed in two chains (even and odd k, 16 products each, ascending),
 // the two chains join and go into a running total; a K of 2,048 or more is cut into four stretches whose totals are added in
-// order, a K of 1,024 to 2,047 beside fewer than 2,048 outputs into two, any other into none. All of this follows from N and K alone, so a row's result depends neither on how many other rows are in the
-// launch nor on the tile, and the rounding error stays small for K in the tens of thousands.
+// order, a K of 1,024 to 2,047 beside fewer than 2,048 outputs into two, any other into none. All of this follows from N and K alone, so a
+// row's result depends neither on how many other rows are in the launch nor on the tile, and the rounding error stays small for K in the tens of thousands.
 //
 // What bounds it is the FMA pipe (128 lanes an SM). A block owns 8 TM rows x 64 outputs, a thread TM x 4 of them: of every
 // 16 bytes that it reads from shared memory (operands stay in [row][k] order, so cp.async brings them without a
@@ -12,10 +12,10 @@
 // 2 TM x 4 / (TM + 4) two-wide FMAs (fma.rn.f32x2: the two k chains in one 64-bit register). A three-stage ring keeps two
 // steps of copies in flight. Few rows or few outputs would leave SMs idle: K is cut among a thread-block cluster whose blocks
 // join their tiles through distributed shared memory.
-// One B200: the four products of a block of width 1,024 on 700 rows 1,057 -> 517 us (700 x 1,024 x 4,096: 152 us, 39 TFLOP/s of
-// 72; 2,048 rows: 43), 20 rows of 1,024 x 4,096 30 us; before, 64 x 64 tiles with two scalar loads a product and no copies in
-// flight. Now the two-wide FMAs of three blocks an SM leave half of the issue slots empty: registers (168 a thread) allow no more
-// warps, and tiles of 8 x 8 a thread, which read less, were as fast (43) at 2,048 rows and slower below.
+// One B200, 700 rows: 40 x 4,096 165 us without stretches, 50 with four; 1,000 x 2,050 132 us; 9,001 x 4,545 1.95 ms (29 TFLOP/s of 72; rows that
+// are no whole 16-byte words come in 4-byte copies). What linear_f32_tc.cu takes now ran here at 39 TFLOP/s (700 x 1,024 x 4,096:
+// 152 us): two-wide FMAs of three blocks an SM leave half of the issue slots empty, registers (168 a thread) allow no more
+// warps, and tiles of 8 x 8 a thread, which read less, were as fast at 2,048 rows and slower below.
 #include <cooperative_groups.h>
 
 #include "linear_f32.cuh"
@@ -183,12 +183,11 @@ PTB_API int ptb_linear_f32(const float* x, const float* w, const float* bias, fl
   // 14 and 17 for 700; 64 x 1,024: 16 and 12, 33 and 23; 256 x 256: 10 and 12, 18 and 23; 512 x 512: 16 and 13, 29 and 27.
   if (K % 4 == 0 && aligned16(w) && ((N >= 64 && K >= 1024) || (N >= 512 && K >= 256)))
     return linear_f32_tensor(x, w, bias, y, M, N, K, ldx, act, error_flag, stream);
-  // stretches of K, by N and K alone (the order of a row's sums must not follow the number of rows). A matrix of 1,024 outputs
-  // and 700 rows has 176 tiles, little more than an SM each, which stretches even out; with one row it has 16. us for one,
-  // two and four stretches: 1 row, N 1,024 K 4,096: 73, 39, 21; 4,096 x 2,048: 38, 22, 17; 18,176 x 4,544: 120, 119, 120. 700
-  // rows, 1,024 x 1,024: 67, 55, 52; 1,024 x 4,096: 256, 189, 181; 2,048 x 2,048: 184, 158, 170; 4,096 x 2,048: 295, 301, 316;
-  // 4,544 x 18,176: 3,047, 2,747, 2,835; 18,176 x 4,544: 2,701, 2,674, 2,852. So long K gains most where rows or outputs are
-  // few, and from some 8,192 outputs on the join costs 3 to 10 % on many rows and gives nothing back on few.
+  // Stretches of K, by N and K alone (the order of a row's sums must not follow the number of rows). us for one, two and four, of
+  // matrices that stay here: 1 row, 40 x 4,096 78, 43, 25; 1,000 x 1,026 33, 23, 16; 4,097 x 2,050 57, 35, 29; 9,000 x 1,026 33, 29, 37; 9,001 x 4,545
+  // 119, 91, 109. 700 rows, 40 x 4,096 165, 92, 50; 1,000 x 1,026 94, 76, 80; 1,000 x 2,050 177, 132, 132; 2,100 x 1,026 126, 121, 139; 4,098 x 1,030
+  // 206, 223, 252; 4,097 x 2,050 388, 401, 436; 18,177 x 4,545 3,673, 3,656, 3,893. So long K gains most where rows or outputs are few, and from
+  // some 2,048 outputs on the join costs many rows 3 to 12 %, which K of 2,048 and more pays for shorter chains of roundings.
   const int ranks = K >= 2048 ? 4 : (K >= 1024 && N < 2048) ? 2 : 1;
   // 16-byte copies where every row starts at a whole word
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && aligned16(x) && aligned16(w);

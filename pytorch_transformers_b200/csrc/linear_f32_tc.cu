@@ -5,12 +5,13 @@
 // out is 2^-27.5 of a product (root mean square) and at most 2^-24. The tensor core cuts its running sums off instead of rounding them, so it
 // sums 32 values of k only, from zero, the small products first; these sums are added in float32 registers with rounded additions, a
 // stretch of K after the other. A sum is 5.1e-8 of itself too small on average, whatever the values (every cut is towards zero), so that share of
-// the result is put back where the stretches' totals join, exactly up to one rounding. The stretches follow from N and K alone and join in order,
-// whoever forms them: a row's result depends neither on the other rows nor on the tile. As many as the multiply-adds of
+// the result is put back where the last stretch's total joins the others, exactly up to one rounding. The stretches follow from N and K alone and
+// join in order, whoever forms them: a row's result depends neither on the other rows nor on the tile. They are as many as the multiply-adds of
 // linear_f32.cu take, or more: a stretch is a chain of roundings. 2-norm off 64 bits in 1e-7, multiply-adds in brackets, normal values and ones
-// between 0 and 1: 1,024 x 1,024 0.71 (1.13) and 0.35 (0.53), 9,216 x 4,096 1.14 (1.38) and 0.48 (0.55), 1,536 x 6,144 1.36 (1.56) and 0.57 (0.65),
-// 65,024 x 4,544 1.20 (1.43) and 0.56 (0.62), 4,544 x 18,176 1.83 (2.35) and 0.68 (0.99). Before, with one or two stretches of a wide
-// matrix and nothing put back, 2.13 and 1.59 at 9,216 x 4,096.
+// between 0 and 1: 1,024 x 1,024 0.78 (1.13) and 0.43 (0.53), 9,216 x 4,096 1.19 (1.38) and 0.54 (0.55), 1,536 x 6,144 1.39 (1.56) and 0.64 (0.65),
+// 65,024 x 4,544 1.24 (1.43) and 0.62 (0.62), 4,544 x 18,176 1.88 (2.35) and 0.74 (0.99). Before, with one or two stretches of a wide
+// matrix and nothing put back, 2.13 and 1.59 at 9,216 x 4,096. (Every join exact, with its rest kept: 0.71 and 0.35 at 1,024 x 1,024, but 45 us
+// where 700 rows of 3,072 x 1,024 take 43. Both sums of a stage added to each other first: 0.75 and 0.44, 49 us, as nothing is summed meanwhile.)
 //
 // A block owns 128 outputs (the M side of tcgen05.mma) x BN rows:
 //   8 warps      take the operands apart: 32-byte words of both matrices from global memory into registers, a stage of 64 k (two of them
@@ -22,8 +23,8 @@
 // the terms' stores are 96 KB and the loads through L1 64 KB, 2,816 clocks at 128 bytes; the instructions themselves are 1,536. With few
 // rows it is the matrix's way from memory. Results leave through shared memory in a loop, whose activations and re-sum of what is no number
 // would else be written out for every register, more than the instruction cache holds (block below 379 -> 330 us).
-// One B200: the four products of a block of width 1,024 on 700 rows 517 -> 220 us (700 x 1,024 x 4,096: 152 -> 80), 2,048 rows of
-// 4,096 x 2,048 880 -> 262 us (131 TFLOP/s), one row of 65,024 x 4,544 420 -> 300 us; before: float32 FMAs (linear_f32.cu). Pairs of
+// One B200: the four products of a block of width 1,024 on 700 rows 517 -> 226 us (700 x 1,024 x 4,096: 152 -> 76), 2,048 rows of
+// 4,096 x 2,048 880 -> 266 us (129 TFLOP/s), one row of 65,024 x 4,544 422 -> 285 us; before: float32 FMAs (linear_f32.cu). Pairs of
 // blocks on one instruction (two SMs, 256 outputs x 128 or 192 rows, half of the x rows each) were no faster: 344.
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -156,13 +157,11 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
                ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
 }
-// The stretches' totals join exactly, as hi + lo (Knuth's sum of two), and round once, with what their sums have lost by being cut
-__device__ __forceinline__ void join(float& hi, float& lo, float t) {
-  const float s = hi + t, b = s - hi;
-  lo += (hi - (s - b)) + (t - b);
-  hi = s;
+// The last stretch's total joins the ones before exactly (Knuth's sum of two) and rounds once, with what all sums have lost by being cut.
+__device__ __forceinline__ float join_last(float before, float last) {
+  const float s = before + last, b = s - before;
+  return s + fmaf(s, F_CUT, (before - (s - b)) + (last - b));
 }
-__device__ __forceinline__ float joined(float hi, float lo) { return hi + fmaf(hi, F_CUT, lo); }
 // v[i] += column i of tensor memory, N a multiple of 8
 template <int N>
 __device__ __forceinline__ void tmem_add(uint32_t taddr, float (&v)[N]) {
@@ -177,36 +176,13 @@ __device__ __forceinline__ void tmem_add(uint32_t taddr, float (&v)[N]) {
     for (int j = 0; j < S; ++j) v[g + j] += __uint_as_float(r[j / 8][j % 8]);
   }
 }
-// v joins the totals in columns 0 .. N of tensor memory (hi) and lo_at .. (lo); LAST: v becomes their sum
-template <bool LAST, int N>
-__device__ __forceinline__ void tmem_join(uint32_t taddr, int lo_at, float (&v)[N]) {
-#pragma unroll
-  for (int g = 0; g < N; g += 8) {
-    uint32_t h[8], l[8];
-    tmem_ld8_nowait(taddr + g, h);
-    tmem_ld8_nowait(taddr + lo_at + g, l);
-    tmem_ld_wait();
-    float hi[8], lo[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      hi[j] = __uint_as_float(h[j]), lo[j] = __uint_as_float(l[j]);
-      join(hi[j], lo[j], v[g + j]);
-      if (LAST) v[g + j] = joined(hi[j], lo[j]);
-    }
-    if (!LAST) {
-      tmem_st8(taddr + g, hi);
-      tmem_st8(taddr + lo_at + g, lo);
-    }
-  }
-}
-
 template <int BN>
 struct LinearF32Tile {
   static constexpr int X_TERM = BN * FK * 2, STAGE = 3 * (F_TERM + X_TERM);
   static constexpr int STAGES = BN <= 64 ? 3 : 2;
   static constexpr int SUMS = BN <= 64 ? 128 : 256, THREADS = F_CONV + SUMS + 32 * F_ISSUE;      // up to 16 warps leave 128 registers a thread
   static constexpr int SMEM = 1024 + STAGES * STAGE;
-  static constexpr int COLS = 4 * BN;      // two sums in turn, the stretches' totals in hi and lo
+  static constexpr int COLS = 4 * BN;      // two sums in turn, the stretches' total; a power of two
 };
 
 template <int BN, bool WIDE>
@@ -341,23 +317,17 @@ linear_f32_tc_kernel(const LinearF32Params p) {
           __syncwarp();
           if (lane == 0) mbar_arrive(read0 + 8 * buf);
         }
-      // the stretches' totals join in order: in one block as they come, waiting in tensor memory; of a cluster's blocks at the end
-      const uint32_t totals = lane_addr + 2 * BN;
-      if (j == 0 && own > 1) {
+      // the stretches' totals join in order: in one block as they come, waiting in tensor memory for the last one; of a cluster's blocks at the end
+      if (j + 1 < own) {
+        if (j > 0) tmem_add(lane_addr + 2 * BN, acc);
 #pragma unroll
-        for (int e = 0; e < SC; e += 8) tmem_st8(totals + e, acc + e);
-        const float none[8] = {};
-#pragma unroll
-        for (int e = 0; e < SC; e += 8) tmem_st8(totals + BN + e, none);
-      } else if (ranks == 1) {
-        if (j + 1 < own) tmem_join<false>(totals, BN, acc);
-        else tmem_join<true>(totals, BN, acc);
+        for (int e = 0; e < SC; e += 8) tmem_st8(lane_addr + 2 * BN + e, acc + e);
+        tmem_st_wait();
       }
-      tmem_st_wait();
     }
     // the ring is free: the last sums are complete, so its last stage has been read. Results leave through it, in a loop of all threads: the
     // activations written out for every register of a tile would be more code than the instruction cache holds
-    const int row = quarter * 32 + lane, tiles = ranks > 1 ? own : 1;
+    const int row = quarter * 32 + lane, tiles = min(own, 2);
     float* tile = reinterpret_cast<float*>(ring) + (tiles - 1) * BN * FM;
 #pragma unroll
     for (int e = 0; e < SC; ++e) tile[(half * SC + e) * FM + row] = acc[e];
@@ -377,14 +347,14 @@ linear_f32_tc_kernel(const LinearF32Params p) {
     for (int at = rank * T::THREADS + tid; at < BN * FM; at += ranks * T::THREADS) {
       const int m = m0 + at / FM, n = n0 + (at - lane) % FM;      // a warp's are of one row
       if (m >= p.M) continue;
-      float v;
+      float v = 0.f;
       if (ranks == 1) {
-        v = tile[at];
+        v = join_last(tile[at], tile[BN * FM + at]);
       } else {
-        float lo = 0.f;
-        v = 0.f;
-        for (int s = 0; s < p.stretches; ++s) join(v, lo, *cluster.map_shared_rank(tile + s % own * BN * FM + at, s / own));
-        v = joined(v, lo);
+        for (int s = 0; s < p.stretches; ++s) {
+          const float t = *cluster.map_shared_rank(tile + s % own * BN * FM + at, s / own);
+          v = s + 1 < p.stretches ? v + t : join_last(v, t);
+        }
       }
       finish_f32(p, m, n, v, lane);
     }
@@ -431,8 +401,8 @@ int linear_f32_tensor(const float* x, const float* w, const float* bias, float* 
   // matrix of few tiles, each of four stages at least (clusters of four blocks: 33 are resident at a time with a block an SM, of three 44,
   // of two 70 and more; 36 clusters of four are two waves: 4,544 x 18,176 and one row 157 us, in clusters of three 108), and then as many as keep
   // a stretch at 64 stages or fewer, at least two, from K of 2,048 on four, since each of its additions rounds (one cluster's block holds two
-  // at most). A stretch more costs a block its totals' way through tensor memory: 700 rows, one or two and now, 4,096 x 1,024 82 -> 86 us,
-  // 9,216 x 4,096 362 -> 354.
+  // at most). A stretch more costs a block its totals' way through tensor memory: 700 rows, with one or two and now, 9,216 x 1,024 110 and 111 us,
+  // 9,216 x 4,096 365 and 357.
   const int shared = tiles <= 33 ? 4 : tiles <= 44 ? 3 : tiles <= 70 ? 2 : 1;
   int most = shared;
   while (most > 1 && total / most < 4) --most;
