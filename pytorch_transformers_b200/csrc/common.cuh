@@ -37,6 +37,19 @@ __device__ __forceinline__ float apply_activation(float v, int act) {
   }
 }
 
+// 1 / (1 + e^-x) where it is formed for every value and a division with its call for odd operands would bind: from e^-|x|, so that the
+// divisor lies in [1, 2]. The hardware's reciprocal gives a quotient, and what the quotient leaves (a Newton step, with the divisor's own
+// rounding) corrects it. 2-norm off 64 bits, the quotient of 1 and 1 + expf(-x) in brackets: normal arguments 2.9e-8 (4.1e-8), three times as
+// wide 2.2e-8 (3.8e-8), evenly to 20 1.8e-8 (3.5e-8); the fast division without the step 4.4e-8, 4.1e-8, 3.6e-8. Times x, as a silu: 3.5e-8
+// (4.0e-8), 3.1e-8 (4.2e-8), 3.0e-8 (3.3e-8).
+__device__ __forceinline__ float sigmoid_of(float x) {
+  const float t = expf(-fabsf(x)), n = x < 0.f ? t : 1.f, d = 1.f + t;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+  const float q = n * r;
+  return fmaf(fmaf((d - 1.f) - t, q, fmaf(-d, q, n)), r, q);      // (d - 1) - t: what 1 + t lost, exactly
+}
+
 // The unit between a gated feed-forward's two products: silu(gate) * up, or with limit > 0 the clamped unit
 // g * sigmoid(alpha g) * (u + 1) of g = min(gate, limit) and u = clamp(up, -limit, limit).
 __device__ __forceinline__ float gated_unit(float gate, float up, float limit, float alpha) {

@@ -133,13 +133,6 @@ __global__ void rglru_conv_run_kernel(const T* __restrict__ proj, const float* _
   }
 }
 
-// 1 / (1 + e^-x) from e^-|x|: the divisor lies in [1, 2], where the fast division is off by two units of 2^-24 at most. The gates of a
-// token and channel are formed by this one expression wherever they are formed.
-__device__ __forceinline__ float sigmoid_of(float x) {
-  const float t = expf(-fabsf(x));
-  return __fdividef(x < 0.f ? t : 1.f, 1.f + t);
-}
-
 // a S + drive with a = exp(log_a), formed as S + ((a - 1) S + drive) with a - 1 = expm1(log_a): a decay close
 // to 1 rounded to float32 is off by up to 3e-8 of itself, which a channel whose decay hardly changes would
 // carry into every step alike (1,000 steps: 3e-5 of the state); a - 1 keeps its digits, and what is left is

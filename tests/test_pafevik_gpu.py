@@ -74,6 +74,20 @@ def test_stream_norm_and_sum(width):
     torch.testing.assert_close(k.add_stream(x.cuda(), a.bfloat16().cuda()).cpu(), x + a.bfloat16().float(), atol=0, rtol=0)
 
 
+@pytest.mark.parametrize("rows", [4, 5000])
+@pytest.mark.parametrize("spread", [1.0, 3.0, 12.0])
+def test_sigmoid_of_a_block_product_errs_no_more_than_a_true_division(rows, spread):
+    """2-norm against 64 bits of float32 results, beside 1 / (1 + exp(-x)) with both operations rounded as IEEE says; ends and NaN."""
+    g = torch.Generator().manual_seed(int(spread))
+    x = (spread * torch.randn(rows, 1000, 1, generator=g)).cuda()
+    x[0, :6, 0] = torch.tensor([math.inf, -math.inf, math.nan, 0.0, 90.0, -90.0])
+    got = K().block_linear(x, torch.ones(1000, 1, 1, device="cuda"), act="sigmoid", out_dtype=torch.float32)[:, :, 0]
+    assert got[0, :5].tolist()[:2] == [1.0, 0.0] and got[0, 2].isnan() and got[0, 3:5].tolist() == [0.5, 1.0] and 0 <= got[0, 5] < 1e-38
+    x, got = x[:, 6:, 0], got[:, 6:]
+    ref = torch.sigmoid(x.double())
+    assert (got.double() - ref).norm() <= (1 / (1 + torch.exp(-x)) - ref).norm()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("m,groups,n,kk", [(1, 3, 20, 24), (70, 5, 14, 10), (130, 1, 80, 80), (9, 18, 64, 32), (300, 4, 40, 24)])
 def test_block_linear(dtype, m, groups, n, kk):

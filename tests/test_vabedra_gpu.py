@@ -184,6 +184,28 @@ def test_what_enters_the_recurrence(m, channel, dtype):
     close(got["l"].exp().reshape(40, -1), plain.delta_decay(x, w, m).reshape(40, -1), dtype, "decays", f32=5e-6, bf16=1.5e-2)
 
 
+@pytest.mark.parametrize("n", [3, 700])
+@pytest.mark.parametrize("spread", [1.0, 3.0, 12.0])
+def test_silu_before_the_recurrence_errs_no_more_than_a_true_division(n, spread):
+    """2-norm against 64 bits of float32 results, beside x / (1 + exp(-x)) with both operations rounded as IEEE says. A filter of one tap
+    of weight one leaves the projections as they are."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.base import StateNeed
+    H, d = 4, 64
+    C = 3 * H * d
+    cache = Cache([(0, None, StateNeed(K().delta_state_floats(H, H, d, d, 1)))], 64, torch.float32, "cuda", max_slots=1)
+    ctx = StepContext(cache, [cache.open()], [[0] * n], 1, [[]], [])
+    state = ctx.state_of(type("E", (), {"cache_entry": 0, "state_offset": 0})(), K().delta_state_floats(H, H, d, d, 1))
+    g = torch.Generator().manual_seed(n)
+    proj = (spread * torch.randn(n, C + H, generator=g)).cuda()
+    act, *_ = K().delta_prepare(proj, torch.ones(1, C, device="cuda"), state, ctx.dev["slots"], ctx.batch_c[0], torch.zeros(H, device="cuda"),
+                                torch.zeros(H * d, device="cuda"), H, H, d, d, C, z=torch.zeros(n, H * d, device="cuda"))
+    x = proj[:, :C]
+    ref = x.double() * torch.sigmoid(x.double())
+    assert (act.double() - ref).norm() <= (x / (1 + torch.exp(-x)) - ref).norm()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("m,channel", [(vm.delta(4, 2, 24, 20, 4), False), (vm.delta(2, 2, 64, 40, 4, rank=5), True),
                                        (vm.delta(2, 1, 9, 6, 4, rank=3), True), (vm.delta(2, 1, 32, 32, 3), False),
