@@ -240,6 +240,32 @@ def test_scan_from_the_gates_product(R, blocks, chunk):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("R,blocks", [(96, 4), (640, 8)])
+def test_scan_in_chunks_forms_a_token_as_the_walk_does(R, blocks):
+    """Outputs of up to half a chunk, where nothing is joined, from a state that an earlier step left: the walk's bits."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.base import StateNeed
+    k, bw, taps, news = K(), R // blocks, 4, [32, 1, 19]
+    g = torch.Generator(device="cuda").manual_seed(R)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    n = sum(news)
+    proj, w, b = rand(n, 2 * R), rand(blocks, 2 * bw, bw) / math.sqrt(bw), 0.3 * rand(blocks, 2 * bw)
+    bias, conv, lam, before = [0.3 * rand(R) for _ in range(3)], 0.5 * rand(R, taps), 1.5 * rand(R) - 1, rand(3, R * taps)
+    got = []
+    for chunked in (False, True):
+        cache = Cache([(0, None, StateNeed(R * taps))], 64 * 16, torch.float32, "cuda", max_slots=3)
+        ctx = StepContext(cache, [cache.open() for _ in news], [[0] * m for m in news], 1, [[] for _ in news])
+        state = cache.entry_state(0)
+        state[:3, :R * taps] = before
+        y_act, u = k.rglru_conv(proj, bias[0], bias[1], conv, bias[2], state, ctx.dev["slots"], ctx.batch_c[0])
+        gates = k.block_linear(u.view(n, blocks, bw), w, b, act="sigmoid", out_dtype=torch.float32)
+        args = (gates, u, y_act, lam, proj, bias[1], state, ctx.dev["slots"], ctx.batch_c[0], blocks, taps, 8.0)
+        ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        got.append(k.rglru_scan_chunks(*args, ints([0, 1, 2]), ints([0, 0, 0]), ints([0, 1, 2]), 3, 64) if chunked else k.rglru_scan(*args))
+    assert torch.equal(*got)
+
+
 def rglru_case(dtype, R, blocks, taps, pasts, news, seed=0, chunk=0):
     """The recurrence's kernels from random branch projections in two steps; (kernel output, plain) for the
     second step, and the state rows of the slots."""
