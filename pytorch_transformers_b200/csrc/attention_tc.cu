@@ -4,7 +4,7 @@
 // is for head size 64; with 128 the tiles of Q, K and V are two blocks of 64 dims, S takes two groups
 // of matrix instructions, O is 128 columns, and one block fits on an SM (two with TWO, below). Above 64 the matrix
 // instructions of S and of O += P V are issued by a warp each (APART), and extras and weights of two terms have two
-// softmax threads a row.
+// softmax threads a row, where walks are not short (SHORT).
 //
 // One block = 128 consecutive new tokens of one sequence x one query head. 128 softmax threads, one per
 // query row (tensor-memory lane t = row t). One more warp's first lane issues every matrix
@@ -138,39 +138,46 @@ struct TcParams {
 // O += P V needs 1,810 clocks a page (weights of two terms): a wait costs a hundred and more also where what it waits for is there, a
 // commit 44, a request for a page some hundreds; the instructions are 900. So each product has a thread, and keys and values of a page
 // have a barrier each. With two threads a softmax row (each takes 32 keys of a page; they exchange their maxima through shared memory
-// and share the work on O by columns) the softmax is no longer the longest part: 1,500. us before and with both: full context
+// and share the work on O by columns) the softmax is no longer the longest part: 1,500. us with one of each and with both: full context
 // of 2,048 tokens, 16 heads 41 -> 38, latent keys of 192 at 3,000 tokens 99 -> 82, 32 heads of 3,400 tokens (TWO) 165 -> 131, window of
-// 1,024 in 2,048 tokens 37 -> 31; two threads a row alone 41 -> 41 and 38 -> 37. A walk of three pages (window of 100) 18 -> 19. Head size
-// 64 is bound by the exponential unit: 3 to 7 % slower with two issuing threads or two barriers a page.
+// 1,024 in 2,048 tokens 37 -> 31; two threads a row alone 41 -> 41 and 38 -> 37. Head size 64 is bound by the exponential unit: 3 to 7 % slower with two issuing threads or two barriers a page.
+// SHORT: one issuing thread and one softmax thread a row, as at head size 64. Short walks are their first and last pages, which hands from one thread to
+// the next only lengthen; and where the softmax has little to do beside its waits, or the exponential unit binds it (a cap), two threads a row
+// win nothing. us with one and with two: window of 64 in 2,048 tokens 12.2 / 13.0, of 100 13.4 / 14.8, of 160 15.3 / 16.3, of 200 17.0 / 17.4 (3,000
+// tokens: 24.9 / 24.2 at 160, 28.4 / 26.2 at 200); capped, 100 17.1 / 19.1, 300 23.5 / 25.3, 512 30.0 / 30.8, 700 36.6 / 37.1, 1,024 42.1 / 40.9, without
+// a window 54 / 50; full context of 300 tokens 9.3 / 9.8 (weights of two terms without extras 8.8 / 9.1, of one 8.5 / 8.8), 512 12.5 / 12.3 (12.2 / 11.3, 11.0 /
+// 10.9), 700 14.9 / 15.7 (14.6 / 14.6, 13.3 / 13.8), 1,000 19.7 / 20.2 (19.4 / 18.8, 17.4 / 17.4), 1,024 20.3 / 18.9 (19.8 / 17.4, 17.3 / 16.3). Weights of
+// one term with extras at any length: 1,280 tokens 20.5 / 21.2, 2,048 32.5 / 33.6. So windows up to 160, or 512 under a cap, and steps of few tiles,
+// whose walks are as short. (Keys of 192: window of 128 19.7 / 20.2, full context of 300 tokens and of 64 9.9 / 9.7 and 6.4 / 6.1, so windows alone.)
 // TWO (head size 128 with weights of two terms): two S buffers and two page stages instead of three and four, 99 KB and 256
 // columns of tensor memory a block, so that two blocks fit on an SM and one's softmax runs under the other's waits. A stage of keys is
 // asked for again when its S is complete, not only when its O += P V is (before, S waited 1,000 of a page's 2,560 clocks for its keys),
 // and by the thread that issues from it: a third warp would leave 80 registers a thread (2 to 4 % slower). Taken where
 // the blocks make more than two waves, or more than one with a window, whose walks are alike long; with fewer blocks and the
 // triangle of a full context the longest chain counts, and a block with an SM of its own runs it faster. us, one an SM
-// against two: full context 208 blocks 32 / 36, 256 37 / 42, 288 44 / 47, 320 56 / 49, 864 (32 heads) 167 / 131; capped 240 51 / 54, 304 73 /
+// against two (two softmax threads a row): full context 208 blocks 32 / 36, 256 37 / 42, 288 44 / 47, 320 56 / 49, 864 (32 heads) 167 / 131; capped 240 51 / 54, 304 73 /
 // 71, 864 245 / 187; window of 300: 160 20 / 16; of 1,024: 256 (2,048 tokens) 38 / 31. Where most of a prompt fits into its window the
 // walks are a triangle again and one an SM would be the faster: 160 blocks of 1,024 in 2,560 tokens 23 / 27 (the rule does not
 // look at lengths).
-template <int DK, bool WIDE, bool EXTRAS, bool TWO> struct TcThreads {
-  static constexpr int PER = DK > 64 && (WIDE || EXTRAS) ? 2 : 1, SOFTMAX = TQ * PER;
-  static constexpr bool APART = DK > 64;      // S and O += P V by a thread each; and (not TWO) a third for the pages
-  static constexpr int BLOCK = SOFTMAX + (APART && !TWO ? 96 : 64);
+template <int DK, bool WIDE, bool EXTRAS, bool TWO, bool SHORT> struct TcThreads {
+  static constexpr int PER = DK > 64 && (WIDE || EXTRAS) && !SHORT ? 2 : 1, SOFTMAX = TQ * PER;
+  static constexpr bool APART = DK > 64 && !SHORT;      // S and O += P V by a thread each; and (not TWO) a third for the pages
+  static constexpr int BLOCK = SOFTMAX + (APART && !TWO ? 96 : 64);      // not APART: one that issues, one for the pages
 };
 template <bool TWO> struct TcShape {
   static constexpr int BUFS = TWO ? 2 : 3;                 // S buffers
   static constexpr int STAGES = TWO ? 2 : STAGES_TC;       // page stages
 };
-template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS, bool TWO>
-__global__ void __launch_bounds__(TcThreads<DK, WIDE, EXTRAS, TWO>::BLOCK, DK == 64 || TWO ? 2 : 1)
+template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS, bool TWO, bool SHORT>
+__global__ void __launch_bounds__(TcThreads<DK, WIDE, EXTRAS, TWO, SHORT>::BLOCK, DK == 64 || TWO ? 2 : 1)
 attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_pool,
                     const __nv_bfloat16* __restrict__ v_pool, __nv_bfloat16* __restrict__ out, StepBatch sb,
                     const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, TcParams p,
                     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                     int* __restrict__ error_flag) {
-  constexpr bool APART = TcThreads<DK, WIDE, EXTRAS, TWO>::APART;
+  constexpr bool APART = TcThreads<DK, WIDE, EXTRAS, TWO, SHORT>::APART;
   constexpr int BUFS = TcShape<TWO>::BUFS, STAGES = TcShape<TWO>::STAGES;
-  constexpr int PER = TcThreads<DK, WIDE, EXTRAS, TWO>::PER, SOFTMAX_THREADS = TcThreads<DK, WIDE, EXTRAS, TWO>::SOFTMAX, MINE = KEYS / PER;
+  constexpr int PER = TcThreads<DK, WIDE, EXTRAS, TWO, SHORT>::PER, SOFTMAX_THREADS = TcThreads<DK, WIDE, EXTRAS, TWO, SHORT>::SOFTMAX, MINE = KEYS / PER;
   __shared__ float row_words[PER == 2 ? 2 : 1][2][PER == 2 ? TQ : 1];      // what a row's two threads tell each other
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte alignment: the swizzle pattern is a function of address bits 4..9
@@ -196,7 +203,7 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool score_warp = warp == SOFTMAX_THREADS / 32;
   const bool value_warp = APART && warp == SOFTMAX_THREADS / 32 + 1;
-  const bool copy_warp = !TWO && warp == SOFTMAX_THREADS / 32 + (APART ? 2 : 1);
+  const bool copy_warp = !(TWO && APART) && warp == SOFTMAX_THREADS / 32 + (APART ? 2 : 1);
   const int row = tid & (TQ - 1);        // query row of a softmax thread (= its tensor-memory lane)
   // heads are the fast index of the grid: the blocks of one tile start together (they read the same
   // pages), and tiles come in the order of the list, which the caller sorts by falling key count so that
@@ -248,10 +255,10 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
     for (int blk = 0; blk < DV / 64; ++blk)
       tma_load_2d(smem_u32(v_ring + st * TILE_V_BYTES + blk * (KEYS * 128)), &v_map, blk * 64, y, full);
   };
-  // The first lane of the copy warp (TWO: of the one that issues S) sets the barriers up and asks for the first pages at once (their numbers
+  // The first lane of the copy warp (TWO and APART: of the one that issues S) sets the barriers up and asks for the first pages at once (their numbers
   // read by the warp's lanes, one each): they are on their way while the other warps fetch Q and tensor
   // memory is allocated. Nobody else touches a barrier before the block-wide barrier below.
-  if (TWO ? score_warp : copy_warp) {
+  if (TWO && APART ? score_warp : copy_warp) {
     const int first_pages = lane < n_blocks ? pages[block_of(lane)] : 0;   // lane b: the number of page b
     if (lane == 0) {
       for (int b = 0; b < 3; ++b) {
@@ -455,7 +462,7 @@ attention_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
       if (capped) {      // cap * tanh(score / cap), in powers of two
         // Where none of the visible ones reaches the cap, by multiply-adds: the exponential unit, with its exponential and its
         // reciprocal here beside the softmax's exponential, is 1,536 clocks of a capped page (32 heads of 3,400 tokens, two blocks an SM 202
-        // -> 187 us; one block an SM 49 -> 51 of 1,900 tokens). Else tanh(x) = 1 - 2 / (1 + exp(2 x)). Which one follows from what the
+        // -> 187 us; one block an SM, 2,048 tokens 52 -> 50, 1,000 tokens 28.9 -> 29.7). Else tanh(x) = 1 - 2 / (1 + exp(2 x)). Which one follows from what the
         // thread's row sees of the page.
         const float to_x = p.scale / p.softcap, out2 = p.softcap * 1.4426950408889634f;
         bool inside = false;
@@ -1002,26 +1009,35 @@ PTB_API int ptb_attention_tc_supports_sizes(int head_dim, int v_dim) {
 PTB_API int ptb_attention_tc_tile_tokens() { return TQ; }
 
 namespace {
-template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS = false, bool TWO = false>
+template <int DK, int DV, bool BIAS, bool WIDE, bool EXTRAS = false, bool TWO = false, bool SHORT = false>
 int launch_tc(const void* q, const void* k_pool, const void* v_pool, int pool_pages, void* out, const StepBatch& sb,
               const int* tile_seq, const int* tile_q0, int n_tiles, const TcParams& p, int* error_flag,
               cudaStream_t stream) {
-  if constexpr (DK == 128 && DV == 128 && WIDE && !TWO) {      // the rule of TWO
-    const long long blocks = (long long)p.heads * n_tiles, sms = sm_count();
-    if (blocks > 2 * sms || (p.window > 0 && blocks > sms))
-      return launch_tc<DK, DV, BIAS, WIDE, EXTRAS, true>(q, k_pool, v_pool, pool_pages, out, sb, tile_seq, tile_q0, n_tiles, p,
-                                                         error_flag, stream);
+  constexpr bool NARROW_EXTRAS = DK == 128 && EXTRAS && !WIDE;
+  if constexpr (DK > 64 && !SHORT && !TWO) {      // the rule of SHORT
+    const int few = DK > 128 ? 0 : WIDE && !EXTRAS ? 3 : 6;
+    if (NARROW_EXTRAS || (p.softcap > 0.f ? DK == 128 && p.window > 0 && p.window <= 512 : (p.window > 0 && p.window <= 160) || n_tiles <= few))
+      return launch_tc<DK, DV, BIAS, WIDE, EXTRAS, TWO, true>(q, k_pool, v_pool, pool_pages, out, sb, tile_seq, tile_q0, n_tiles, p,
+                                                              error_flag, stream);
   }
-  const CUtensorMap* km = pool_map(k_pool, pool_pages, p.kv_heads, DK);
-  const CUtensorMap* vm = pool_map(v_pool, pool_pages, p.kv_heads, DV);
-  if (km == nullptr || vm == nullptr) return PTB_ERR_LAUNCH;
-  const size_t smem = 1024 + TQ * DK * 2 + TcShape<TWO>::STAGES * KEYS * (DK + DV) * 2 + 192;
-  static SharedLimit limit;
-  if (!limit.allows(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO>, smem)) return PTB_ERR_LAUNCH;
-  dim3 grid(p.heads, n_tiles);
-  attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO><<<grid, TcThreads<DK, WIDE, EXTRAS, TWO>::BLOCK, smem, stream>>>(
-      (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, sb,
-      tile_seq, tile_q0, p, *km, *vm, error_flag);
+  if constexpr (!NARROW_EXTRAS || SHORT) {
+    if constexpr (DK == 128 && DV == 128 && WIDE && !TWO) {      // the rule of TWO
+      const long long blocks = (long long)p.heads * n_tiles, sms = sm_count();
+      if (blocks > 2 * sms || (p.window > 0 && blocks > sms))
+        return launch_tc<DK, DV, BIAS, WIDE, EXTRAS, true, SHORT>(q, k_pool, v_pool, pool_pages, out, sb, tile_seq, tile_q0, n_tiles, p,
+                                                                  error_flag, stream);
+    }
+    const CUtensorMap* km = pool_map(k_pool, pool_pages, p.kv_heads, DK);
+    const CUtensorMap* vm = pool_map(v_pool, pool_pages, p.kv_heads, DV);
+    if (km == nullptr || vm == nullptr) return PTB_ERR_LAUNCH;
+    const size_t smem = 1024 + TQ * DK * 2 + TcShape<TWO>::STAGES * KEYS * (DK + DV) * 2 + 192;
+    static SharedLimit limit;
+    if (!limit.allows(attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO, SHORT>, smem)) return PTB_ERR_LAUNCH;
+    dim3 grid(p.heads, n_tiles);
+    attention_tc_kernel<DK, DV, BIAS, WIDE, EXTRAS, TWO, SHORT><<<grid, TcThreads<DK, WIDE, EXTRAS, TWO, SHORT>::BLOCK, smem, stream>>>(
+        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pool, (const __nv_bfloat16*)v_pool, (__nv_bfloat16*)out, sb,
+        tile_seq, tile_q0, p, *km, *vm, error_flag);
+  }
   return launch_status();
 }
 }  // namespace

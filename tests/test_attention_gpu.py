@@ -494,6 +494,39 @@ def test_tc_cap_inside_and_beyond(K, heads, d, window, softcap):
     K.check_device_errors("cuda:0")
 
 
+@pytest.mark.parametrize("heads", [4, 60])
+@pytest.mark.parametrize("news,window,softcap,wide", [
+    ([768], 0, 0.0, True), ([769], 0, 0.0, True), ([300, 83, 129], 0, 0.0, False), ([900, 50], 160, 0.0, True), ([900, 50], 161, 0.0, True),
+    ([900, 50], 512, 9.0, True), ([900, 50], 513, 9.0, True), ([900, 1], 600, 0.0, False)])
+def test_tc_on_both_sides_of_the_short_walks(K, heads, news, window, softcap, wide):
+    """Head size 128 with one thread that issues and one a row, or more of both, and with one or two blocks an SM, around the sizes where the
+    choice changes; against the general kernel, bound as for test_tc_extras, for weights of one bfloat16 term with their rounding (2^-9 of a
+    mean of values)."""
+    from pytorch_transformers_b200.cache.paged import Cache
+    from pytorch_transformers_b200.engine.batch import StepContext
+    from pytorch_transformers_b200.parts.attention import AttentionTiles
+    from pytorch_transformers_b200.parts.base import CacheNeed
+    kv, d = 2, 128
+    cache = Cache([(0, CacheNeed("full", kv, d), None)], sum((n + 63) // 64 * 64 for n in news), BF, "cuda")
+    ctx = StepContext(cache, [cache.open() for _ in news], [[0] * n for n in news], 1, [[] for _ in news], [AttentionTiles(K)])
+    g = torch.Generator(device="cuda").manual_seed(window + heads)
+    k_pool, v_pool, gi = cache.entry_storage(0)
+    k_pool.normal_(generator=g), v_pool.normal_(generator=g)
+    q = torch.randn(sum(news), heads, d, generator=g, device="cuda").to(BF)
+    tiles, batch = ctx.plan(AttentionTiles.plan_key), ctx.batch_c[gi]
+    at = lambda seq, q0, count: (q, k_pool, v_pool, batch, tiles.dev[seq], tiles.dev[q0], tiles.facts[count])
+    ref = torch.empty(sum(news), heads * d, dtype=BF, device="cuda")
+    K.attention_generic(*at("tile_seq", "tile_q0", "n_tiles"), None, kv, d ** -0.5, window, softcap=softcap, out=ref)
+    ref, mma = ref.double(), at("mtile_seq", "mtile_q0", "n_mma_tiles")
+    got = [(wide, K.attention_tc_extras(*mma, kv, d ** -0.5, window, softcap=softcap, wide_weights=wide))]
+    if window == 0 and softcap == 0:
+        got += [(w, K.attention_tc(*mma, kv, d ** -0.5, None, w)) for w in (False, True)]
+    for two_terms, out in got:
+        bound = 2.0 ** -7 * ref.abs() + (2e-4 if two_terms else 2.0 ** -9 * v_pool.abs().max().item())
+        assert ((out.double() - ref).abs() <= bound).all(), (out.double() - ref).abs().max()
+    K.check_device_errors("cuda:0")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("d,vd", [(8, 8), (8, 16), (16, 12), (72, 136), (128, 64), (256, 256), (250, 256)])
 def test_general_attention_reads_words_and_values_alike(K, dtype, d, vd):
