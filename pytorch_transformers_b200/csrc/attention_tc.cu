@@ -51,6 +51,7 @@
 // dependent steps per page (about 1,500 clocks with two chains an SM, of which the exponential unit is
 // busy 1,024) plus 6 us of set-up and drain; blocks that stay and draw one tile after another from a
 // counter saved the set-up but ran their pages 10 to 25 % slower, and were taken out again.
+#include "f32x2.cuh"
 #include "mma_common.cuh"
 #include "tc_common.cuh"
 
@@ -60,31 +61,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   float m;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(m) : "f"(a), "f"(b), "f"(c));
   return m;
-}
-// two float32 values in one 64-bit register for the packed multiply-add and add instructions
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
-  return r;
 }
 // tanh(x) / x of z = x^2 up to 1: the polynomial of degree 6 whose largest relative error is smallest (5e-8; 1.6e-7 with float32 roundings)
 __device__ __forceinline__ uint64_t tanh_ratio2(uint64_t z) {

@@ -16,34 +16,11 @@
 // state, decayed keys and queries, T, P, W, U_0) enter the products split in two bfloat16 terms, hi hi + hi lo + lo hi, but for
 // the scores inside a sub-block, which keep 32 bits; projections are bfloat16 as they are, their unit norms factors of the results.
 #include "chunk_mma.cuh"
+#include "f32x2.cuh"
 
 namespace {
 
 constexpr float LOG2E_F = 1.4426950408889634f;
-
-// two float32 values in a 64-bit register: the two-wide multiply-adds
-__device__ __forceinline__ unsigned long long pack2(float x, float y) {
-  unsigned long long v;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
-  return v;
-}
-__device__ __forceinline__ float2 halves2(unsigned long long v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ unsigned long long wide2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ unsigned long long minus2(unsigned long long a, unsigned long long b) { return fma2(b, 0xbf800000bf800000ull, a); }
 
 // hi and lo terms of two neighbouring values of a row of a swizzled [rows][D] tile
 template <int D>
@@ -378,7 +355,7 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
       const int task = eight * 8 + (lane >> 2), b = task / 36, pr = task % 36, ra = pr / 9, rb = pr % 9;
       const int r = rb <= ra ? ra : 7 - ra, s = rb <= ra ? rb : rb - ra - 1;     // s <= r
       const int row = b * 8 + r, col = b * 8 + s;
-      unsigned long long a2 = 0ull, p2 = 0ull;      // the even and the odd channels' sums
+      uint64_t a2 = 0ull, p2 = 0ull;      // the even and the odd channels' sums
 #pragma unroll 4
       for (int d = sub * 4; d < DK; d += 16) {
         const ulonglong2 ct = *reinterpret_cast<const ulonglong2*>(cb + row * CP + d);
@@ -387,8 +364,8 @@ delta_chunk_local_kernel(const __nv_bfloat16* __restrict__ act, const float* __r
         const uint2 k2 = *reinterpret_cast<const uint2*>(ks + col * KP + d);
         const uint2 qt = *reinterpret_cast<const uint2*>(qs + row * KP + d);
         const float2 x = halves2(minus2(ct.x, cs.x)), y = halves2(minus2(ct.y, cs.y));
-        const unsigned long long e0 = mul2(wide2(k2.x), pack2(fast_exp2(x.x), fast_exp2(x.y)));
-        const unsigned long long e1 = mul2(wide2(k2.y), pack2(fast_exp2(y.x), fast_exp2(y.y)));
+        const uint64_t e0 = mul2(wide2(k2.x), pack2(fast_exp2(x.x), fast_exp2(x.y)));
+        const uint64_t e1 = mul2(wide2(k2.y), pack2(fast_exp2(y.x), fast_exp2(y.y)));
         a2 = fma2(wide2(kt.x), e0, a2);
         a2 = fma2(wide2(kt.y), e1, a2);
         p2 = fma2(wide2(qt.x), e0, p2);

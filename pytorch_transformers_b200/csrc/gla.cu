@@ -17,6 +17,7 @@
 // and 3 run on the tensor cores instead (csrc/gla_mma.cu): there float32 operands enter a product as bfloat16 terms, two
 // in pass 1 (the decayed keys, 16 bits) and three in pass 3 (24 bits).
 #include "common.cuh"
+#include "f32x2.cuh"
 
 namespace {
 
@@ -30,19 +31,7 @@ enum { GLA_WALK = 0, GLA_CHUNK_SUM = 1, GLA_CHUNK_OUT = 2 };
 // registers that hold the next batch, and 48 KB of shared memory)
 __host__ __device__ constexpr int walk_batch(int rows, int cols) { return (rows == 32 || cols == 2) ? 8 : 16; }
 
-// Two float32 lanes in one 64-bit register and their fused multiply-add in one instruction (each lane rounds as fmaf does).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
+typedef uint64_t f32x2;
 
 // z <- logsigmoid(z + bias) / tau: the logarithm of sigmoid(z + bias)^(1 / tau)
 __global__ void gla_decay_kernel(float* __restrict__ z, const float* __restrict__ bias, long long total, int width,

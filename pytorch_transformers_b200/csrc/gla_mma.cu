@@ -10,6 +10,7 @@
 // The result has the layout of the walk's pass 1 (csrc/gla.cu): sums [chunks][heads][dim][v_dim], chunk_decay
 // [chunks][heads][dim].
 #include "chunk_mma.cuh"
+#include "f32x2.cuh"
 
 namespace {
 
@@ -133,12 +134,12 @@ int launch_sum(const void* proj, int stride, const float* log_decay, const StepB
 // the whole sub-blocks between, and w up to t: the first goes into the keys, the others into the queries, all factors are at
 // most 1, nothing is subtracted, and the scores are a product. Inside a sub-block every (t, i, channel) has an exponent of its
 // own: a warp takes four keys and walks the tokens, its lanes' channels' sums for each key in registers; no branch on the keys' places, so that
-// the loads run ahead (117 -> 109 us). What bounds this part is the exponential unit: 136 (t, i) pairs a sub-block and channel, 70,000
-// exponentials a block against 16 a clock and SM. Decaying the four keys to their last one's token, and one exponential for all four from there
+// the loads run ahead (117 -> 109 us). What bounds this part is the exponential unit: 160 (t, i) pairs a sub-block and channel (ten squares of
+// four by four; 24 of them lie before their key and count as zero), 82,000 exponentials a block against 16 a clock and SM. Decaying the four keys to their last one's token, and one exponential for all four from there
 // on, took 100 us, but two roundings and an exponential more a term: 1.48e-7 off 64 bits (one chunk, 2-norm) instead of 1.43e-7. 2,900
 // tokens of 16 heads of 128 x 128; with operands of two terms 94 (before), the walk on the CUDA cores 175.
 // Operands of a product that are float32 (scaled queries and keys, scores, the state) enter it as three bfloat16 terms, 24 bits: what
-// a product leaves out (second x third, third x third) is 2^-26 of it, below the rounding of its float32 sum. A matrix instruction
+// a product leaves out (second x third, third x third) is 2^-27.5 of it (root mean square; 2^-24 at most), below the rounding of its float32 sum. A matrix instruction
 // cuts its sum off instead of rounding it, so the six products of 16 entries are summed from zero, the small ones first, and
 // join the running sum by a rounded addition. With two terms the outputs of one chunk from a given state were 4e-6 off 64
 // bits, with three into one running sum 1e-6, where the walk in float32 is 2e-7 off.
@@ -158,30 +159,6 @@ struct OutShape {
       size_t(CH) * DK * 2 + 2 * size_t(A_BYTES) + C_BYTES + size_t(CH) * LP * 4 + size_t(SUBS - 1) * DK * 4 + size_t(CH) * SPITCH * 4;
 };
 
-// two float32 values in a 64-bit register
-__device__ __forceinline__ unsigned long long pack2(float x, float y) {
-  unsigned long long v;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
-  return v;
-}
-__device__ __forceinline__ float2 halves2(unsigned long long v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ unsigned long long wide2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(c) : "l"(a), "l"(b));
-  return c;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(a) : "l"(b));
-  return a;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  asm("add.rn.f32x2 %0, %0, %1;\n" : "+l"(a) : "l"(b));
-  return a;
-}
 __device__ __forceinline__ float2 pair_f(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
 template <int DK, int DV>
@@ -228,7 +205,7 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
   {   // scores inside sub-block `warp`, in groups of four keys
     constexpr int PAIRS = DK / 64;      // a lane's channels, two in a register pair: half the multiply-adds
     const int c0 = lane * 2 * PAIRS;
-    auto load_row = [&](const unsigned char* tile, int row, unsigned long long (&f)[PAIRS]) {
+    auto load_row = [&](const unsigned char* tile, int row, uint64_t (&f)[PAIRS]) {
       const unsigned char* p = tile + swz<DK>(row, c0 / 8) + (c0 % 8) * 2;
       if constexpr (PAIRS == 2) {
         const uint2 v = *reinterpret_cast<const uint2*>(p);
@@ -239,8 +216,8 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
     };
     const int r0 = warp * SUB;
     // a lane's part of sum_c q[c] k[c] exp2(e[c])
-    auto score = [&](const unsigned long long (&q)[PAIRS], const unsigned long long (&k)[PAIRS], const unsigned long long (&e)[PAIRS]) {
-      unsigned long long sum = 0ull;
+    auto score = [&](const uint64_t (&q)[PAIRS], const uint64_t (&k)[PAIRS], const uint64_t (&e)[PAIRS]) {
+      uint64_t sum = 0ull;
 #pragma unroll
       for (int u = 0; u < PAIRS; ++u) {
         const float2 x = halves2(e[u]);
@@ -249,8 +226,8 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
       const float2 v = halves2(sum);
       return v.x + v.y;
     };
-    auto load_logs = [&](int row, unsigned long long (&l)[PAIRS]) {
-      const unsigned long long* from = reinterpret_cast<const unsigned long long*>(l_s + row * LP + c0);
+    auto load_logs = [&](int row, uint64_t (&l)[PAIRS]) {
+      const uint64_t* from = reinterpret_cast<const uint64_t*>(l_s + row * LP + c0);
       if constexpr (PAIRS == 2) {
         const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(from);
         l[0] = v.x, l[1] = v.y;
@@ -277,7 +254,7 @@ gla_chunk_out_mma_kernel(const __nv_bfloat16* __restrict__ proj, int stride, con
 #pragma unroll 1
     for (int gi = 0; gi < 2; ++gi) {
       const int g = half ? 1 + gi : 3 * gi;      // 20 tokens a warp: groups 0 and 3, or 1 and 2
-      unsigned long long k[4][PAIRS], e[4][PAIRS], q[PAIRS], l[PAIRS];      // e: a key's logarithms after it, up to the token
+      uint64_t k[4][PAIRS], e[4][PAIRS], q[PAIRS], l[PAIRS];      // e: a key's logarithms after it, up to the token
       float p[16];
 #pragma unroll
       for (int a = 0; a < 4; ++a) load_row(k_s, r0 + 4 * g + a, k[a]);

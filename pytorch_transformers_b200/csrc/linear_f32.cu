@@ -18,6 +18,7 @@
 // warps, and tiles of 8 x 8 a thread, which read less, were as fast at 2,048 rows and slower below.
 #include <cooperative_groups.h>
 
+#include "f32x2.cuh"
 #include "linear_f32.cuh"
 #include "mma_common.cuh"
 
@@ -27,14 +28,6 @@ namespace cg = cooperative_groups;
 
 constexpr int TN = 4, LBN = 16 * TN, LBK = 32, LPITCH = LBK + 4, LSTAGES = 3, LTHREADS = 128;
 
-__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float2 halves(unsigned long long v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
 // copies that leave zeros where `bytes` is 0 (a row or a k past the end; the address is then any valid one)
 __device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
@@ -104,16 +97,16 @@ linear_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, cons
       for (int i = 0; i < TM; ++i) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + 8 * i * LPITCH + k);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma2(part[i][j], a.x, b[j].x);
+        for (int j = 0; j < TN; ++j) part[i][j] = fma2(a.x, b[j].x, part[i][j]);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma2(part[i][j], a.y, b[j].y);
+        for (int j = 0; j < TN; ++j) part[i][j] = fma2(a.y, b[j].y, part[i][j]);
       }
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const float2 p = halves(part[i][j]);
+        const float2 p = halves2(part[i][j]);
         acc[i][j] += p.x + p.y;
       }
   }

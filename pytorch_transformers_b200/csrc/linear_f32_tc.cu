@@ -30,6 +30,7 @@
 #include "tc_common.cuh"
 #include <cooperative_groups.h>
 
+#include "f32x2.cuh"
 #include "linear_f32.cuh"
 
 namespace {
@@ -71,26 +72,16 @@ __device__ __forceinline__ void load8(float (&f)[8], const float* p, int vec) {
 }
 
 // the three terms of two values times F_SCALE, packed
-__device__ __forceinline__ void scale2(float& x, float& y) {
-  unsigned long long v;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
-  asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(v) : "l"(0x4800000048000000ull));
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v));
-}
-__device__ __forceinline__ void minus2(float& x, float& y, uint32_t pair) {      // x - low half, y - high half
-  unsigned long long v, t;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y));
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(t) : "r"(pair << 16), "r"(pair & 0xffff0000u));
-  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(v) : "l"(t), "l"(0xbf800000bf800000ull));
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v));
-}
 __device__ __forceinline__ void three_terms(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-  scale2(x, y);
-  a = pack_bf16(x, y);
-  minus2(x, y, a);
-  b = pack_bf16(x, y);
-  minus2(x, y, b);
-  c = pack_bf16(x, y);
+  auto pair = [](uint64_t v) {
+    const float2 f = halves2(v);
+    return pack_bf16(f.x, f.y);
+  };
+  uint64_t v = mul2(pack2(x, y), pack2(F_SCALE, F_SCALE));
+  a = pair(v);
+  v = minus2(v, wide2(a));
+  b = pair(v);
+  c = pair(minus2(v, wide2(b)));
 }
 
 // ... of eight values, to the same place of three tiles
