@@ -46,7 +46,10 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream(t: torch.Tensor):
-    # the current stream's handle as torch keeps it: 0.1 us, where current_stream(device) makes an object in 2.5
+    # the current stream's handle as torch keeps it: 0.1 us, where current_stream(device) makes an object in 2.5. Of no device (a tensor in
+    # host memory) it would be the current device's, and the kernel would read the host's address.
+    if not t.is_cuda:
+        raise KernelError("the kernels run on a CUDA device only; got a tensor on " + str(t.device))
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(t.get_device()))
 
 

@@ -111,6 +111,11 @@ def test_block_linear(dtype, m, groups, n, kk):
     torch.testing.assert_close(y.double().cpu(), want, **tol)
 
 
+def test_block_linear_refuses_rows_in_host_memory():
+    with pytest.raises(K().KernelError):
+        K().block_linear(torch.zeros(3, 2, 8), torch.zeros(2, 4, 8, device="cuda"))
+
+
 def latent_case(dtype, heads, rank, rot, pasts, news, needle=None, base=10000.0, scale=0.2, seed=0):
     """Cache rows from random down-projections in two steps (``pasts``, then ``news`` tokens per sequence), then
     the latent attention of the second step; returns (kernel output, plain output) for the second step's rows.

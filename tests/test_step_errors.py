@@ -94,3 +94,10 @@ def test_a_model_without_weights_says_so():
     cache = bare.new_cache(64)
     with pytest.raises(RuntimeError, match="no weights"):
         bare.step(cache, [cache.open()], [[1]])
+
+
+def test_no_kernel_is_launched_for_a_tensor_in_host_memory():
+    """The stream that a launch asks for is that of its tensor's device; a tensor of none has no stream."""
+    from pytorch_transformers_b200 import kernels
+    with pytest.raises(kernels.KernelError, match="cpu"):
+        kernels._stream(torch.zeros(1))
