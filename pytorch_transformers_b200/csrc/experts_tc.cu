@@ -27,9 +27,10 @@
 // Every wait on a barrier is bounded: when one runs out, the error flag is raised and the block carries on to its end without
 // waiting again.
 //
-// One B200, 64 experts of 1,408, width 2,048, both products: 12,288 rows (about 192 an expert, tiles of 256) 334 -> 289 us (735 TFLOP/s),
-// 21,000 rows 500 -> 438, 4,200 rows 241 -> 220, 48 rows 136 -> 124 (4.9 TB/s of the matrices of the experts in use); before, a block a
-// tile and one ring of three stages. With many rows shared memory's bandwidth bounds it (a stage of 192 rows: 56 KB in, 80 KB
+// One B200, 64 experts of 1,408, width 2,048, chosen evenly, plan and both products: 12,288 rows (about 192 an expert, tiles of 256) 322 -> 281 us
+// (790 TFLOP/s without the plan), 21,000 rows 487 -> 434, 4,200 rows 223 -> 206, 48 rows 108 -> 102;
+// before, a block a tile and one ring of three stages. A router that chooses unevenly leaves a last round of few tiles: 328 -> 318 of such 12,288 rows.
+// With many rows shared memory's bandwidth bounds it (a stage of 192 rows: 56 KB in, 80 KB
 // read by the matrix instructions, 1,090 of its clocks), then the results of a tile and a last round of few tiles. Boxes asked into L2 eight
 // stages ahead cost a third with few rows (67 -> 90 us).
 #include <cudaTypedefs.h>
@@ -46,10 +47,10 @@ constexpr int XK = 64;                     // k per stage: 128 bytes, one swizzl
 constexpr int X_BOX_BYTES = XM * XK * 2;   // 16 KB
 constexpr int X_MAX_W = 7, X_MAX_X = 4;   // stages of the rings of matrix boxes and of x rows
 constexpr int MAX_BOXES = 2;               // boxes of a tile, each with an accumulator and a thread that issues for it
-// TWO: two blocks an SM, for tiles of few rows
-template <bool TWO>
+// TWO: two blocks an SM, for tiles of few rows (the first product's units leave registers for four storing warps then)
+template <int MODE, bool TWO>
 struct ExpertThreads {
-  static constexpr int GATHER = TWO ? 64 : 256, STORE = TWO ? 128 : 256, ALL = 32 * (1 + MAX_BOXES) + GATHER + STORE;
+  static constexpr int GATHER = TWO ? 64 : 256, STORE = TWO && MODE == 0 ? 128 : 256, ALL = 32 * (1 + MAX_BOXES) + GATHER + STORE;
   static constexpr int RING = (TWO ? 111 : 225) * 1024;
 };
 
@@ -87,17 +88,22 @@ struct ExpertTcParams {
   float glu_limit, glu_alpha;
 };
 
-template <int MODE, bool TWO>
-__global__ void __launch_bounds__(ExpertThreads<TWO>::ALL, TWO ? 2 : 1)
+// PER: rows of a tile that a gathering thread copies a chunk of
+template <int MODE, bool TWO, int PER>
+__global__ void __launch_bounds__(ExpertThreads<MODE, TWO>::ALL, TWO ? 2 : 1)
 expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertTcParams p) {
   pdl_entry();
-  constexpr int X_GATHER = ExpertThreads<TWO>::GATHER, X_STORE = ExpertThreads<TWO>::STORE;
+  constexpr int X_GATHER = ExpertThreads<MODE, TWO>::GATHER, X_STORE = ExpertThreads<MODE, TWO>::STORE;
   constexpr int TMEM_COLS = TWO ? 256 : 512;
   constexpr int BOXES = MODE != 0 && TWO ? 1 : 2;
   constexpr int COLS = MODE == 0 ? XM : BOXES * XM;      // output columns of a tile
-  const int m_tiles = (p.N + COLS - 1) / COLS, total = p.plan[0] * m_tiles;
-  if (int(blockIdx.x) >= total) return;
+  const int m_tiles = (p.N + COLS - 1) / COLS;
   const int *tile_expert = p.plan + 1, *tile_row0 = tile_expert + p.max_tiles, *tile_n = tile_row0 + p.max_tiles;
+  // the first tile is asked for with the number of tiles (a way from memory less before the first box), whether there is one or not: no block lies past
+  // the plan's room
+  const int tile0 = blockIdx.x / m_tiles, expert0 = tile_expert[tile0], first0 = tile_row0[tile0], rows0 = tile_n[tile0];
+  const int total = p.plan[0] * m_tiles;
+  if (int(blockIdx.x) >= total) return;
   const int* pair_of_row = tile_n + p.max_tiles + p.pairs;
   extern __shared__ unsigned char smem_dyn[];
   // 1024-byte alignment: the swizzle pattern is a function of address bits 4..9
@@ -140,7 +146,7 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
       uint32_t st = 0, parity = 1;                     // parity of the round before
       int filled = 0;
       bool alive = true;
-      int expert = tile_expert[blockIdx.x / m_tiles];
+      int expert = expert0;
       for (int t = blockIdx.x; t < total && alive; t += gridDim.x) {
         const int m0 = t % m_tiles * COLS, wrow = expert * (MODE == 0 ? 2 : 1) * p.N + m0;      // rows past an expert's own come along and are not stored
         if (t + int(gridDim.x) < total) expert = tile_expert[(t + gridDim.x) / m_tiles];
@@ -166,7 +172,7 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
       const uint64_t wdesc0 = smem_desc(wring + box * X_BOX_BYTES, 16, 1024), xdesc0 = smem_desc(xring, 16, 1024);
       uint32_t ws = 0, wpar = 0, xs = 0, xpar = 0, n = 0;      // n: tiles so far
       bool alive = true;
-      int rows = tile_n[blockIdx.x / m_tiles];
+      int rows = rows0;
       for (int t = blockIdx.x; t < total && alive; t += gridDim.x, ++n) {
         const uint32_t set = p.sets == 2 ? n & 1 : 0, round = p.sets == 2 ? n >> 1 : n;
         const uint32_t idesc = idesc_bf16(XM, (rows + 15) / 16 * 16, false), acc = tmem_base + (set * BOXES + box) * p.acc2;
@@ -192,28 +198,31 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
   } else if (warp < 1 + MAX_BOXES + X_GATHER / 32) {
     const int gt = tid - 32 * (1 + MAX_BOXES), c = gt % 8;      // chunk c (8 values) of rows gt / 8 + X_GATHER / 8 j
     // a tile's rows; those of the block's next tile are looked up while this one's are copied
-    int row[8], next[8], rows = 0, next_rows = 0;
-    auto look_up = [&](int t, int (&to)[8]) {
-      const int tile = t / m_tiles, row0 = tile_row0[tile], n = tile_n[tile];
+    int row[PER], next[PER], rows = 0, next_rows = 0;
+    auto look_up = [&](int row0, int n, int (&to)[PER]) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < PER; ++j) {
         const int r = gt / 8 + X_GATHER / 8 * j;
         to[j] = r < n ? (MODE == 1 ? row0 + r : pair_of_row[row0 + r]) : -1;
       }
-      return n;
     };
-    rows = look_up(blockIdx.x, row);
+    rows = rows0;
+    look_up(first0, rows, row);
     const uint32_t dst0 = xring + (gt / 8) * 128 + ((c ^ ((gt / 8) & 7)) << 4);
     uint32_t st = 0, parity = 1;
     int filled = 0;
     bool alive = true;
     for (int t = blockIdx.x; t < total && alive; t += gridDim.x) {
       const bool more = t + int(gridDim.x) < total;
-      if (more) next_rows = look_up(t + gridDim.x, next);
+      if (more) {
+        const int tile = (t + gridDim.x) / m_tiles;
+        next_rows = tile_n[tile];
+        look_up(tile_row0[tile], next_rows, next);
+      }
       const int n16 = (rows + 15) / 16 * 16;
-      const __nv_bfloat16* src[8];
+      const __nv_bfloat16* src[PER];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) src[j] = row[j] >= 0 ? p.x + size_t(MODE == 1 ? row[j] : row[j] / p.top) * p.K + c * 8 : nullptr;
+      for (int j = 0; j < PER; ++j) src[j] = row[j] >= 0 ? p.x + size_t(MODE == 1 ? row[j] : row[j] / p.top) * p.K + c * 8 : nullptr;
       for (int i = 0; i < n_iter; ++i, ++filled) {
         if (filled >= p.x_stages && !mbar_wait(xempty0 + 8 * st, parity, p.error_flag, 34)) {
           alive = false;
@@ -222,14 +231,14 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
         const bool k_ok = i * XK + c * 8 < p.K;
         const uint32_t dst = dst0 + st * p.x_stage_bytes;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < PER; ++j)
           if (gt / 8 + X_GATHER / 8 * j < n16)
             copy16_or_zero(dst + j * (X_GATHER * 16), src[j] && k_ok ? src[j] + i * XK : p.x, src[j] && k_ok);
         arrive_when_copied(xfull0 + 8 * st);
         if (++st == uint32_t(p.x_stages)) { st = 0; parity ^= 1; }
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) row[j] = next[j];
+      for (int j = 0; j < PER; ++j) row[j] = next[j];
       rows = next_rows;
     }
     cp_async_wait_all();
@@ -240,7 +249,7 @@ expert_linear_tc_kernel(const __grid_constant__ CUtensorMap w_map, const ExpertT
     uint32_t n = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++n) {
       const uint32_t set = p.sets == 2 ? n & 1 : 0, round = p.sets == 2 ? n >> 1 : n;
-      const int tile = t / m_tiles, row0 = tile_row0[tile], rows = tile_n[tile];
+      const int tile = t / m_tiles, row0 = n == 0 ? first0 : tile_row0[tile], rows = n == 0 ? rows0 : tile_n[tile];
       const int f0 = t % m_tiles * COLS + quarter * 32 + lane;      // output column = lane of tensor memory
       if (!mbar_wait(done0 + 8 * set, round & 1, p.error_flag, 33)) break;
       tc_fence_after();
@@ -318,30 +327,39 @@ bool make_expert_map(CUtensorMap* map, const void* base, long long rows, int K) 
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int MODE, bool TWO>
+template <int MODE, bool TWO, int PER>
 int launch_expert_tc(const CUtensorMap& map, ExpertTcParams p, int tile_rows, cudaStream_t stream) {
-  constexpr int RING = ExpertThreads<TWO>::RING, BOXES = MODE != 0 && TWO ? 1 : 2, COLS = MODE == 0 ? XM : BOXES * XM;
+  constexpr int RING = ExpertThreads<MODE, TWO>::RING, BOXES = MODE != 0 && TWO ? 1 : 2, COLS = MODE == 0 ? XM : BOXES * XM;
   p.acc2 = tile_rows < 32 ? 32 : tile_rows;
   p.sets = 2 * BOXES * p.acc2 <= (TWO ? 256 : 512) ? 2 : 1;
   p.x_stage_bytes = tile_rows * XK * 2;
-  p.x_stages = tile_rows >= 128 ? 3 : TWO && tile_rows == 32 ? 3 : X_MAX_X;
+  p.x_stages = TWO && MODE == 0 && tile_rows == 128 ? 2 : tile_rows >= 128 ? 3 : TWO && tile_rows == 32 ? 3 : X_MAX_X;
   p.w_stages = min(X_MAX_W, (RING - p.x_stages * p.x_stage_bytes) / (BOXES * X_BOX_BYTES));
   const size_t smem = 1024 + size_t(RING);
   static SharedLimit limit;
-  if (!limit.allows(expert_linear_tc_kernel<MODE, TWO>, smem)) return PTB_ERR_LAUNCH;
+  if (!limit.allows(expert_linear_tc_kernel<MODE, TWO, PER>, smem)) return PTB_ERR_LAUNCH;
   const long long most = (long long)p.max_tiles * ((p.N + COLS - 1) / COLS), slots = (long long)sm_count() * (TWO ? 2 : 1);
-  launch_pdl(expert_linear_tc_kernel<MODE, TWO>, int(most < slots ? most : slots), ExpertThreads<TWO>::ALL, smem, stream, map, p);
+  launch_pdl(expert_linear_tc_kernel<MODE, TWO, PER>, int(most < slots ? most : slots), ExpertThreads<MODE, TWO>::ALL, smem, stream, map, p);
   return launch_status();
 }
 
 template <int MODE>
-int launch_expert_tc(const CUtensorMap& map, const ExpertTcParams& p, int tile_rows, cudaStream_t stream) {
-  // Two blocks an SM, each with half of its shared memory, for tiles of up to 32 rows, and of 64 where all tiles are resident then: what
-  // counts there is the matrices' stream, which a last round of few tiles on a block an SM each leaves slack in (16 experts of 1,408, 40
-  // tokens of 6 choices: 68 us with one block an SM, 58 with two; 64 experts, 300 tokens, tiles of 64: 187 with one)
-  const long long most = (long long)p.max_tiles * ((p.N + XM - 1) / XM);
-  const bool two = tile_rows <= 32 || (tile_rows == 64 && most <= 2 * sm_count());
-  return two ? launch_expert_tc<MODE, true>(map, p, tile_rows, stream) : launch_expert_tc<MODE, false>(map, p, tile_rows, stream);
+int launch_expert_tc(const CUtensorMap& map, const ExpertTcParams& p, int n_experts, int tile_rows, cudaStream_t stream) {
+  // Two blocks an SM, each with half of its shared memory and, in the second product, with tiles of half the columns, where what counts are blocks
+  // and the matrices' stream: tiles of up to 32 rows; of 64 in the second product; of 64 and 128 in the first where a block an SM would leave a last
+  // round of few tiles, and of 64 where tiles are few at all. Else the first product's deeper rings win. Tiles counted as one an expert. us
+  // with one and with two: first product, tiles of 64 rows, 64 tiles 13.3 / 12.8, 88 22.3 / 30.3, 128 48.2 / 58.4, 176 45.1 / 37.9, 256 48.8 / 50.9, 704 115 /
+  // 122 (768 of less K 134 / 129); tiles of 128, 176 tiles 48.9 / 41.9, 256 52.8 / 53.0; tiles of 16, 88 to 768 tiles 20.0 / 17.4, 42.3 / 30.1, 113 / 112, 127 / 123. Second
+  // product, tiles of 64, 32 tiles of 128 columns 19.9 / 17.0, 128 15.9 / 14.1, 512 29.3 / 27.3, 1,024 65.0 / 62.9; tiles of 128, 32 tiles 21.4 / 24.1, 256 21.7 / 22.1,
+  // 512 30.8 / 29.5 (not taken).
+  const int sms = sm_count();
+  const long long tiles = (long long)min(p.pairs, n_experts) * ((p.N + XM - 1) / XM);
+  const bool last_round = tiles > sms && tiles <= 3 * sms / 2;
+  if (tile_rows <= 32 || (tile_rows == 64 && (MODE != 0 || tiles <= sms / 2 || last_round)))
+    return launch_expert_tc<MODE, true, 8>(map, p, tile_rows, stream);
+  if constexpr (MODE == 0)
+    if (tile_rows == 128 && last_round) return launch_expert_tc<MODE, true, 16>(map, p, tile_rows, stream);
+  return launch_expert_tc<MODE, false, 8>(map, p, tile_rows, stream);
 }
 
 }  // namespace
@@ -363,6 +381,6 @@ PTB_API int ptb_expert_linear_tc(int mode, const void* x, const void* w, void* o
   p.x = (const __nv_bfloat16*)x; p.out = out; p.plan = plan; p.row_scale = row_scale; p.error_flag = error_flag;
   p.pairs = pairs; p.max_tiles = max_tiles; p.top = top; p.N = N; p.K = K; p.act = act;
   p.glu_limit = glu_limit; p.glu_alpha = glu_alpha;
-  return mode == 0 ? launch_expert_tc<0>(map, p, tile_rows, stream) : mode == 1 ? launch_expert_tc<1>(map, p, tile_rows, stream)
-                                                                                : launch_expert_tc<2>(map, p, tile_rows, stream);
+  return mode == 0 ? launch_expert_tc<0>(map, p, n_experts, tile_rows, stream) : mode == 1 ? launch_expert_tc<1>(map, p, n_experts, tile_rows, stream)
+                                                                                : launch_expert_tc<2>(map, p, n_experts, tile_rows, stream);
 }

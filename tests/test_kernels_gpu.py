@@ -471,11 +471,12 @@ def test_expert_tiles(K, kind, width, inner, tile_rows):
 
 @pytest.mark.parametrize("kind", ["gated", "plain"])
 @pytest.mark.parametrize("tile_rows", [16, 32, 64, 128, 256])
-def test_expert_tiles_beyond_the_blocks(K, kind, tile_rows):
+@pytest.mark.parametrize("n_experts", [40, 16, 6])
+def test_expert_tiles_beyond_the_blocks(K, kind, tile_rows, n_experts):
     """More tiles than blocks stay on the device, so that a block walks several: its rings carry on from tile to tile at any
-    stage (9 and 21 stages of k, each with a remainder), and tiles of different rows take turns in tensor memory. The bound
-    is that of test_expert_tiles."""
-    width, inner, n_experts = 520, 1304, 40
+    stage (9 and 21 stages of k, each with a remainder), and tiles of different rows take turns in tensor memory; with fewer experts a
+    little more than one round of tiles, and less than half of one, which choose other forms. The bound is that of test_expert_tiles."""
+    width, inner = 520, 1304
     counts = [(1, 16, 17, 64, 65, 130, 0, 200)[e % 8] for e in range(n_experts)]
     h = rnd(sum(counts), width, dtype=torch.bfloat16, seed=1)
     ids = torch.repeat_interleave(torch.arange(n_experts), torch.tensor(counts))[torch.randperm(sum(counts), generator=torch.Generator().manual_seed(5))]
