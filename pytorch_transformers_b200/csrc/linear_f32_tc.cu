@@ -392,8 +392,8 @@ int linear_f32_tensor(const float* x, const float* w, const float* bias, float* 
   // matrix of few tiles, each of four stages at least (clusters of four blocks: 33 are resident at a time with a block an SM, of three 44,
   // of two 70 and more; 36 clusters of four are two waves: 4,544 x 18,176 and one row 157 us, in clusters of three 108), and then as many as keep
   // a stretch at 64 stages or fewer, at least two, from K of 2,048 on four, since each of its additions rounds (one cluster's block holds two
-  // at most). A stretch more costs a block its totals' way through tensor memory: 700 rows, with one or two and now, 9,216 x 1,024 110 and 111 us,
-  // 9,216 x 4,096 365 and 357.
+  // at most). A stretch more costs a block its totals' way through tensor memory: with one or two and now, 128 rows of 9,216 x 1,024 47 and 49 us,
+  // 700 rows of 9,216 x 4,096 365 and 357, one row of 65,024 x 4,544 279 and 285.
   const int shared = tiles <= 33 ? 4 : tiles <= 44 ? 3 : tiles <= 70 ? 2 : 1;
   int most = shared;
   while (most > 1 && total / most < 4) --most;
